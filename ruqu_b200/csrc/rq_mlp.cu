@@ -6,16 +6,19 @@
 // qaoa.rs:221-222); it is trained on angles the batched simulator optimises.
 //
 // k_gemm_bf16 computes C[M x N] = A[M x K] * B[N x K]^T (+ epilogue) on the
-// 5th-generation tensor cores: each CTA owns a 128-row tile of C and up to 256
-// columns; K is consumed in chunks of 64.  Operands are copied from global
-// memory into shared memory in the no-swizzle K-major "core matrix" layout
-// (8 rows x 16 bytes per core matrix; element (r, k) of a tile at byte
-// (r/8)*SBO + (k/8)*LBO + (r%8)*16 + (k%8)*2 with LBO = 128, SBO = 1024),
-// one elected thread issues tcgen05.mma (kind::f16, BF16 inputs, FP32
-// accumulator in tensor memory), tcgen05.commit signals an mbarrier, and the
-// epilogue reads the accumulator back with tcgen05.ld.  Every wait on the
-// mbarrier is bounded; on expiry the kernel records an error and returns after
-// freeing its tensor memory.
+// 5th-generation tensor cores: each CTA owns a 128-row tile of C and NT
+// columns; K is consumed in chunks of KC through two shared-memory buffers, so
+// a chunk loads while the previous one's MMAs run.  Operands sit in shared
+// memory in the no-swizzle K-major "core matrix" layout (8 rows x 16 bytes per
+// core matrix; element (r, k) of a tile at byte (r/8)*SBO + (k/8)*128 +
+// (r%8)*16 + (k%8)*2, SBO = 16 KC); an operand stored the other way round
+// (K rows of M or N values) is transposed in registers on the way in, one 8x8
+// block per thread, so no transposed copies exist in memory.  One thread
+// issues tcgen05.mma (kind::f16, BF16 inputs, FP32 accumulator in tensor
+// memory), tcgen05.commit signals the buffer's mbarrier, and the epilogue reads
+// the accumulator back with tcgen05.ld and applies the layer's elementwise work.
+// Every wait on an mbarrier is bounded; on expiry the kernel records an error
+// and returns after freeing its tensor memory.
 #include "rq_internal.cuh"
 
 #include <cuda_bf16.h>
@@ -29,9 +32,8 @@
 namespace {
 
 constexpr int BM = 128;      // rows per CTA (UMMA M)
-constexpr int BK = 64;       // K per shared-memory chunk
+constexpr int GT = 256;      // threads per CTA
 constexpr int LBO = 128;     // bytes between core matrices along K
-constexpr int SBO = (BK / 8) * 128;   // bytes between 8-row groups
 
 __device__ int g_mma_timeout = 0;   // set when a bounded wait expires
 
@@ -40,11 +42,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // shared-memory matrix descriptor, no swizzle, K-major (sm_100 version 1)
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
+__device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t sbo) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
     d |= (uint64_t)(LBO >> 4) << 16;
-    d |= (uint64_t)(SBO >> 4) << 32;
+    d |= (uint64_t)(sbo >> 4) << 32;
     d |= (uint64_t)1 << 46;   // descriptor version for sm_100
     return d;                 // base offset 0, lbo mode 0, layout type 0 (no swizzle)
 }
@@ -86,46 +88,120 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 
 enum Epi : int {
     EPI_F32 = 0,         // C (f32) = acc
-    EPI_BIAS_RELU = 1,   // Z (f32) = acc + bias; H (bf16) = relu(Z)
-    EPI_BIAS = 2         // C (f32) = acc + bias
+    EPI_BIAS_RELU = 1,   // H (bf16) = relu(acc + bias)
+    EPI_BIAS = 2,        // C (f32) = acc + bias
+    EPI_RELU_BACK = 3,   // H (bf16) = acc where mask > 0 and row < valid, else 0; colpart = column sums
+    EPI_MSE = 4          // d = acc + bias - target: H (bf16) = 2 d / (valid * out), colpart = column
+                         // sums of that, losspart = sum of d^2
 };
 
 struct GemmArgs {
-    const __nv_bfloat16* A;   // [M x K] row-major
-    const __nv_bfloat16* B;   // [N x K] row-major
-    int M, N, K;              // M % 128 == 0, N % 16 == 0, K % 16 == 0
-    int lda, ldb;             // row strides (elements)
+    const __nv_bfloat16* A;   // [M x K] row-major, or [K x M] with at
+    const __nv_bfloat16* B;   // [N x K] row-major, or [K x N] with bt
+    int M, N, K;              // K % 16 == 0
+    int lda, ldb;             // row strides (elements, multiples of 8)
+    int at, bt;               // operand stored transposed (M / N then a multiple of 8)
+    int arows;                // rows of A that exist (the rest of M reads as zeros); at: K rows of A and B
     float* C;                 // [M x N] f32 (row stride ldc)
     int ldc;
-    const float* bias;        // [N]
-    __nv_bfloat16* H;         // [M x N] bf16 (row stride ldh), EPI_BIAS_RELU
+    const float* bias;        // [nbias]
+    int nbias;
+    __nv_bfloat16* H;         // [M x N] bf16 (row stride ldh)
     int ldh;
     int epi;
+    const __nv_bfloat16* mask;   // EPI_RELU_BACK: [M x N] bf16 (row stride ldh)
+    int valid;                   // EPI_RELU_BACK, EPI_MSE: rows that count
+    const float* target;         // EPI_MSE: [valid x out] f32
+    int out;                     // EPI_MSE: columns that count
+    float* colpart;              // EPI_RELU_BACK, EPI_MSE: [row tiles][ldh] column sums
+    float* losspart;             // EPI_MSE: [row tiles * column tiles]
 };
 
-// Tile of C: rows [blockIdx.x*128, +128), cols [blockIdx.y*NT, +NT).  128 threads.
-template <int NT>
-__global__ void __launch_bounds__(128, 1) k_gemm_bf16(GemmArgs g) {
-    static_assert(NT % 16 == 0 && NT >= 32 && NT <= 256, "tile N");
-    extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* sA = smem;                        // 128 x 64 bf16 = 16 KB
-    unsigned char* sB = smem + BM * BK * 2;          // NT x 64 bf16
-    __shared__ __align__(8) uint64_t mbar;
+__device__ __forceinline__ void gcp_async16(void* dst, const void* src, bool take) {
+    const uint32_t n = take ? 16u : 0u;   // 0: the 16 bytes are zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+}
+
+// rows [row0, +R) x k [k0, +kw) of an operand stored [rows x K] into the core-matrix layout.
+// Eight neighbouring threads fill one core matrix (128 contiguous bytes of shared memory, no
+// bank conflicts); a warp reads 64 contiguous bytes of each of its eight rows.
+template <int R, int KC>
+__device__ __forceinline__ void load_k_major(unsigned char* dst, const __nv_bfloat16* __restrict__ src, int ld, int row0,
+                                             int row_lim, int k0, int kw, int tid) {
+    const int kch = kw >> 3, total = R * kch;
+    for (int u = tid; u < total; u += GT) {
+        const int cm = u >> 3, rg = cm / kch, kc = cm - rg * kch, r = rg * 8 + (u & 7);
+        const bool ok = row0 + r < row_lim;
+        const __nv_bfloat16* g = src + (ok ? (size_t)(row0 + r) * ld + k0 + kc * 8 : 0);
+        gcp_async16(dst + rg * (KC * 16) + kc * 128 + (u & 7) * 16, g, ok);
+    }
+}
+
+// the same tile of an operand stored [K x rows]: 8x8 blocks transposed in registers, one core
+// matrix per thread and step (eight 16-byte loads in flight, eight contiguous 16-byte stores)
+template <int R, int KC>
+__device__ __forceinline__ void load_mn_major(unsigned char* dst, const __nv_bfloat16* __restrict__ src, int ld, int row0,
+                                              int row_lim, int k0, int kw, int k_lim, int tid) {
+    const int kch = kw >> 3, total = (R / 8) * kch;
+    for (int u = tid; u < total; u += GT) {
+        const int kc = u / (R / 8), rg = u - kc * (R / 8);   // neighbouring threads: neighbouring 16 bytes of a row
+        const bool ok = row0 + rg * 8 < row_lim;
+        uint4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = k0 + kc * 8 + j;
+            v[j] = ok && k < k_lim ? *reinterpret_cast<const uint4*>(src + (size_t)k * ld + row0 + rg * 8)
+                                   : make_uint4(0u, 0u, 0u, 0u);
+        }
+        unsigned char* d = dst + rg * (KC * 16) + kc * 128;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t* x = reinterpret_cast<const uint32_t*>(&v[2 * j]);
+                const uint32_t* y = reinterpret_cast<const uint32_t*>(&v[2 * j + 1]);
+                o[j] = __byte_perm(x[r >> 1], y[r >> 1], (r & 1) ? 0x7632 : 0x5410);
+            }
+            *reinterpret_cast<uint4*>(d + r * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+}
+
+// One launch covers the tiles of g0 and, after them, those of g1 (independent products that
+// become ready together; tiles0 = the tiles of g0).  A tile is rows [128 i, +128) x columns
+// [NT j, +NT) of C.  The warm-start products are small (256 x 256 x 256-336): what bounds them is
+// the latency of load -> MMA -> epilogue, so narrow tiles (more CTAs, each loading little) and the
+// whole K in at most two chunks.  The products of a training step (batch 256, 336 -> 256 -> 256 ->
+// 8) took 80 us each on a B200 with 256-column tiles and 64-wide chunks (two CTAs, a wait after
+// every chunk) and take 8 us; the ReLU mask and the bias gradients, two kernels of 135 us that
+// walked the batch serially per column, run in this epilogue.  A step with Adam: 900 -> 65 us.
+template <int NT, int KC>
+__global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, int tiles0) {
+    static_assert(NT % 32 == 0 && NT >= 32 && NT <= 256, "tile N");
+    constexpr int ABYTES = BM * KC * 2, BBYTES = NT * KC * 2;
+    extern __shared__ __align__(1024) unsigned char smem[];   // two buffers of A | B
+    __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_base;
     __shared__ int timed_out;
+    __shared__ float colred[GT / 32][NT / 2];
 
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int row0 = blockIdx.x * BM, col0 = blockIdx.y * NT;
-    const int ncols = NT < 32 ? 32 : NT;   // tensor-memory columns (power of two >= 32)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const GemmArgs g = (int)blockIdx.x < tiles0 ? g0 : g1;
+    const int tile = (int)blockIdx.x < tiles0 ? blockIdx.x : blockIdx.x - tiles0;
+    const int mt = (g.M + BM - 1) / BM;
+    const int tm = tile % mt, tn = tile / mt;
+    const int row0 = tm * BM, col0 = tn * NT;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(ncols)
+                     "r"(NT)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(&mbar, 1);
+        mbar_init(&mbar[0], 1);
+        mbar_init(&mbar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         timed_out = 0;
     }
@@ -134,26 +210,24 @@ __global__ void __launch_bounds__(128, 1) k_gemm_bf16(GemmArgs g) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
 
-    const int nk = g.K / BK + ((g.K % BK) ? 1 : 0);
-    uint32_t phase = 0;
+    const int nk = (g.K + KC - 1) / KC;
+    int issued = 0;                       // chunks whose MMAs have been issued
     for (int kc = 0; kc < nk; ++kc) {
-        const int k0 = kc * BK;
-        const int kw = min(BK, g.K - k0);   // multiple of 16
-        // stage A (128 x kw) and B (NT x kw) into the core-matrix layout, 16 bytes per access
-        const int chunksA = BM * (kw / 8), chunksB = NT * (kw / 8);
-        for (int c = tid; c < chunksA + chunksB; c += blockDim.x) {
-            const bool isA = c < chunksA;
-            const int cc = isA ? c : c - chunksA;
-            const int r = cc / (kw / 8), kk = (cc % (kw / 8)) * 8;
-            const int grow = isA ? row0 + r : col0 + r;   // rows past M / N read as zeros
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (grow < (isA ? g.M : g.N)) {
-                const __nv_bfloat16* src = isA ? g.A + (size_t)grow * g.lda + k0 + kk : g.B + (size_t)grow * g.ldb + k0 + kk;
-                v = *reinterpret_cast<const uint4*>(src);
-            }
-            unsigned char* dst = (isA ? sA : sB) + (r >> 3) * SBO + (kk >> 3) * LBO + (r & 7) * 16;
-            *reinterpret_cast<uint4*>(dst) = v;
+        const int buf = kc & 1;
+        unsigned char* sA = smem + buf * (ABYTES + BBYTES);
+        unsigned char* sB = sA + ABYTES;
+        if (kc >= 2) {                    // the MMAs of chunk kc - 2 read this buffer
+            if (!mbar_wait(&mbar[buf], (uint32_t)((kc >> 1) - 1) & 1u, g_mma_wait_polls)) timed_out = 1;
+            __syncthreads();
+            if (timed_out) break;
         }
+        const int k0 = kc * KC;
+        const int kw = min(KC, g.K - k0);   // multiple of 16
+        if (g.at) load_mn_major<BM, KC>(sA, g.A, g.lda, row0, g.M, k0, kw, g.arows, tid);
+        else load_k_major<BM, KC>(sA, g.A, g.lda, row0, g.arows, k0, kw, tid);
+        if (g.bt) load_mn_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, g.at ? g.arows : g.K, tid);
+        else load_k_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, tid);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         // make the generic-proxy writes visible to the tensor core (async proxy)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -162,8 +236,8 @@ __global__ void __launch_bounds__(128, 1) k_gemm_bf16(GemmArgs g) {
         if (tid == 0) {
             const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
             for (int ks = 0; ks < kw / 16; ++ks) {
-                const uint64_t ad = sdesc(a0 + ks * 2 * LBO);
-                const uint64_t bd = sdesc(b0 + ks * 2 * LBO);
+                const uint64_t ad = sdesc(a0 + ks * 2 * LBO, KC * 16);
+                const uint64_t bd = sdesc(b0 + ks * 2 * LBO, KC * 16);
                 const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
@@ -173,91 +247,172 @@ __global__ void __launch_bounds__(128, 1) k_gemm_bf16(GemmArgs g) {
                     : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&mbar))
+                             smem_u32(&mbar[buf]))
                          : "memory");
         }
-        // the chunk's MMAs must finish before the buffers are overwritten (and before the epilogue)
-        if (!mbar_wait(&mbar, phase, g_mma_wait_polls)) {
-            timed_out = 1;
-        }
-        phase ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (timed_out) {
-            // the MMAs of this chunk may still be in flight: let them land (bounded) before the
-            // shared and tensor memory they use are released
-            if (tid == 0) mbar_wait(&mbar, phase ^ 1u);
-            break;
-        }
+        issued = kc + 1;
     }
-
+    // the last chunk's commit covers every earlier MMA of the issuing thread
     if (!timed_out) {
-        // epilogue: warp w holds rows 32w..32w+31 in tensor-memory lanes 32w..
-        const int r = row0 + warp * 32 + (tid & 31);
-        for (int c0 = 0; c0 < NT; c0 += 16) {
+        if (!mbar_wait(&mbar[(nk - 1) & 1], (uint32_t)((nk - 1) >> 1) & 1u, g_mma_wait_polls)) timed_out = 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    if (timed_out) {
+        // MMAs may still be in flight: let them land (bounded) before the shared and tensor memory
+        // they use are released
+        if (tid == 0) {
+            mbar_wait(&mbar[(issued - 1) & 1], (uint32_t)((issued - 1) >> 1) & 1u);
+            atomicExch(&g_mma_timeout, 1);
+        }
+    } else {
+        // epilogue: warps w and w + 4 read the tensor-memory lanes 32 (w % 4).. (rows of the tile),
+        // the lower four warps the first half of the columns, the upper four the second
+        const int rl = (warp & 3) * 32 + lane, r = row0 + rl, half = warp >> 2;
+        float loss = 0.f;
+        const float inv = g.epi == EPI_MSE ? 1.f / (float)(g.valid * g.out) : 0.f;
+        for (int c0 = half * (NT / 2); c0 < (half + 1) * (NT / 2); c0 += 16) {
             uint32_t v[16];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (r < g.M) {
+            float x[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
+            const int c = col0 + c0;
+            const bool in = r < g.M && c < g.N;
+            const bool full = in && c + 16 <= g.N;
+            if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (c + j < g.nbias) x[j] += g.bias[c + j];
+            }
+            if (g.epi == EPI_F32 || g.epi == EPI_BIAS) {
+                float* o = g.C + (size_t)r * g.ldc + c;
+                if (full && (g.ldc & 3) == 0) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4*>(o + j) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+                } else if (in) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (c + j < g.N) o[j] = x[j];
+                }
+                continue;
+            }
+            if (g.epi == EPI_BIAS_RELU) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] = x[j] > 0.f ? x[j] : 0.f;
+            } else if (g.epi == EPI_RELU_BACK) {
+                uint4 mk[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+                if (in && r < g.valid) {   // N is a multiple of 16 here
+                    const uint4* mp = reinterpret_cast<const uint4*>(g.mask + (size_t)r * g.ldh + c);
+                    mk[0] = mp[0];
+                    mk[1] = mp[1];
+                }
+                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(mk);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] = __bfloat162float(mb[j]) > 0.f ? x[j] : 0.f;
+            } else {   // EPI_MSE
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int c = col0 + c0 + j;
-                    if (c >= g.N) continue;
-                    float x = __uint_as_float(v[j]);
-                    if (g.epi != EPI_F32) x += g.bias[c];
-                    g.C[(size_t)r * g.ldc + c] = x;
-                    if (g.epi == EPI_BIAS_RELU) g.H[(size_t)r * g.ldh + c] = __float2bfloat16_rn(x > 0.f ? x : 0.f);
+                    float gr = 0.f;
+                    if (r < g.valid && c + j < g.out) {
+                        const float d = x[j] - g.target[(size_t)r * g.out + c + j];
+                        loss += d * d;
+                        gr = 2.f * d * inv;
+                    }
+                    x[j] = gr;
+                }
+            }
+            if (r < g.M) {
+                __nv_bfloat16 h[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(x[j]);
+                __nv_bfloat16* o = g.H + (size_t)r * g.ldh + c;
+                if (c + 16 <= g.ldh) {     // ldh is a multiple of 16: whole 16-column groups
+                    reinterpret_cast<uint4*>(o)[0] = reinterpret_cast<const uint4*>(h)[0];
+                    reinterpret_cast<uint4*>(o)[1] = reinterpret_cast<const uint4*>(h)[1];
+                }
+            }
+            if (g.epi != EPI_BIAS_RELU) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float t = x[j];
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                    if (lane == j) colred[warp][c0 - half * (NT / 2) + j] = t;
                 }
             }
         }
-    } else if (tid == 0) {
-        atomicExch(&g_mma_timeout, 1);
+        if (g.epi == EPI_RELU_BACK || g.epi == EPI_MSE) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+            __shared__ float lred[GT / 32];
+            if (lane == 0) lred[warp] = loss;
+            __syncthreads();
+            for (int j = tid; j < NT; j += GT) {
+                const int w0 = (j / (NT / 2)) * 4, cc = j % (NT / 2);
+                if (col0 + j < g.ldh)
+                    g.colpart[(size_t)tm * g.ldh + col0 + j] =
+                        (colred[w0][cc] + colred[w0 + 1][cc]) + (colred[w0 + 2][cc] + colred[w0 + 3][cc]);
+            }
+            if (g.epi == EPI_MSE && tid == 0) {
+                float s = 0.f;
+                for (int k = 0; k < GT / 32; ++k) s += lred[k];
+                g.losspart[tile] = s;
+            }
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NT) : "memory");
+}
+
+template <int NT, int KC>
+int launch_gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1) {
+    auto tiles = [](const GemmArgs& g) { return ((g.M + BM - 1) / BM) * ((g.N + NT - 1) / NT); };
+    constexpr int smem = 2 * (BM + NT) * KC * 2;
+    const int t0 = tiles(g0);
+    RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<NT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_gemm_bf16<NT, KC><<<t0 + (g1 ? tiles(*g1) : 0), GT, smem, stream>>>(g0, g1 ? *g1 : g0, t0);
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
+// Tile width by the number of CTAs it leaves: the widest tile whose grid still has a CTA for
+// every SM (A is re-read once per column tile, so large products want wide tiles), else 32
+// columns, where a small product spreads over the most SMs.
+int gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1 = nullptr) {
+    const long mt = (g0.M + BM - 1) / BM;
+    if (!g1 && mt * ((g0.N + 255) / 256) >= 148) return launch_gemm<256, 128>(stream, g0, g1);
+    if (!g1 && mt * ((g0.N + 127) / 128) >= 148) return launch_gemm<128, 192>(stream, g0, g1);
+    if (!g1 && mt * ((g0.N + 63) / 64) >= 148) return launch_gemm<64, 192>(stream, g0, g1);
+    return launch_gemm<32, 256>(stream, g0, g1);
 }
 
 }  // namespace
 
 namespace rq {
 
-// C = A * B^T with the given epilogue, on `stream`.  Shapes are checked here.
+// C = A * B^T on `stream`.  Shapes are checked here.
 int gemm_bf16(cudaStream_t stream, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N,
-              int K, float* C, int ldc, int epi, const float* bias, __nv_bfloat16* H, int ldh) {
+              int K, float* C, int ldc) {
     if (M < 1 || N < 1 || K < 16 || K % 16)
         return fail(RQ_ERR_INVALID_ARGUMENT, "gemm_bf16: M, N >= 1 and K a positive multiple of 16");
     if (lda % 8 || ldb % 8) return fail(RQ_ERR_INVALID_ARGUMENT, "gemm_bf16: row strides must be multiples of 8");
-    GemmArgs g{A, B, M, N, K, lda, ldb, C, ldc, bias, H, ldh, epi};
-    const int nt = N > 128 ? 256 : (N > 64 ? 128 : (N > 32 ? 64 : 32));
-    dim3 grid((M + BM - 1) / BM, (N + nt - 1) / nt);
-    const size_t smem = (size_t)(BM + nt) * BK * 2;
-    switch (nt) {
-        case 256:
-            RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_gemm_bf16<256><<<grid, 128, smem, stream>>>(g);
-            break;
-        case 128:
-            RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_gemm_bf16<128><<<grid, 128, smem, stream>>>(g);
-            break;
-        case 64:
-            RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_gemm_bf16<64><<<grid, 128, smem, stream>>>(g);
-            break;
-        default:
-            RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_gemm_bf16<32><<<grid, 128, smem, stream>>>(g);
-            break;
-    }
-    RQ_CUDA(cudaGetLastError());
-    return RQ_OK;
+    GemmArgs g{};
+    g.A = A; g.lda = lda; g.B = B; g.ldb = ldb;
+    g.M = M; g.N = N; g.K = K;
+    g.arows = M;
+    g.C = C; g.ldc = ldc;
+    g.epi = EPI_F32;
+    return gemm(stream, g);
 }
 
 int mma_timeout_flag(int* out) {
@@ -295,7 +450,7 @@ int rq_gemm_bf16(const uint16_t* A, const uint16_t* B, int32_t M, int32_t N, int
     cudaError_t e = cudaMemcpy(dA, A, (size_t)M * K * 2, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(dB, B, (size_t)N * K * 2, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) rc = rq::cuda_fail(e, "cudaMemcpy");
-    if (rc == RQ_OK) rc = rq::gemm_bf16(0, dA, K, dB, K, M, N, K, dC, N, EPI_F32, nullptr, nullptr, 0);
+    if (rc == RQ_OK) rc = rq::gemm_bf16(0, dA, K, dB, K, M, N, K, dC, N);
     if (rc == RQ_OK) {
         e = cudaMemcpy(C, dC, (size_t)M * N * 4, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = rq::cuda_fail(e, "cudaMemcpy");
@@ -329,94 +484,80 @@ __global__ void k_pad_bf16(const float* __restrict__ src, int rows, int cols, in
     }
 }
 
-// dst[c][r] = src[r][c]  (rows x cols -> cols x rows)
-__global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ src, int rows, int cols, int lds,
-                                 __nv_bfloat16* __restrict__ dst, int ldd) {
-    __shared__ __nv_bfloat16 t[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int r = by + j, c = bx + threadIdx.x;
-        t[j][threadIdx.x] = (r < rows && c < cols) ? src[(long)r * lds + c] : __float2bfloat16_rn(0.f);
+// Where the parameters, their gradients and their BF16 copies lie (flat parameter index order:
+// W1, b1, W2, b2, W3, b3).
+struct ParamMap {
+    int in, h1, h2, out, inp, outp;
+    long b1, w2, b2, w3, b3, total;       // first parameter of each later block
+    const float *g1, *g2, *g3t;           // dW1 [h1 x inp], dW2 [h2 x h1], dW3^T [h2 x outp]
+    const float *db1, *db2, *db3;         // per-row-tile column sums: [ntile][h1 | h2 | outp]
+    int ntile;
+    __nv_bfloat16 *W1b, *W2b, *W3b;
+};
+
+// gradient of parameter w; *copy = where its BF16 copy lives (null for a bias)
+__device__ __forceinline__ float grad_of(const ParamMap& m, long w, __nv_bfloat16** copy) {
+    const float* part;
+    int width, c;
+    *copy = nullptr;
+    if (w < m.b1) {
+        const int r = (int)(w / m.in), k = (int)(w - (long)r * m.in);
+        *copy = m.W1b + (long)r * m.inp + k;
+        return m.g1[(long)r * m.inp + k];
+    } else if (w < m.w2) {
+        part = m.db1; width = m.h1; c = (int)(w - m.b1);
+    } else if (w < m.b2) {
+        *copy = m.W2b + (w - m.w2);
+        return m.g2[w - m.w2];
+    } else if (w < m.w3) {
+        part = m.db2; width = m.h2; c = (int)(w - m.b2);
+    } else if (w < m.b3) {
+        const int r = (int)((w - m.w3) / m.h2), k = (int)((w - m.w3) - (long)r * m.h2);
+        *copy = m.W3b + (long)r * m.h2 + k;
+        return m.g3t[(long)k * m.outp + r];
+    } else {
+        part = m.db3; width = m.outp; c = (int)(w - m.b3);
     }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int c = bx + j, r = by + threadIdx.x;
-        if (c < cols && r < rows) dst[(long)c * ldd + r] = t[threadIdx.x][j];
-    }
+    float s = 0.f;
+    for (int t = 0; t < m.ntile; ++t) s += part[(long)t * width + c];
+    return s;
 }
 
-// MSE over the valid B x out block; dY (bf16, Bp x ldy) = 2 (Y - T) / (B out); db = column sums of dY (f32)
-__global__ void k_mse_grad(const float* __restrict__ Y, int ldy, const float* __restrict__ T, int B, int out,
-                           __nv_bfloat16* __restrict__ dY, int Bp, int outp, float* __restrict__ db,
-                           float* __restrict__ loss) {
-    __shared__ float red[32];
-    const float inv = 1.f / (float)(B * out);
-    float l = 0.f;
-    for (int w = threadIdx.x; w < Bp * outp; w += blockDim.x) {
-        const int r = w / outp, c = w - r * outp;
-        float g = 0.f;
-        if (r < B && c < out) {
-            const float d = Y[(long)r * ldy + c] - T[(long)r * out + c];
-            l += d * d;
-            g = 2.f * d * inv;
-        }
-        dY[(long)r * outp + c] = __float2bfloat16_rn(g);
-    }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+// One Adam step over every parameter, and the BF16 copies the next step's products read.  One
+// launch for the six blocks (they were six Adam launches, three copies and two transposes); the
+// loss of the step from its per-tile sums on the way.
+__global__ void k_adam(ParamMap map, float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float lr,
+                       float b1, float b2, float eps, float c1, float c2, const float* __restrict__ losspart, int nloss,
+                       float inv, float* __restrict__ loss) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         float s = 0.f;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += red[k];
+        for (int k = 0; k < nloss; ++k) s += losspart[k];
         *loss = s * inv;
     }
-    // bias gradient of the output layer (same scaling as dY)
-    for (int c = threadIdx.x; c < out; c += blockDim.x) {
-        float s = 0.f;
-        for (int r = 0; r < B; ++r) s += 2.f * (Y[(long)r * ldy + c] - T[(long)r * out + c]) * inv;
-        db[c] = s;
-    }
-}
-
-// dZ = dH * (Z > 0) (bf16, rows >= B zeroed); db[c] = sum over the B valid rows
-__global__ void k_relu_back(const float* __restrict__ dH, const float* __restrict__ Z, int B, int Bp, int cols,
-                            __nv_bfloat16* __restrict__ dZ, float* __restrict__ db) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int r = 0; r < Bp; ++r) {
-            float g = 0.f;
-            if (r < B) {
-                g = Z[(long)r * cols + c] > 0.f ? dH[(long)r * cols + c] : 0.f;
-                s += g;
-            }
-            dZ[(long)r * cols + c] = __float2bfloat16_rn(g);
-        }
-        db[c] = s;
-    }
-}
-
-// Adam on a [rows x cols] parameter block whose gradient sits at g[(r * gsr) + c * gsc]
-__global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
-                       int rows, int cols, long gsr, long gsc, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-    const long total = (long)rows * cols;
-    for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long)gridDim.x * blockDim.x) {
-        const long r = w / cols, c = w - r * cols;
-        const float gr = g[r * gsr + c * gsc];
+    for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < map.total; w += (long)gridDim.x * blockDim.x) {
+        __nv_bfloat16* copy;
+        const float gr = grad_of(map, w, &copy);
         const float mm = b1 * m[w] + (1.f - b1) * gr;
         const float vv = b2 * v[w] + (1.f - b2) * gr * gr;
         m[w] = mm;
         v[w] = vv;
-        p[w] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+        const float np = p[w] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+        p[w] = np;
+        if (copy) *copy = __float2bfloat16_rn(np);
     }
 }
 
-// gradient block copy into the caller's flat layout
-__global__ void k_gather(const float* __restrict__ g, int rows, int cols, long gsr, long gsc, float* __restrict__ out) {
-    const long total = (long)rows * cols;
-    for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long)gridDim.x * blockDim.x) {
-        const long r = w / cols, c = w - r * cols;
-        out[w] = g[r * gsr + c * gsc];
+// gradients in the caller's flat layout, and the loss
+__global__ void k_gather(ParamMap map, const float* __restrict__ losspart, int nloss, float inv, float* __restrict__ out,
+                         float* __restrict__ loss) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        float s = 0.f;
+        for (int k = 0; k < nloss; ++k) s += losspart[k];
+        *loss = s * inv;
+    }
+    for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < map.total; w += (long)gridDim.x * blockDim.x) {
+        __nv_bfloat16* copy;
+        out[w] = grad_of(map, w, &copy);
     }
 }
 
@@ -433,15 +574,19 @@ struct rq_mlp {
     float *P = nullptr, *Mo = nullptr, *Vo = nullptr;
     long off_w1 = 0, off_b1 = 0, off_w2 = 0, off_b2 = 0, off_w3 = 0, off_b3 = 0, nparam = 0;
     long step = 0;
-    // BF16 copies: W1b [h1 x inp], W2b [h2 x h1], W3b [outp x h2], W2t [h1 x h2], W3t [h2 x outp]
-    __nv_bfloat16 *W1b = nullptr, *W2b = nullptr, *W3b = nullptr, *W2t = nullptr, *W3t = nullptr;
+    // BF16 copies: W1b [h1 x inp], W2b [h2 x h1], W3b [outp x h2]
+    __nv_bfloat16 *W1b = nullptr, *W2b = nullptr, *W3b = nullptr;
     // batch workspace
     int cap = 0;
-    __nv_bfloat16 *X = nullptr, *Xt = nullptr, *H1 = nullptr, *H1t = nullptr, *H2 = nullptr, *H2t = nullptr;
-    __nv_bfloat16 *dY = nullptr, *dYt = nullptr, *dZ2 = nullptr, *dZ2t = nullptr, *dZ1 = nullptr, *dZ1t = nullptr;
-    float *Xf = nullptr, *Tf = nullptr, *Z1 = nullptr, *Z2 = nullptr, *Y = nullptr, *dH2 = nullptr, *dH1 = nullptr;
-    float *G = nullptr;           // gradients: dW1 [h1 x inp], db1, dW2 [h2 x h1], db2, dW3t [h2 x outp], db3
-    long g_w1 = 0, g_b1 = 0, g_w2 = 0, g_b2 = 0, g_w3t = 0, g_b3 = 0, g_total = 0;
+    __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dY = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
+    float *Xf = nullptr, *Tf = nullptr, *Y = nullptr;
+    float *db1 = nullptr, *db2 = nullptr, *db3 = nullptr, *losspart = nullptr;   // per-row-tile sums
+    // a training set on the device (kept between calls up to TRAIN_KEEP_BYTES)
+    float *tx = nullptr, *tt = nullptr;
+    __nv_bfloat16* txb = nullptr;
+    size_t train_rows = 0;
+    float* G = nullptr;           // gradients: dW1 [h1 x inp], dW2 [h2 x h1], dW3t [h2 x outp]
+    long g_w1 = 0, g_w2 = 0, g_w3t = 0, g_total = 0;
     float* loss = nullptr;
 };
 
@@ -457,6 +602,8 @@ int dalloc(P** p, size_t n) {
     return RQ_OK;
 }
 
+constexpr size_t TRAIN_KEEP_BYTES = (size_t)256 << 20;
+
 int mlp_refresh_bf16(rq_mlp* m) {
     const int sms = rq::num_sms(m->device);
     const float* P = m->P;
@@ -466,11 +613,6 @@ int mlp_refresh_bf16(rq_mlp* m) {
                                                                                     m->W2b, m->h2, m->h1, m->h1);
     k_pad_bf16<<<rq::grid_for((uint64_t)m->outp * m->h2, 256, sms), 256, 0, m->stream>>>(P + m->off_w3, m->out, m->h2,
                                                                                       m->h2, m->W3b, m->outp, m->h2, m->h2);
-    dim3 tb(32, 8);
-    k_transpose_bf16<<<dim3((m->h1 + 31) / 32, (m->h2 + 31) / 32), tb, 0, m->stream>>>(m->W2b, m->h2, m->h1, m->h1, m->W2t,
-                                                                                       m->h2);
-    k_transpose_bf16<<<dim3((m->h2 + 31) / 32, (m->outp + 31) / 32), tb, 0, m->stream>>>(m->W3b, m->outp, m->h2, m->h2,
-                                                                                         m->W3t, m->outp);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -478,103 +620,157 @@ int mlp_refresh_bf16(rq_mlp* m) {
 int mlp_reserve(rq_mlp* m, int B) {
     const int Bp = (B + 127) & ~127;
     if (Bp <= m->cap) return RQ_OK;
-    void* bufs[] = {m->X, m->Xt, m->H1, m->H1t, m->H2, m->H2t, m->dY, m->dYt, m->dZ2, m->dZ2t, m->dZ1, m->dZ1t,
-                    m->Xf, m->Tf, m->Z1, m->Z2, m->Y, m->dH2, m->dH1};
-    for (void* b : bufs) if (b) cudaFree(b);
-    const size_t b = (size_t)Bp;
-    RQ_TRY(dalloc(&m->X, b * m->inp));
-    RQ_TRY(dalloc(&m->Xt, b * m->inp));
-    RQ_TRY(dalloc(&m->H1, b * m->h1));
-    RQ_TRY(dalloc(&m->H1t, b * m->h1));
-    RQ_TRY(dalloc(&m->H2, b * m->h2));
-    RQ_TRY(dalloc(&m->H2t, b * m->h2));
-    RQ_TRY(dalloc(&m->dY, b * m->outp));
-    RQ_TRY(dalloc(&m->dYt, b * m->outp));
-    RQ_TRY(dalloc(&m->dZ2, b * m->h2));
-    RQ_TRY(dalloc(&m->dZ2t, b * m->h2));
-    RQ_TRY(dalloc(&m->dZ1, b * m->h1));
-    RQ_TRY(dalloc(&m->dZ1t, b * m->h1));
-    RQ_TRY(dalloc(&m->Xf, b * m->in));
-    RQ_TRY(dalloc(&m->Tf, b * m->out));
-    RQ_TRY(dalloc(&m->Z1, b * m->h1));
-    RQ_TRY(dalloc(&m->Z2, b * m->h2));
-    RQ_TRY(dalloc(&m->Y, b * m->outp));
-    RQ_TRY(dalloc(&m->dH2, b * m->h2));
-    RQ_TRY(dalloc(&m->dH1, b * m->h1));
+    m->cap = 0;
+    auto regrow = [](auto** p, size_t n) {
+        if (*p) cudaFree(*p);
+        *p = nullptr;
+        return dalloc(p, n);
+    };
+    const size_t b = (size_t)Bp, nt = b / BM;
+    RQ_TRY(regrow(&m->X, b * m->inp));
+    RQ_TRY(regrow(&m->H1, b * m->h1));
+    RQ_TRY(regrow(&m->H2, b * m->h2));
+    RQ_TRY(regrow(&m->dY, b * m->outp));
+    RQ_TRY(regrow(&m->dZ2, b * m->h2));
+    RQ_TRY(regrow(&m->dZ1, b * m->h1));
+    RQ_TRY(regrow(&m->Xf, b * m->in));
+    RQ_TRY(regrow(&m->Tf, b * m->out));
+    RQ_TRY(regrow(&m->Y, b * m->outp));
+    RQ_TRY(regrow(&m->db1, nt * m->h1));
+    RQ_TRY(regrow(&m->db2, nt * m->h2));
+    RQ_TRY(regrow(&m->db3, nt * m->outp));
+    RQ_TRY(regrow(&m->losspart, nt * (size_t)((m->outp + 31) / 32)));
     m->cap = Bp;
     return RQ_OK;
 }
 
-// forward on m->Xf (B x in, f32 on device): Z1, H1, Z2, H2, Y
-int mlp_forward_dev(rq_mlp* m, int B) {
-    const int Bp = (B + 127) & ~127;
-    const int sms = rq::num_sms(m->device);
-    k_pad_bf16<<<rq::grid_for((uint64_t)Bp * m->inp, 256, sms), 256, 0, m->stream>>>(m->Xf, B, m->in, m->in, m->X, Bp,
-                                                                                  m->inp, m->inp);
-    RQ_CUDA(cudaGetLastError());
-    RQ_TRY(rq::gemm_bf16(m->stream, m->X, m->inp, m->W1b, m->inp, Bp, m->h1, m->inp, m->Z1, m->h1, EPI_BIAS_RELU,
-                         m->P + m->off_b1, m->H1, m->h1));
-    RQ_TRY(rq::gemm_bf16(m->stream, m->H1, m->h1, m->W2b, m->h1, Bp, m->h2, m->h1, m->Z2, m->h2, EPI_BIAS_RELU,
-                         m->P + m->off_b2, m->H2, m->h2));
-    RQ_TRY(rq::gemm_bf16(m->stream, m->H2, m->h2, m->W3b, m->h2, Bp, m->out, m->h2, m->Y, m->outp, EPI_BIAS,
-                         m->P + m->off_b3, nullptr, 0));
+void train_release(rq_mlp* m) {
+    void* bufs[] = {m->tx, m->tt, m->txb};
+    for (void* b : bufs) if (b) cudaFree(b);
+    m->tx = m->tt = nullptr;
+    m->txb = nullptr;
+    m->train_rows = 0;
+}
+
+int train_reserve(rq_mlp* m, size_t n) {
+    if (n <= m->train_rows) return RQ_OK;
+    train_release(m);
+    RQ_TRY(dalloc(&m->tx, n * m->in));
+    RQ_TRY(dalloc(&m->tt, n * m->out));
+    RQ_TRY(dalloc(&m->txb, n * m->inp));
+    m->train_rows = n;
     return RQ_OK;
 }
 
-// backward after mlp_forward_dev with targets in m->Tf: gradients into m->G, loss into m->loss
-int mlp_backward_dev(rq_mlp* m, int B) {
-    const int Bp = (B + 127) & ~127;
-    dim3 tb(32, 8);
-    k_mse_grad<<<1, 1024, 0, m->stream>>>(m->Y, m->outp, m->Tf, B, m->out, m->dY, Bp, m->outp, m->G + m->g_b3, m->loss);
-    RQ_CUDA(cudaGetLastError());
-    // dW3^T [h2 x outp] = H2^T [h2 x Bp] * (dY^T [outp x Bp])^T
-    k_transpose_bf16<<<dim3((m->h2 + 31) / 32, (Bp + 31) / 32), tb, 0, m->stream>>>(m->H2, Bp, m->h2, m->h2, m->H2t, Bp);
-    k_transpose_bf16<<<dim3((m->outp + 31) / 32, (Bp + 31) / 32), tb, 0, m->stream>>>(m->dY, Bp, m->outp, m->outp, m->dYt, Bp);
-    RQ_TRY(rq::gemm_bf16(m->stream, m->H2t, Bp, m->dYt, Bp, m->h2, m->outp, Bp, m->G + m->g_w3t, m->outp, EPI_F32,
-                         nullptr, nullptr, 0));
-    // dH2 [Bp x h2] = dY [Bp x outp] * (W3^T [h2 x outp])^T
-    RQ_TRY(rq::gemm_bf16(m->stream, m->dY, m->outp, m->W3t, m->outp, Bp, m->h2, m->outp, m->dH2, m->h2, EPI_F32,
-                         nullptr, nullptr, 0));
-    k_relu_back<<<(m->h2 + 127) / 128, 128, 0, m->stream>>>(m->dH2, m->Z2, B, Bp, m->h2, m->dZ2, m->G + m->g_b2);
-    // dW2 [h2 x h1] = dZ2^T [h2 x Bp] * (H1^T [h1 x Bp])^T
-    k_transpose_bf16<<<dim3((m->h2 + 31) / 32, (Bp + 31) / 32), tb, 0, m->stream>>>(m->dZ2, Bp, m->h2, m->h2, m->dZ2t, Bp);
-    k_transpose_bf16<<<dim3((m->h1 + 31) / 32, (Bp + 31) / 32), tb, 0, m->stream>>>(m->H1, Bp, m->h1, m->h1, m->H1t, Bp);
-    RQ_TRY(rq::gemm_bf16(m->stream, m->dZ2t, Bp, m->H1t, Bp, m->h2, m->h1, Bp, m->G + m->g_w2, m->h1, EPI_F32, nullptr,
-                         nullptr, 0));
-    // dH1 [Bp x h1] = dZ2 [Bp x h2] * (W2^T [h1 x h2])^T
-    RQ_TRY(rq::gemm_bf16(m->stream, m->dZ2, m->h2, m->W2t, m->h2, Bp, m->h1, m->h2, m->dH1, m->h1, EPI_F32, nullptr,
-                         nullptr, 0));
-    k_relu_back<<<(m->h1 + 127) / 128, 128, 0, m->stream>>>(m->dH1, m->Z1, B, Bp, m->h1, m->dZ1, m->G + m->g_b1);
-    // dW1 [h1 x inp] = dZ1^T [h1 x Bp] * (X^T [inp x Bp])^T
-    k_transpose_bf16<<<dim3((m->h1 + 31) / 32, (Bp + 31) / 32), tb, 0, m->stream>>>(m->dZ1, Bp, m->h1, m->h1, m->dZ1t, Bp);
-    k_transpose_bf16<<<dim3((m->inp + 31) / 32, (Bp + 31) / 32), tb, 0, m->stream>>>(m->X, Bp, m->inp, m->inp, m->Xt, Bp);
-    RQ_TRY(rq::gemm_bf16(m->stream, m->dZ1t, Bp, m->Xt, Bp, m->h1, m->inp, Bp, m->G + m->g_w1, m->inp, EPI_F32, nullptr,
-                         nullptr, 0));
+// rows of f32 inputs as padded BF16 rows
+int mlp_pack_rows(rq_mlp* m, const float* src, size_t rows, __nv_bfloat16* dst) {
+    k_pad_bf16<<<rq::grid_for((uint64_t)rows * m->inp, 256, rq::num_sms(m->device)), 256, 0, m->stream>>>(
+        src, (int)rows, m->in, m->in, dst, (int)rows, m->inp, m->inp);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
 
-// one Adam step over every parameter block from m->G
-int mlp_adam(rq_mlp* m, float lr, float b1, float b2, float eps) {
+// hidden layers on B packed rows X: H1, H2
+int mlp_hidden(rq_mlp* m, const __nv_bfloat16* X, int B) {
+    const int Bp = (B + 127) & ~127;
+    GemmArgs g{};
+    g.A = X; g.lda = m->inp; g.arows = B;
+    g.B = m->W1b; g.ldb = m->inp;
+    g.M = Bp; g.N = m->h1; g.K = m->inp;
+    g.bias = m->P + m->off_b1; g.nbias = m->h1;
+    g.H = m->H1; g.ldh = m->h1;
+    g.epi = EPI_BIAS_RELU;
+    RQ_TRY(gemm(m->stream, g));
+    g.A = m->H1; g.lda = m->h1; g.arows = Bp;
+    g.B = m->W2b; g.ldb = m->h1;
+    g.N = m->h2; g.K = m->h1;
+    g.bias = m->P + m->off_b2; g.nbias = m->h2;
+    g.H = m->H2; g.ldh = m->h2;
+    return gemm(m->stream, g);
+}
+
+GemmArgs output_layer(rq_mlp* m, int B) {
+    GemmArgs g{};
+    g.M = (B + 127) & ~127;
+    g.A = m->H2; g.lda = m->h2; g.arows = g.M;
+    g.B = m->W3b; g.ldb = m->h2;
+    g.N = m->out; g.K = m->h2;
+    g.bias = m->P + m->off_b3; g.nbias = m->out;
+    g.C = m->Y; g.ldc = m->outp;
+    g.epi = EPI_BIAS;
+    return g;
+}
+
+// forward and backward pass on B packed rows X with targets T (device): weight gradients into m->G,
+// bias gradients and the loss as per-tile sums
+int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) {
+    const int Bp = (B + 127) & ~127;
+    RQ_TRY(mlp_hidden(m, X, B));
+    // output layer with the loss: dY = 2 (Y - T) / (B out)
+    GemmArgs y = output_layer(m, B);
+    y.N = m->outp;                     // W3b's padding rows are zero; columns past out become zero in dY
+    y.H = m->dY; y.ldh = m->outp;
+    y.epi = EPI_MSE;
+    y.nbias = m->out;
+    y.valid = B; y.out = m->out; y.target = T;
+    y.colpart = m->db3; y.losspart = m->losspart;
+    RQ_TRY((launch_gemm<32, 256>(m->stream, y, nullptr)));
+    // dW3^T [h2 x outp] = H2^T dY, and dZ2 [Bp x h2] = (dY W3) where H2 > 0
+    GemmArgs w{};
+    w.A = m->H2; w.lda = m->h2; w.at = 1;
+    w.B = m->dY; w.ldb = m->outp; w.bt = 1;
+    w.M = m->h2; w.N = m->outp; w.K = Bp; w.arows = B;
+    w.C = m->G + m->g_w3t; w.ldc = m->outp;
+    w.epi = EPI_F32;
+    GemmArgs d{};
+    d.A = m->dY; d.lda = m->outp; d.arows = Bp;
+    d.B = m->W3b; d.ldb = m->h2; d.bt = 1;
+    d.M = Bp; d.N = m->h2; d.K = m->outp;
+    d.H = m->dZ2; d.ldh = m->h2; d.mask = m->H2;
+    d.valid = B; d.colpart = m->db2;
+    d.epi = EPI_RELU_BACK;
+    RQ_TRY(gemm(m->stream, w, &d));
+    // dW2 [h2 x h1] = dZ2^T H1, and dZ1 [Bp x h1] = (dZ2 W2) where H1 > 0
+    w.A = m->dZ2; w.lda = m->h2;
+    w.B = m->H1; w.ldb = m->h1;
+    w.M = m->h2; w.N = m->h1;
+    w.C = m->G + m->g_w2; w.ldc = m->h1;
+    d.A = m->dZ2; d.lda = m->h2;
+    d.B = m->W2b; d.ldb = m->h1;
+    d.N = m->h1; d.K = m->h2;
+    d.H = m->dZ1; d.ldh = m->h1; d.mask = m->H1;
+    d.colpart = m->db1;
+    RQ_TRY(gemm(m->stream, w, &d));
+    // dW1 [h1 x inp] = dZ1^T X
+    w.A = m->dZ1; w.lda = m->h1;
+    w.B = X; w.ldb = m->inp;
+    w.M = m->h1; w.N = m->inp;
+    w.C = m->G + m->g_w1; w.ldc = m->inp;
+    return gemm(m->stream, w);
+}
+
+ParamMap param_map(const rq_mlp* m, int B) {
+    ParamMap k{};
+    k.in = m->in; k.h1 = m->h1; k.h2 = m->h2; k.out = m->out; k.inp = m->inp; k.outp = m->outp;
+    k.b1 = m->off_b1; k.w2 = m->off_w2; k.b2 = m->off_b2; k.w3 = m->off_w3; k.b3 = m->off_b3; k.total = m->nparam;
+    k.g1 = m->G + m->g_w1; k.g2 = m->G + m->g_w2; k.g3t = m->G + m->g_w3t;
+    k.db1 = m->db1; k.db2 = m->db2; k.db3 = m->db3;
+    k.ntile = (B + BM - 1) / BM;
+    k.W1b = m->W1b; k.W2b = m->W2b; k.W3b = m->W3b;
+    return k;
+}
+
+int loss_tiles(const rq_mlp* m, int B) { return ((B + BM - 1) / BM) * ((m->outp + 31) / 32); }
+
+// one Adam step over every parameter from the gradients of the last mlp_gradients_dev (B rows)
+int mlp_adam(rq_mlp* m, int B, float lr, float b1, float b2, float eps) {
     m->step += 1;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    const int sms = rq::num_sms(m->device);
-    struct Blk { long off, goff; int rows, cols; long gsr, gsc; };
-    const Blk blks[] = {
-        {m->off_w1, m->g_w1, m->h1, m->in, m->inp, 1},
-        {m->off_b1, m->g_b1, 1, m->h1, 0, 1},
-        {m->off_w2, m->g_w2, m->h2, m->h1, m->h1, 1},
-        {m->off_b2, m->g_b2, 1, m->h2, 0, 1},
-        {m->off_w3, m->g_w3t, m->out, m->h2, 1, m->outp},   // dW3 is stored transposed
-        {m->off_b3, m->g_b3, 1, m->out, 0, 1},
-    };
-    for (const auto& b : blks) {
-        k_adam<<<rq::grid_for((uint64_t)b.rows * b.cols, 256, sms), 256, 0, m->stream>>>(
-            m->P + b.off, m->Mo + b.off, m->Vo + b.off, m->G + b.goff, b.rows, b.cols, b.gsr, b.gsc, lr, b1, b2, eps, c1,
-            c2);
-    }
+    k_adam<<<rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0, m->stream>>>(
+        param_map(m, B), m->P, m->Mo, m->Vo, lr, b1, b2, eps, c1, c2, m->losspart, loss_tiles(m, B),
+        1.f / (float)(B * m->out), m->loss);
     RQ_CUDA(cudaGetLastError());
-    return mlp_refresh_bf16(m);
+    return RQ_OK;
 }
 
 }  // namespace
@@ -598,12 +794,9 @@ int rq_mlp_create(int32_t in, int32_t h1, int32_t h2, int32_t out, uint64_t seed
     m->off_b3 = m->off_w3 + (long)out * h2;
     m->nparam = m->off_b3 + out;
     m->g_w1 = 0;
-    m->g_b1 = m->g_w1 + (long)h1 * m->inp;
-    m->g_w2 = m->g_b1 + h1;
-    m->g_b2 = m->g_w2 + (long)h2 * h1;
-    m->g_w3t = m->g_b2 + h2;
-    m->g_b3 = m->g_w3t + (long)h2 * m->outp;
-    m->g_total = m->g_b3 + m->outp;
+    m->g_w2 = m->g_w1 + (long)h1 * m->inp;
+    m->g_w3t = m->g_w2 + (long)h2 * h1;
+    m->g_total = m->g_w3t + (long)h2 * m->outp;
     RQ_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     RQ_TRY(dalloc(&m->P, m->nparam));
     RQ_TRY(dalloc(&m->Mo, m->nparam));
@@ -613,8 +806,6 @@ int rq_mlp_create(int32_t in, int32_t h1, int32_t h2, int32_t out, uint64_t seed
     RQ_TRY(dalloc(&m->W1b, (size_t)h1 * m->inp));
     RQ_TRY(dalloc(&m->W2b, (size_t)h2 * h1));
     RQ_TRY(dalloc(&m->W3b, (size_t)m->outp * h2));
-    RQ_TRY(dalloc(&m->W2t, (size_t)h1 * h2));
-    RQ_TRY(dalloc(&m->W3t, (size_t)h2 * m->outp));
     RQ_CUDA(cudaMemset(m->G, 0, m->g_total * sizeof(float)));
     RQ_CUDA(cudaMemset(m->Mo, 0, m->nparam * sizeof(float)));
     RQ_CUDA(cudaMemset(m->Vo, 0, m->nparam * sizeof(float)));
@@ -640,10 +831,10 @@ int rq_mlp_destroy(rq_mlp* m) {
     if (!m) return RQ_OK;
     cudaSetDevice(m->device);
     if (m->stream) cudaStreamSynchronize(m->stream);
-    void* bufs[] = {m->P, m->Mo, m->Vo, m->G, m->loss, m->W1b, m->W2b, m->W3b, m->W2t, m->W3t, m->X, m->Xt, m->H1,
-                    m->H1t, m->H2, m->H2t, m->dY, m->dYt, m->dZ2, m->dZ2t, m->dZ1, m->dZ1t, m->Xf, m->Tf, m->Z1,
-                    m->Z2, m->Y, m->dH2, m->dH1};
+    void* bufs[] = {m->P, m->Mo, m->Vo, m->G, m->loss, m->W1b, m->W2b, m->W3b, m->X, m->H1, m->H2, m->dY, m->dZ2,
+                    m->dZ1, m->Xf, m->Tf, m->Y, m->db1, m->db2, m->db3, m->losspart};
     for (void* b : bufs) if (b) cudaFree(b);
+    train_release(m);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return RQ_OK;
@@ -680,7 +871,9 @@ int rq_mlp_forward(rq_mlp* m, const float* x, int32_t B, float* y) {
     RQ_CUDA(cudaSetDevice(m->device));
     RQ_TRY(mlp_reserve(m, B));
     RQ_CUDA(cudaMemcpyAsync(m->Xf, x, (size_t)B * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    RQ_TRY(mlp_forward_dev(m, B));
+    RQ_TRY(mlp_pack_rows(m, m->Xf, B, m->X));
+    RQ_TRY(mlp_hidden(m, m->X, B));
+    RQ_TRY(gemm(m->stream, output_layer(m, B)));
     RQ_CUDA(cudaMemcpy2DAsync(y, m->out * sizeof(float), m->Y, m->outp * sizeof(float), m->out * sizeof(float), B,
                               cudaMemcpyDeviceToHost, m->stream));
     RQ_CUDA(cudaStreamSynchronize(m->stream));
@@ -697,20 +890,12 @@ int rq_mlp_gradients(rq_mlp* m, const float* x, const float* t, int32_t B, float
     RQ_TRY(mlp_reserve(m, B));
     RQ_CUDA(cudaMemcpyAsync(m->Xf, x, (size_t)B * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     RQ_CUDA(cudaMemcpyAsync(m->Tf, t, (size_t)B * m->out * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    RQ_TRY(mlp_forward_dev(m, B));
-    RQ_TRY(mlp_backward_dev(m, B));
+    RQ_TRY(mlp_pack_rows(m, m->Xf, B, m->X));
+    RQ_TRY(mlp_gradients_dev(m, m->X, m->Tf, B));
     float* dflat = nullptr;
     RQ_TRY(dalloc(&dflat, m->nparam));
-    const int sms = rq::num_sms(m->device);
-    struct Blk { long off, goff; int rows, cols; long gsr, gsc; };
-    const Blk blks[] = {
-        {m->off_w1, m->g_w1, m->h1, m->in, m->inp, 1},  {m->off_b1, m->g_b1, 1, m->h1, 0, 1},
-        {m->off_w2, m->g_w2, m->h2, m->h1, m->h1, 1},   {m->off_b2, m->g_b2, 1, m->h2, 0, 1},
-        {m->off_w3, m->g_w3t, m->out, m->h2, 1, m->outp}, {m->off_b3, m->g_b3, 1, m->out, 0, 1},
-    };
-    for (const auto& b : blks)
-        k_gather<<<rq::grid_for((uint64_t)b.rows * b.cols, 256, sms), 256, 0, m->stream>>>(m->G + b.goff, b.rows, b.cols,
-                                                                                         b.gsr, b.gsc, dflat + b.off);
+    k_gather<<<rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0, m->stream>>>(
+        param_map(m, B), m->losspart, loss_tiles(m, B), 1.f / (float)(B * m->out), dflat, m->loss);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(grads, dflat, m->nparam * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream);
@@ -730,32 +915,26 @@ int rq_mlp_train(rq_mlp* m, const float* x, const float* t, int32_t n, int32_t B
     if (!m || !x || !t || n < 1 || B < 1 || steps < 0) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "bad argument");
     RQ_CUDA(cudaSetDevice(m->device));
     RQ_TRY(mlp_reserve(m, B));
-    float *dx = nullptr, *dt = nullptr;
-    RQ_TRY(dalloc(&dx, (size_t)n * m->in));
-    RQ_TRY(dalloc(&dt, (size_t)n * m->out));
+    RQ_TRY(train_reserve(m, n));
     int rc = RQ_OK;
-    cudaError_t e = cudaMemcpyAsync(dx, x, (size_t)n * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, (size_t)n * m->out * sizeof(float), cudaMemcpyHostToDevice, m->stream);
+    cudaError_t e = cudaMemcpyAsync(m->tx, x, (size_t)n * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(m->tt, t, (size_t)n * m->out * sizeof(float), cudaMemcpyHostToDevice, m->stream);
     if (e != cudaSuccess) rc = rq::cuda_fail(e, "cudaMemcpyAsync");
+    // every row in BF16 once; a minibatch is a range of those rows
+    if (rc == RQ_OK) rc = mlp_pack_rows(m, m->tx, n, m->txb);
     for (int s = 0; s < steps && rc == RQ_OK; ++s) {
         const long r0 = ((long)s * B) % n;
         const int take = (int)std::min<long>(B, n - r0);
-        e = cudaMemcpyAsync(m->Xf, dx + r0 * m->in, (size_t)take * m->in * sizeof(float), cudaMemcpyDeviceToDevice, m->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(m->Tf, dt + r0 * m->out, (size_t)take * m->out * sizeof(float), cudaMemcpyDeviceToDevice,
-                                m->stream);
-        if (e != cudaSuccess) { rc = rq::cuda_fail(e, "cudaMemcpyAsync"); break; }
-        rc = mlp_forward_dev(m, take);
-        if (rc == RQ_OK) rc = mlp_backward_dev(m, take);
-        if (rc == RQ_OK) rc = mlp_adam(m, lr, 0.9f, 0.999f, 1e-8f);
+        rc = mlp_gradients_dev(m, m->txb + r0 * m->inp, m->tt + r0 * m->out, take);
+        if (rc == RQ_OK) rc = mlp_adam(m, take, lr, 0.9f, 0.999f, 1e-8f);
     }
     if (rc == RQ_OK && last_loss) {
         e = cudaMemcpyAsync(last_loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream);
         if (e != cudaSuccess) rc = rq::cuda_fail(e, "cudaMemcpyAsync");
     }
     e = cudaStreamSynchronize(m->stream);
-    cudaFree(dx);
-    cudaFree(dt);
+    if ((size_t)n * (m->in * 4 + m->out * 4 + m->inp * 2) > TRAIN_KEEP_BYTES) train_release(m);
     RQ_TRY(rc);
     RQ_CUDA(e);
     int to = 0;

@@ -107,3 +107,28 @@ def test_mlp_training_reduces_loss():
     last = net.train(x, t, batch=256, steps=300, lr=1e-3)
     l1, _ = net.gradients(x[:256], t[:256])
     assert last < 0.3 * l0 and l1 < 0.3 * l0, (l0, last, l1)
+
+
+@pytest.mark.parametrize("dims,B", [((5, 16, 16, 2), 1), ((17, 48, 16, 8), 127), ((325, 16, 272, 33), 129),
+                                    ((100, 272, 64, 40), 700), ((40, 1040, 32, 2), 256)])
+def test_mlp_edge_shapes_match_oracle(dims, B):
+    """Widths and batches at the edges of the GEMM tiles: fewer rows than a tile, one row past
+    it, more column tiles than one, two and more K chunks (also along the batch), a remainder
+    chunk.  Same tolerances as the default widths above (BF16 operands rounded alike, FP32 sums
+    in another order)."""
+    net = Mlp(*dims, seed=11)
+    r = np.random.default_rng(B)
+    x = r.normal(size=(B, dims[0])).astype(np.float32)
+    t = r.uniform(0, 1.5, size=(B, dims[3])).astype(np.float32)
+    p = net.get_params()
+    y_ref, loss_ref, g_ref = omlp.forward_backward(p, dims, x, t, mimic_bf16=True)
+    assert np.max(np.abs(net.forward(x) - y_ref)) < 1e-3 * (1 + np.max(np.abs(y_ref)))
+    loss, g = net.gradients(x, t)
+    assert abs(loss - loss_ref) < 1e-4 * (1 + loss_ref)
+    i, h1, h2, o = dims
+    k = 0
+    for n in (h1 * i, h1, h2 * h1, h2, o * h2, o):
+        a, b = g[k:k + n], g_ref[k:k + n]
+        # an activation whose BF16 rounding or ReLU sign differs moves single entries: 1e-2 of the norm
+        assert np.linalg.norm(a - b) <= 1e-2 * (np.linalg.norm(b) + 1e-12), (n, np.linalg.norm(a - b), np.linalg.norm(b))
+        k += n
