@@ -90,9 +90,18 @@ enum Epi : int {
     EPI_F32 = 0,         // C (f32) = acc
     EPI_BIAS_RELU = 1,   // H (bf16) = relu(acc + bias)
     EPI_BIAS = 2,        // C (f32) = acc + bias
-    EPI_RELU_BACK = 3,   // H (bf16) = acc where mask > 0 and row < valid, else 0; colpart = column sums
-    EPI_MSE = 4          // d = acc + bias - target: H (bf16) = 2 d / (valid * out), colpart = column
-                         // sums of that, losspart = sum of d^2
+    EPI_RELU_BACK = 3,   // F (f32) = acc where mask > 0 and row < valid, else 0; H (bf16) = F
+    EPI_MSE = 4          // d = acc + bias - target: F (f32) = 2 d, H (bf16) = 2 d / (valid * out),
+                         // losspart = sum of d^2
+};
+
+// Column sums of an f32 matrix, dst[c] = scale * sum over the rows, added in row order: the bias
+// gradients, computed by extra CTAs (32 columns each) of a launch of products that is ready anyway.
+struct ColSum {
+    const float* src;
+    int ld, cols, rows;
+    float scale;
+    float* dst;
 };
 
 struct GemmArgs {
@@ -113,9 +122,18 @@ struct GemmArgs {
     int valid;                   // EPI_RELU_BACK, EPI_MSE: rows that count
     const float* target;         // EPI_MSE: [valid x out] f32
     int out;                     // EPI_MSE: columns that count
-    float* colpart;              // EPI_RELU_BACK, EPI_MSE: [row tiles][ldh] column sums
+    float* F;                    // EPI_RELU_BACK, EPI_MSE: [M x N] f32 (row stride ldh)
     float* losspart;             // EPI_MSE: [row tiles * column tiles]
 };
+
+// Programmatic dependent launch: a kernel of the training chain starts while its predecessor
+// drains, sets up its tensor memory and barriers, and waits here for the predecessor's results
+// (griddepcontrol.wait returns once every earlier grid of the chain has finished and its writes are
+// visible; it returns at once in a kernel launched without the attribute).  What a predecessor
+// writes is read past the L1 cache (cp.async.cg, __ldcg): the reading kernel may have begun before
+// the write, so the read-only path would be free to return or to fetch early a stale line.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ void gcp_async16(void* dst, const void* src, bool take) {
     const uint32_t n = take ? 16u : 0u;   // 0: the 16 bytes are zero-filled
@@ -126,23 +144,33 @@ __device__ __forceinline__ void gcp_async16(void* dst, const void* src, bool tak
 // Eight neighbouring threads fill one core matrix (128 contiguous bytes of shared memory, no
 // bank conflicts); a warp reads 64 contiguous bytes of each of its eight rows.
 template <int R, int KC>
-__device__ __forceinline__ void load_k_major(unsigned char* dst, const __nv_bfloat16* __restrict__ src, int ld, int row0,
+__device__ __forceinline__ void load_k_major(unsigned char* dst, const __nv_bfloat16* src, int ld, int row0,
                                              int row_lim, int k0, int kw, int tid) {
-    const int kch = kw >> 3, total = R * kch;
-    for (int u = tid; u < total; u += GT) {
-        const int cm = u >> 3, rg = cm / kch, kc = cm - rg * kch, r = rg * 8 + (u & 7);
-        const bool ok = row0 + r < row_lim;
-        const __nv_bfloat16* g = src + (ok ? (size_t)(row0 + r) * ld + k0 + kc * 8 : 0);
-        gcp_async16(dst + rg * (KC * 16) + kc * 128 + (u & 7) * 16, g, ok);
+    // core matrix (rg, kc) of this thread's eight, stepped by GT / 8 without further divisions
+    const int kch = kw >> 3, sg = (GT / 8) / kch, sc = (GT / 8) - sg * kch;
+    int rg = (tid >> 3) / kch, kc = (tid >> 3) - rg * kch;
+#pragma unroll 4
+    while (rg < R / 8) {
+        const int r = row0 + rg * 8 + (tid & 7);
+        const bool ok = r < row_lim;
+        const __nv_bfloat16* g = src + (ok ? (size_t)r * ld + k0 + kc * 8 : 0);
+        gcp_async16(dst + rg * (KC * 16) + kc * 128 + (tid & 7) * 16, g, ok);
+        rg += sg;
+        kc += sc;
+        if (kc >= kch) {
+            kc -= kch;
+            ++rg;
+        }
     }
 }
 
 // the same tile of an operand stored [K x rows]: 8x8 blocks transposed in registers, one core
 // matrix per thread and step (eight 16-byte loads in flight, eight contiguous 16-byte stores)
 template <int R, int KC>
-__device__ __forceinline__ void load_mn_major(unsigned char* dst, const __nv_bfloat16* __restrict__ src, int ld, int row0,
+__device__ __forceinline__ void load_mn_major(unsigned char* dst, const __nv_bfloat16* src, int ld, int row0,
                                               int row_lim, int k0, int kw, int k_lim, int tid) {
     const int kch = kw >> 3, total = (R / 8) * kch;
+#pragma unroll 2
     for (int u = tid; u < total; u += GT) {
         const int kc = u / (R / 8), rg = u - kc * (R / 8);   // neighbouring threads: neighbouring 16 bytes of a row
         const bool ok = row0 + rg * 8 < row_lim;
@@ -150,7 +178,7 @@ __device__ __forceinline__ void load_mn_major(unsigned char* dst, const __nv_bfl
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int k = k0 + kc * 8 + j;
-            v[j] = ok && k < k_lim ? *reinterpret_cast<const uint4*>(src + (size_t)k * ld + row0 + rg * 8)
+            v[j] = ok && k < k_lim ? __ldcg(reinterpret_cast<const uint4*>(src + (size_t)k * ld + row0 + rg * 8))
                                    : make_uint4(0u, 0u, 0u, 0u);
         }
         unsigned char* d = dst + rg * (KC * 16) + kc * 128;
@@ -168,25 +196,56 @@ __device__ __forceinline__ void load_mn_major(unsigned char* dst, const __nv_bfl
     }
 }
 
+// One thread's serial sum keeps the rounding of one long addition chain; the rows come in through
+// shared memory, 256 at a time with every load of the block in flight (a chain of dependent
+// global loads took 135 us for 256 rows).
+__device__ void column_sums(const ColSum& s, int block, float* stage, int tid) {
+    const int c0 = block * 32;
+    float acc = 0.f;
+    for (int r0 = 0; r0 < s.rows; r0 += 256) {
+        const int nr = min(256, s.rows - r0);
+#pragma unroll 8
+        for (int k = tid; k < 256 * 8; k += GT) {   // 8 float4 per row (ld and c0 are multiples of 16)
+            const int r = k >> 3, c = (k & 7) * 4;
+            if (r < nr && c0 + c < s.ld)
+                *reinterpret_cast<float4*>(stage + r * 32 + c) =
+                    __ldcg(reinterpret_cast<const float4*>(s.src + (size_t)(r0 + r) * s.ld + c0 + c));
+        }
+        __syncthreads();
+        if (tid < 32)
+#pragma unroll 16
+            for (int r = 0; r < nr; ++r) acc = fmaf(stage[r * 32 + tid], s.scale, acc);
+        __syncthreads();
+    }
+    if (tid < 32 && c0 + tid < s.cols) s.dst[c0 + tid] = acc;
+}
+
 // One launch covers the tiles of g0 and, after them, those of g1 (independent products that
-// become ready together; tiles0 = the tiles of g0).  A tile is rows [128 i, +128) x columns
+// become ready together; tiles0 and tiles1 = their tiles), then the column sums cs.  A tile is rows [128 i, +128) x columns
 // [NT j, +NT) of C.  The warm-start products are small (256 x 256 x 256-336): what bounds them is
 // the latency of load -> MMA -> epilogue, so narrow tiles (more CTAs, each loading little) and the
 // whole K in at most two chunks.  The products of a training step (batch 256, 336 -> 256 -> 256 ->
 // 8) took 80 us each on a B200 with 256-column tiles and 64-wide chunks (two CTAs, a wait after
 // every chunk) and take 8 us; the ReLU mask and the bias gradients, two kernels of 135 us that
-// walked the batch serially per column, run in this epilogue.  A step with Adam: 900 -> 65 us.
+// walked the batch serially per column, run in this epilogue and beside the products.  A step with
+// Adam: 900 -> 65 us, and 50 us with each launch's set-up overlapping its predecessor (pdl_wait).
 template <int NT, int KC>
-__global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, int tiles0) {
+__global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, const ColSum cs, int tiles0,
+                                                     int tiles1) {
     static_assert(NT % 32 == 0 && NT >= 32 && NT <= 256, "tile N");
     constexpr int ABYTES = BM * KC * 2, BBYTES = NT * KC * 2;
     extern __shared__ __align__(1024) unsigned char smem[];   // two buffers of A | B
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_base;
     __shared__ int timed_out;
-    __shared__ float colred[GT / 32][NT / 2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if ((int)blockIdx.x >= tiles0 + tiles1) {
+        pdl_wait();
+        pdl_go();
+        column_sums(cs, blockIdx.x - tiles0 - tiles1, reinterpret_cast<float*>(smem), tid);
+        return;
+    }
     const GemmArgs g = (int)blockIdx.x < tiles0 ? g0 : g1;
     const int tile = (int)blockIdx.x < tiles0 ? blockIdx.x : blockIdx.x - tiles0;
     const int mt = (g.M + BM - 1) / BM;
@@ -209,6 +268,8 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
+    pdl_wait();
+    pdl_go();
 
     const int nk = (g.K + KC - 1) / KC;
     int issued = 0;                       // chunks whose MMAs have been issued
@@ -289,7 +350,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
             if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
-                    if (c + j < g.nbias) x[j] += g.bias[c + j];
+                    if (c + j < g.nbias) x[j] += __ldcg(g.bias + c + j);
             }
             if (g.epi == EPI_F32 || g.epi == EPI_BIAS) {
                 float* o = g.C + (size_t)r * g.ldc + c;
@@ -311,8 +372,8 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
                 uint4 mk[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
                 if (in && r < g.valid) {   // N is a multiple of 16 here
                     const uint4* mp = reinterpret_cast<const uint4*>(g.mask + (size_t)r * g.ldh + c);
-                    mk[0] = mp[0];
-                    mk[1] = mp[1];
+                    mk[0] = __ldcg(mp);
+                    mk[1] = __ldcg(mp + 1);
                 }
                 const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(mk);
 #pragma unroll
@@ -324,44 +385,33 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
                     if (r < g.valid && c + j < g.out) {
                         const float d = x[j] - g.target[(size_t)r * g.out + c + j];
                         loss += d * d;
-                        gr = 2.f * d * inv;
+                        gr = 2.f * d;
                     }
                     x[j] = gr;
                 }
             }
-            if (r < g.M) {
+            if (r < g.M && c + 16 <= g.ldh) {     // ldh is a multiple of 16: whole 16-column groups
+                const size_t at = (size_t)r * g.ldh + c;
+                if (g.epi != EPI_BIAS_RELU) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4*>(g.F + at + j) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+                }
+                const float f = g.epi == EPI_MSE ? inv : 1.f;
                 __nv_bfloat16 h[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(x[j]);
-                __nv_bfloat16* o = g.H + (size_t)r * g.ldh + c;
-                if (c + 16 <= g.ldh) {     // ldh is a multiple of 16: whole 16-column groups
-                    reinterpret_cast<uint4*>(o)[0] = reinterpret_cast<const uint4*>(h)[0];
-                    reinterpret_cast<uint4*>(o)[1] = reinterpret_cast<const uint4*>(h)[1];
-                }
-            }
-            if (g.epi != EPI_BIAS_RELU) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    float t = x[j];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-                    if (lane == j) colred[warp][c0 - half * (NT / 2) + j] = t;
-                }
+                for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(x[j] * f);
+                reinterpret_cast<uint4*>(g.H + at)[0] = reinterpret_cast<const uint4*>(h)[0];
+                reinterpret_cast<uint4*>(g.H + at)[1] = reinterpret_cast<const uint4*>(h)[1];
             }
         }
-        if (g.epi == EPI_RELU_BACK || g.epi == EPI_MSE) {
+        if (g.epi == EPI_MSE) {
+            __shared__ float lred[GT / 32];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-            __shared__ float lred[GT / 32];
             if (lane == 0) lred[warp] = loss;
             __syncthreads();
-            for (int j = tid; j < NT; j += GT) {
-                const int w0 = (j / (NT / 2)) * 4, cc = j % (NT / 2);
-                if (col0 + j < g.ldh)
-                    g.colpart[(size_t)tm * g.ldh + col0 + j] =
-                        (colred[w0][cc] + colred[w0 + 1][cc]) + (colred[w0 + 2][cc] + colred[w0 + 3][cc]);
-            }
-            if (g.epi == EPI_MSE && tid == 0) {
+            if (tid == 0) {
                 float s = 0.f;
                 for (int k = 0; k < GT / 32; ++k) s += lred[k];
                 g.losspart[tile] = s;
@@ -374,26 +424,42 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NT) : "memory");
 }
 
+// launch with the programmatic-serialization attribute (see pdl_wait)
+template <typename... KA, typename... A>
+int launch_chained(cudaStream_t stream, void (*kern)(KA...), unsigned grid, unsigned threads, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    RQ_CUDA(cudaLaunchKernelEx(&cfg, kern, KA(args)...));
+    return RQ_OK;
+}
+
 template <int NT, int KC>
-int launch_gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1) {
+int launch_gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1, const ColSum* cs) {
     auto tiles = [](const GemmArgs& g) { return ((g.M + BM - 1) / BM) * ((g.N + NT - 1) / NT); };
     constexpr int smem = 2 * (BM + NT) * KC * 2;
-    const int t0 = tiles(g0);
+    const int t0 = tiles(g0), t1 = g1 ? tiles(*g1) : 0, tc = cs ? (cs->cols + 31) / 32 : 0;
     RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<NT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k_gemm_bf16<NT, KC><<<t0 + (g1 ? tiles(*g1) : 0), GT, smem, stream>>>(g0, g1 ? *g1 : g0, t0);
-    RQ_CUDA(cudaGetLastError());
-    return RQ_OK;
+    return launch_chained(stream, k_gemm_bf16<NT, KC>, t0 + t1 + tc, GT, smem, g0, g1 ? *g1 : g0,
+                          cs ? *cs : ColSum{}, t0, t1);
 }
 
 // Tile width by the number of CTAs it leaves: the widest tile whose grid still has a CTA for
 // every SM (A is re-read once per column tile, so large products want wide tiles), else 32
 // columns, where a small product spreads over the most SMs.
-int gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1 = nullptr) {
+int gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1 = nullptr, const ColSum* cs = nullptr) {
     const long mt = (g0.M + BM - 1) / BM;
-    if (!g1 && mt * ((g0.N + 255) / 256) >= 148) return launch_gemm<256, 128>(stream, g0, g1);
-    if (!g1 && mt * ((g0.N + 127) / 128) >= 148) return launch_gemm<128, 192>(stream, g0, g1);
-    if (!g1 && mt * ((g0.N + 63) / 64) >= 148) return launch_gemm<64, 192>(stream, g0, g1);
-    return launch_gemm<32, 256>(stream, g0, g1);
+    if (!g1 && mt * ((g0.N + 255) / 256) >= 148) return launch_gemm<256, 128>(stream, g0, g1, cs);
+    if (!g1 && mt * ((g0.N + 127) / 128) >= 148) return launch_gemm<128, 192>(stream, g0, g1, cs);
+    if (!g1 && mt * ((g0.N + 63) / 64) >= 148) return launch_gemm<64, 192>(stream, g0, g1, cs);
+    return launch_gemm<32, 256>(stream, g0, g1, cs);
 }
 
 }  // namespace
@@ -490,58 +556,53 @@ struct ParamMap {
     int in, h1, h2, out, inp, outp;
     long b1, w2, b2, w3, b3, total;       // first parameter of each later block
     const float *g1, *g2, *g3t;           // dW1 [h1 x inp], dW2 [h2 x h1], dW3^T [h2 x outp]
-    const float *db1, *db2, *db3;         // per-row-tile column sums: [ntile][h1 | h2 | outp]
-    int ntile;
+    const float *db1, *db2, *db3;         // [h1], [h2], [out]
     __nv_bfloat16 *W1b, *W2b, *W3b;
 };
 
 // gradient of parameter w; *copy = where its BF16 copy lives (null for a bias)
 __device__ __forceinline__ float grad_of(const ParamMap& m, long w, __nv_bfloat16** copy) {
-    const float* part;
-    int width, c;
     *copy = nullptr;
     if (w < m.b1) {
         const int r = (int)(w / m.in), k = (int)(w - (long)r * m.in);
         *copy = m.W1b + (long)r * m.inp + k;
-        return m.g1[(long)r * m.inp + k];
+        return __ldcg(m.g1 + (long)r * m.inp + k);
     } else if (w < m.w2) {
-        part = m.db1; width = m.h1; c = (int)(w - m.b1);
+        return __ldcg(m.db1 + (w - m.b1));
     } else if (w < m.b2) {
         *copy = m.W2b + (w - m.w2);
-        return m.g2[w - m.w2];
+        return __ldcg(m.g2 + (w - m.w2));
     } else if (w < m.w3) {
-        part = m.db2; width = m.h2; c = (int)(w - m.b2);
+        return __ldcg(m.db2 + (w - m.b2));
     } else if (w < m.b3) {
         const int r = (int)((w - m.w3) / m.h2), k = (int)((w - m.w3) - (long)r * m.h2);
         *copy = m.W3b + (long)r * m.h2 + k;
-        return m.g3t[(long)k * m.outp + r];
-    } else {
-        part = m.db3; width = m.outp; c = (int)(w - m.b3);
+        return __ldcg(m.g3t + (long)k * m.outp + r);
     }
-    float s = 0.f;
-    for (int t = 0; t < m.ntile; ++t) s += part[(long)t * width + c];
-    return s;
+    return __ldcg(m.db3 + (w - m.b3));
 }
 
 // One Adam step over every parameter, and the BF16 copies the next step's products read.  One
 // launch for the six blocks (they were six Adam launches, three copies and two transposes); the
 // loss of the step from its per-tile sums on the way.
-__global__ void k_adam(ParamMap map, float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float lr,
-                       float b1, float b2, float eps, float c1, float c2, const float* __restrict__ losspart, int nloss,
-                       float inv, float* __restrict__ loss) {
+__global__ void k_adam(ParamMap map, float* p, float* m, float* v, float lr,
+                       float b1, float b2, float eps, float c1, float c2, const float* losspart, int nloss,
+                       float inv, float* loss) {
+    pdl_wait();
+    pdl_go();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         float s = 0.f;
-        for (int k = 0; k < nloss; ++k) s += losspart[k];
+        for (int k = 0; k < nloss; ++k) s += __ldcg(losspart + k);
         *loss = s * inv;
     }
     for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < map.total; w += (long)gridDim.x * blockDim.x) {
         __nv_bfloat16* copy;
         const float gr = grad_of(map, w, &copy);
-        const float mm = b1 * m[w] + (1.f - b1) * gr;
-        const float vv = b2 * v[w] + (1.f - b2) * gr * gr;
+        const float mm = b1 * __ldcg(m + w) + (1.f - b1) * gr;
+        const float vv = b2 * __ldcg(v + w) + (1.f - b2) * gr * gr;
         m[w] = mm;
         v[w] = vv;
-        const float np = p[w] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+        const float np = __ldcg(p + w) - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
         p[w] = np;
         if (copy) *copy = __float2bfloat16_rn(np);
     }
@@ -552,7 +613,7 @@ __global__ void k_gather(ParamMap map, const float* __restrict__ losspart, int n
                          float* __restrict__ loss) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         float s = 0.f;
-        for (int k = 0; k < nloss; ++k) s += losspart[k];
+        for (int k = 0; k < nloss; ++k) s += __ldcg(losspart + k);
         *loss = s * inv;
     }
     for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < map.total; w += (long)gridDim.x * blockDim.x) {
@@ -580,7 +641,9 @@ struct rq_mlp {
     int cap = 0;
     __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dY = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
     float *Xf = nullptr, *Tf = nullptr, *Y = nullptr;
-    float *db1 = nullptr, *db2 = nullptr, *db3 = nullptr, *losspart = nullptr;   // per-row-tile sums
+    float *F1 = nullptr, *F2 = nullptr, *F3 = nullptr;     // f32 dZ1, dZ2 and 2 (Y - T): summed over rows into
+    float *db1 = nullptr, *db2 = nullptr, *db3 = nullptr;  // the bias gradients
+    float* losspart = nullptr;                             // per-tile sums of squares
     // a training set on the device (kept between calls up to TRAIN_KEEP_BYTES)
     float *tx = nullptr, *tt = nullptr;
     __nv_bfloat16* txb = nullptr;
@@ -636,9 +699,9 @@ int mlp_reserve(rq_mlp* m, int B) {
     RQ_TRY(regrow(&m->Xf, b * m->in));
     RQ_TRY(regrow(&m->Tf, b * m->out));
     RQ_TRY(regrow(&m->Y, b * m->outp));
-    RQ_TRY(regrow(&m->db1, nt * m->h1));
-    RQ_TRY(regrow(&m->db2, nt * m->h2));
-    RQ_TRY(regrow(&m->db3, nt * m->outp));
+    RQ_TRY(regrow(&m->F1, b * m->h1));
+    RQ_TRY(regrow(&m->F2, b * m->h2));
+    RQ_TRY(regrow(&m->F3, b * m->outp));
     RQ_TRY(regrow(&m->losspart, nt * (size_t)((m->outp + 31) / 32)));
     m->cap = Bp;
     return RQ_OK;
@@ -702,7 +765,7 @@ GemmArgs output_layer(rq_mlp* m, int B) {
 }
 
 // forward and backward pass on B packed rows X with targets T (device): weight gradients into m->G,
-// bias gradients and the loss as per-tile sums
+// bias gradients into m->db1..3, the loss as per-tile sums
 int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) {
     const int Bp = (B + 127) & ~127;
     RQ_TRY(mlp_hidden(m, X, B));
@@ -713,8 +776,8 @@ int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) 
     y.epi = EPI_MSE;
     y.nbias = m->out;
     y.valid = B; y.out = m->out; y.target = T;
-    y.colpart = m->db3; y.losspart = m->losspart;
-    RQ_TRY((launch_gemm<32, 256>(m->stream, y, nullptr)));
+    y.F = m->F3; y.losspart = m->losspart;
+    RQ_TRY((launch_gemm<32, 256>(m->stream, y, nullptr, nullptr)));
     // dW3^T [h2 x outp] = H2^T dY, and dZ2 [Bp x h2] = (dY W3) where H2 > 0
     GemmArgs w{};
     w.A = m->H2; w.lda = m->h2; w.at = 1;
@@ -727,9 +790,10 @@ int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) 
     d.B = m->W3b; d.ldb = m->h2; d.bt = 1;
     d.M = Bp; d.N = m->h2; d.K = m->outp;
     d.H = m->dZ2; d.ldh = m->h2; d.mask = m->H2;
-    d.valid = B; d.colpart = m->db2;
+    d.valid = B; d.F = m->F2;
     d.epi = EPI_RELU_BACK;
-    RQ_TRY(gemm(m->stream, w, &d));
+    const ColSum b3{m->F3, m->outp, m->out, B, 1.f / (float)(B * m->out), m->db3};
+    RQ_TRY(gemm(m->stream, w, &d, &b3));
     // dW2 [h2 x h1] = dZ2^T H1, and dZ1 [Bp x h1] = (dZ2 W2) where H1 > 0
     w.A = m->dZ2; w.lda = m->h2;
     w.B = m->H1; w.ldb = m->h1;
@@ -739,23 +803,24 @@ int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) 
     d.B = m->W2b; d.ldb = m->h1;
     d.N = m->h1; d.K = m->h2;
     d.H = m->dZ1; d.ldh = m->h1; d.mask = m->H1;
-    d.colpart = m->db1;
-    RQ_TRY(gemm(m->stream, w, &d));
+    d.F = m->F1;
+    const ColSum b2{m->F2, m->h2, m->h2, B, 1.f, m->db2};
+    RQ_TRY(gemm(m->stream, w, &d, &b2));
     // dW1 [h1 x inp] = dZ1^T X
     w.A = m->dZ1; w.lda = m->h1;
     w.B = X; w.ldb = m->inp;
     w.M = m->h1; w.N = m->inp;
     w.C = m->G + m->g_w1; w.ldc = m->inp;
-    return gemm(m->stream, w);
+    const ColSum b1{m->F1, m->h1, m->h1, B, 1.f, m->db1};
+    return gemm(m->stream, w, nullptr, &b1);
 }
 
-ParamMap param_map(const rq_mlp* m, int B) {
+ParamMap param_map(const rq_mlp* m) {
     ParamMap k{};
     k.in = m->in; k.h1 = m->h1; k.h2 = m->h2; k.out = m->out; k.inp = m->inp; k.outp = m->outp;
     k.b1 = m->off_b1; k.w2 = m->off_w2; k.b2 = m->off_b2; k.w3 = m->off_w3; k.b3 = m->off_b3; k.total = m->nparam;
     k.g1 = m->G + m->g_w1; k.g2 = m->G + m->g_w2; k.g3t = m->G + m->g_w3t;
     k.db1 = m->db1; k.db2 = m->db2; k.db3 = m->db3;
-    k.ntile = (B + BM - 1) / BM;
     k.W1b = m->W1b; k.W2b = m->W2b; k.W3b = m->W3b;
     return k;
 }
@@ -766,11 +831,9 @@ int loss_tiles(const rq_mlp* m, int B) { return ((B + BM - 1) / BM) * ((m->outp 
 int mlp_adam(rq_mlp* m, int B, float lr, float b1, float b2, float eps) {
     m->step += 1;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    k_adam<<<rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0, m->stream>>>(
-        param_map(m, B), m->P, m->Mo, m->Vo, lr, b1, b2, eps, c1, c2, m->losspart, loss_tiles(m, B),
-        1.f / (float)(B * m->out), m->loss);
-    RQ_CUDA(cudaGetLastError());
-    return RQ_OK;
+    return launch_chained(m->stream, k_adam, rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0,
+                          param_map(m), m->P, m->Mo, m->Vo, lr, b1, b2, eps, c1, c2, m->losspart, loss_tiles(m, B),
+                          1.f / (float)(B * m->out), m->loss);
 }
 
 }  // namespace
@@ -803,6 +866,9 @@ int rq_mlp_create(int32_t in, int32_t h1, int32_t h2, int32_t out, uint64_t seed
     RQ_TRY(dalloc(&m->Vo, m->nparam));
     RQ_TRY(dalloc(&m->G, m->g_total));
     RQ_TRY(dalloc(&m->loss, 1));
+    RQ_TRY(dalloc(&m->db1, h1));
+    RQ_TRY(dalloc(&m->db2, h2));
+    RQ_TRY(dalloc(&m->db3, out));
     RQ_TRY(dalloc(&m->W1b, (size_t)h1 * m->inp));
     RQ_TRY(dalloc(&m->W2b, (size_t)h2 * h1));
     RQ_TRY(dalloc(&m->W3b, (size_t)m->outp * h2));
@@ -832,7 +898,7 @@ int rq_mlp_destroy(rq_mlp* m) {
     cudaSetDevice(m->device);
     if (m->stream) cudaStreamSynchronize(m->stream);
     void* bufs[] = {m->P, m->Mo, m->Vo, m->G, m->loss, m->W1b, m->W2b, m->W3b, m->X, m->H1, m->H2, m->dY, m->dZ2,
-                    m->dZ1, m->Xf, m->Tf, m->Y, m->db1, m->db2, m->db3, m->losspart};
+                    m->dZ1, m->Xf, m->Tf, m->Y, m->F1, m->F2, m->F3, m->db1, m->db2, m->db3, m->losspart};
     for (void* b : bufs) if (b) cudaFree(b);
     train_release(m);
     if (m->stream) cudaStreamDestroy(m->stream);
@@ -895,7 +961,7 @@ int rq_mlp_gradients(rq_mlp* m, const float* x, const float* t, int32_t B, float
     float* dflat = nullptr;
     RQ_TRY(dalloc(&dflat, m->nparam));
     k_gather<<<rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0, m->stream>>>(
-        param_map(m, B), m->losspart, loss_tiles(m, B), 1.f / (float)(B * m->out), dflat, m->loss);
+        param_map(m), m->losspart, loss_tiles(m, B), 1.f / (float)(B * m->out), dflat, m->loss);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(grads, dflat, m->nparam * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream);
