@@ -177,6 +177,9 @@ RQ_API int rq_state_from_amplitudes(const double* interleaved, uint64_t len,
                              uint32_t num_qubits, int32_t precision,
                              uint64_t seed, rq_state** out);
 
+/* Ends the state.  Its stream and small device buffers are kept for a later state of the
+ * same size on that device (bounded; freed when idle or when memory runs out), unless
+ * rq_state_device_ptr handed the memory out. */
 RQ_API int rq_state_destroy(rq_state* s);
 
 /* Back to |0...0>, measurement stream rewound to draw 0 of the same seed.

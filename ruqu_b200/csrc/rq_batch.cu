@@ -1376,7 +1376,7 @@ int grow(P** ptr, size_t* cap, size_t need_elems) {
     if (*ptr) cudaFree(*ptr);
     *ptr = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc((void**)ptr, need_elems * sizeof(P));
+    cudaError_t e = rq::device_malloc((void**)ptr, need_elems * sizeof(P));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return rq::fail(RQ_ERR_MEMORY_ALLOCATION,
@@ -1388,7 +1388,7 @@ int grow(P** ptr, size_t* cap, size_t need_elems) {
 
 template <typename P>
 int dalloc_b(P** p, size_t n) {
-    cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(1, n) * sizeof(P));
+    cudaError_t e = rq::device_malloc((void**)p, std::max<size_t>(1, n) * sizeof(P));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return rq::fail(RQ_ERR_MEMORY_ALLOCATION, "memory allocation failed: need " + std::to_string(n * sizeof(P)) + " bytes");
@@ -1401,7 +1401,7 @@ int grow_bytes(void** ptr, size_t* cap, size_t bytes) {
     if (*ptr) cudaFree(*ptr);
     *ptr = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc(ptr, bytes);
+    cudaError_t e = rq::device_malloc(ptr, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return rq::fail(RQ_ERR_MEMORY_ALLOCATION, "memory allocation failed: need " + std::to_string(bytes) + " bytes");

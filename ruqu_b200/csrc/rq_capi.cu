@@ -9,7 +9,7 @@
 #include "rq_internal.cuh"
 
 #include <algorithm>
-
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -102,6 +102,156 @@ int check_create(uint32_t nq, int32_t prec) {
     return RQ_OK;
 }
 
+// What a destroyed state leaves for the next one: its stream, its pinned staging and its small
+// device buffers.  A driver that evaluates one circuit per state (evaluate_energy,
+// evaluate_qaoa_cost, run_shots) spent 3-30 ms per evaluation in cudaMalloc, cudaFree,
+// cudaMallocHost, cudaFreeHost and stream creation -- the calls serialise with every process on
+// the machine's GPUs -- against 0.2 ms on the device.  Bounds: POOL_ENTRIES sets, POOL_STATE_BYTES
+// of device memory each, POOL_TOTAL_BYTES in all; sets unused for POOL_IDLE_S are freed at the next
+// create or destroy, all of them when an allocation fails (device_malloc).  A set enters the pool
+// with its stream drained, and never with amplitudes whose device pointer was handed out
+// (rq_state_device_ptr): another stream may still use those.
+constexpr size_t POOL_ENTRIES = 16;
+constexpr size_t POOL_STATE_BYTES = (size_t)64 << 20;
+constexpr size_t POOL_TOTAL_BYTES = (size_t)256 << 20;
+constexpr double POOL_IDLE_S = 30.0;
+constexpr size_t AMPS_MIN_BYTES = (size_t)64 << 10;   // small states share one size
+
+struct PoolEntry {
+    rq_state r;                       // the resources only: stream, buffers and their sizes
+    unsigned long long ctx = 0;       // context they belong to
+    double since = 0.0;
+    size_t bytes() const {
+        return (r.amps ? r.amps_cap : 0) + r.scratch_cap + (r.partials_cap + r.tree_cap) * sizeof(double);
+    }
+};
+
+struct Pool {
+    std::mutex mu;
+    std::vector<PoolEntry> entries;   // oldest first
+};
+
+Pool& pool() {
+    static Pool* p = new Pool();      // never destroyed: the driver releases everything at exit
+    return *p;
+}
+
+double now_s() {
+    return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
+}
+
+// free a set's resources (its device current); a set of a context that is gone is only forgotten
+void release_resources(rq_state& r, unsigned long long ctx) {
+    if (ctx != rq::current_context_id()) return;
+    if (r.amps) cudaFree(r.amps);
+    if (r.partials) cudaFree(r.partials);
+    if (r.tree) cudaFree(r.tree);
+    if (r.scratch) cudaFree(r.scratch);
+    if (r.hbuf) cudaFreeHost(r.hbuf);
+    if (r.stream) cudaStreamDestroy(r.stream);
+}
+
+// free the entries for which `drop` holds, on their devices
+template <class F>
+void pool_drop(F drop) {
+    std::vector<PoolEntry> out;
+    {
+        std::lock_guard<std::mutex> lk(pool().mu);
+        auto& e = pool().entries;
+        for (size_t k = 0; k < e.size();)
+            if (drop(e[k])) {
+                out.push_back(e[k]);
+                e.erase(e.begin() + k);
+            } else {
+                ++k;
+            }
+    }
+    if (out.empty()) return;
+    int cur = 0;
+    cudaGetDevice(&cur);
+    for (auto& e : out) {
+        cudaSetDevice(e.r.device);
+        release_resources(e.r, e.ctx);
+    }
+    cudaSetDevice(cur);
+}
+
+void pool_drop_idle() {
+    const double t = now_s();
+    pool_drop([t](const PoolEntry& e) { return t - e.since > POOL_IDLE_S; });
+}
+
+// a set for `amps_bytes` on the current device: one with amplitudes of that size, else one without
+// amplitudes
+bool pool_take(int device, size_t amps_bytes, rq_state* s) {
+    const unsigned long long ctx = rq::current_context_id();
+    if (ctx == 0) return false;
+    pool_drop([device, ctx](const PoolEntry& e) { return e.r.device == device && e.ctx != ctx; });
+    std::lock_guard<std::mutex> lk(pool().mu);
+    auto& es = pool().entries;
+    for (int pass = 0; pass < 2; ++pass)
+        for (size_t k = es.size(); k-- > 0;) {
+            const rq_state& r = es[k].r;
+            if (r.device != device || (pass == 0 ? !r.amps || r.amps_cap != amps_bytes : r.amps != nullptr)) continue;
+            s->stream = r.stream;
+            s->amps = r.amps;
+            s->amps_cap = r.amps ? r.amps_cap : 0;
+            s->partials = r.partials;
+            s->partials_cap = r.partials_cap;
+            s->tree = r.tree;
+            s->tree_cap = r.tree_cap;
+            s->hbuf = r.hbuf;
+            s->hbuf_cap = r.hbuf_cap;
+            s->scratch = r.scratch;
+            s->scratch_cap = r.scratch_cap;
+            es.erase(es.begin() + k);
+            return true;
+        }
+    return false;
+}
+
+// the resources of a destroyed state (its device current, its stream drained)
+void pool_give(rq_state* s) {
+    PoolEntry e;
+    e.r = *s;
+    e.ctx = rq::current_context_id();
+    e.since = now_s();
+    rq_state rest;                    // what does not enter the pool
+    if (s->exported || s->amps_cap > POOL_STATE_BYTES) {
+        rest.amps = e.r.amps;
+        e.r.amps = nullptr;
+        e.r.amps_cap = 0;
+    }
+    if (e.bytes() > POOL_STATE_BYTES) {
+        rest.tree = e.r.tree;
+        e.r.tree = nullptr;
+        e.r.tree_cap = 0;
+    }
+    if (s->exported || e.ctx == 0 || e.bytes() > POOL_STATE_BYTES) {   // an exported stream is not reused either
+        release_resources(e.r, e.ctx);
+    } else {
+        std::vector<PoolEntry> out;
+        {
+            std::lock_guard<std::mutex> lk(pool().mu);
+            auto& es = pool().entries;
+            es.push_back(e);
+            size_t total = 0;
+            for (const auto& x : es) total += x.bytes();
+            while (es.size() > POOL_ENTRIES || total > POOL_TOTAL_BYTES) {
+                total -= es.front().bytes();
+                out.push_back(es.front());
+                es.erase(es.begin());
+            }
+        }
+        for (auto& x : out) {
+            cudaSetDevice(x.r.device);
+            release_resources(x.r, x.ctx);
+        }
+        cudaSetDevice(s->device);
+    }
+    release_resources(rest, e.ctx);
+}
+
 int alloc_state(uint32_t nq, int32_t prec, uint64_t seed, rq_state** out) {
     rq_state* s = new rq_state();
     s->nq = nq;
@@ -109,18 +259,26 @@ int alloc_state(uint32_t nq, int32_t prec, uint64_t seed, rq_state** out) {
     s->n = 1ull << nq;
     s->seed = seed;
     s->device = device_of_current();
-    cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
-    if (e != cudaSuccess) {
-        delete s;
-        return rq::cuda_fail(e, "cudaStreamCreateWithFlags");
+    const size_t need = s->bytes(), cap = std::max(need, AMPS_MIN_BYTES);
+    pool_drop_idle();
+    cudaError_t e = cudaSuccess;
+    if (!pool_take(s->device, cap, s)) {
+        e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+        if (e != cudaSuccess) {
+            delete s;
+            return rq::cuda_fail(e, "cudaStreamCreateWithFlags");
+        }
     }
-    e = cudaMalloc(&s->amps, s->bytes());
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        size_t need = s->bytes();
-        cudaStreamDestroy(s->stream);
-        delete s;
-        return rq::fail(RQ_ERR_MEMORY_ALLOCATION, "memory allocation failed: need " + std::to_string(need) + " bytes");
+    if (!s->amps) {
+        e = rq::device_malloc(&s->amps, cap);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            s->amps = nullptr;
+            release_resources(*s, rq::current_context_id());
+            delete s;
+            return rq::fail(RQ_ERR_MEMORY_ALLOCATION, "memory allocation failed: need " + std::to_string(need) + " bytes");
+        }
+        s->amps_cap = cap;
     }
     *out = s;
     return RQ_OK;
@@ -247,7 +405,7 @@ int ensure_partials(rq_state* s, size_t nd) {
         s->partials_cap = 0;
     }
     size_t cap = nd < 4096 ? 4096 : nd;
-    RQ_CUDA(cudaMalloc(&s->partials, cap * sizeof(double)));
+    RQ_CUDA(device_malloc((void**)&s->partials, cap * sizeof(double)));
     s->partials_cap = cap;
     return RQ_OK;
 }
@@ -274,7 +432,7 @@ int ensure_tree(rq_state* s, size_t nd) {
         s->tree = nullptr;
         s->tree_cap = 0;
     }
-    cudaError_t e = cudaMalloc(&s->tree, nd * sizeof(double));
+    cudaError_t e = device_malloc((void**)&s->tree, nd * sizeof(double));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(RQ_ERR_MEMORY_ALLOCATION, "memory allocation failed: need " + std::to_string(nd * sizeof(double)) +
@@ -282,6 +440,62 @@ int ensure_tree(rq_state* s, size_t nd) {
     }
     s->tree_cap = nd;
     return RQ_OK;
+}
+
+int scratch_get(rq_state* s, size_t bytes, void** out) {
+    if (bytes > SCRATCH_KEEP_BYTES) {
+        RQ_CUDA(cudaMallocAsync(out, bytes, s->stream));
+        return RQ_OK;
+    }
+    if (s->scratch_cap < bytes) {
+        if (s->scratch) {
+            RQ_CUDA(cudaStreamSynchronize(s->stream));
+            cudaFree(s->scratch);
+            s->scratch = nullptr;
+            s->scratch_cap = 0;
+        }
+        size_t cap = (size_t)64 << 10;
+        while (cap < bytes) cap <<= 1;
+        RQ_CUDA(device_malloc(&s->scratch, cap));
+        s->scratch_cap = cap;
+    }
+    *out = s->scratch;
+    return RQ_OK;
+}
+
+void scratch_put(rq_state* s, void* p) {
+    if (p && p != s->scratch) cudaFreeAsync(p, s->stream);
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    pool_drop([](const PoolEntry&) { return true; });
+    return cudaMalloc(p, bytes);
+}
+
+// Unique id of the current CUDA context (cuCtxGetId, reached through the runtime's
+// driver entry points so the library needs no libcuda link); 0 when unavailable.
+unsigned long long current_context_id() {
+    using GetCurrent = int (*)(void**);
+    using GetId = int (*)(void*, unsigned long long*);
+    static GetCurrent get_current = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess ? reinterpret_cast<GetCurrent>(f) : nullptr;
+    }();
+    static GetId get_id = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(f) : nullptr;
+    }();
+    void* ctx = nullptr;
+    unsigned long long id = 0;
+    if (!get_current || !get_id || get_current(&ctx) != 0 || !ctx || get_id(ctx, &id) != 0) return 0;
+    return id;
 }
 
 }  // namespace rq
@@ -474,13 +688,11 @@ int rq_plan_destroy(rq_plan* p) {
 int rq_state_destroy(rq_state* s) {
     if (!s) return RQ_OK;
     cudaSetDevice(s->device);
-    if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->amps) cudaFree(s->amps);
-    if (s->partials) cudaFree(s->partials);
-    if (s->tree) cudaFree(s->tree);
-    if (s->hbuf) cudaFreeHost(s->hbuf);
-    if (s->stream) cudaStreamDestroy(s->stream);
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) pool_give(s);
+    else release_resources(*s, rq::current_context_id());
     delete s;
+    pool_drop_idle();
     return RQ_OK;
 }
 
@@ -505,6 +717,7 @@ int rq_state_precision(const rq_state* s, int32_t* out) {
 
 int rq_state_device_ptr(const rq_state* s, void** out_ptr, void** out_stream) {
     if (!s) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "null state");
+    const_cast<rq_state*>(s)->exported = true;
     if (out_ptr) *out_ptr = s->amps;
     if (out_stream) *out_stream = (void*)s->stream;
     return RQ_OK;
@@ -716,11 +929,11 @@ int rq_state_probabilities(rq_state* s, double* out) {
     if (!s || !out) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "null pointer");
     RQ_TRY(set_device(s));
     double* d = nullptr;
-    RQ_CUDA(cudaMallocAsync((void**)&d, s->n * sizeof(double), s->stream));
+    RQ_TRY(rq::scratch_get(s, s->n * sizeof(double), (void**)&d));
     int rc = rq::probabilities_dev(s, d);
     cudaError_t e = cudaSuccess;
     if (rc == RQ_OK) e = cudaMemcpyAsync(out, d, s->n * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-    cudaFreeAsync(d, s->stream);
+    rq::scratch_put(s, d);
     RQ_TRY(rc);
     RQ_CUDA(e);
     RQ_CUDA(cudaStreamSynchronize(s->stream));
@@ -853,11 +1066,11 @@ int rq_state_download(rq_state* s, double* out) {
         return rq::sync_checked(s);
     }
     double* d = nullptr;
-    RQ_CUDA(cudaMallocAsync((void**)&d, bytes, s->stream));
+    RQ_TRY(rq::scratch_get(s, bytes, (void**)&d));
     int rc = rq::download_f64(s, d);
     cudaError_t e = cudaSuccess;
     if (rc == RQ_OK) e = cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, s->stream);
-    cudaFreeAsync(d, s->stream);
+    rq::scratch_put(s, d);
     RQ_TRY(rc);
     RQ_CUDA(e);
     return rq::sync_checked(s);
@@ -873,10 +1086,10 @@ int rq_state_upload(rq_state* s, const double* in) {
         return RQ_OK;
     }
     double* d = nullptr;
-    RQ_CUDA(cudaMallocAsync((void**)&d, bytes, s->stream));
+    RQ_TRY(rq::scratch_get(s, bytes, (void**)&d));
     cudaError_t e = cudaMemcpyAsync(d, in, bytes, cudaMemcpyHostToDevice, s->stream);
     int rc = e == cudaSuccess ? rq::upload_f64(s, d) : rq::cuda_fail(e, "cudaMemcpyAsync");
-    cudaFreeAsync(d, s->stream);
+    rq::scratch_put(s, d);
     RQ_TRY(rc);
     RQ_CUDA(cudaStreamSynchronize(s->stream));
     return RQ_OK;

@@ -29,6 +29,11 @@ struct rq_state {
     bool tree_ready = false;      // tree holds the levels of tree_order (rq_state_tree_build / sample)
     double* hbuf = nullptr;       // pinned host staging for small results
     size_t hbuf_cap = 0;          // in doubles
+    void* scratch = nullptr;      // device scratch of the calls that return arrays (scratch_get)
+    size_t scratch_cap = 0;       // in bytes
+    size_t amps_cap = 0;          // bytes allocated for amps
+    bool exported = false;        // the device pointer was handed out: its memory is never reused
+    bool tc_ran = false;          // a tensor-core sweep was launched since the last check of its waits
     int32_t exec_mode = RQ_EXEC_AUTO;
     size_t elem_bytes() const { return prec == RQ_F32 ? 8 : 16; }
     size_t bytes() const { return (size_t)n * elem_bytes(); }
@@ -52,6 +57,8 @@ int cuda_fail(cudaError_t e, const char* what);
 
 // ---- device facts --------------------------------------------------------
 int num_sms(int device);
+// unique id of the current CUDA context, 0 when unavailable
+unsigned long long current_context_id();
 
 // Grid for a grid-stride loop over `work` items: at most 8 resident
 // 256-thread blocks per SM, never more blocks than needed.
@@ -66,6 +73,13 @@ inline unsigned grid_for(uint64_t work, int threads, int sms, int per_sm = 8) {
 int ensure_partials(rq_state* s, size_t ndoubles);
 int ensure_hbuf(rq_state* s, size_t ndoubles);
 int ensure_tree(rq_state* s, size_t ndoubles);
+// `bytes` of device scratch for one call on s's stream: the state's own buffer up to
+// SCRATCH_KEEP_BYTES (kept for the next call), a stream-ordered allocation above that.
+constexpr size_t SCRATCH_KEEP_BYTES = (size_t)64 << 20;
+int scratch_get(rq_state* s, size_t bytes, void** out);
+void scratch_put(rq_state* s, void* p);
+// cudaMalloc that gives the memory of destroyed states back and tries again before it fails
+cudaError_t device_malloc(void** p, size_t bytes);
 
 // ---- kernels' host launchers (rq_gates.cu) --------------------------------
 int init_basis(rq_state* s, uint64_t index);

@@ -657,7 +657,7 @@ namespace {
 
 template <typename P>
 int dalloc(P** p, size_t n) {
-    cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(1, n) * sizeof(P));
+    cudaError_t e = rq::device_malloc((void**)p, std::max<size_t>(1, n) * sizeof(P));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return rq::fail(RQ_ERR_MEMORY_ALLOCATION, "memory allocation failed: need " + std::to_string(n * sizeof(P)) + " bytes");

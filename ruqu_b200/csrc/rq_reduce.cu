@@ -422,29 +422,6 @@ std::mutex g_noalloc_mu;
 double* g_noalloc_addr[kMaxDevices] = {nullptr};
 unsigned long long g_noalloc_ctx[kMaxDevices] = {0};   // context the address belongs to
 
-// Unique id of the current CUDA context (cuCtxGetId, reached through the runtime's
-// driver entry points so the library needs no libcuda link); 0 when unavailable.
-unsigned long long current_context_id() {
-    using GetCurrent = int (*)(void**);
-    using GetId = int (*)(void*, unsigned long long*);
-    static GetCurrent get_current = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        return cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-                       q == cudaDriverEntryPointSuccess ? reinterpret_cast<GetCurrent>(f) : nullptr;
-    }();
-    static GetId get_id = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        return cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-                       q == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(f) : nullptr;
-    }();
-    void* ctx = nullptr;
-    unsigned long long id = 0;
-    if (!get_current || !get_id || get_current(&ctx) != 0 || !ctx || get_id(ctx, &id) != 0) return 0;
-    return id;
-}
-
 // Device address of g_noalloc_scratch on the current device.  In host code
 // the array's name is only a host-side stand-in, so the address is looked up
 // with that device current, once per device and context: the first call on a
@@ -454,7 +431,7 @@ unsigned long long current_context_id() {
 int noalloc_scratch_address(int device, double** out) {
     if (device < 0 || device >= kMaxDevices) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "device index out of range");
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
-    const unsigned long long ctx = current_context_id();
+    const unsigned long long ctx = rq::current_context_id();
     if (!g_noalloc_addr[device] || ctx == 0 || ctx != g_noalloc_ctx[device]) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);

@@ -203,7 +203,7 @@ int sample(rq_state* s, const uint32_t* qubits, uint32_t nqm, uint64_t base_seed
     RQ_TRY(build_tree(s, P));
     const int sms = num_sms(s->device);
     uint64_t* dout = nullptr;
-    RQ_CUDA(cudaMallocAsync((void**)&dout, shots * sizeof(uint64_t), s->stream));
+    RQ_TRY(scratch_get(s, shots * sizeof(uint64_t), (void**)&dout));
     unsigned gs = grid_for(shots, 128, sms);
     if (s->prec == RQ_F32)
         k_sample<float><<<gs, 128, 0, s->stream>>>((const float2*)s->amps, s->tree, P, plan, base_seed, shots, dout);
@@ -211,7 +211,7 @@ int sample(rq_state* s, const uint32_t* qubits, uint32_t nqm, uint64_t base_seed
         k_sample<double><<<gs, 128, 0, s->stream>>>((const double2*)s->amps, s->tree, P, plan, base_seed, shots, dout);
     cudaError_t le = cudaGetLastError();
     cudaError_t ce = cudaMemcpyAsync(host_out, dout, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream);
-    cudaFreeAsync(dout, s->stream);
+    scratch_put(s, dout);
     RQ_CUDA(le);
     RQ_CUDA(ce);
     return rq::sync_checked(s);
@@ -231,15 +231,11 @@ int tree_lookup(rq_state* s, uint32_t level, const uint64_t* index, uint64_t cou
         if (index[i] >= lim) return fail(RQ_ERR_INVALID_ARGUMENT, "tree index out of range for its level");
     if (count == 0) return RQ_OK;
     const Perm P = stored_perm(s);
+    static_assert(sizeof(uint64_t) == sizeof(double), "one buffer holds the indices, then the results");
     uint64_t* didx = nullptr;
-    double* dout = nullptr;
-    RQ_CUDA(cudaMallocAsync((void**)&didx, count * sizeof(uint64_t), s->stream));
-    cudaError_t e = cudaMallocAsync((void**)&dout, count * sizeof(double), s->stream);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(didx, s->stream);
-        return cuda_fail(e, "tree lookup buffers");
-    }
-    e = cudaMemcpyAsync(didx, index, count * sizeof(uint64_t), cudaMemcpyHostToDevice, s->stream);
+    RQ_TRY(scratch_get(s, 2 * count * sizeof(uint64_t), (void**)&didx));
+    double* dout = reinterpret_cast<double*>(didx + count);
+    cudaError_t e = cudaMemcpyAsync(didx, index, count * sizeof(uint64_t), cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess) {
         const unsigned g = grid_for(count, TPB, num_sms(s->device));
         if (s->prec == RQ_F32)
@@ -249,8 +245,7 @@ int tree_lookup(rq_state* s, uint32_t level, const uint64_t* index, uint64_t cou
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_out, dout, count * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-    cudaFreeAsync(didx, s->stream);
-    cudaFreeAsync(dout, s->stream);
+    scratch_put(s, didx);
     RQ_CUDA(e);
     return rq::sync_checked(s);
 }
