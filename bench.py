@@ -330,7 +330,7 @@ def vqe_batch_leg(a, ws, rank, with_cpu):
                         "peak_kind": peak_kind, "bytes": prof["sweep_bytes"], "kernel_ms": prof["sweep_ms"],
                         "note": "waves of ~96 MB of states are sized to stay in L2, so these bytes are mostly "
                                 "L2 traffic: a fraction above 1 of the HBM copy peak is possible and expected"},
-           "energy_pass": {"kernel": "k_vqe_energy_tiles", "flops": prof["energy_flops"],
+           "energy_pass": {"kernel": "k_vqe_energy", "flops": prof["energy_flops"],
                            "kernel_ms": prof["energy_ms"],
                            "achieved_tflops": prof["energy_flops"] / (prof["energy_ms"] / 1e3) / 1e12,
                            "flops_definition": "8 per Pauli string and amplitude: one complex product "

@@ -213,6 +213,21 @@ __device__ __forceinline__ void op_ry(V* reg, T c, T s) {
     }
 }
 
+// Ry on the packed qubit: (x, y) -> (c x - s y, s x + c y) in every element
+template <int NR, typename V, typename T>
+__device__ __forceinline__ void op_ry0(V* reg, T c, T s) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const V v = reg[i];
+        if constexpr (std::is_same<T, float>::value) {
+            reg[i] = pk_fma(make_float2(c, s), make_float2(v.x, v.x), pk_mul(make_float2(-s, c), make_float2(v.y, v.y)));
+        } else {
+            reg[i].x = c * v.x - s * v.y;
+            reg[i].y = s * v.x + c * v.y;
+        }
+    }
+}
+
 template <int NR, typename V, typename T>
 __device__ __forceinline__ void dispatch_ry(int k, V* reg, T c, T s) {
     switch (k) {
@@ -362,6 +377,14 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
                         const int b1 = k1 >= 0 ? ((i >> k1) & 1) : u1;
                         if (b0 & b1) { reg[i].x = -reg[i].x; reg[i].y = -reg[i].y; }
                     }
+                } else if (op.type == OP_RY0) {
+                    const T* r = a.rot + ((size_t)gcirc * a.nparam + op.param) * 2;
+                    op_ry0<NR>(reg, r[0], r[1]);
+                } else if (op.type == OP_CZ0) {
+                    const int u0 = (int)((U >> op.q0) & 1ull);
+#pragma unroll
+                    for (int i = 0; i < NR; ++i)
+                        if (op.k0 >= 0 ? ((i >> op.k0) & 1) : u0) reg[i].y = -reg[i].y;
                 } else if (op.type == OP_CPH) {
                     CutNb<RB> cp;
                     cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
@@ -661,6 +684,22 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                     flush(dispatch_im_y<NR>(op.k0, rp, rl), op.param);
                     dispatch_ry<NR>(op.k0, rp, r[0], -r[1]);
                     dispatch_ry<NR>(op.k0, rl, r[0], -r[1]);
+                } else if (op.type == OP_RY0) {
+                    const T* r = a.rot + ((size_t)gcirc * a.nparam + op.param) * 2;
+                    T acc = 0;   // Im <lambda|Y|psi> on the packed qubit
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) acc += rl[i].y * rp[i].x - rl[i].x * rp[i].y;
+                    flush((double)acc, op.param);
+                    op_ry0<NR>(rp, r[0], -r[1]);
+                    op_ry0<NR>(rl, r[0], -r[1]);
+                } else if (op.type == OP_CZ0) {
+                    const int u0 = (int)((U >> op.q0) & 1ull);
+#pragma unroll
+                    for (int i = 0; i < NR; ++i)
+                        if (op.k0 >= 0 ? ((i >> op.k0) & 1) : u0) {
+                            rp[i].y = -rp[i].y;
+                            rl[i].y = -rl[i].y;
+                        }
                 } else if (op.type == OP_CZ) {   // self-inverse
                     const int k0 = op.k0, k1 = op.k1;
                     const int u0 = (int)((U >> op.q0) & 1ull), u1 = (int)((U >> op.q1) & 1ull);
@@ -857,250 +896,277 @@ __global__ void k_bsample(const typename C2<T>::t* __restrict__ amps, const doub
 
 
 // ---- batched VQE -------------------------------------------------------------
-
-// Pauli strings sharing one X/Y pattern (same rules as rq_reduce.cu):
-// x == 0: acc += s(i)|a_i|^2 over all i; x != 0: over pairs (i, i^x) with the
-// top bit h of x clear, acc += s(i) * (odd ? Im : Re) of conj(a_{i^x}) a_i.
-struct VGroup {
-    uint64_t x;
-    uint32_t h, t0, nt, pad;
+//
+// The ansatz (Ry rotations and CZ signs on |0...0>) never leaves the real numbers, so a state of
+// n qubits is kept as 2^(n-1) elements (x, y) = the real amplitudes of qubit 0 = 0 and 1: half the
+// memory, half the arithmetic and half the shared-memory traffic of complex amplitudes with zero
+// imaginary parts, and the same kernels (Ry on any other qubit acts on both parts alike; OP_RY0
+// and OP_CZ0 handle qubit 0).  A string with an odd number of Y factors is imaginary and
+// antisymmetric: its expectation in a real state is zero, and it adds nothing to a gradient.
+//
+// On an element index j (the qubits above 0) and part b (qubit 0) a string with X/Y mask
+// x = 2X + x0, Y/Z mask z = 2Z + z0 and an even number of Y factors has, up to its factor,
+//   <P> = sum_j (-1)^|j & Z| (A.x B.x' + (-1)^z0 A.y B.y'),  A = a_j, B = a_(j ^ X),
+// with B's parts swapped when x0 = 1.
+struct PTerm {
+    uint32_t xl;      // X inside a tile of 2^M elements
+    uint32_t z;       // Z
+    uint32_t z0;      // sign bit (bit 31) of (-1)^z0
+    uint32_t pad;
+    double f;         // energy pass: coefficient and pair factors; H pass: coefficient
 };
-struct VTerm {
-    uint64_t pmask;
-    uint32_t odd, pad;
-    double factor;   // coeff * the ny / pairing factor
+// strings of one kind, [begin, end): top part t of X, x0, and (energy pass) how their pairs are
+// walked -- mode b < RBITS: X has register bit b, walk the elements where it is 0; RBITS: walk all;
+// RBITS + 1 + v: X crosses tiles and its top bit inside the tile is v
+struct PSeg {
+    uint32_t x0, mode, begin, end;
 };
 
-template <typename T>
-__global__ void k_vqe_energy(const typename C2<T>::t* __restrict__ states, uint32_t n, uint64_t ncirc, uint64_t circ0,
-                             const VGroup* __restrict__ groups, uint32_t ngroups, const VTerm* __restrict__ terms,
-                             double* __restrict__ energies) {
-    __shared__ double red[8][8];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const uint64_t N = 1ull << n;
-    for (uint64_t c = blockIdx.x; c < ncirc; c += gridDim.x) {
-        const typename C2<T>::t* a = states + c * N;
-        double E = 0.0;
-        for (uint32_t g = 0; g < ngroups; ++g) {
-            const VGroup G = groups[g];
-            uint64_t pm[8];
-            uint32_t od[8];
-            double acc[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                pm[k] = k < (int)G.nt ? terms[G.t0 + k].pmask : 0;
-                od[k] = k < (int)G.nt ? terms[G.t0 + k].odd : 0;
-                acc[k] = 0.0;
-            }
-            const uint64_t count = G.x ? N >> 1 : N;
-            for (uint64_t q = threadIdx.x; q < count; q += blockDim.x) {
-                uint64_t i;
-                double re, im;
-                if (G.x == 0) {
-                    i = q;
-                    const auto v = a[i];
-                    const double vr = v.x, vi = v.y;
-                    re = vr * vr + vi * vi;
-                    im = 0.0;
-                } else {
-                    i = rqd::insert0(q, G.h);
-                    const auto ai = a[i];
-                    const auto aj = a[i ^ G.x];
-                    const double air = ai.x, aii = ai.y, ajr = aj.x, aji = aj.y;
-                    re = ajr * air + aji * aii;
-                    im = ajr * aii - aji * air;
-                }
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const double v = od[k] ? im : re;
-                    acc[k] += (__popcll(i & pm[k]) & 1) ? -v : v;
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                double v = warp_sum_d(acc[k]);
-                if (lane == 0) red[warp][k] = v;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                for (uint32_t k = 0; k < G.nt; ++k) {
-                    double sum = 0.0;
-                    for (uint32_t w = 0; w < nw; ++w) sum += red[w][k];
-                    E += terms[G.t0 + k].factor * sum;
-                }
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) energies[circ0 + c] = E;
-    }
+// threads of the two kernels below; element e = tid + (register index << PK_TB)
+constexpr int PK_THREADS = 512, PK_TB = 9;
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return pk_mul(a, b); }
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ float2 fma2(float s, float2 b, float2 c) { return pk_fma(make_float2(s, s), b, c); }
+__device__ __forceinline__ double2 fma2(double s, double2 b, double2 c) { return make_double2(fma(s, b.x, c.x), fma(s, b.y, c.y)); }
+
+template <typename V>
+__device__ __forceinline__ void pk_load_tile(V* dst, const V* __restrict__ src, uint32_t L, uint32_t tid) {
+    constexpr uint32_t EPC = 16 / sizeof(V);
+    if (L >= EPC)
+        for (uint32_t e = tid * EPC; e < L; e += PK_THREADS * EPC) bcp_async16(dst + e, src + e);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-
-// One Pauli group of a tile pass: NT strings (NT = 8 for 5..8), per-warp sums
-// into wsum.  Products of amplitudes in the state's precision, every product
-// added to an FP64 accumulator; indices fit 32 bits (at most 30 qubits).
-// need: 1 = only Re of conj(a_j) a_i is used, 2 = only Im, 3 = both.
-// a group's pairs are split into this many work units, so that the warps of a CTA finish a
-// partner tile together (groups alone are too few and too coarse to balance 16 warps)
-constexpr uint32_t VQE_CHUNKS = 4;
-
-template <typename T, int NT>
-__device__ __forceinline__ void tile_group(const VGroup& G, const VTerm* __restrict__ terms,
-                                           const typename C2<T>::t* own, const typename C2<T>::t* src, uint32_t r,
-                                           uint32_t rp, uint32_t t, uint32_t M, double* wsum, uint32_t nterms,
-                                           uint32_t lane, uint32_t warp, uint32_t chunk, uint32_t nchunk) {
+// The strings [begin, end) of one segment over the register elements A: per string the products of
+// the walked elements (one shared-memory load each), a tree over the register bits with each bit's
+// sign as a factor (at most 16 products in the state's type), then FP64.
+// BIT >= 0: walk the elements whose register bit BIT is HI; BIT < 0: all.
+template <typename T, int RBITS, int BIT, int HI>
+__device__ __forceinline__ double pk_walk(const typename C2<T>::t* A, const typename C2<T>::t* src,
+                                          const PTerm* __restrict__ terms, uint32_t begin, uint32_t end, uint32_t own,
+                                          uint32_t tid, uint32_t L) {
     using V = typename C2<T>::t;
-    const uint32_t L = 1u << M;
-    uint32_t pm[NT];
-    bool od[NT];
-    double acc[NT];
-    int need = 0;
+    constexpr int NB = BIT >= 0 ? RBITS - 1 : RBITS;   // free register bits
+    constexpr int NW = 1 << NB;
+    const bool in = tid < L;
+    double acc = 0.0;
+    PTerm nt = terms[begin];
+    for (uint32_t k = begin; k < end; ++k) {
+        const PTerm t = nt;
+        if (k + 1 < end) nt = terms[k + 1];
+        const uint32_t P = in ? tid ^ t.xl : 0u;
+        V v[NW];
 #pragma unroll
-    for (int k = 0; k < NT; ++k) {
-        pm[k] = k < (int)G.nt ? (uint32_t)terms[G.t0 + k].pmask : 0u;
-        od[k] = k < (int)G.nt ? terms[G.t0 + k].odd != 0 : false;
-        if (k < (int)G.nt) need |= od[k] ? 2 : 1;
-        acc[k] = 0.0;
-    }
-    const uint32_t x = (uint32_t)G.x;
-    const uint32_t xl = x & (L - 1);
-    const uint32_t count = x == 0 ? L : L >> 1;
-    // this call's share of the group's pairs: chunk `chunk` of `nchunk` equal parts
-    const uint32_t qlo = (uint32_t)(((uint64_t)count * chunk) / nchunk), qhi = (uint32_t)(((uint64_t)count * (chunk + 1)) / nchunk);
-    const uint32_t sel = r < rp ? 0u : (1u ^ ((xl >> (M - 1)) & 1u));
-    const uint32_t rbase = r << M, pbase = rp << M;
-    // one warp owns the group: its lanes walk all pairs, one warp reduction per group.  The
-    // products are summed in T over 16 pairs of a lane, then added into the FP64 accumulators
-    // (16 terms in f32 keep the partial within ~1e-6 relative).
-    for (uint32_t q0 = qlo + lane; q0 < qhi; q0 += 32 * 16) {
-        T part[NT];
-#pragma unroll
-        for (int k = 0; k < NT; ++k) part[k] = (T)0;
-#pragma unroll 4
-        for (uint32_t u = 0; u < 16; ++u) {
-            const uint32_t q = q0 + 32 * u;
-            if (q >= qhi) break;
-            T re = 0, im = 0;
-            uint32_t i;
-            if (x == 0) {
-                i = rbase | q;
-                const V v = own[q];
-                re = v.x * v.x + v.y * v.y;
-            } else {
-                V af, as;
-                if (t == 0) {
-                    const uint32_t e = (uint32_t)rqd::insert0(q, G.h);
-                    i = rbase | e;
-                    af = own[e];
-                    as = own[e ^ xl];
-                } else {
-                    const uint32_t e = (uint32_t)rqd::insert0(q, M - 1) | (sel << (M - 1));
-                    const uint32_t ep = e ^ xl;
-                    const uint32_t im_ = rbase | e;
-                    const V ao = own[e], ap = src[ep];
-                    const bool first_is_mine = !((im_ >> G.h) & 1u);
-                    i = first_is_mine ? im_ : (pbase | ep);
-                    af = first_is_mine ? ao : ap;
-                    as = first_is_mine ? ap : ao;
-                }
-                if (need & 1) re = as.x * af.x + as.y * af.y;
-                if (need & 2) im = as.x * af.y - as.y * af.x;
-            }
-#pragma unroll
-            for (int k = 0; k < NT; ++k) {
-                const T v = od[k] ? im : re;
-                part[k] += (__popc(i & pm[k]) & 1) ? -v : v;
-            }
+        for (int w = 0; w < NW; ++w) {
+            const int i = BIT < 0 ? w : ((w >> BIT) << (BIT + 1)) | (HI << BIT) | (w & ((1 << (BIT < 0 ? 0 : BIT)) - 1));
+            v[w] = mul2(A[i], src[P ^ ((uint32_t)i << PK_TB)]);
         }
 #pragma unroll
-        for (int k = 0; k < NT; ++k) acc[k] += (double)part[k];
-    }
+        for (int b = 0; b < NB; ++b) {
+            const int gb = BIT >= 0 && b >= BIT ? b + 1 : b;
+            const T sg = ((t.z >> (PK_TB + gb)) & 1u) ? (T)-1 : (T)1;
 #pragma unroll
-    for (int k = 0; k < NT; ++k) {
-        const double v = warp_sum_d(acc[k]);
-        if (lane == 0 && k < (int)G.nt) wsum[warp * nterms + G.t0 + k] += v;
+            for (int w = 0; w < NW; w += 2 << b) v[w] = fma2(sg, v[w + (1 << b)], v[w]);
+        }
+        const uint32_t st = (uint32_t)__popc((own | tid | ((uint32_t)(HI && BIT >= 0 ? 1 : 0) << (PK_TB + (BIT < 0 ? 0 : BIT)))) & t.z) & 1u;
+        const T s0 = t.z0 ? (T)-1 : (T)1;
+        const T s = v[0].x + s0 * v[0].y;
+        acc += (st ? -t.f : t.f) * (double)s;
     }
+    return acc;
 }
 
-// Tiled form: the state of a circuit is split into ntile tiles of 2^M
-// amplitudes; the CTA of (circuit, tile r) keeps tile r in shared memory and
-// loads every partner tile r ^ t once, evaluating all Pauli groups whose X/Y
-// pattern has top part x >> M == t from on-chip memory.  Pairs inside tile r
-// (t = 0) are all counted by that CTA; pairs between tiles lo < hi are split
-// by bit M-1 of their element in tile lo (0: CTA lo, 1: CTA hi), so each pair
-// is counted once.  Each group is walked by one warp (groups dealt round-robin
-// to the warps), whose per-string sums land in shared memory; the CTA writes one
-// partial per string, and k_vqe_finalize adds the tiles and the strings in a
-// fixed order.
-template <typename T>
-__global__ void __launch_bounds__(512, 1) k_vqe_energy_tiles(const typename C2<T>::t* __restrict__ states, uint32_t n,
-                                                             uint32_t M, uint64_t ncirc,
-                                                             const VGroup* __restrict__ groups,
-                                                             const uint32_t* __restrict__ gofs, uint32_t nterms,
-                                                             const VTerm* __restrict__ terms,
-                                                             double* __restrict__ part) {
+template <typename T, int RBITS>
+__device__ __forceinline__ double pk_segment(const PSeg& g, const typename C2<T>::t* A, const typename C2<T>::t* src,
+                                             const PTerm* __restrict__ terms, uint32_t own, bool lower, uint32_t tid,
+                                             uint32_t L) {
+    if constexpr (RBITS > 0) {
+        if (g.mode > RBITS) {   // pairs across two tiles: the lower tile's CTA takes its elements with top bit 0
+            const uint32_t hi = lower ? 0u : 1u ^ (g.mode - RBITS - 1);
+            return hi ? pk_walk<T, RBITS, RBITS - 1, 1>(A, src, terms, g.begin, g.end, own, tid, L)
+                      : pk_walk<T, RBITS, RBITS - 1, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+        }
+        if (g.mode == 0) return pk_walk<T, RBITS, 0, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+        if constexpr (RBITS > 1)
+            if (g.mode == 1) return pk_walk<T, RBITS, 1, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+        if constexpr (RBITS > 2)
+            if (g.mode == 2) return pk_walk<T, RBITS, 2, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+        if constexpr (RBITS > 3)
+            if (g.mode == 3) return pk_walk<T, RBITS, 3, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+    }
+    return pk_walk<T, RBITS, -1, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+}
+
+// Energy of every (circuit, tile) of a wave: a thread keeps its 2^RBITS elements of the tile in
+// registers for all strings; the partner tiles r ^ t (t = 0: the tile itself) come in turn through
+// two shared-memory buffers, the next loading while one is in use.  Per string and thread one load
+// and two packed FP32x2 instructions per element walked, and one FP64 FMA: strings add up in FP64
+// per thread and are reduced over the CTA once.  Pairs inside the tile are walked once by a register
+// bit of X (where X has none, all elements are walked and f is halved), pairs between two tiles half
+// by each tile's CTA.  Bound by instruction issue.  The one-warp-per-string walk of complex tiles this
+// replaces was bound by its index and sign arithmetic: 13.6 us per 16-qubit circuit and 200 strings
+// (2056 circuits), now 1.1 us.
+template <typename T, int RBITS>
+__global__ void __launch_bounds__(PK_THREADS, 1)
+    k_vqe_energy(const typename C2<T>::t* __restrict__ states, uint32_t n, uint32_t M, uint64_t ncirc,
+                 const PSeg* __restrict__ segs, const uint32_t* __restrict__ sofs, const PTerm* __restrict__ terms,
+                 double e0, double* __restrict__ part) {
     using V = typename C2<T>::t;
+    constexpr int NR = 1 << RBITS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint64_t L = 1ull << M;
-    V* own = reinterpret_cast<V*>(smem_raw);
-    V* par = own + L;
-    double* wsum = reinterpret_cast<double*>(par + L);   // [warps][nterms]
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    __shared__ double red[PK_THREADS / 32];
+    const uint32_t L = 1u << M, tid = threadIdx.x;
+    V* buf[2] = {reinterpret_cast<V*>(smem_raw), reinterpret_cast<V*>(smem_raw) + L};
     const uint32_t ntile = 1u << (n - M);
-    const uint64_t N = 1ull << n;
     const uint64_t nwork = ncirc * ntile;
     for (uint64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
         const uint64_t c = w / ntile;
         const uint32_t r = (uint32_t)(w - c * ntile);
-        const V* a = states + c * N;
-        for (uint32_t k = threadIdx.x; k < nw * nterms; k += blockDim.x) wsum[k] = 0.0;
-        for (uint64_t e = threadIdx.x; e < L; e += blockDim.x) own[e] = a[((uint64_t)r << M) | e];
-        __syncthreads();
-        for (uint32_t t = 0; t < ntile; ++t) {
-            if (gofs[t] == gofs[t + 1]) continue;
-            const uint32_t rp = r ^ t;
-            const V* src = own;
-            if (t) {
-                for (uint64_t e = threadIdx.x; e < L; e += blockDim.x) par[e] = a[((uint64_t)rp << M) | e];
-                __syncthreads();
-                src = par;
-            }
-            // work units: each group's pairs in VQE_CHUNKS equal parts, dealt to the warps in turn
-            // (a warp's partial sums of a term add up in its own row of wsum)
-            const uint32_t nunits = (gofs[t + 1] - gofs[t]) * VQE_CHUNKS;
-            for (uint32_t u = warp; u < nunits; u += nw) {
-                const VGroup G = groups[gofs[t] + u / VQE_CHUNKS];
-                const uint32_t ch = u % VQE_CHUNKS;
-                switch (G.nt) {
-                    case 1: tile_group<T, 1>(G, terms, own, src, r, rp, t, M, wsum, nterms, lane, warp, ch, VQE_CHUNKS); break;
-                    case 2: tile_group<T, 2>(G, terms, own, src, r, rp, t, M, wsum, nterms, lane, warp, ch, VQE_CHUNKS); break;
-                    case 3: tile_group<T, 3>(G, terms, own, src, r, rp, t, M, wsum, nterms, lane, warp, ch, VQE_CHUNKS); break;
-                    case 4: tile_group<T, 4>(G, terms, own, src, r, rp, t, M, wsum, nterms, lane, warp, ch, VQE_CHUNKS); break;
-                    default: tile_group<T, 8>(G, terms, own, src, r, rp, t, M, wsum, nterms, lane, warp, ch, VQE_CHUNKS); break;
-                }
+        const V* a = states + (c << n);
+        const uint32_t own = r << M;
+        V A[NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const uint32_t e = tid | ((uint32_t)i << PK_TB);
+            A[i] = e < L ? a[own | e] : V{0, 0};
+        }
+        auto next_t = [&](uint32_t t) {
+            while (t < ntile && sofs[t] == sofs[t + 1]) ++t;
+            return t;
+        };
+        double acc = 0.0;
+        uint32_t t = next_t(0), at = 0;
+        if (t < ntile) pk_load_tile<V>(buf[0], a + ((uint64_t)(r ^ t) << M), L, tid);
+        while (t < ntile) {
+            const uint32_t tn = next_t(t + 1);
+            if (tn < ntile) {
+                pk_load_tile<V>(buf[at ^ 1], a + ((uint64_t)(r ^ tn) << M), L, tid);
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             }
             __syncthreads();
+            uint32_t swapped = 0;
+            for (uint32_t g = sofs[t]; g < sofs[t + 1]; ++g) {
+                const PSeg sg = segs[g];
+                if (sg.x0 != swapped) {   // strings with x0 = 1 follow those with x0 = 0
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) A[i] = V{A[i].y, A[i].x};
+                    swapped = sg.x0;
+                }
+                acc += pk_segment<T, RBITS>(sg, A, buf[at], terms, own, r < (r ^ t), tid, L);
+            }
+            if (swapped) {
+#pragma unroll
+                for (int i = 0; i < NR; ++i) A[i] = V{A[i].y, A[i].x};
+            }
+            __syncthreads();
+            at ^= 1u;
+            t = tn;
         }
-        for (uint32_t k = threadIdx.x; k < nterms; k += blockDim.x) {
-            double sum = 0.0;
-            for (uint32_t wv = 0; wv < nw; ++wv) sum += wsum[wv * nterms + k];
-            part[w * nterms + k] = sum;
+        acc = warp_sum_d(acc);
+        if ((tid & 31u) == 0) red[tid >> 5] = acc;
+        __syncthreads();
+        if (tid == 0) {
+            double e = r == 0 ? e0 : 0.0;
+            for (int k = 0; k < PK_THREADS / 32; ++k) e += red[k];
+            part[w] = e;
         }
         __syncthreads();
     }
 }
 
-// energies[circ0 + c] = sum over strings (in order) of factor * sum over tiles
-__global__ void k_vqe_finalize(const double* __restrict__ part, uint64_t ncirc, uint32_t ntile, uint32_t nterms,
-                               const VTerm* __restrict__ terms, uint64_t circ0, double* __restrict__ energies) {
-    for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncirc; c += (uint64_t)gridDim.x * blockDim.x) {
-        double E = 0.0;
-        for (uint32_t k = 0; k < nterms; ++k) {
-            double s = 0.0;
-            for (uint32_t r = 0; r < ntile; ++r) s += part[(c * ntile + r) * nterms + k];
-            E += terms[k].factor * s;
+// lambda = H psi for every (circuit, tile) of a wave (the start of the VQE adjoint pass): a thread
+// owns 2^RBITS output elements (both parts summed in FP64 over the strings), the source tiles r ^ t
+// come through shared memory as in the energy pass.  Per string and element one shared-memory load,
+// the sign flips, two conversions and two FP64 FMAs; the grid-stride kernel this replaces read every
+// source amplitude from L2 and summed both complex parts of every string: 19.7 us per 16-qubit
+// circuit and 200 strings (512 circuits), now 3.3 us.
+template <typename T> struct SignBits;
+template <> struct SignBits<float> {
+    static __device__ __forceinline__ float flip(float v, uint32_t m) { return __uint_as_float(__float_as_uint(v) ^ m); }
+};
+template <> struct SignBits<double> {
+    static __device__ __forceinline__ double flip(double v, uint32_t m) {
+        return __hiloint2double(__double2hiint(v) ^ (int)m, __double2loint(v));
+    }
+};
+
+template <typename T, int RBITS>
+__global__ void __launch_bounds__(PK_THREADS, 1)
+    k_vqe_apply_h(const typename C2<T>::t* __restrict__ states, typename C2<T>::t* __restrict__ lam, uint32_t n,
+                  uint32_t M, uint64_t ncirc, const PSeg* __restrict__ segs, const uint32_t* __restrict__ sofs,
+                  const PTerm* __restrict__ terms) {
+    using V = typename C2<T>::t;
+    constexpr int NR = 1 << RBITS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t L = 1u << M, tid = threadIdx.x;
+    const bool in = tid < L;
+    V* buf[2] = {reinterpret_cast<V*>(smem_raw), reinterpret_cast<V*>(smem_raw) + L};
+    const uint32_t ntile = 1u << (n - M);
+    const uint64_t nwork = ncirc * ntile;
+    for (uint64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
+        const uint64_t c = w / ntile;
+        const uint32_t r = (uint32_t)(w - c * ntile);
+        const V* a = states + (c << n);
+        double hx[NR], hy[NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) hx[i] = hy[i] = 0.0;
+        auto next_t = [&](uint32_t t) {
+            while (t < ntile && sofs[t] == sofs[t + 1]) ++t;
+            return t;
+        };
+        uint32_t t = next_t(0), at = 0;
+        if (t < ntile) pk_load_tile<V>(buf[0], a + ((uint64_t)(r ^ t) << M), L, tid);
+        while (t < ntile) {
+            const uint32_t tn = next_t(t + 1);
+            if (tn < ntile) {
+                pk_load_tile<V>(buf[at ^ 1], a + ((uint64_t)(r ^ tn) << M), L, tid);
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            }
+            __syncthreads();
+            const V* src = buf[at];
+            const uint32_t top = (r ^ t) << M;
+            for (uint32_t g = sofs[t]; g < sofs[t + 1]; ++g) {
+                const PSeg sg = segs[g];
+                PTerm nt = terms[sg.begin];
+                for (uint32_t k = sg.begin; k < sg.end; ++k) {
+                    const PTerm tm = nt;
+                    if (k + 1 < sg.end) nt = terms[k + 1];
+                    const uint32_t P = in ? tid ^ tm.xl : 0u;
+                    // sign of the source element (index parity with Z); part b of the source
+                    // carries (-1)^(b z0) and lands in part b ^ x0
+                    uint32_t m = (uint32_t)(__popc((top | P) & tm.z) & 1) << 31;
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) {
+                        const int i = q ^ (q >> 1);   // Gray-code order: one sign bit changes per element
+                        if (q) m ^= ((tm.z >> (PK_TB + gray_bit(q))) & 1u) << 31;
+                        const V v = src[P ^ ((uint32_t)i << PK_TB)];
+                        const double vx = (double)SignBits<T>::flip(v.x, m);
+                        const double vy = (double)SignBits<T>::flip(v.y, m ^ tm.z0);
+                        if (sg.x0) {
+                            hx[i] = fma(tm.f, vy, hx[i]);
+                            hy[i] = fma(tm.f, vx, hy[i]);
+                        } else {
+                            hx[i] = fma(tm.f, vx, hx[i]);
+                            hy[i] = fma(tm.f, vy, hy[i]);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            at ^= 1u;
+            t = tn;
         }
-        energies[circ0 + c] = E;
+        V* o = lam + (c << n) + ((uint64_t)r << M);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const uint32_t e = tid | ((uint32_t)i << PK_TB);
+            if (e < L) o[e] = V{(T)hx[i], (T)hy[i]};
+        }
     }
 }
 
@@ -1127,44 +1193,6 @@ __global__ void k_vqe_rot(const double* __restrict__ params, uint64_t ncirc, uin
 constexpr int TPB = 256;
 
 }  // namespace
-
-// One Hamiltonian string as the operator i^ny X^x Z^pm: (P psi)[i] = c_k (-1)^popc((i^x) & pm) psi[i ^ x]
-// with c_k = coeff * i^ny (ny = number of Y factors); (cr, ci) = c_k.
-struct HTerm {
-    uint64_t x, pm;
-    double cr, ci;
-};
-
-// lambda = H psi for every circuit of a wave (the start of the VQE adjoint pass).  One
-// output amplitude per thread and grid-stride step; the strings are read in order by
-// every thread (uniform loads), psi[i ^ x] from L2 (a warp's 32 indices map to one
-// aligned 32-amplitude block), the sum over strings in FP64.
-template <typename T>
-__global__ void __launch_bounds__(256) k_vqe_apply_h(const typename C2<T>::t* __restrict__ psi,
-                                                     typename C2<T>::t* __restrict__ lam, uint32_t n, uint64_t ncirc,
-                                                     const HTerm* __restrict__ terms, uint32_t nterms) {
-    using V = typename C2<T>::t;
-    const uint64_t N = 1ull << n;
-    const uint64_t total = ncirc * N;
-    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t c = w >> n, i = w & (N - 1);
-        const V* src = psi + c * N;
-        double re = 0.0, im = 0.0;
-        for (uint32_t k = 0; k < nterms; ++k) {
-            const HTerm t = terms[k];
-            const uint64_t j = i ^ t.x;
-            const V v = src[j];
-            const double sg = (__popcll(j & t.pm) & 1) ? -1.0 : 1.0;
-            const double cr = sg * t.cr, ci = sg * t.ci;
-            re += cr * (double)v.x - ci * (double)v.y;
-            im += cr * (double)v.y + ci * (double)v.x;
-        }
-        V o;
-        o.x = (T)re;
-        o.y = (T)im;
-        lam[w] = o;
-    }
-}
 
 // ===========================================================================
 // batch object
@@ -2323,11 +2351,13 @@ struct rq_vqe_batch {
     size_t off_ops = 0, smem = 0;
     uint64_t ntiles = 0;
     uint32_t m = 0;
-    VGroup* d_groups = nullptr;
-    VTerm* d_terms = nullptr;
-    uint32_t* d_gofs = nullptr;   // groups of top pattern t: [gofs[t], gofs[t+1])
-    uint32_t ngroups = 0, nterms = 0;
-    uint32_t em = 0;              // log2 amplitudes of an energy tile
+    uint32_t pn = 0;              // qubits of the packed real state (n - 1)
+    uint32_t em = 0;              // log2 elements of a tile of the energy and H passes
+    uint32_t nterms = 0;          // strings as given
+    double e0 = 0.0;              // what the strings without a real expectation add (0, or NaN)
+    PTerm* d_terms = nullptr;     // energy strings, then H strings, by segment
+    PSeg* d_segs = nullptr;
+    uint32_t* d_sofs = nullptr;   // segments of top part t: [sofs[t], sofs[t + 1]); H pass: after ntile + 1
     double* d_part = nullptr;
     size_t part_cap = 0;
     double* d_params = nullptr;
@@ -2348,8 +2378,6 @@ struct rq_vqe_batch {
     std::vector<SweepDesc> adescs;
     unsigned char* aprog = nullptr;
     size_t aoff_ops = 0;
-    HTerm* d_hterms = nullptr;
-    uint32_t nhterms = 0;
     void* d_lam = nullptr;
     size_t lam_cap = 0;
     double* d_gpart = nullptr;
@@ -2360,29 +2388,90 @@ struct rq_vqe_batch {
 
 namespace {
 
-// energy of every circuit of a wave through the tiled kernel
+// The sweeps of a list of Ry and CZ gates on n qubits for the packed real state of n - 1 (qubit
+// q > 0 is its qubit q - 1, qubit 0 its two parts).  The gates are planned as sweeps over the
+// 2^n amplitudes (mloc local qubits) and run in exactly that order, so every amplitude goes
+// through the same roundings as unpacked: planning the packed gates afresh saves a sweep in four
+// on 16 qubits (5.5 instead of 5.8 ms for 2056 circuits) but its other order of the rotations moves
+// single f32 energies by their whole rounding error.  The order is cut into sweeps of m local packed
+// qubits and phases of rb slots; qubit 0 needs neither.
+void packed_program(const std::vector<PGate>& gates, uint32_t n, uint32_t mloc, uint32_t m, uint32_t rb, uint32_t epv,
+                    std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
+    const uint32_t m0 = std::min(n, mloc), c = std::min<uint32_t>(m, 5);
+    std::vector<PGate> order;
+    for (const auto& sw : plan_sweeps(gates, n, m0, std::min<uint32_t>(m0, 5)))
+        for (const auto& pp : plan_phases(sw, rb))
+            for (int k : pp.ops) {
+                PGate g = sw.ops[k];
+                if (g.type == OP_RYP && g.q0 == 0) {
+                    g.type = OP_RY0;
+                } else if (g.type == OP_CZ && g.q0 == 0) {
+                    g.type = OP_CZ0;
+                    g.q0 = g.q1 - 1;
+                } else {
+                    g.q0 -= 1;
+                    if (g.type == OP_CZ) g.q1 -= 1;
+                }
+                order.push_back(g);
+            }
+    const uint64_t base = (1ull << c) - 1;
+    std::vector<Sweep> sweeps;
+    std::vector<std::vector<PhasePlan>> pplans;
+    for (const auto& g : order) {
+        const uint64_t nd = needs(g);
+        if (sweeps.empty() || (uint32_t)__builtin_popcountll(sweeps.back().L | nd) > m) {
+            sweeps.push_back(Sweep{base, {}});
+            pplans.push_back({PhasePlan{0, {}}});
+        }
+        Sweep& sw = sweeps.back();
+        auto& pp = pplans.back();
+        sw.L |= nd;
+        if ((uint32_t)__builtin_popcountll(pp.back().R | nd) > rb) pp.push_back(PhasePlan{0, {}});
+        pp.back().R |= nd;
+        pp.back().ops.push_back((int)sw.ops.size());
+        sw.ops.push_back(g);
+    }
+    for (size_t k = 0; k < sweeps.size(); ++k) {   // fill up the local qubits, then each phase's slots
+        for (uint32_t q = 0; q < n - 1 && (uint32_t)__builtin_popcountll(sweeps[k].L) < m; ++q) sweeps[k].L |= 1ull << q;
+        for (auto& pp : pplans[k])
+            for (uint32_t q = n - 1; q-- > 0 && (uint32_t)__builtin_popcountll(pp.R) < rb;) pp.R |= (1ull << q) & sweeps[k].L;
+    }
+    std::vector<double> mats;
+    build_program(sweeps, n - 1, m, c, rb, epv, descs, phases, ops, mats, false, &pplans);
+}
+
+// calls f(std::integral_constant<int, RBITS>) for the register bits of a tile of 2^M elements
+template <typename T, class F>
+int with_register_bits(uint32_t M, F f) {
+    switch (M > (uint32_t)PK_TB ? M - PK_TB : 0) {
+        case 0: return f(std::integral_constant<int, 0>());
+        case 1: return f(std::integral_constant<int, 1>());
+        case 2: return f(std::integral_constant<int, 2>());
+        case 3: return f(std::integral_constant<int, 3>());
+        default: break;
+    }
+    if constexpr (std::is_same<T, float>::value) return f(std::integral_constant<int, 4>());
+    return rq::fail(RQ_ERR_CUDA, "energy tile too large");
+}
+
+// energy of every circuit of a wave
 template <typename T>
 int vqe_energy(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     using V = typename C2<T>::t;
-    const uint32_t n = b->n;
-    const uint32_t M = b->em;
-    const uint32_t ntile = 1u << (n - M);
-    const uint32_t threads = 512;
-    const size_t smem = 2 * ((size_t)1 << M) * sizeof(V) + (size_t)(threads / 32) * b->nterms * sizeof(double);
-    if (smem > 227 * 1024) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "Hamiltonian has too many strings for the energy kernel");
-    auto kern = k_vqe_energy_tiles<T>;
-    RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    RQ_TRY(grow(&b->d_part, &b->part_cap, ncirc * ntile * std::max<uint32_t>(1, b->nterms)));
-    int per_sm = 0;
-    RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
-    if (per_sm < 1) return rq::fail(RQ_ERR_CUDA, "energy kernel does not fit on an SM");
+    const uint32_t ntile = 1u << (b->pn - b->em);
+    const size_t smem = 2 * ((size_t)1 << b->em) * sizeof(V);
+    RQ_TRY(grow(&b->d_part, &b->part_cap, ncirc * ntile));
     const int sms = rq::num_sms(b->device);
-    const unsigned grid = (unsigned)std::min<uint64_t>(ncirc * ntile, (uint64_t)sms * per_sm);
-    kern<<<grid, threads, smem, b->stream>>>((const V*)b->d_states, n, M, ncirc, b->d_groups, b->d_gofs, b->nterms,
-                                             b->d_terms, b->d_part);
-    RQ_CUDA(cudaGetLastError());
-    k_vqe_finalize<<<rq::grid_for(ncirc, TPB, sms), TPB, 0, b->stream>>>(b->d_part, ncirc, ntile, b->nterms, b->d_terms,
-                                                                         circ0, b->d_energy);
+    const unsigned grid = (unsigned)std::min<uint64_t>(ncirc * ntile, (uint64_t)sms);
+    RQ_TRY(with_register_bits<T>(b->em, [&](auto rbits) {
+        auto kern = k_vqe_energy<T, decltype(rbits)::value>;
+        RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<grid, PK_THREADS, smem, b->stream>>>((const V*)b->d_states, b->pn, b->em, ncirc, b->d_segs, b->d_sofs,
+                                                    b->d_terms, b->e0, b->d_part);
+        RQ_CUDA(cudaGetLastError());
+        return (int)RQ_OK;
+    }));
+    k_energy_finalize<<<rq::grid_for(ncirc, TPB, sms), TPB, 0, b->stream>>>(b->d_part, ncirc, ntile, circ0, b->d_energy);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -2413,7 +2502,7 @@ int vqe_wave(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
         kern<<<grid, threads, b->smem, b->stream>>>(d, ph, op, a);
         RQ_CUDA(cudaGetLastError());
     }
-    const double sb = (double)((size_t)1 << b->n) * sizeof(V);
+    const double sb = (double)((size_t)1 << b->pn) * sizeof(V);
     b->prof.end(ev, b->stream, 0, (double)ncirc * sweep_bytes(b->descs, sb));
     ev = b->prof.begin(b->stream);
     RQ_TRY(vqe_energy<T>(b, ncirc, circ0));
@@ -2431,11 +2520,17 @@ int vqe_adjoint(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     using V = typename C2<T>::t;
     constexpr int RBc = std::is_same<T, float>::value ? 4 : 3;
     const int sms = rq::num_sms(b->device);
-    const uint64_t amps = ncirc << b->n;
-    const unsigned hgrid = (unsigned)std::min<uint64_t>((amps + 255) / 256, (uint64_t)sms * 8);
-    k_vqe_apply_h<T><<<hgrid, 256, 0, b->stream>>>((const V*)b->d_states, (V*)b->d_lam, b->n, ncirc, b->d_hterms,
-                                                   b->nhterms);
-    RQ_CUDA(cudaGetLastError());
+    const uint32_t ntile = 1u << (b->pn - b->em);
+    const size_t hsmem = 2 * ((size_t)1 << b->em) * sizeof(V);
+    const unsigned hgrid = (unsigned)std::min<uint64_t>(ncirc * ntile, (uint64_t)sms);
+    RQ_TRY(with_register_bits<T>(b->em, [&](auto rbits) {
+        auto kern = k_vqe_apply_h<T, decltype(rbits)::value>;
+        RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+        kern<<<hgrid, PK_THREADS, hsmem, b->stream>>>((const V*)b->d_states, (V*)b->d_lam, b->pn, b->em, ncirc,
+                                                      b->d_segs, b->d_sofs + ntile + 1, b->d_terms);
+        RQ_CUDA(cudaGetLastError());
+        return (int)RQ_OK;
+    }));
     QArgs<T> a{};
     a.amps = (V*)b->d_states;
     a.lam = (V*)b->d_lam;
@@ -2452,7 +2547,6 @@ int vqe_adjoint(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     const unsigned threads = 1u << (b->am - RBc);
     const unsigned ngroup = threads < 32 ? threads : threads / 32;
     const size_t smem = 2 * ((size_t)1 << b->am) * sizeof(V) + (size_t)ngroup * b->P * sizeof(double);
-    if (smem > 227 * 1024) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "too many parameters for the adjoint kernel");
     RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
@@ -2465,6 +2559,20 @@ int vqe_adjoint(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
                                                                                    b->P, circ0, b->d_grad);
         RQ_CUDA(cudaGetLastError());
     }
+    return RQ_OK;
+}
+
+// The sizes a run takes: an energy pass of two tiles and a row of strings per warp, and an adjoint
+// pass of two tiles and a row of parameters per warp, fit 227 KB (tiles of up to 2^13 / 2^12 of the
+// 2^n amplitudes).  The packed kernels need less; the limits stay where callers know them.
+int vqe_limits(const rq_vqe_batch* b, int32_t with_gradient) {
+    const uint32_t m = std::min(b->n, b->prec == RQ_F32 ? 13u : 12u), arb = b->prec == RQ_F32 ? 4 : 3;
+    const size_t tiles = 2 * ((size_t)1 << m) * elem_size(b->prec);
+    if (tiles + (size_t)16 * b->nterms * sizeof(double) > 227 * 1024)
+        return rq::fail(RQ_ERR_INVALID_ARGUMENT, "Hamiltonian has too many strings for the energy kernel");
+    const unsigned threads = 1u << (m - arb), ngroup = threads < 32 ? threads : threads / 32;
+    if (with_gradient == RQ_VQE_GRAD_ADJOINT && tiles + (size_t)ngroup * b->P * sizeof(double) > 227 * 1024)
+        return rq::fail(RQ_ERR_INVALID_ARGUMENT, "too many parameters for the adjoint kernel");
     return RQ_OK;
 }
 
@@ -2485,16 +2593,16 @@ int vqe_enqueue(rq_vqe_batch* b, uint64_t ncirc, uint32_t V, uint64_t wave, bool
             if (adj) {
                 const int ev = b->prof.begin(b->stream);
                 RQ_TRY(vqe_adjoint<float>(b, wn, w0));
-                b->prof.end(ev, b->stream, 2, (double)wn * (2.0 * (double)((size_t)8 << b->n) +
-                                                            sweep_bytes(b->adescs, (double)((size_t)8 << b->n), 2.0)));
+                b->prof.end(ev, b->stream, 2, (double)wn * (2.0 * (double)((size_t)8 << b->pn) +
+                                                            sweep_bytes(b->adescs, (double)((size_t)8 << b->pn), 2.0)));
             }
         } else {
             RQ_TRY(vqe_wave<double>(b, wn, w0));
             if (adj) {
                 const int ev = b->prof.begin(b->stream);
                 RQ_TRY(vqe_adjoint<double>(b, wn, w0));
-                b->prof.end(ev, b->stream, 2, (double)wn * (2.0 * (double)((size_t)16 << b->n) +
-                                                            sweep_bytes(b->adescs, (double)((size_t)16 << b->n), 2.0)));
+                b->prof.end(ev, b->stream, 2, (double)wn * (2.0 * (double)((size_t)16 << b->pn) +
+                                                            sweep_bytes(b->adescs, (double)((size_t)16 << b->pn), 2.0)));
             }
         }
     }
@@ -2520,12 +2628,16 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
     b->depth = depth;
     b->P = num_qubits * depth;
     cudaGetDevice(&b->device);
-    // Hamiltonian in mask form, grouped by X/Y pattern, chunks of <= 8 terms
-    std::map<uint64_t, std::vector<std::pair<uint64_t, std::pair<uint32_t, double>>>> by_x;   // x -> (pmask, (ny, coeff))
-    std::vector<HTerm> hterms;
+    b->pn = num_qubits - 1;
+    b->nterms = nterms;
+    // tiles of the energy and H passes: two in shared memory, 2^13 f32 / 2^12 f64 elements each
+    b->em = std::min<uint32_t>(b->pn, precision == RQ_F32 ? 13 : 12);
+    const uint32_t M = b->em, ntile = 1u << (b->pn - M), RBITS = M > (uint32_t)PK_TB ? M - PK_TB : 0;
+    // Hamiltonian in mask form, by segment (top part of X, qubit-0 bit of X, walk mode)
+    std::map<std::vector<uint32_t>, std::vector<PTerm>> eseg, hseg;
     for (uint32_t k = 0; k < nterms; ++k) {
         if (offsets[k + 1] < offsets[k]) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing");
-        uint64_t x = 0, pm = 0;
+        uint64_t x = 0, z = 0;
         uint32_t ny = 0;
         for (uint32_t j = offsets[k]; j < offsets[k + 1]; ++j) {
             const uint32_t q = ops[j].qubit;
@@ -2534,93 +2646,90 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
             if (o == RQ_PAULI_I) continue;
             if (q >= num_qubits) return rq::fail(RQ_ERR_INVALID_QUBIT_INDEX, "Pauli factor on qubit " + std::to_string(q));
             if (o == RQ_PAULI_X || o == RQ_PAULI_Y) x ^= 1ull << q;
-            if (o == RQ_PAULI_Y || o == RQ_PAULI_Z) pm ^= 1ull << q;
+            if (o == RQ_PAULI_Y || o == RQ_PAULI_Z) z ^= 1ull << q;
             if (o == RQ_PAULI_Y) ++ny;
         }
-        by_x[x].push_back({pm, {ny & 3u, coeffs[k]}});
-        // the adjoint pass applies the Hermitian part of H; a string whose operator
-        // i^ny X^x Z^pm is anti-Hermitian (a qubit repeated within the string) has no
-        // real expectation and drops out
-        if (((ny + (uint32_t)__builtin_popcountll(x & pm)) & 1u) == 0) {
-            const double cf = coeffs[k];
-            const uint32_t r = ny & 3u;
-            HTerm h{x, pm, r == 0 ? cf : (r == 2 ? -cf : 0.0), r == 1 ? cf : (r == 3 ? -cf : 0.0)};
-            hterms.push_back(h);
+        // an odd number of Y factors (an imaginary operator), or an anti-Hermitian product (a qubit
+        // repeated within the string): no real expectation and no gradient in a real state
+        if ((ny & 1u) || (__builtin_popcountll(x & z) & 1)) {
+            b->e0 += coeffs[k] * 0.0;   // NaN for a non-finite coefficient
+            continue;
         }
+        const double cf = (ny & 2u) ? -coeffs[k] : coeffs[k];
+        const uint32_t x0 = (uint32_t)(x & 1u), X = (uint32_t)(x >> 1), top = X >> M, xl = X & ((1u << M) - 1);
+        PTerm t{};
+        t.xl = xl;
+        t.z = (uint32_t)(z >> 1);
+        t.z0 = (uint32_t)(z & 1u) << 31;
+        t.f = cf;
+        hseg[{top, x0}].push_back(t);
+        uint32_t mode = RBITS;
+        const uint32_t xr = xl >> PK_TB;
+        if (top) mode = RBITS + 1 + ((xl >> (M - 1)) & 1u);
+        else if (RBITS && xr) mode = 31u - (uint32_t)__builtin_clz(xr);
+        // pairs are summed once (x = 0: single amplitudes), or walked from both ends
+        t.f = cf * (x == 0 ? 1.0 : (top || mode < RBITS) ? 2.0 : 1.0);
+        if (x0 && (z & 1u)) t.f = -t.f;   // A's parts are swapped for x0 = 1: the z0 sign sits on the other one
+        eseg[{top, x0, mode}].push_back(t);
     }
-    auto re_ip = [](uint32_t k) { k &= 3u; return k == 0 ? 1.0 : (k == 2 ? -1.0 : 0.0); };
-    // energy tiles: two tiles (own + partner) in shared memory, 2^13 f32 / 2^12 f64 amplitudes each
-    const uint32_t Mt = std::min<uint32_t>(num_qubits, precision == RQ_F32 ? 13 : 12);
-    b->em = Mt;
-    const uint32_t ntile = 1u << (num_qubits - Mt);
-    std::vector<VGroup> groups;
-    std::vector<VTerm> terms;
-    std::vector<uint32_t> gofs(ntile + 1, 0);
-    for (uint32_t t = 0; t < ntile; ++t) {
-        gofs[t] = (uint32_t)groups.size();
-        for (auto& kv : by_x) {
-            const uint64_t x = kv.first;
-            if ((uint32_t)(x >> Mt) != t) continue;
-            const auto& list = kv.second;
-            for (size_t c0 = 0; c0 < list.size(); c0 += 8) {
-                VGroup G{};
-                G.x = x;
-                G.h = x ? 63 - __builtin_clzll(x) : 0;
-                G.t0 = (uint32_t)terms.size();
-                G.nt = (uint32_t)std::min<size_t>(8, list.size() - c0);
-                for (uint32_t k = 0; k < G.nt; ++k) {
-                    const auto& tt = list[c0 + k];
-                    VTerm vt{};
-                    vt.pmask = tt.first;
-                    const uint32_t ny = tt.second.first;
-                    const bool odd = x && (__builtin_popcountll(x & tt.first) & 1);
-                    vt.odd = odd ? 1u : 0u;
-                    const double f = x == 0 ? re_ip(ny) : (odd ? 2.0 * re_ip(ny + 1) : 2.0 * re_ip(ny));
-                    vt.factor = tt.second.second * f;
-                    terms.push_back(vt);
-                }
-                groups.push_back(G);
+    // a state that is not finite gives NaN through the strings left out, too
+    if (nterms) eseg[{0u, 0u, RBITS}].push_back(PTerm{});
+    std::vector<PTerm> terms;
+    std::vector<PSeg> segs;
+    std::vector<uint32_t> sofs(2 * (ntile + 1), 0);
+    auto lay_out = [&](const std::map<std::vector<uint32_t>, std::vector<PTerm>>& by, uint32_t* ofs) {
+        auto it = by.begin();
+        for (uint32_t t = 0; t < ntile; ++t) {
+            ofs[t] = (uint32_t)segs.size();
+            for (; it != by.end() && it->first[0] == t; ++it) {
+                PSeg g{};
+                g.x0 = it->first[1];
+                g.mode = it->first.size() > 2 ? it->first[2] : 0;
+                g.begin = (uint32_t)terms.size();
+                terms.insert(terms.end(), it->second.begin(), it->second.end());
+                g.end = (uint32_t)terms.size();
+                segs.push_back(g);
             }
         }
-    }
-    gofs[ntile] = (uint32_t)groups.size();
-    b->ngroups = (uint32_t)groups.size();
-    b->nterms = (uint32_t)terms.size();
-    if (groups.empty()) groups.push_back(VGroup{});
-    if (terms.empty()) terms.push_back(VTerm{});
-    RQ_CUDA(cudaMalloc((void**)&b->d_gofs, gofs.size() * sizeof(uint32_t)));
-    RQ_CUDA(cudaMemcpy(b->d_gofs, gofs.data(), gofs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    RQ_CUDA(cudaMalloc((void**)&b->d_groups, groups.size() * sizeof(VGroup)));
-    RQ_CUDA(cudaMemcpy(b->d_groups, groups.data(), groups.size() * sizeof(VGroup), cudaMemcpyHostToDevice));
-    RQ_CUDA(cudaMalloc((void**)&b->d_terms, terms.size() * sizeof(VTerm)));
-    RQ_CUDA(cudaMemcpy(b->d_terms, terms.data(), terms.size() * sizeof(VTerm), cudaMemcpyHostToDevice));
+        ofs[ntile] = (uint32_t)segs.size();
+    };
+    lay_out(eseg, sofs.data());
+    lay_out(hseg, sofs.data() + ntile + 1);
+    if (segs.empty()) segs.push_back(PSeg{});
+    if (terms.empty()) terms.push_back(PTerm{});
+    RQ_CUDA(cudaMalloc((void**)&b->d_sofs, sofs.size() * sizeof(uint32_t)));
+    RQ_CUDA(cudaMemcpy(b->d_sofs, sofs.data(), sofs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    RQ_CUDA(cudaMalloc((void**)&b->d_segs, segs.size() * sizeof(PSeg)));
+    RQ_CUDA(cudaMemcpy(b->d_segs, segs.data(), segs.size() * sizeof(PSeg), cudaMemcpyHostToDevice));
+    RQ_CUDA(cudaMalloc((void**)&b->d_terms, terms.size() * sizeof(PTerm)));
+    RQ_CUDA(cudaMemcpy(b->d_terms, terms.data(), terms.size() * sizeof(PTerm), cudaMemcpyHostToDevice));
     // the ansatz program
-    b->m = std::min(num_qubits, precision == RQ_F32 ? 13u : 12u);
-    const uint32_t c = std::min<uint32_t>(b->m, 5);
-    b->ntiles = 1ull << (num_qubits - b->m);
+    const uint32_t mloc = precision == RQ_F32 ? 13u : 12u;
+    b->m = std::min(b->pn, mloc);
+    b->ntiles = 1ull << (b->pn - b->m);
     b->smem = ((size_t)1 << b->m) * elem_size(precision);
+    auto ry_gate = [&](uint32_t l, uint32_t q) {
+        PGate r{};
+        r.type = OP_RYP;
+        r.q0 = q;
+        r.param = (uint16_t)(l * num_qubits + q);
+        return r;
+    };
+    auto cz_gate = [&](uint32_t q) {
+        PGate z{};
+        z.type = OP_CZ;
+        z.q0 = q;
+        z.q1 = q + 1;
+        return z;
+    };
     std::vector<PGate> g;
     for (uint32_t l = 0; l < depth; ++l) {
-        for (uint32_t q = 0; q < num_qubits; ++q) {
-            PGate r{};
-            r.type = OP_RYP;
-            r.q0 = q;
-            r.param = (uint16_t)(l * num_qubits + q);
-            g.push_back(r);
-        }
-        for (uint32_t q = 0; q + 1 < num_qubits; ++q) {
-            PGate z{};
-            z.type = OP_CZ;
-            z.q0 = q;
-            z.q1 = q + 1;
-            g.push_back(z);
-        }
+        for (uint32_t q = 0; q < num_qubits; ++q) g.push_back(ry_gate(l, q));
+        for (uint32_t q = 0; q + 1 < num_qubits; ++q) g.push_back(cz_gate(q));
     }
-    auto sweeps = plan_sweeps(g, num_qubits, b->m, c);
     std::vector<PhaseDesc> phases;
     std::vector<SwOp> opsv;
-    std::vector<double> mats;
-    build_program(sweeps, num_qubits, b->m, c, rb, precision == RQ_F32 ? 2 : 1, b->descs, phases, opsv, mats);
+    packed_program(g, num_qubits, mloc, b->m, rb, precision == RQ_F32 ? 2 : 1, b->descs, phases, opsv);
     if (precision == RQ_F32) retable_f16(b->descs, phases, rb);   // the conflict-free layout (k_batch_sweep<float>)
     b->smem += max_phases(b->descs) * sizeof(PhaseDesc);   // the phase descriptors after the tile
     b->descs.front().flags |= SWEEP_INIT_ZERO;
@@ -2633,36 +2742,17 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
     RQ_CUDA(cudaMemcpy(b->prog, host.data(), total, cudaMemcpyHostToDevice));
     {
         // the adjoint program: per layer in reverse, the CZ ladder, then Ry^-1 on every qubit
-        b->nhterms = (uint32_t)hterms.size();
-        if (hterms.empty()) hterms.push_back(HTerm{});
-        RQ_CUDA(cudaMalloc((void**)&b->d_hterms, hterms.size() * sizeof(HTerm)));
-        RQ_CUDA(cudaMemcpy(b->d_hterms, hterms.data(), hterms.size() * sizeof(HTerm), cudaMemcpyHostToDevice));
         const uint32_t arb = precision == RQ_F32 ? 4 : 3;
-        b->am = std::min(num_qubits, precision == RQ_F32 ? 13u : 12u);
-        b->antiles = 1ull << (num_qubits - b->am);
-        const uint32_t ac = std::min<uint32_t>(b->am, 5);
+        b->am = std::min(b->pn, mloc);
+        b->antiles = 1ull << (b->pn - b->am);
         std::vector<PGate> ga;
         for (uint32_t l = depth; l-- > 0;) {
-            for (uint32_t q = num_qubits - 1; q-- > 0;) {
-                PGate z{};
-                z.type = OP_CZ;
-                z.q0 = q;
-                z.q1 = q + 1;
-                ga.push_back(z);
-            }
-            for (uint32_t q = num_qubits; q-- > 0;) {
-                PGate r{};
-                r.type = OP_RYP;
-                r.q0 = q;
-                r.param = (uint16_t)(l * num_qubits + q);
-                ga.push_back(r);
-            }
+            for (uint32_t q = num_qubits - 1; q-- > 0;) ga.push_back(cz_gate(q));
+            for (uint32_t q = num_qubits; q-- > 0;) ga.push_back(ry_gate(l, q));
         }
-        auto asw = plan_sweeps(ga, num_qubits, b->am, ac);
         std::vector<PhaseDesc> aph;
         std::vector<SwOp> aops;
-        std::vector<double> amats;
-        build_program(asw, num_qubits, b->am, ac, arb, precision == RQ_F32 ? 2 : 1, b->adescs, aph, aops, amats);
+        packed_program(ga, num_qubits, mloc, b->am, arb, precision == RQ_F32 ? 2 : 1, b->adescs, aph, aops);
         b->aoff_ops = (aph.size() * sizeof(PhaseDesc) + 255) & ~size_t(255);
         const size_t atotal = b->aoff_ops + aops.size() * sizeof(SwOp);
         std::vector<unsigned char> ah(atotal);
@@ -2690,6 +2780,7 @@ int rq_vqe_batch_run(rq_vqe_batch* b, uint32_t nsets, const double* params, int3
         return rq::fail(RQ_ERR_INVALID_ARGUMENT, "with_gradient must be RQ_VQE_GRAD_NONE, _SHIFT or _ADJOINT");
     RQ_CUDA(cudaSetDevice(b->device));
     const uint32_t P = b->P;
+    RQ_TRY(vqe_limits(b, with_gradient));
     const bool adj = with_gradient == RQ_VQE_GRAD_ADJOINT;
     const uint32_t V = with_gradient == RQ_VQE_GRAD_SHIFT ? 1 + 2 * P : 1;
     const uint64_t ncirc = (uint64_t)nsets * V;
@@ -2697,7 +2788,7 @@ int rq_vqe_batch_run(rq_vqe_batch* b, uint32_t nsets, const double* params, int3
     RQ_TRY(grow(&b->d_params, &b->params_cap, (size_t)nsets * P));
     RQ_TRY(grow_bytes(&b->d_rot, &b->rot_cap, ncirc * P * 2 * es));
     RQ_TRY(grow(&b->d_energy, &b->energy_cap, ncirc));
-    const size_t state_bytes = ((size_t)1 << b->n) * elem_size(b->prec);
+    const size_t state_bytes = ((size_t)1 << b->pn) * elem_size(b->prec);
     const uint64_t wave = std::max<uint64_t>(1, std::min<uint64_t>(ncirc, b->wave_bytes / state_bytes));
     RQ_TRY(grow_bytes(&b->d_states, &b->states_cap, wave * state_bytes));
     if (adj) {
@@ -2723,6 +2814,8 @@ int rq_vqe_batch_run(rq_vqe_batch* b, uint32_t nsets, const double* params, int3
     RQ_CUDA(cudaStreamSynchronize(b->stream));
     RQ_CUDA(cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1));
     b->graph.collect(b->prof);
+    if (adj && b->e0 != 0.0)   // not finite: so are the gradients
+        for (size_t k = 0; k < (size_t)nsets * P; ++k) gradients[k] += b->e0;
     for (uint32_t s = 0; s < nsets; ++s) {
         energies[s] = e[(uint64_t)s * V];
         if (with_gradient == RQ_VQE_GRAD_SHIFT)
@@ -2769,8 +2862,8 @@ int rq_vqe_batch_destroy(rq_vqe_batch* b) {
     if (!b) return RQ_OK;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    void* ptrs[] = {b->prog,     b->d_groups, b->d_terms, b->d_gofs,  b->d_part, b->d_params, b->d_rot,
-                    b->d_states, b->d_energy, b->aprog,   b->d_hterms, b->d_lam,  b->d_gpart,  b->d_grad};
+    void* ptrs[] = {b->prog,     b->d_segs,   b->d_terms, b->d_sofs, b->d_part,  b->d_params, b->d_rot,
+                    b->d_states, b->d_energy, b->aprog,   b->d_lam,  b->d_gpart, b->d_grad};
     for (void* q : ptrs) if (q) cudaFree(q);
     b->graph.drop();
     b->prof.release();

@@ -27,8 +27,10 @@ namespace rqp {
 // (param = its index there).
 // DENSE: a 32x32 complex unitary on the phase's five register slots, applied
 // on the tensor cores (param = index of its operand image).
+// RY0, CZ0: Ry on, and CZ with, the qubit that a packed real state keeps in the real and
+// imaginary part of each element (q0 = the other qubit of CZ0); they need no register slot.
 enum OpType : uint8_t { OP_U1 = 0, OP_D1 = 1, OP_CX = 2, OP_CZ = 3, OP_ZZ = 4, OP_CPH = 5, OP_RXP = 6, OP_RYP = 7,
-                        OP_DENSE = 8 };
+                        OP_DENSE = 8, OP_RY0 = 9, OP_CZ0 = 10 };
 
 constexpr int RBMAX = 5;
 constexpr int MMAX = 14;

@@ -100,3 +100,42 @@ def test_vqe_runs_replay_one_graph_with_identical_results(gradient):
         else:
             assert np.array_equal(x, y)
     assert flags == [False, True, True]
+
+
+@pytest.mark.parametrize("prec,n", [("f32", 7), ("f32", 10), ("f32", 11), ("f32", 14), ("f32", 15), ("f64", 6),
+                                    ("f64", 12), ("f64", 13), ("f64", 15)])
+def test_vqe_batch_tile_edges(prec, n):
+    """States of one partly filled block, of one tile, of a tile without and with one register
+    bit, and of several tiles; strings whose X pattern is empty, only qubit 0, only inside a warp,
+    on a register bit, and across tiles, each with and without Z on qubit 0, and strings with one
+    and two Y factors.  Tolerances as above."""
+    top = n - 1
+    strings = [[], [(0, 3)], [(0, 1)], [(0, 1), (2, 3)], [(1, 1)], [(1, 1), (0, 3)], [(0, 1), (3, 1)],
+               [(0, 2), (3, 2)], [(0, 2), (4, 1)], [(top, 1)], [(top, 1), (0, 1)], [(top, 2), (0, 2), (1, 3)],
+               [(top - 1, 1), (2, 3)], [(top - 1, 2), (top, 2)], [(top - 2, 1), (top, 3), (0, 1)],
+               [(q, 3) for q in range(n)], [(q, 1) for q in range(n)], [(0, 2), (1, 2), (top, 2)]]
+    coeffs = np.linspace(-1.0, 1.3, len(strings))
+    depth = 2
+    params = np.random.default_rng(n).uniform(-math.pi, math.pi, size=(3, n * depth))
+    vb = VqeBatch(n, depth, coeffs, strings, prec)
+    e, g = vb.run(params, gradient="adjoint")
+    tol = 1e-10 if prec == "f64" else 1e-5 * float(np.sum(np.abs(coeffs)))
+    for s in range(3):
+        assert abs(e[s] - _energy(n, depth, params[s], coeffs, strings)) < tol
+    for k in (0, 1, n - 1, n, 2 * n - 1):
+        pp, pm = params[0].copy(), params[0].copy()
+        pp[k] += math.pi / 2
+        pm[k] -= math.pi / 2
+        want = (_energy(n, depth, pp, coeffs, strings) - _energy(n, depth, pm, coeffs, strings)) / 2
+        assert abs(g[0, k] - want) < tol, (k, g[0, k], want)
+
+
+def test_vqe_batch_non_finite_inputs_stay_non_finite():
+    """NaN or infinite coefficients and angles give NaN energies, also through a string with one
+    Y factor, which adds nothing otherwise."""
+    p = np.full((2, 14), 0.3)
+    e, g = VqeBatch(7, 2, [1.0, np.inf], [[(0, 3)], [(1, 2)]], "f32").run(p, gradient="adjoint")
+    assert np.all(np.isnan(e)) and np.all(np.isnan(g))
+    p[1, 3] = np.nan
+    e = VqeBatch(7, 2, [1.0], [[(1, 2)]], "f32").run(p)
+    assert e[0] == 0.0 and np.isnan(e[1])
