@@ -8,7 +8,6 @@
 #include "rq_internal.cuh"
 
 #include <algorithm>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -19,7 +18,6 @@ using rqd::C2;
 using rqd::insert0;
 
 constexpr int TPB = 256;
-constexpr int KMAX = 8;   // Pauli strings per pass
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -63,150 +61,295 @@ __global__ void k_prob(const typename C2<T>::t* __restrict__ a, uint64_t count, 
     if (threadIdx.x == 0) partials[blockIdx.x] = r;
 }
 
-struct TermChunk {
-    uint64_t pmask[KMAX];
-    int odd[KMAX];
-    int k;
+// ---- Pauli strings ------------------------------------------------------------
+//
+// A string is (x, z): x = XOR of its X/Y qubits, z = XOR of its Y/Z qubits.
+//   x == 0: sum over i of (-1)^|i & z| |a_i|^2
+//   x != 0: sum over the pairs {i, j = i ^ x} of (-1)^|i & z| times Re (|x & z| even) or Im (odd) of
+//           conj(a_j) a_i, which is the same from either end of the pair.
+// Products and sums in FP64 for either state type.  Three kernels:
+//   k_pauli_small  a string per CTA (states of at most SMALL_QUBITS: latency, not bandwidth);
+//   k_pauli_z      up to ZK strings with x == 0 per read of the state;
+//   k_pauli_span   up to SK strings with x != 0 per read of the state.
+
+constexpr uint32_t SMALL_QUBITS = 13;
+constexpr int SMALL_STRINGS = 480;
+struct SmallStrings {
+    uint32_t x[SMALL_STRINGS], z[SMALL_STRINGS];
 };
 
-// Pauli strings sharing one xmask.  x == 0: acc_k += s_k(i)|a_i|^2.
-// x != 0: pairs (i, j = i^x) with the top bit h of x clear in i,
-// z = conj(a_j) a_i, acc_k += s_k(i) * (odd_k ? Im z : Re z).
+// One launch for all strings, each summed by one CTA straight into out[]: the 8-qubit VQE energy's
+// 32 strings took 30 launches of 3.1 us and a reduction.
 template <typename T>
-__global__ void k_pauli(const typename C2<T>::t* __restrict__ a, uint64_t count, uint64_t x, uint32_t h,
-                        TermChunk tc, double* __restrict__ partials, uint32_t slot0, uint32_t stride) {
+__global__ void k_pauli_small(const typename C2<T>::t* __restrict__ a, uint32_t n, const __grid_constant__ SmallStrings ss,
+                              double* __restrict__ out) {
     __shared__ double sh[32];
-    double acc[KMAX];
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) acc[k] = 0.0;
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < count;
-         p += (uint64_t)gridDim.x * blockDim.x) {
-        double re, im;
-        uint64_t i;
+    const uint32_t x = ss.x[blockIdx.x], z = ss.z[blockIdx.x];
+    const bool odd = __popc(x & z) & 1;
+    const uint32_t h = x ? 31 - __clz(x) : 0, count = x ? 1u << (n - 1) : 1u << n;
+    double acc = 0.0;
+#pragma unroll 4
+    for (uint32_t p = threadIdx.x; p < count; p += blockDim.x) {
+        uint32_t i = p;
+        double v;
         if (x == 0) {
-            i = p;
-            re = norm2(a[i]);
-            im = 0.0;
+            v = norm2(a[i]);
         } else {
-            i = insert0(p, h);
-            auto ai = a[i];
-            auto aj = a[i ^ x];
-            double air = ai.x, aii = ai.y, ajr = aj.x, aji = aj.y;
-            re = ajr * air + aji * aii;
-            im = ajr * aii - aji * air;
+            i = (uint32_t)insert0(p, h);
+            const auto ai = a[i], aj = a[i ^ x];
+            const double air = ai.x, aii = ai.y, ajr = aj.x, aji = aj.y;
+            v = odd ? ajr * aii - aji * air : ajr * air + aji * aii;
+        }
+        acc += (__popc(i & z) & 1) ? -v : v;
+    }
+    const double r = block_sum(acc, sh);
+    if (threadIdx.x == 0) out[blockIdx.x] = r;
+}
+
+// Strings with x == 0.  A thread takes 16 amplitudes whose indices differ in four fixed bits (f32: bit
+// 0 and bits 9-11, f64: bits 8-11 of a tile of 2^12), forms the 16 signed sums of their probabilities
+// over those bits (a Walsh-Hadamard transform, 64 additions), and every string adds the one that its
+// mask on those bits selects, with the sign of the other bits: five instructions per string and 16
+// amplitudes.  The sums go through the thread's own column of shared memory, as a register cannot be
+// selected at run time.  Bound by HBM: 30 single-Z strings of 30 qubits f32 in 1.43 ms (a copy-rate read takes
+// 1.31 ms) against 2.65 ms
+// for per-string sums of each warp's 1024 amplitudes.
+constexpr int ZK = 32, ZPASSES = 11, ZT = 256;
+struct ZPass {
+    uint64_t z[ZK];
+    uint16_t col[ZK];   // offset of the selected sum in a thread's column of sums
+    uint32_t k;
+    uint32_t pad;
+};
+struct ZPasses {
+    ZPass p[ZPASSES];
+};
+
+template <typename T> struct Vec16;
+template <> struct Vec16<float> { using t = float4; };
+template <> struct Vec16<double> { using t = double2; };
+
+template <typename T, int KT>
+__global__ void __launch_bounds__(ZT, KT > 16 ? 2 : 3) k_pauli_z(const typename C2<T>::t* __restrict__ a, uint64_t ntiles,
+                                                   const __grid_constant__ ZPasses zp, double* __restrict__ partials,
+                                                   uint32_t stride) {
+    using VV = typename Vec16<T>::t;
+    constexpr bool F = sizeof(T) == 4;
+    __shared__ double W[16 * ZT];
+    const ZPass& P = zp.p[blockIdx.y];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, K = P.k;
+    const uint32_t ebits = F ? tid << 1 : tid;          // this thread's part of the element index
+    uint64_t zl = lane < K ? P.z[lane] : 0ull;          // lane k keeps string k's mask
+    uint32_t tpar = 0;                                  // bit k: parity of ebits & z_k
+    for (uint32_t k = 0; k < K; ++k) tpar |= (uint32_t)(__popc(ebits & (uint32_t)P.z[k]) & 1) << k;
+    double acc[KT];   // strings past K have mask 0 and are not written
+#pragma unroll
+    for (int k = 0; k < KT; ++k) acc[k] = 0.0;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const VV* src = reinterpret_cast<const VV*>(a + (tile << 12));
+        double p[16];
+        if constexpr (F) {   // register bit 0 = element bit 0, register bits 1-3 = element bits 9-11
+            VV v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = __ldcs(src + u * ZT + tid);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                p[2 * u] = (double)v[u].x * v[u].x + (double)v[u].y * v[u].y;
+                p[2 * u + 1] = (double)v[u].z * v[u].z + (double)v[u].w * v[u].w;
+            }
+        } else {             // register bits 0-3 = element bits 8-11
+            VV v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) v[u] = __ldcs(src + u * ZT + tid);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) p[u] = v[u].x * v[u].x + v[u].y * v[u].y;
         }
 #pragma unroll
-        for (int k = 0; k < KMAX; ++k) {
-            if (k < tc.k) {
-                double v = tc.odd[k] ? im : re;
-                acc[k] += (__popcll(i & tc.pmask[k]) & 1) ? -v : v;
+        for (int b = 1; b < 16; b <<= 1)
+#pragma unroll
+            for (int m = 0; m < 16; ++m)
+                if (!(m & b)) {
+                    const double s = p[m], d = p[m | b];
+                    p[m] = s + d;
+                    p[m | b] = s - d;
+                }
+#pragma unroll
+        for (int m = 0; m < 16; ++m) W[m * ZT + tid] = p[m];
+        const uint32_t sg = tpar ^ __ballot_sync(0xffffffffu, __popcll((tile << 12) & zl) & 1);
+#pragma unroll
+        for (int k0 = 0; k0 < KT; k0 += 8) {
+            double w[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = W[P.col[k0 + k] + tid];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int flip = (int)((sg << (31 - k0 - k)) & 0x80000000u);
+                acc[k0 + k] += __hiloint2double(__double2hiint(w[k]) ^ flip, __double2loint(w[k]));
             }
         }
     }
-    for (int k = 0; k < tc.k; ++k) {
-        double r = block_sum(acc[k], sh);
-        if (threadIdx.x == 0) partials[(size_t)(slot0 + k) * stride + blockIdx.x] = r;
+    double* red = W;   // [warp][string]
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        const double r = warp_sum(acc[k]);
+        if (lane == 0) red[(tid >> 5) * ZK + k] = r;
+    }
+    __syncthreads();
+    if (tid < K) {
+        double r = 0.0;
+        for (int w = 0; w < ZT / 32; ++w) r += red[w * ZK + tid];
+        partials[(size_t)(blockIdx.y * ZK + tid) * stride + blockIdx.x] = r;
     }
 }
 
-// Single-qubit Z strings (and the identity) in one pass: <Z_q> = sum_x p(x)(1 - 2 bit_q(x)).
-// Each thread owns chunks of 32 consecutive amplitudes: per chunk it forms the total
-// probability and the five sums over the amplitudes whose low index bit b is set;
-// a string on a low qubit (q < 5) adds total - 2 s_q, one on a high qubit adds
-// +-total by bit q of the chunk's index, the identity adds total.  Up to ZMAX
-// strings per pass; FP64 accumulation, fixed-order block and grid reductions.
-constexpr int ZMAX = 32;
-struct ZChunk {
-    uint8_t q[ZMAX];   // qubit of the string, 64 = identity
-    int k;
+// Strings with x != 0.  A pass owns eight independent X patterns (of the bits above the contiguous
+// low ones): a tile is a coset of their span, 2^8 runs of 256 bytes, so for every string whose x lies
+// in the span both ends of each pair are in the tile, and one read of the state serves them all
+// (at least eight strings of a Hamiltonian of unrelated patterns; the X fields of an Ising model).
+// The basis is in reduced echelon form: index = rep ^ sum_k u_k basis_k with rep zero at the pivot bits,
+// so a string's local X mask is its pivot bits, and its local sign mask the parities of basis_k & z.
+// A thread keeps 16 / 8 elements in registers as doubles and reads the partners from shared memory; a
+// pair is walked once, by a register bit of the local X mask held at 0 (all elements where it has none:
+// the sum is then halved by the caller).  Sums per string and thread live in shared memory across the
+// CTA's tiles.  Bound by the FP64 conversions (XU 60 %, issue 47 %): 64 random strings of 24 qubits
+// f32 in 0.59 ms against 2.8 ms for a read of the state
+// per string.
+constexpr int SK = 16, SPASSES = 10, ST = 512, STB = 9;
+struct SpanString {
+    uint64_t z;
+    uint16_t lx, lz;     // X and sign masks on the tile's local bits
+    uint8_t mode, odd;   // mode: register bit held at 0, or the number of register bits: walk all
+    uint16_t pad;
 };
+struct SpanPass {
+    uint64_t basis[8];   // bits above the run
+    uint8_t free_bit[24];   // the other bits above the run, low to high: the tile number's bits
+    uint32_t k, row0;       // its strings, and the row of the first
+    SpanString s[SK];
+};
+struct SpanPasses {
+    SpanPass p[SPASSES];
+};
+template <typename T> struct SpanShape;
+template <> struct SpanShape<float> { static constexpr int C = 5, RB = 4; };    // 2^13 elements of 8 bytes
+template <> struct SpanShape<double> { static constexpr int C = 4, RB = 3; };   // 2^12 elements of 16 bytes
 
-template <typename T> struct ZVec;
-template <> struct ZVec<float> { using t = float4; static constexpr int EPV = 2; };
-template <> struct ZVec<double> { using t = double2; static constexpr int EPV = 1; };
-
-// Warp-cooperative: warp w of the grid owns segments of 1024 consecutive amplitudes;
-// in each, lane l loads the 16-byte vectors it*32 + l (coalesced), so the low index bits
-// of every element it sees are fixed by (lane, position in the vector) and the next bits
-// by the unrolled `it`: the lane keeps its total, the sum with index bit 0 set (f32) and
-// the sums by the bits of `it`; a string's value per segment follows from those
-// (bits 0..9) or from the segment index (bits >= 10).
-template <typename T>
-__global__ void __launch_bounds__(256, 2) k_zsingle(const typename C2<T>::t* __restrict__ a, uint64_t nseg,
-                                                    ZChunk zc, double* __restrict__ partials, uint32_t slot0,
-                                                    uint32_t stride) {
-    using VV = typename ZVec<T>::t;
-    constexpr int EPV = ZVec<T>::EPV;
-    constexpr int NIT = 1024 / (32 * EPV);    // vectors per lane per segment: 16 (f32) or 32 (f64)
-    constexpr int LB = EPV == 2 ? 1 : 0;      // element bits below the lane bits
-    constexpr int ITB = EPV == 2 ? 4 : 5;     // bits of `it`
-    __shared__ double sh[32];
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    double acc[ZMAX];
+template <typename T, int RB, int BIT, bool ODD>
+__device__ __forceinline__ double span_walk(const double* ar, const double* ai, const typename C2<T>::t* tile,
+                                            uint32_t tid, const SpanString& s) {
+    constexpr int NB = BIT >= 0 ? RB - 1 : RB, NW = 1 << NB, B0 = BIT < 0 ? 0 : BIT;
+    const uint32_t P = tid ^ s.lx;
+    double v[NW];
 #pragma unroll
-    for (int k = 0; k < ZMAX; ++k) acc[k] = 0.0;
-    for (uint64_t sg = warp; sg < nseg; sg += nwarps) {
-        const VV* src = reinterpret_cast<const VV*>(a + sg * 1024);
-        double tot = 0.0, odd = 0.0, r[ITB];
-#pragma unroll
-        for (int k = 0; k < ITB; ++k) r[k] = 0.0;
-#pragma unroll
-        for (int h = 0; h < NIT; h += 8) {
-            VV v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = __ldcs(src + (h + u) * 32 + lane);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int it = h + u;
-                double pit;
-                if constexpr (EPV == 2) {
-                    const double p0 = (double)v[u].x * v[u].x + (double)v[u].y * v[u].y;
-                    const double p1 = (double)v[u].z * v[u].z + (double)v[u].w * v[u].w;
-                    odd += p1;
-                    pit = p0 + p1;
-                } else {
-                    pit = (double)v[u].x * v[u].x + (double)v[u].y * v[u].y;
-                }
-                tot += pit;
-#pragma unroll
-                for (int k = 0; k < ITB; ++k)
-                    if ((it >> k) & 1) r[k] += pit;
-            }
-        }
-        // element index bits inside the segment: [0, LB) vector slot, [LB, LB + 5) lane, then `it`
-#pragma unroll
-        for (int k = 0; k < ZMAX; ++k) {
-            if (k < zc.k) {
-                const uint32_t q = zc.q[k];
-                double v;
-                if (q >= 64) {
-                    v = tot;
-                } else if (q < (uint32_t)LB) {
-                    v = tot - 2.0 * odd;
-                } else if (q < (uint32_t)LB + 5) {
-                    v = ((lane >> (q - LB)) & 1u) ? -tot : tot;
-                } else if (q < 10) {
-                    const uint32_t kb = q - LB - 5;
-                    double s = r[0];
-#pragma unroll
-                    for (int t = 1; t < ITB; ++t)
-                        if (kb == (uint32_t)t) s = r[t];
-                    v = tot - 2.0 * s;
-                } else {
-                    v = ((sg >> (q - 10)) & 1ull) ? -tot : tot;
-                }
-                acc[k] += v;
-            }
-        }
+    for (int w = 0; w < NW; ++w) {
+        const int i = BIT < 0 ? w : ((w >> B0) << (B0 + 1)) | (w & ((1 << B0) - 1));
+        const auto b = tile[P ^ ((uint32_t)i << STB)];
+        const double br = b.x, bi = b.y;
+        v[w] = ODD ? br * ai[i] - bi * ar[i] : br * ar[i] + bi * ai[i];
     }
 #pragma unroll
-    for (int k = 0; k < ZMAX; ++k) {
-        if (k < zc.k) {
-            double rr = block_sum(acc[k], sh);
-            if (threadIdx.x == 0) partials[(size_t)(slot0 + k) * stride + blockIdx.x] = rr;
+    for (int b = 0; b < NB; ++b) {
+        const int gb = BIT >= 0 && b >= BIT ? b + 1 : b;
+        const double sg = ((s.lz >> (STB + gb)) & 1u) ? -1.0 : 1.0;
+#pragma unroll
+        for (int w = 0; w < NW; w += 2 << b) v[w] = fma(sg, v[w + (1 << b)], v[w]);
+    }
+    return v[0];
+}
+
+template <typename T, int RB, bool ODD>
+__device__ __forceinline__ double span_string(const double* ar, const double* ai, const typename C2<T>::t* tile,
+                                              uint32_t tid, const SpanString& s) {
+    switch (s.mode) {
+        case 0: return span_walk<T, RB, 0, ODD>(ar, ai, tile, tid, s);
+        case 1: return span_walk<T, RB, 1, ODD>(ar, ai, tile, tid, s);
+        case 2: return span_walk<T, RB, 2, ODD>(ar, ai, tile, tid, s);
+        case 3: if constexpr (RB > 3) return span_walk<T, RB, 3, ODD>(ar, ai, tile, tid, s); break;
+        default: break;
+    }
+    return span_walk<T, RB, -1, ODD>(ar, ai, tile, tid, s);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(ST, 1) k_pauli_span(const typename C2<T>::t* __restrict__ a, uint32_t tile_bits,
+                                                      const __grid_constant__ SpanPasses sp,
+                                                      double* __restrict__ partials, uint32_t stride) {
+    using V = typename C2<T>::t;
+    constexpr int C = SpanShape<T>::C, RB = SpanShape<T>::RB, NR = 1 << RB;
+    constexpr uint32_t L = 1u << (C + 8), EPV = 16 / sizeof(V);   // elements of a tile, per 16 bytes
+    extern __shared__ __align__(16) unsigned char smem[];
+    V* buf = reinterpret_cast<V*>(smem);                           // two tiles
+    double* sums = reinterpret_cast<double*>(smem + 2 * L * sizeof(V));   // [string][thread]
+    const SpanPass& P = sp.p[blockIdx.y];
+    const uint32_t tid = threadIdx.x;
+    for (uint32_t k = 0; k < P.k; ++k) sums[k * ST + tid] = 0.0;
+    // this thread's 16-byte piece of a run: runs u = (tid >> 4) + 32 j, the piece tid & 15
+    const uint32_t piece = (tid & 15u) * EPV;
+    uint64_t ut = 0;
+#pragma unroll
+    for (int b = 0; b < 5; ++b)
+        if ((tid >> (4 + b)) & 1u) ut ^= P.basis[b];
+    const uint64_t ntiles = 1ull << tile_bits;
+    auto rep_of = [&](uint64_t t) {
+        uint64_t r = 0;
+        for (uint32_t b = 0; b < tile_bits; ++b) r |= ((t >> b) & 1ull) << P.free_bit[b];
+        return r;
+    };
+    auto load = [&](uint64_t rep, V* dst) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            uint64_t g = rep ^ ut;
+            if (j & 1) g ^= P.basis[5];
+            if (j & 2) g ^= P.basis[6];
+            if (j & 4) g ^= P.basis[7];
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + (((tid >> 4) + 32 * j) << C) + piece);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(a + g + piece) : "memory");
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint64_t tile = blockIdx.x;
+    uint64_t rep = rep_of(tile);
+    uint32_t at = 0;
+    if (tile < ntiles) load(rep, buf);
+    while (tile < ntiles) {
+        const uint64_t next = tile + gridDim.x;
+        uint64_t nrep = 0;
+        if (next < ntiles) {
+            nrep = rep_of(next);
+            load(nrep, buf + (at ^ 1u) * L);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const V* tl = buf + at * L;
+        double ar[NR], ai[NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const V v = tl[tid | ((uint32_t)i << STB)];
+            ar[i] = v.x;
+            ai[i] = v.y;
+        }
+        for (uint32_t k = 0; k < P.k; ++k) {
+            const SpanString& s = P.s[k];
+            const double v = s.odd ? span_string<T, RB, true>(ar, ai, tl, tid, s) : span_string<T, RB, false>(ar, ai, tl, tid, s);
+            const bool neg = (__popcll(rep & s.z) + __popc(tid & s.lz)) & 1;
+            sums[k * ST + tid] += neg ? -v : v;
+        }
+        __syncthreads();
+        tile = next;
+        rep = nrep;
+        at ^= 1u;
+    }
+    // the CTA's sum of each string: a warp per string, fixed order
+    __syncthreads();
+    const uint32_t lane = tid & 31u;
+    for (uint32_t k = tid >> 5; k < P.k; k += ST / 32) {
+        double r = 0.0;
+        for (uint32_t t = lane; t < ST; t += 32) r += sums[k * ST + t];
+        r = warp_sum(r);
+        if (lane == 0) partials[(size_t)(P.row0 + k) * stride + blockIdx.x] = r;
     }
 }
 
@@ -230,11 +373,13 @@ __global__ void k_inner(const typename C2<TA>::t* __restrict__ a, const typename
     if (threadIdx.x == 0) partials[stride + blockIdx.x] = r;
 }
 
-// out[k] = sum_b partials[k*stride + b], fixed order
-__global__ void k_finalize(const double* __restrict__ partials, uint32_t nblocks, uint32_t stride,
+// out[k] = sum_b partials[k*stride + b] over the first na blocks for k < ka, nb for the others, in a
+// fixed order.  out may be pinned host memory.
+__global__ void k_finalize(const double* __restrict__ partials, uint32_t ka, uint32_t na, uint32_t nb, uint32_t stride,
                            double* __restrict__ out) {
     __shared__ double sh[32];
     const double* p = partials + (size_t)blockIdx.x * stride;
+    const uint32_t nblocks = blockIdx.x < ka ? na : nb;
     double acc = 0.0;
     for (uint32_t b = threadIdx.x; b < nblocks; b += blockDim.x) acc += p[b];
     double r = block_sum(acc, sh);
@@ -254,13 +399,11 @@ __global__ void k_probs(const typename C2<T>::t* __restrict__ a, uint64_t n, dou
 
 int reduction_grid(rq_state* s) { return rq::num_sms(s->device) * 4; }
 
-// finalize `nout` partial rows and copy them to host
+// finalize `nout` partial rows into the pinned staging, read by the host after one synchronisation
 int finish(rq_state* s, unsigned nblocks, unsigned stride, unsigned nout, double* host) {
-    double* dout = s->partials + (size_t)nout * stride;
-    k_finalize<<<nout, TPB, 0, s->stream>>>(s->partials, nblocks, stride, dout);
-    RQ_CUDA(cudaGetLastError());
     RQ_TRY(rq::ensure_hbuf(s, nout));
-    RQ_CUDA(cudaMemcpyAsync(s->hbuf, dout, nout * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    k_finalize<<<nout, TPB, 0, s->stream>>>(s->partials, nout, nblocks, nblocks, stride, s->hbuf);
+    RQ_CUDA(cudaGetLastError());
     RQ_TRY(rq::sync_checked(s));
     for (unsigned k = 0; k < nout; ++k) host[k] = s->hbuf[k];
     return RQ_OK;
@@ -272,6 +415,164 @@ inline double re_ipow(uint32_t k) {
         case 2: return -1.0;
         default: return 0.0;
     }
+}
+
+// Which kernel sums which string, into which row of the partials.
+struct PauliPlan {
+    bool small = false;
+    std::vector<uint32_t> zs;             // strings of k_pauli_z in row order
+    std::vector<SpanPass> spans;
+    uint32_t rows = 0;                    // one per string
+    uint32_t zblocks = 0, sblocks = 0, stride = 0;
+    std::vector<uint32_t> row_of;         // string -> row
+    std::vector<double> factor;           // string -> factor of its sum
+    const rq::PauliMask* terms = nullptr;
+};
+
+void plan_strings(uint32_t n, int32_t prec, int sms, const rq::PauliMask* terms, uint32_t nterms, PauliPlan& P) {
+    P.terms = terms;
+    P.rows = nterms;
+    P.row_of.assign(nterms, 0);
+    P.factor.resize(nterms);
+    for (uint32_t k = 0; k < nterms; ++k) {
+        const rq::PauliMask& t = terms[k];
+        const bool odd = __builtin_popcountll(t.xmask & t.pmask) & 1;
+        P.factor[k] = t.xmask == 0 ? re_ipow(t.ny) : 2.0 * re_ipow(odd ? t.ny + 1 : t.ny);
+    }
+    if (n <= SMALL_QUBITS) {
+        P.small = true;
+        for (uint32_t k = 0; k < nterms; ++k) P.row_of[k] = k;
+        return;
+    }
+    std::vector<uint32_t> left;
+    for (uint32_t k = 0; k < nterms; ++k) {
+        if (terms[k].xmask == 0) {
+            P.row_of[k] = (uint32_t)P.zs.size();
+            P.zs.push_back(k);
+        } else {
+            left.push_back(k);
+        }
+    }
+    uint32_t row = (uint32_t)P.zs.size();
+    const uint32_t C = prec == RQ_F32 ? 5 : 4, RB = prec == RQ_F32 ? 4 : 3;
+    const uint64_t low = (1ull << C) - 1;
+    while (!left.empty()) {
+        SpanPass sp{};
+        sp.row0 = row;
+        uint64_t pivot[8];
+        uint32_t dim = 0;
+        auto reduced = [&](uint64_t x) {
+            for (uint32_t b = 0; b < dim; ++b)
+                if (x & pivot[b]) x ^= sp.basis[b];
+            return x;
+        };
+        auto add = [&](uint64_t v) {   // v reduced and not zero: clear its pivot from the others
+            const uint64_t pv = 1ull << (63 - __builtin_clzll(v));
+            for (uint32_t b = 0; b < dim; ++b)
+                if (sp.basis[b] & pv) sp.basis[b] ^= v;
+            pivot[dim] = pv;
+            sp.basis[dim++] = v;
+        };
+        std::vector<uint32_t> take, rest;
+        for (uint32_t k : left) {
+            const uint64_t r = take.size() < (size_t)SK ? reduced(terms[k].xmask & ~low) : ~0ull;
+            if (take.size() == (size_t)SK || (r && dim == 8)) {
+                rest.push_back(k);
+                continue;
+            }
+            if (r) add(r);
+            take.push_back(k);
+        }
+        for (uint32_t q = C; dim < 8; ++q)
+            if (const uint64_t r = reduced(1ull << q)) add(r);
+        uint64_t pivots = 0;
+        for (uint32_t b = 0; b < 8; ++b) pivots |= pivot[b];
+        uint32_t nf = 0;
+        for (uint32_t q = C; q < n; ++q)
+            if (!((pivots >> q) & 1)) sp.free_bit[nf++] = (uint8_t)q;
+        for (uint32_t k : take) {
+            const rq::PauliMask& t = terms[k];
+            SpanString& ss = sp.s[sp.k];
+            uint32_t lx = (uint32_t)(t.xmask & low), lz = (uint32_t)(t.pmask & low);
+            for (uint32_t b = 0; b < 8; ++b) {
+                if (t.xmask & pivot[b]) lx |= 1u << (C + b);
+                if (__builtin_popcountll(sp.basis[b] & t.pmask) & 1) lz |= 1u << (C + b);
+            }
+            ss.z = t.pmask;
+            ss.lx = (uint16_t)lx;
+            ss.lz = (uint16_t)lz;
+            ss.odd = (uint8_t)(__builtin_popcountll(t.xmask & t.pmask) & 1);
+            const uint32_t xr = lx >> STB;
+            ss.mode = (uint8_t)(xr ? 31 - __builtin_clz(xr) : RB);
+            if (!xr) P.factor[k] *= 0.5;   // walked from both ends
+            P.row_of[k] = row++;
+            ++sp.k;
+        }
+        P.spans.push_back(sp);
+        left.swap(rest);
+    }
+    P.zblocks = P.zs.empty() ? 0 : (uint32_t)std::min<uint64_t>(1ull << (n - 12), (uint64_t)sms * 2);
+    P.sblocks = P.spans.empty() ? 0 : (uint32_t)std::min<uint64_t>(1ull << (n - C - 8), (uint64_t)sms);
+    P.stride = std::max(P.zblocks, P.sblocks);
+}
+
+template <typename T>
+int launch_strings_t(const PauliPlan& P, const void* amps, uint32_t n, cudaStream_t st, double* partials, double* out) {
+    using V = typename C2<T>::t;
+    const V* a = (const V*)amps;
+    if (P.small) {
+        for (uint32_t k0 = 0; k0 < P.rows; k0 += SMALL_STRINGS) {
+            SmallStrings ss{};
+            const uint32_t k1 = std::min<uint32_t>(P.rows, k0 + SMALL_STRINGS);
+            for (uint32_t k = k0; k < k1; ++k) {
+                ss.x[k - k0] = (uint32_t)P.terms[k].xmask;
+                ss.z[k - k0] = (uint32_t)P.terms[k].pmask;
+            }
+            k_pauli_small<T><<<k1 - k0, TPB, 0, st>>>(a, n, ss, out + k0);
+            RQ_CUDA(cudaGetLastError());
+        }
+        return RQ_OK;
+    }
+    const uint32_t nz = (uint32_t)P.zs.size(), zpasses = (nz + ZK - 1) / ZK;
+    for (uint32_t p0 = 0; p0 < zpasses; p0 += ZPASSES) {
+        ZPasses zp{};
+        const uint32_t np = std::min<uint32_t>(ZPASSES, zpasses - p0);
+        for (uint32_t p = 0; p < np; ++p) {
+            const uint32_t k0 = (p0 + p) * ZK;
+            zp.p[p].k = std::min<uint32_t>(ZK, nz - k0);
+            for (uint32_t k = 0; k < zp.p[p].k; ++k) {
+                const uint64_t z = P.terms[P.zs[k0 + k]].pmask;
+                zp.p[p].z[k] = z;
+                zp.p[p].col[k] = (uint16_t)(ZT * (sizeof(T) == 4 ? (z & 1u) | ((z >> 8) & 14u) : (z >> 8) & 15u));
+            }
+        }
+        double* part = partials + (size_t)p0 * ZK * P.stride;
+        auto kern = nz <= 8 ? k_pauli_z<T, 8> : nz <= 16 ? k_pauli_z<T, 16> : k_pauli_z<T, ZK>;
+        kern<<<dim3(P.zblocks, np), ZT, 0, st>>>(a, 1ull << (n - 12), zp, part, P.stride);
+        RQ_CUDA(cudaGetLastError());
+    }
+    constexpr int smem = 2 * (1 << (SpanShape<T>::C + 8)) * (int)sizeof(V) + SK * ST * (int)sizeof(double);
+    if (!P.spans.empty())
+        RQ_CUDA(cudaFuncSetAttribute(k_pauli_span<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    for (size_t p0 = 0; p0 < P.spans.size(); p0 += SPASSES) {
+        SpanPasses sp{};
+        const size_t np = std::min<size_t>(SPASSES, P.spans.size() - p0);
+        for (size_t p = 0; p < np; ++p) sp.p[p] = P.spans[p0 + p];
+        k_pauli_span<T><<<dim3(P.sblocks, (unsigned)np), ST, smem, st>>>(a, n - SpanShape<T>::C - 8, sp, partials,
+                                                                       P.stride);
+        RQ_CUDA(cudaGetLastError());
+    }
+    k_finalize<<<P.rows, TPB, 0, st>>>(partials, nz, P.zblocks, P.sblocks, P.stride, out);
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
+// the sums of every string on `st`: out[row] (device or pinned host memory), partials of
+// P.rows * P.stride doubles
+int launch_strings(const PauliPlan& P, const void* amps, uint32_t n, int32_t prec, cudaStream_t st, double* partials,
+                   double* out) {
+    return prec == RQ_F32 ? launch_strings_t<float>(P, amps, n, st, partials, out)
+                          : launch_strings_t<double>(P, amps, n, st, partials, out);
 }
 
 }  // namespace
@@ -295,78 +596,13 @@ int norm_sq(rq_state* s, double* out) { return prob_bit(s, 64, 0, out); }
 
 int pauli_expect(rq_state* s, const PauliMask* terms, uint32_t nterms, double* out) {
     if (nterms == 0) return RQ_OK;
-    unsigned G = reduction_grid(s);
-    RQ_TRY(ensure_partials(s, (size_t)nterms * G + nterms + 8));
-    std::vector<uint32_t> slot_of(nterms);
-    uint32_t slot = 0;
-    // single-qubit Z strings and identities: one pass for up to ZMAX of them
-    std::vector<uint32_t> zs;
-    if (s->nq >= 10)
-        for (uint32_t k = 0; k < nterms; ++k)
-            if (terms[k].xmask == 0 && __builtin_popcountll(terms[k].pmask) <= 1) zs.push_back(k);
-    for (size_t c0 = 0; c0 < zs.size(); c0 += ZMAX) {
-        ZChunk zc{};
-        zc.k = (int)std::min<size_t>(ZMAX, zs.size() - c0);
-        for (int k = 0; k < zc.k; ++k) {
-            const uint64_t pm = terms[zs[c0 + k]].pmask;
-            zc.q[k] = (uint8_t)(pm ? __builtin_ctzll(pm) : 64);
-            slot_of[zs[c0 + k]] = slot + k;
-        }
-        const uint64_t nseg = s->n >> 10;     // segments of 1024 amplitudes, one warp each
-        const unsigned Gz = std::min<unsigned>(G, grid_for(nseg * 32, TPB, num_sms(s->device), 4));
-        if (s->prec == RQ_F32)
-            k_zsingle<float><<<Gz, TPB, 0, s->stream>>>((const float2*)s->amps, nseg, zc, s->partials, slot, G);
-        else
-            k_zsingle<double><<<Gz, TPB, 0, s->stream>>>((const double2*)s->amps, nseg, zc, s->partials, slot, G);
-        RQ_CUDA(cudaGetLastError());
-        // blocks past Gz contribute nothing to these rows
-        if (Gz < G)
-            for (int k = 0; k < zc.k; ++k)
-                RQ_CUDA(cudaMemsetAsync(s->partials + (size_t)(slot + k) * G + Gz, 0, (G - Gz) * sizeof(double),
-                                        s->stream));
-        slot += zc.k;
-    }
-    std::vector<char> done(nterms, 0);
-    for (uint32_t k : zs) done[k] = 1;
-    // the other strings: group by xmask (stable), chunks of KMAX
-    std::map<uint64_t, std::vector<uint32_t>> groups;
-    for (uint32_t k = 0; k < nterms; ++k)
-        if (!done[k]) groups[terms[k].xmask].push_back(k);
-    for (auto& kv : groups) {
-        uint64_t x = kv.first;
-        uint32_t h = x ? 63 - __builtin_clzll(x) : 0;
-        uint64_t count = x ? s->n >> 1 : s->n;
-        const auto& idx = kv.second;
-        for (size_t c0 = 0; c0 < idx.size(); c0 += KMAX) {
-            TermChunk tc{};
-            tc.k = (int)std::min<size_t>(KMAX, idx.size() - c0);
-            for (int k = 0; k < tc.k; ++k) {
-                const PauliMask& t = terms[idx[c0 + k]];
-                tc.pmask[k] = t.pmask;
-                tc.odd[k] = x ? (__builtin_popcountll(x & t.pmask) & 1) : 0;
-                slot_of[idx[c0 + k]] = slot + k;
-            }
-            if (s->prec == RQ_F32)
-                k_pauli<float><<<G, TPB, 0, s->stream>>>((const float2*)s->amps, count, x, h, tc, s->partials, slot, G);
-            else
-                k_pauli<double><<<G, TPB, 0, s->stream>>>((const double2*)s->amps, count, x, h, tc, s->partials, slot, G);
-            RQ_CUDA(cudaGetLastError());
-            slot += tc.k;
-        }
-    }
-    std::vector<double> sums(nterms);
-    RQ_TRY(finish(s, G, G, nterms, sums.data()));
-    for (uint32_t k = 0; k < nterms; ++k) {
-        const PauliMask& t = terms[k];
-        double acc = sums[slot_of[k]];
-        if (t.xmask == 0) {
-            out[k] = acc * re_ipow(t.ny);
-        } else if (!(__builtin_popcountll(t.xmask & t.pmask) & 1)) {
-            out[k] = 2.0 * acc * re_ipow(t.ny);
-        } else {
-            out[k] = 2.0 * acc * re_ipow(t.ny + 1);
-        }
-    }
+    PauliPlan plan;
+    plan_strings(s->nq, s->prec, num_sms(s->device), terms, nterms, plan);
+    RQ_TRY(ensure_partials(s, (size_t)plan.rows * plan.stride));
+    RQ_TRY(ensure_hbuf(s, plan.rows));
+    RQ_TRY(launch_strings(plan, s->amps, s->nq, s->prec, s->stream, s->partials, s->hbuf));
+    RQ_TRY(sync_checked(s));
+    for (uint32_t k = 0; k < nterms; ++k) out[k] = s->hbuf[plan.row_of[k]] * plan.factor[k];
     return RQ_OK;
 }
 
@@ -488,47 +724,20 @@ extern "C" int rq_expectation_batch_noalloc(const void* device_amps, uint32_t nu
     double* scratch = nullptr;
     RQ_TRY(noalloc_scratch_address(device, &scratch));
     cudaStream_t st = static_cast<cudaStream_t>(stream_handle);
-    const uint64_t n = 1ull << num_qubits;
-    unsigned G = (unsigned)std::min<int>(rq::num_sms(device) * 4, (int)RQ_NOALLOC_MAX_BLOCKS);
-    // partials occupy [0, nstrings*G); the finalised sums follow at nstrings*G
-    std::map<uint64_t, std::vector<uint32_t>> groups;
-    for (uint32_t k = 0; k < nstrings; ++k) groups[terms[k].xmask].push_back(k);
-    std::vector<uint32_t> slot_of(nstrings);
-    uint32_t slot = 0;
-    for (auto& kv : groups) {
-        uint64_t x = kv.first;
-        uint32_t h = x ? 63 - __builtin_clzll(x) : 0;
-        uint64_t count = x ? n >> 1 : n;
-        const auto& idx = kv.second;
-        for (size_t c0 = 0; c0 < idx.size(); c0 += KMAX) {
-            TermChunk tc{};
-            tc.k = (int)std::min<size_t>(KMAX, idx.size() - c0);
-            for (int k = 0; k < tc.k; ++k) {
-                const rq::PauliMask& t = terms[idx[c0 + k]];
-                tc.pmask[k] = t.pmask;
-                tc.odd[k] = x ? (__builtin_popcountll(x & t.pmask) & 1) : 0;
-                slot_of[idx[c0 + k]] = slot + k;
-            }
-            if (precision == RQ_F32)
-                k_pauli<float><<<G, TPB, 0, st>>>((const float2*)device_amps, count, x, h, tc, scratch, slot, G);
-            else
-                k_pauli<double><<<G, TPB, 0, st>>>((const double2*)device_amps, count, x, h, tc, scratch, slot, G);
-            RQ_CUDA(cudaGetLastError());
-            slot += tc.k;
-        }
+    // partials occupy [0, nstrings * stride), at most RQ_NOALLOC_MAX_STRINGS * RQ_NOALLOC_MAX_BLOCKS;
+    // the finalised sums follow
+    PauliPlan plan;
+    plan_strings(num_qubits, precision, rq::num_sms(device), terms.data(), nstrings, plan);
+    if (plan.stride > RQ_NOALLOC_MAX_BLOCKS) {   // fewer CTAs take more tiles each
+        plan.zblocks = std::min<uint32_t>(plan.zblocks, RQ_NOALLOC_MAX_BLOCKS);
+        plan.sblocks = std::min<uint32_t>(plan.sblocks, RQ_NOALLOC_MAX_BLOCKS);
+        plan.stride = RQ_NOALLOC_MAX_BLOCKS;
     }
-    double* sums = scratch + (size_t)nstrings * G;
-    k_finalize<<<nstrings, TPB, 0, st>>>(scratch, G, G, sums);
-    RQ_CUDA(cudaGetLastError());
+    double* sums = scratch + (size_t)nstrings * plan.stride;
+    RQ_TRY(launch_strings(plan, device_amps, num_qubits, precision, st, scratch, sums));
     std::vector<double> host(nstrings);
     RQ_CUDA(cudaMemcpyAsync(host.data(), sums, nstrings * sizeof(double), cudaMemcpyDeviceToHost, st));
     RQ_CUDA(cudaStreamSynchronize(st));
-    for (uint32_t k = 0; k < nstrings; ++k) {
-        const rq::PauliMask& t = terms[k];
-        double acc = host[slot_of[k]];
-        if (t.xmask == 0) out[k] = acc * re_ipow(t.ny);
-        else if (!(__builtin_popcountll(t.xmask & t.pmask) & 1)) out[k] = 2.0 * acc * re_ipow(t.ny);
-        else out[k] = 2.0 * acc * re_ipow(t.ny + 1);
-    }
+    for (uint32_t k = 0; k < nstrings; ++k) out[k] = host[plan.row_of[k]] * plan.factor[k];
     return RQ_OK;
 }
