@@ -738,6 +738,42 @@ int rq_debug_set_wait_limit(uint32_t polls) {
 
 namespace {
 
+// one unitary gate of a validated list for the small-circuit kernel
+rq::SmallCircuitOp small_op(const rq_gate& g) {
+    rq::SmallCircuitOp o{};
+    o.q0 = g.q0;
+    o.q1 = g.q1;
+    switch (g.kind) {
+        case RQ_GATE_CNOT: o.kind = rq::SmallCircuitOp::CNOT; return o;
+        case RQ_GATE_CZ: o.kind = rq::SmallCircuitOp::CZ; return o;
+        case RQ_GATE_SWAP: o.kind = rq::SmallCircuitOp::SWAP; return o;
+        case RQ_GATE_RZZ: {
+            const double h = g.angle / 2.0;
+            o.kind = rq::SmallCircuitOp::ZZ;
+            o.m[0] = std::cos(-h);
+            o.m[1] = std::sin(-h);
+            o.m[2] = std::cos(h);
+            o.m[3] = std::sin(h);
+            return o;
+        }
+        default: break;
+    }
+    double m[8] = {0};
+    matrix_1q(g, m);
+    o.q1 = 0;
+    if (is_diag_1q(g.kind)) {
+        o.kind = rq::SmallCircuitOp::D1;
+        o.m[0] = m[0];
+        o.m[1] = m[1];
+        o.m[2] = m[6];
+        o.m[3] = m[7];
+    } else {
+        o.kind = rq::SmallCircuitOp::U1;
+        std::memcpy(o.m, m, sizeof(m));
+    }
+    return o;
+}
+
 // The gate loop of run_with_config (simulator.rs:67-78) over a validated list:
 // measurements and resets in order, every maximal run of unitary gates through the
 // sweep path (or per-gate kernels).  With mdraw, the k-th measurement / reset of the
@@ -777,6 +813,12 @@ int run_gate_list(rq_state* s, const rq_gate* gates, uint64_t n, int32_t mode, r
             uint32_t m = 0;
             if (mode == RQ_EXEC_AUTO) RQ_TRY(rq::autotune_tc(s, run.data(), run.size(), &passes, &m));
             RQ_TRY(rq::apply_sweeps(s, run.data(), run.size(), passes, m));
+        } else if (mode == RQ_EXEC_AUTO && s->nq <= rq::SMALL_CIRCUIT_QUBITS) {
+            std::vector<rq::SmallCircuitOp> ops;
+            ops.reserve(e - k);
+            for (uint64_t j = k; j < e; ++j)
+                if (gates[j].kind != RQ_GATE_BARRIER) ops.push_back(small_op(gates[j]));
+            RQ_TRY(rq::apply_small(s, ops));
         } else {
             for (uint64_t j = k; j < e; ++j)
                 if (gates[j].kind != RQ_GATE_BARRIER) RQ_TRY(rq::apply_one_gate(s, gates[j]));

@@ -8,6 +8,9 @@
 // touching only the amplitudes they change.
 #include "rq_internal.cuh"
 
+#include <algorithm>
+#include <vector>
+
 namespace {
 
 using rqd::C2;
@@ -20,12 +23,26 @@ struct CM4 { T v[32]; };   // 4x4 complex
 template <typename T>
 struct CD4 { T v[8]; };    // 4 complex diagonal entries
 
+__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fmar(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fmar(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// d * x with the roundings spelled out: the per-gate and the small-circuit kernels agree bit for bit
+template <typename V, typename T>
+__device__ __forceinline__ V cmulr(T dr, T di, V x) {
+    V r;
+    r.x = fmar(dr, x.x, -mulr(di, x.y));
+    r.y = fmar(di, x.x, mulr(dr, x.y));
+    return r;
+}
+
 template <typename V, typename T>
 __device__ __forceinline__ V cmac2(T ar, T ai, V x, T br, T bi, V y) {
     // (a*x + b*y) with a=(ar,ai), b=(br,bi)
-    V r;
-    r.x = ar * x.x - ai * x.y + br * y.x - bi * y.y;
-    r.y = ar * x.y + ai * x.x + br * y.y + bi * y.x;
+    V r = cmulr<V, T>(ar, ai, x);
+    r.x = fmar(-bi, y.y, fmar(br, y.x, r.x));
+    r.y = fmar(bi, y.x, fmar(br, y.y, r.y));
     return r;
 }
 
@@ -63,11 +80,7 @@ __global__ void k_diag1q(typename C2<T>::t* __restrict__ a, uint64_t count, uint
         uint64_t i = half_only ? (insert0(p, q) | (1ull << q)) : p;
         int b = (int)((i >> q) & 1);
         T dr = d.v[2 * b], di = d.v[2 * b + 1];
-        V x = a[i];
-        V r;
-        r.x = dr * x.x - di * x.y;
-        r.y = dr * x.y + di * x.x;
-        a[i] = r;
+        a[i] = cmulr<V, T>(dr, di, a[i]);
     }
 }
 
@@ -102,11 +115,7 @@ __global__ void k_diag2q(typename C2<T>::t* __restrict__ a, uint64_t n, uint32_t
          i += (uint64_t)gridDim.x * blockDim.x) {
         int k = (int)(((i >> q1) & 1) * 2 + ((i >> q2) & 1));
         T dr = d.v[2 * k], di = d.v[2 * k + 1];
-        V x = a[i];
-        V r;
-        r.x = dr * x.x - di * x.y;
-        r.y = dr * x.y + di * x.x;
-        a[i] = r;
+        a[i] = cmulr<V, T>(dr, di, a[i]);
     }
 }
 
@@ -256,6 +265,98 @@ __global__ void k_basis(typename C2<T>::t* __restrict__ a, uint64_t n, uint64_t 
     }
 }
 
+// A run of gates on a state of at most 2^SMALL_CIRCUIT_QUBITS amplitudes: one CTA keeps the state in
+// shared memory, the gates and their matrices come as kernel parameters (no table to upload), one
+// barrier per gate.  Every amplitude sees the arithmetic of the per-gate kernels above.  What bounds
+// such a circuit is latency: 69 gates on 8 qubits took 69 launches, 110 us on the device and 160 us of
+// launch calls, and take one launch of 17 us.
+enum SmallOp : uint8_t { SM_U1, SM_D1, SM_D1_HALF, SM_CNOT, SM_CZ, SM_SWAP, SM_ZZ };
+struct SmallGate {
+    uint8_t op, q0, q1, pad;
+    uint32_t m;                  // first matrix entry
+};
+template <int G, int M>
+struct SmallRun {
+    uint32_t n, count;
+    SmallGate g[G];
+    double m[M];
+};
+using SmallRun4K = SmallRun<96, 400>;      // 4 KB of parameters
+using SmallRun16K = SmallRun<384, 1600>;   // 16 KB
+
+template <typename T, typename R>
+__global__ void __launch_bounds__(512) k_small_circuit(typename C2<T>::t* __restrict__ a,
+                                                       const __grid_constant__ R run) {
+    using V = typename C2<T>::t;
+    __shared__ V st[1 << rq::SMALL_CIRCUIT_QUBITS];
+    const uint32_t N = 1u << run.n, tid = threadIdx.x, nt = blockDim.x;
+    for (uint32_t i = tid; i < N; i += nt) st[i] = a[i];
+    __syncthreads();
+    for (uint32_t k = 0; k < run.count; ++k) {
+        const SmallGate g = run.g[k];
+        const double* m = run.m + g.m;
+        const uint32_t lo = g.q0 < g.q1 ? g.q0 : g.q1, hi = g.q0 < g.q1 ? g.q1 : g.q0;
+        switch (g.op) {
+            case SM_U1: {
+                T c[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) c[j] = (T)m[j];
+                for (uint32_t p = tid; p < N >> 1; p += nt) {
+                    const uint32_t i0 = (uint32_t)insert0(p, g.q0), i1 = i0 | (1u << g.q0);
+                    const V x = st[i0], y = st[i1];
+                    st[i0] = cmac2<V, T>(c[0], c[1], x, c[2], c[3], y);
+                    st[i1] = cmac2<V, T>(c[4], c[5], x, c[6], c[7], y);
+                }
+                break;
+            }
+            case SM_D1:
+            case SM_D1_HALF: {
+                const bool half = g.op == SM_D1_HALF;
+                const T d0r = (T)m[0], d0i = (T)m[1], d1r = (T)m[2], d1i = (T)m[3];
+                for (uint32_t p = tid; p < (half ? N >> 1 : N); p += nt) {
+                    const uint32_t i = half ? (uint32_t)insert0(p, g.q0) | (1u << g.q0) : p;
+                    const bool b = (i >> g.q0) & 1u;
+                    const T dr = b ? d1r : d0r, di = b ? d1i : d0i;
+                    st[i] = cmulr<V, T>(dr, di, st[i]);
+                }
+                break;
+            }
+            case SM_ZZ: {
+                const T er = (T)m[0], ei = (T)m[1], pr = (T)m[2], pi = (T)m[3];
+                for (uint32_t i = tid; i < N; i += nt) {
+                    const bool diff = ((i >> g.q0) ^ (i >> g.q1)) & 1u;
+                    const T dr = diff ? pr : er, di = diff ? pi : ei;
+                    st[i] = cmulr<V, T>(dr, di, st[i]);
+                }
+                break;
+            }
+            case SM_CZ:
+                for (uint32_t p = tid; p < N >> 2; p += nt) {
+                    const uint32_t i = (uint32_t)insert0(insert0(p, lo), hi) | (1u << g.q0) | (1u << g.q1);
+                    const V x = st[i];
+                    V r;
+                    r.x = -x.x;
+                    r.y = -x.y;
+                    st[i] = r;
+                }
+                break;
+            default: {   // CNOT: swap the target pair where the control is 1; SWAP: swap 01 and 10
+                for (uint32_t p = tid; p < N >> 2; p += nt) {
+                    const uint32_t b = (uint32_t)insert0(insert0(p, lo), hi);
+                    const uint32_t i = g.op == SM_CNOT ? b | (1u << g.q0) : b | (1u << g.q1);
+                    const uint32_t j = g.op == SM_CNOT ? i | (1u << g.q1) : b | (1u << g.q0);
+                    const V x = st[i], y = st[j];
+                    st[i] = y;
+                    st[j] = x;
+                }
+                break;
+            }
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = tid; i < N; i += nt) a[i] = st[i];
+}
+
 template <typename T>
 CM2<T> cm2(const double* m8) {
     CM2<T> r;
@@ -349,6 +450,54 @@ int gate_cz(rq_state* s, uint32_t q1, uint32_t q2) {
     uint64_t ng = s->n >> 2;
     if (s->prec == RQ_F32) RQ_LAUNCH(k_cz<float>, ng, (float2*)s->amps, ng, q1, q2);
     else RQ_LAUNCH(k_cz<double>, ng, (double2*)s->amps, ng, q1, q2);
+    return RQ_OK;
+}
+
+namespace {
+
+// as many of the gates [k, n) as one launch's parameters hold
+template <typename R>
+int launch_small(rq_state* s, const std::vector<SmallCircuitOp>& ops, size_t* k) {
+    constexpr size_t G = sizeof(R::g) / sizeof(SmallGate), M = sizeof(R::m) / sizeof(double);
+    R r{};
+    r.n = s->nq;
+    size_t nm = 0;
+    for (; *k < ops.size() && r.count < G; ++*k) {
+        const SmallCircuitOp& o = ops[*k];
+        const size_t cnt = o.kind == SmallCircuitOp::U1 ? 8 : o.kind == SmallCircuitOp::D1 || o.kind == SmallCircuitOp::ZZ ? 4 : 0;
+        if (nm + cnt > M) break;
+        SmallGate& g = r.g[r.count++];
+        switch (o.kind) {
+            case SmallCircuitOp::U1: g.op = SM_U1; break;
+            case SmallCircuitOp::D1: g.op = o.m[0] == 1.0 && o.m[1] == 0.0 ? SM_D1_HALF : SM_D1; break;
+            case SmallCircuitOp::CNOT: g.op = SM_CNOT; break;
+            case SmallCircuitOp::CZ: g.op = SM_CZ; break;
+            case SmallCircuitOp::SWAP: g.op = SM_SWAP; break;
+            case SmallCircuitOp::ZZ: g.op = SM_ZZ; break;
+        }
+        g.q0 = (uint8_t)o.q0;
+        g.q1 = (uint8_t)o.q1;
+        g.m = (uint32_t)nm;
+        for (size_t j = 0; j < cnt; ++j) r.m[nm++] = o.m[j];
+    }
+    const unsigned threads = std::min<unsigned>(512, std::max<unsigned>(32, (unsigned)(s->n >> 1)));
+    if (s->prec == RQ_F32) k_small_circuit<float, R><<<1, threads, 0, s->stream>>>((float2*)s->amps, r);
+    else k_small_circuit<double, R><<<1, threads, 0, s->stream>>>((double2*)s->amps, r);
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
+}  // namespace
+
+int apply_small(rq_state* s, const std::vector<SmallCircuitOp>& ops) {
+    size_t k = 0;
+    while (k < ops.size()) {
+        size_t m = 0;
+        for (size_t j = k; j < ops.size(); ++j)
+            m += ops[j].kind == SmallCircuitOp::U1 ? 8 : ops[j].kind == SmallCircuitOp::D1 || ops[j].kind == SmallCircuitOp::ZZ ? 4 : 0;
+        if (ops.size() - k <= 96 && m <= 400) RQ_TRY(launch_small<SmallRun4K>(s, ops, &k));
+        else RQ_TRY(launch_small<SmallRun16K>(s, ops, &k));
+    }
     return RQ_OK;
 }
 

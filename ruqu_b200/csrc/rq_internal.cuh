@@ -90,6 +90,15 @@ int gate2q_diag(rq_state* s, uint32_t q1, uint32_t q2, const double* d8);
 int gate_cnot(rq_state* s, uint32_t c, uint32_t t);
 int gate_swap(rq_state* s, uint32_t q1, uint32_t q2);
 int gate_cz(rq_state* s, uint32_t q1, uint32_t q2);
+// A run of gates on a state of at most SMALL_CIRCUIT_QUBITS qubits as one kernel (or one per 384
+// gates): the execution RQ_EXEC_AUTO picks below the sweeps' 12 qubits.
+constexpr uint32_t SMALL_CIRCUIT_QUBITS = 11;
+struct SmallCircuitOp {
+    enum Kind { U1, D1, CNOT, CZ, SWAP, ZZ } kind;   // q0 = control of CNOT
+    uint32_t q0, q1;
+    double m[8];                                      // U1: 2x2; D1: d0, d1; ZZ: equal, different bits
+};
+int apply_small(rq_state* s, const std::vector<SmallCircuitOp>& ops);
 int scale_all(rq_state* s, double f);
 int negate_except(rq_state* s, uint64_t keep);
 int half_copy(rq_state* s, uint32_t q, uint32_t v, void* device_buf, int unpack);
