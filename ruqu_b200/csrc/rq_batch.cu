@@ -10,6 +10,9 @@
 //  * circuits with the same qubit count form a class and share one planned
 //    program (rq_plan.cuh); a launch covers (circuit, tile) pairs of a class;
 //  * H^n|0> is synthesised by the first sweep (uniform amplitude 2^(-n/2));
+//  * flipping every bit leaves a cut, the start and the mixer unchanged, so
+//    psi(x) = psi(~x) throughout and only the 2^(n-1) amplitudes with qubit
+//    n-1 = 0 are kept (symmetric_program): half the memory and half the work;
 //  * the product of all Rzz of a layer is one diagonal phase
 //    exp(-i*gamma*(|E| - 2 cut(x))) (unit weights): each thread derives
 //    cut(x) for its 2^RB register amplitudes from the graph's neighbour masks
@@ -120,19 +123,6 @@ __device__ __forceinline__ int cut_nb(const CutNb<RB>& cp, int i) {   // i: a co
         for (int t = s + 1; t < RB; ++t)
             if (((i >> s) & 1) && ((i >> t) & 1)) c -= 2 * (int)((cp.adj >> (s * RB + t)) & 1u);
     return c;
-}
-
-// v * i^k (exact: a swap and sign changes)
-template <typename V>
-__device__ __forceinline__ V mul_ipow(V v, int k) {
-    V r;
-    switch (k & 3) {
-        case 0: r = v; break;
-        case 1: r.x = -v.y; r.y = v.x; break;
-        case 2: r.x = -v.x; r.y = -v.y; break;
-        default: r.x = v.y; r.y = -v.x; break;
-    }
-    return r;
 }
 
 template <typename V, typename T>
@@ -308,7 +298,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
             // all of the tile's copies in flight at once (cp.async, element-granular for the swizzle)
 #pragma unroll
             for (int j = 0; j < VPT; ++j) {
-                const V* g = amps + (base | dep_tid | d.gj[j]);
+                const V* g = amps + ((base ^ d.gj[j]) | dep_tid);
                 const uint32_t se = stid ^ d.sgj[j];
                 if constexpr (EPV == 2) {
                     bcp_async8(sm + se, g);
@@ -332,6 +322,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
                     ebase |= 1u << ph.tbit_local[b];
                     U |= 1ull << ph.tbit_global[b];
                 }
+            if (U >> SELECTOR) U = (U ^ d.selmask) & ~(1ull << SELECTOR);
             const uint32_t sb = F16L ? swz16(ebase) : swzb<T>(ebase);
             // register i sits at sb ^ (XOR of S[k] over the set bits k of i): visited in
             // Gray-code order, each address is one XOR from the previous one
@@ -343,11 +334,6 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
                 if (d.flags & SWEEP_INIT_UNIFORM) {
 #pragma unroll
                     for (int i = 0; i < NR; ++i) { reg[i].x = a.amp0; reg[i].y = (T)0; }
-                    if (d.flags & SWEEP_PHASE_IN) {   // S^n H^n |0>: amplitude i^popc(x)
-                        const int pu = __popcll(U);
-#pragma unroll
-                        for (int i = 0; i < NR; ++i) reg[i] = mul_ipow(reg[i], pu + __popc(i));
-                    }
                 } else {   // |0...0>
 #pragma unroll
                     for (int i = 0; i < NR; ++i) { reg[i].x = (i == 0 && U == 0) ? (T)1 : (T)0; reg[i].y = (T)0; }
@@ -396,11 +382,6 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
                     }
                 }
             }
-            if ((d.flags & SWEEP_PHASE_OUT) && p + 1 == d.phase_end) {   // S^dag on every qubit
-                const int pu = __popcll(U);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) reg[i] = mul_ipow(reg[i], -(pu + __popc(i)));
-            }
             if ((d.flags & SWEEP_ENERGY) && p + 1 == d.phase_end) {
                 CutNb<RB> cp;
                 cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
@@ -408,7 +389,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
 #pragma unroll
                 for (int i = 0; i < NR; ++i)
                     e += (reg[i].x * reg[i].x + reg[i].y * reg[i].y) * (T)cut_nb<RB>(cp, i);
-                energy += (double)e;
+                energy += 2.0 * (double)e;   // the other half of the state mirrors this one
             }
             {
                 uint32_t ad = sb;
@@ -436,7 +417,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
 #pragma unroll
         for (int j = 0; j < VPT; ++j) {
             const uint32_t se = stid ^ d.sgj[j];
-            const uint64_t g = base | dep_tid | d.gj[j];
+            const uint64_t g = (base ^ d.gj[j]) | dep_tid;
             VV v;
             if constexpr (EPV == 2) {
                 float2 x = sm[se], y = sm[se ^ 1u];
@@ -595,7 +576,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
             VV v[4], u[4];
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
-                const uint64_t g = base | dep_tid | d.gj[j0 + jj];
+                const uint64_t g = (base ^ d.gj[j0 + jj]) | dep_tid;
                 v[jj] = __ldcs(reinterpret_cast<const VV*>(psi + g));
                 if (!initl) u[jj] = __ldcs(reinterpret_cast<const VV*>(lam + g));
             }
@@ -626,6 +607,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                     ebase |= 1u << ph.tbit_local[b];
                     U |= 1ull << ph.tbit_global[b];
                 }
+            if (U >> SELECTOR) U = (U ^ d.selmask) & ~(1ull << SELECTOR);
             const uint32_t sb = swzb<T>(ebase);
             // register i sits at sb ^ (XOR of S[k] over the set bits k of i): Gray-code order
             uint32_t S[RB];
@@ -661,7 +643,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                 const SwOp op = ops[o];
                 if (op.type == OP_RXP) {
                     const T* r = a.rot + ((size_t)gcirc * a.nparam + op.param) * 2;
-                    flush(2.0 * dispatch_im_x<NR>(op.k0, rp, rl), a.p + op.param);
+                    flush(4.0 * dispatch_im_x<NR>(op.k0, rp, rl), a.p + op.param);   // both halves
                     dispatch_rx<NR>(op.k0, rp, r[0], -r[1]);
                     dispatch_rx<NR>(op.k0, rl, r[0], -r[1]);
                 } else if (op.type == OP_CPH) {
@@ -677,7 +659,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                         rp[i] = cmulv(rp[i], tab[2 * c], -tab[2 * c + 1]);
                         rl[i] = cmulv(rl[i], tab[2 * c], -tab[2 * c + 1]);
                     }
-                    flush(2.0 * (double)acc, op.param);
+                    flush(4.0 * (double)acc, op.param);
                 } else if (op.type == OP_RYP) {
                     // Ry(theta) = exp(-i theta Y / 2): dE/dtheta = Im <lambda|Y|psi>
                     const T* r = a.rot + ((size_t)gcirc * a.nparam + op.param) * 2;
@@ -736,7 +718,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
 #pragma unroll
         for (int j = 0; j < VPT; ++j) {
             const uint32_t se = stid ^ d.sgj[j];
-            const uint64_t g = base | dep_tid | d.gj[j];
+            const uint64_t g = (base ^ d.gj[j]) | dep_tid;
             VV v, u;
             if constexpr (EPV == 2) {
                 float2 x = smp[se], y = smp[se ^ 1u];
@@ -804,7 +786,9 @@ __device__ __forceinline__ double pr(const typename C2<T>::t* a, uint64_t i) {
     return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
 }
 
-// level n-1 of every circuit's tree (tree of circuit c at tree + c * 2^n)
+// Prefix trees over the kept half of each state (n = its index bits, one less than the qubits; tree of
+// circuit c at tree + c * 2^n): level L holds 2^L sums over the indices with the same low L bits.
+// Level n-1 comes from the amplitudes:
 template <typename T>
 __global__ void k_bleaf(const typename C2<T>::t* __restrict__ amps, uint32_t n, uint64_t ncirc, double* __restrict__ tree) {
     const uint64_t half = 1ull << (n - 1), per = 1ull << n;
@@ -827,7 +811,8 @@ __global__ void k_bfold(double* __restrict__ tree, uint32_t n, uint64_t ncirc, u
     }
 }
 
-// one block per circuit: shots, cut of each, best (max cut, lowest shot)
+// one block per circuit: shots, cut of each, best (max cut, lowest shot).  A shot measures the n + 1
+// qubits in order; p(x) = p(~x), so the mass of a prefix j of L bits is level L at j plus level L at ~j.
 template <typename T>
 __global__ void k_bsample(const typename C2<T>::t* __restrict__ amps, const double* __restrict__ tree, uint32_t n,
                           uint64_t ncirc, uint64_t circ0, const uint32_t* __restrict__ circ_inst,
@@ -851,15 +836,19 @@ __global__ void k_bsample(const typename C2<T>::t* __restrict__ amps, const doub
         for (uint32_t s = threadIdx.x; s < shots; s += blockDim.x) {
             const uint64_t key = base_seed + (user_of[gc] << 32) + s;
             uint64_t prefix = 0;
-            for (uint32_t q = 0; q < n; ++q) {
+            for (uint32_t q = 0; q <= n; ++q) {
                 double m0, m1;
-                if (q + 1 == n) {
+                const uint64_t mask = (1ull << (q + 1)) - 1, one = prefix | (1ull << q);
+                if (q == n) {
                     m0 = pr<T>(a, prefix);
-                    m1 = pr<T>(a, prefix | (1ull << q));
+                    m1 = pr<T>(a, one ^ mask);
+                } else if (q + 1 == n) {
+                    m0 = __dadd_rn(pr<T>(a, prefix), pr<T>(a, prefix ^ mask));
+                    m1 = __dadd_rn(pr<T>(a, one), pr<T>(a, one ^ mask));
                 } else {
-                    const double* L = t + ((1ull << (q + 1)) - 1);
-                    m0 = L[prefix];
-                    m1 = L[prefix | (1ull << q)];
+                    const double* L = t + mask;
+                    m0 = __dadd_rn(L[prefix], L[prefix ^ mask]);
+                    m1 = __dadd_rn(L[one], L[one ^ mask]);
                 }
                 const double p0 = m0 / __dadd_rn(m0, m1);
                 const double u = rqd::uniform(key, 0, q);
@@ -1532,7 +1521,7 @@ template <typename T>
 int sample_class(rq_qaoa_batch* b, QClass& K, uint64_t ncirc, uint64_t circ0, void* states, uint32_t shots,
                  uint64_t seed) {
     using V = typename C2<T>::t;
-    const uint32_t n = K.n;
+    const uint32_t n = K.n - 1;   // index bits of the kept half
     const uint64_t per = 1ull << n;
     // trees for as many circuits as the tree scratch allows
     const size_t tree_budget = (size_t)8 << 30;
@@ -1610,13 +1599,10 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
         QClass K;
         K.n = kv.first;
         K.insts = kv.second;
-        K.m = std::min(K.n, mloc);
-        K.c = std::min<uint32_t>(K.m, 5);
-        K.ntiles = 1ull << (K.n - K.m);
+        K.m = std::min(K.n - 1, mloc);
+        K.ntiles = 1ull << (K.n - 1 - K.m);
         K.smem = ((size_t)1 << K.m) * elem_size(precision);
-        // the circuit of qaoa.rs:125-153 after H^n: per layer the cost phase, then Rx on every
-        // qubit, run as Ry between the phases S^n H^n |0> and a final S^dag n (SWEEP_PHASE_IN /
-        // _OUT): a real rotation costs half the arithmetic of Rx
+        // the circuit of qaoa.rs:125-153 after H^n: per layer the cost phase, then Rx on every qubit
         std::vector<PGate> g;
         for (uint32_t l = 0; l < p; ++l) {
             PGate ph{};
@@ -1628,21 +1614,19 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
             g.push_back(ph);
             for (uint32_t q = 0; q < K.n; ++q) {
                 PGate rx{};
-                rx.type = OP_RYP;
+                rx.type = OP_RXP;
                 rx.q0 = q;
                 rx.param = (uint16_t)l;
                 g.push_back(rx);
             }
         }
-        auto sweeps = plan_sweeps(g, K.n, K.m, K.c);
         std::vector<PhaseDesc> phases;
         std::vector<SwOp> ops;
-        std::vector<double> mats;
-        build_program(sweeps, K.n, K.m, K.c, rb, precision == RQ_F32 ? 2 : 1, K.descs, phases, ops, mats);
+        symmetric_program(g, K.n, K.m, rb, precision == RQ_F32 ? 2 : 1, K.descs, phases, ops);
         if (precision == RQ_F32) retable_f16(K.descs, phases, rb);   // the conflict-free layout (k_batch_sweep<float>)
         K.smem += max_phases(K.descs) * sizeof(PhaseDesc);   // the phase descriptors after the tile
-        K.descs.front().flags |= SWEEP_INIT_UNIFORM | SWEEP_PHASE_IN;
-        K.descs.back().flags |= SWEEP_ENERGY | SWEEP_PHASE_OUT;
+        K.descs.front().flags |= SWEEP_INIT_UNIFORM;
+        K.descs.back().flags |= SWEEP_ENERGY;
         K.off_ops = (phases.size() * sizeof(PhaseDesc) + 255) & ~size_t(255);
         size_t total = K.off_ops + ops.size() * sizeof(SwOp);
         std::vector<unsigned char> host(total);
@@ -1653,9 +1637,8 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
         {
             // adjoint: per layer in reverse, Rx^-1 on every qubit, then the inverse cost phase
             const uint32_t arb = precision == RQ_F32 ? 4 : 3;
-            K.am = std::min(K.n, mloc);
-            K.antiles = 1ull << (K.n - K.am);
-            const uint32_t ac = std::min<uint32_t>(K.am, 5);
+            K.am = std::min(K.n - 1, mloc);
+            K.antiles = 1ull << (K.n - 1 - K.am);
             std::vector<PGate> ga;
             for (uint32_t l = p; l-- > 0;) {
                 for (uint32_t q = 0; q < K.n; ++q) {
@@ -1671,11 +1654,9 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
                 ph.span = (K.n >= 64) ? ~0ull : ((1ull << K.n) - 1);
                 ga.push_back(ph);
             }
-            auto asw = plan_sweeps(ga, K.n, K.am, ac);
             std::vector<PhaseDesc> aph;
             std::vector<SwOp> aops;
-            std::vector<double> amats;
-            build_program(asw, K.n, K.am, ac, arb, precision == RQ_F32 ? 2 : 1, K.adescs, aph, aops, amats);
+            symmetric_program(ga, K.n, K.am, arb, precision == RQ_F32 ? 2 : 1, K.adescs, aph, aops);
             K.adescs.front().flags |= SWEEP_INIT_LAMBDA;
             K.aoff_ops = (aph.size() * sizeof(PhaseDesc) + 255) & ~size_t(255);
             const size_t atotal = K.aoff_ops + aops.size() * sizeof(SwOp);
@@ -1764,7 +1745,7 @@ int qaoa_prepare(rq_qaoa_batch* b, uint32_t nsets, const double* gammas, const d
     RQ_TRY(grow(&b->d_circ_inst, &cap_ci, ncirc));
     size_t cap_u = b->circ_cap;
     RQ_TRY(grow(&b->d_user, &cap_u, ncirc));
-    size_t cap_a = b->circ_cap;
+    size_t cap_a = b->circ_cap * 2 * p;
     RQ_TRY(grow(&b->d_ang, &cap_a, 2 * ncirc * p));
     size_t es = b->prec == RQ_F32 ? sizeof(float) : sizeof(double);
     size_t cap_rx = b->circ_cap ? b->circ_cap * p * 2 * es : 0;
@@ -1825,8 +1806,9 @@ int qaoa_launch(rq_qaoa_batch* b, uint32_t nsets, uint32_t shots, uint64_t base_
         auto& K = b->classes[ki];
         const uint64_t kc = (per_class ? (*per_class)[ki] : (uint64_t)K.insts.size()) * nsets;
         if (kc == 0) continue;
-        const size_t state_bytes = ((size_t)1 << K.n) * elem_size(b->prec);
-        const size_t per_circ = adjoint ? 2 * state_bytes : state_bytes;
+        // waves are counted in whole states, as callers who set a budget count them
+        const size_t state_bytes = ((size_t)1 << (K.n - 1)) * elem_size(b->prec);
+        const size_t per_circ = (adjoint ? 2 : 1) * 2 * state_bytes;
         const uint64_t wave = std::max<uint64_t>(1, std::min<uint64_t>(kc, b->state_budget / per_circ));
         RQ_TRY(grow_bytes(&b->d_states, &b->states_cap, wave * state_bytes));
         RQ_TRY(grow(&b->d_epart, &b->epart_cap, wave * K.ntiles));
@@ -1845,9 +1827,9 @@ int qaoa_launch(rq_qaoa_batch* b, uint32_t nsets, uint32_t shots, uint64_t base_
                 ev = b->prof.begin(b->stream);
                 if (b->prec == RQ_F32) RQ_TRY(sample_class<float>(b, K, wn, pos + w0, b->d_states, shots, base_seed));
                 else RQ_TRY(sample_class<double>(b, K, wn, pos + w0, b->d_states, shots, base_seed));
-                // the tree's leaf level reads the state and writes 2^n doubles; the folds read and
+                // the tree's leaf level reads the kept half and writes half as many doubles; the folds read and
                 // write the levels above once more (the walks touch n entries per shot)
-                b->prof.end(ev, b->stream, 1, (double)wn * (sb + 2.0 * (double)((size_t)1 << K.n) * 8.0));
+                b->prof.end(ev, b->stream, 1, (double)wn * (sb + 2.0 * (double)((size_t)1 << (K.n - 1)) * 8.0));
             }
             if (adjoint) {
                 ev = b->prof.begin(b->stream);
@@ -2281,7 +2263,7 @@ int rq_qaoa_batch_state(rq_qaoa_batch* b, uint64_t circuit, double* interleaved)
     if (pos == UINT64_MAX || pos < b->last_wave_first || pos >= b->last_wave_first + b->last_wave_count)
         return rq::fail(RQ_ERR_INVALID_ARGUMENT, "circuit " + std::to_string(circuit) +
                                                      " is not held on the device (only the last wave of the last run is)");
-    const uint64_t per = 1ull << b->last_wave_n;
+    const uint64_t per = 1ull << (b->last_wave_n - 1);   // kept amplitudes
     const size_t es = elem_size(b->prec);
     const unsigned char* src = (const unsigned char*)b->d_states + (pos - b->last_wave_first) * per * es;
     if (b->prec == RQ_F64) {
@@ -2290,6 +2272,10 @@ int rq_qaoa_batch_state(rq_qaoa_batch* b, uint64_t circuit, double* interleaved)
         std::vector<float> tmp(2 * per);
         RQ_CUDA(cudaMemcpy(tmp.data(), src, per * es, cudaMemcpyDeviceToHost));
         for (uint64_t i = 0; i < 2 * per; ++i) interleaved[i] = tmp[i];
+    }
+    for (uint64_t i = 0; i < per; ++i) {   // psi(~x) = psi(x)
+        interleaved[2 * (2 * per - 1 - i)] = interleaved[2 * i];
+        interleaved[2 * (2 * per - 1 - i) + 1] = interleaved[2 * i + 1];
     }
     return RQ_OK;
 }
@@ -2387,58 +2373,6 @@ struct rq_vqe_batch {
 };
 
 namespace {
-
-// The sweeps of a list of Ry and CZ gates on n qubits for the packed real state of n - 1 (qubit
-// q > 0 is its qubit q - 1, qubit 0 its two parts).  The gates are planned as sweeps over the
-// 2^n amplitudes (mloc local qubits) and run in exactly that order, so every amplitude goes
-// through the same roundings as unpacked: planning the packed gates afresh saves a sweep in four
-// on 16 qubits (5.5 instead of 5.8 ms for 2056 circuits) but its other order of the rotations moves
-// single f32 energies by their whole rounding error.  The order is cut into sweeps of m local packed
-// qubits and phases of rb slots; qubit 0 needs neither.
-void packed_program(const std::vector<PGate>& gates, uint32_t n, uint32_t mloc, uint32_t m, uint32_t rb, uint32_t epv,
-                    std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
-    const uint32_t m0 = std::min(n, mloc), c = std::min<uint32_t>(m, 5);
-    std::vector<PGate> order;
-    for (const auto& sw : plan_sweeps(gates, n, m0, std::min<uint32_t>(m0, 5)))
-        for (const auto& pp : plan_phases(sw, rb))
-            for (int k : pp.ops) {
-                PGate g = sw.ops[k];
-                if (g.type == OP_RYP && g.q0 == 0) {
-                    g.type = OP_RY0;
-                } else if (g.type == OP_CZ && g.q0 == 0) {
-                    g.type = OP_CZ0;
-                    g.q0 = g.q1 - 1;
-                } else {
-                    g.q0 -= 1;
-                    if (g.type == OP_CZ) g.q1 -= 1;
-                }
-                order.push_back(g);
-            }
-    const uint64_t base = (1ull << c) - 1;
-    std::vector<Sweep> sweeps;
-    std::vector<std::vector<PhasePlan>> pplans;
-    for (const auto& g : order) {
-        const uint64_t nd = needs(g);
-        if (sweeps.empty() || (uint32_t)__builtin_popcountll(sweeps.back().L | nd) > m) {
-            sweeps.push_back(Sweep{base, {}});
-            pplans.push_back({PhasePlan{0, {}}});
-        }
-        Sweep& sw = sweeps.back();
-        auto& pp = pplans.back();
-        sw.L |= nd;
-        if ((uint32_t)__builtin_popcountll(pp.back().R | nd) > rb) pp.push_back(PhasePlan{0, {}});
-        pp.back().R |= nd;
-        pp.back().ops.push_back((int)sw.ops.size());
-        sw.ops.push_back(g);
-    }
-    for (size_t k = 0; k < sweeps.size(); ++k) {   // fill up the local qubits, then each phase's slots
-        for (uint32_t q = 0; q < n - 1 && (uint32_t)__builtin_popcountll(sweeps[k].L) < m; ++q) sweeps[k].L |= 1ull << q;
-        for (auto& pp : pplans[k])
-            for (uint32_t q = n - 1; q-- > 0 && (uint32_t)__builtin_popcountll(pp.R) < rb;) pp.R |= (1ull << q) & sweeps[k].L;
-    }
-    std::vector<double> mats;
-    build_program(sweeps, n - 1, m, c, rb, epv, descs, phases, ops, mats, false, &pplans);
-}
 
 // calls f(std::integral_constant<int, RBITS>) for the register bits of a tile of 2^M elements
 template <typename T, class F>

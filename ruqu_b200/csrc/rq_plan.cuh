@@ -67,18 +67,16 @@ struct SweepDesc {
     uint64_t gj[1 << RBMAX];    // deposit of the per-thread vector offsets
     uint32_t sgj[1 << RBMAX];   // swz((tid-independent part of) the vector's first element)
     uint32_t img_begin, img_count;   // dense operand images of this sweep (tensor-core sweeps)
+    uint64_t selmask;           // symmetric states: qubits that thread bit SELECTOR flips (all outside the tile)
 };
+
+// tbit_global of the thread bit that selects a tile or its complement (symmetric states)
+constexpr uint8_t SELECTOR = 63;
 
 constexpr uint32_t SWEEP_INIT_UNIFORM = 1u;   // synthesise |+>^n instead of loading the tile
 constexpr uint32_t SWEEP_ENERGY = 2u;         // reduce sum |a|^2 cut(x) after the last phase
 constexpr uint32_t SWEEP_INIT_ZERO = 4u;      // synthesise |0...0> instead of loading the tile
 constexpr uint32_t SWEEP_INIT_LAMBDA = 8u;    // adjoint sweeps: build lambda = C psi instead of loading it
-// batched QAOA: Rx(t) = S^dag Ry(t) S, and the S of one layer cancels the S^dag of the next
-// across the diagonal cost phase, so the forward program runs Ry and carries the phases
-// i^popc(x) from the start (PHASE_IN, with INIT_UNIFORM) to the end (PHASE_OUT: (-i)^popc(x)
-// after the last phase)
-constexpr uint32_t SWEEP_PHASE_IN = 16u;
-constexpr uint32_t SWEEP_PHASE_OUT = 32u;
 
 
 struct PGate {
@@ -931,6 +929,156 @@ inline void build_program(std::vector<Sweep>& sweeps, uint32_t nq, uint32_t m, u
     if (mats.empty()) mats.push_back(0.0);
     if (ops.empty()) ops.push_back(SwOp{});
     if (phases.empty()) phases.push_back(PhaseDesc{});
+}
+
+// ---- programs of the batched engines --------------------------------------
+
+// The sweeps of a QAOA circuit on the kept half of a symmetric state, psi(x) = psi(~x): 2^(n-1) amplitudes,
+// indices with qubit n-1 = 0.  A rotation of qubit q < n-1 pairs indices that differ in bit q; one of
+// qubit n-1 pairs x with the index that stands for its flip, the complement of x in all n-1 bits.  The
+// planner sees n qubits; here the complement becomes a direction like the others:
+//  * a register slot of qubit n-1 is the local offset with every bit set;
+//  * a sweep that rotates qubit n-1 needs each tile's complement at hand.  Where tiles are not the whole
+//    state, its tiles have m-1 local qubits and a selector bit (the highest local offset bit): 0 the tile,
+//    1 its complement, whose outside qubits are all flipped;
+//  * flipping the n-1 index bits changes the cut as flipping vertex n-1 does, so for the cost phase the
+//    complement slot is that vertex.
+// Rx is the same from either end of a pair, so no signs change.
+inline void symmetric_program(const std::vector<PGate>& gates, uint32_t n, uint32_t m, uint32_t rb, uint32_t epv,
+                       std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
+    const uint32_t N = n - 1, c = std::min<uint32_t>(m, 5), cb = epv == 2 ? 4 : 3, t = m - rb;
+    const bool whole = m == N;
+    const uint64_t G = 1ull << N;
+    for (auto& sw : plan_sweeps(gates, n, whole ? n : m, c)) {
+        const bool pairs = (sw.L & G) && !whole;          // tiles with their complements
+        uint64_t real = sw.L & (G - 1);
+        const uint32_t want = pairs ? m - 1 : m;
+        for (uint32_t q = 0; q < N && (uint32_t)__builtin_popcountll(real) < want; ++q) real |= 1ull << q;
+        SweepDesc d{};
+        d.n = N;
+        d.m = m;
+        d.c = c;
+        uint8_t local_index[64];
+        uint32_t li = 0, ni = 0;
+        const uint64_t outside = (G - 1) & ~real;
+        const uint32_t sel = pairs ? 63 - (uint32_t)__builtin_clzll(outside) : 64;
+        for (uint32_t q = 0; q < N; ++q) {
+            if ((real >> q) & 1) { local_index[q] = (uint8_t)li; d.local_global[li++] = (uint8_t)q; }
+            else if (q != sel) d.nonlocal[ni++] = (uint8_t)q;
+        }
+        d.nonlocal_count = ni;
+        d.selmask = pairs ? outside : 0;
+        for (uint32_t j = 0; j < (1u << rb) / epv; ++j) {
+            const uint64_t x = (uint64_t)j * (1ull << t) * epv;
+            uint64_t g = 0;
+            for (uint32_t b = 0; b < li; ++b)
+                if ((x >> b) & 1) g |= 1ull << d.local_global[b];
+            if (pairs && ((x >> (m - 1)) & 1)) g ^= outside;
+            d.gj[j] = g;
+            d.sgj[j] = swz_host((uint32_t)x, cb);
+        }
+        d.phase_begin = (uint32_t)phases.size();
+        Sweep s2{real | (whole ? G : sw.L & G), sw.ops};
+        for (const auto& pp : plan_phases(s2, rb)) {
+            PhaseDesc P{};
+            P.op_begin = (uint32_t)ops.size();
+            int slot_of[64];
+            for (int q = 0; q < 64; ++q) slot_of[q] = -1;
+            uint32_t off[RBMAX], ns = 0;
+            for (uint32_t q = 0; q < n; ++q)
+                if ((pp.R >> q) & 1) {
+                    slot_of[q] = (int)ns;
+                    P.slot_global[ns] = (uint8_t)q;
+                    off[ns++] = q == N ? (1u << m) - 1 : 1u << local_index[q];
+                }
+            const bool flips = (pp.R & G) != 0;
+            std::vector<uint32_t> tb;                       // thread bits: the local bits that are no slots
+            for (uint32_t b = 0; b < li; ++b)
+                if (slot_of[d.local_global[b]] < 0) tb.push_back(b);
+            if (flips && whole) tb.pop_back();              // the complement replaces one of them
+            for (uint32_t b : tb) {
+                P.tbit_local[P.nt] = (uint8_t)b;
+                P.tbit_global[P.nt++] = d.local_global[b];
+            }
+            if (pairs && !flips) {
+                P.tbit_local[P.nt] = (uint8_t)(m - 1);
+                P.tbit_global[P.nt++] = SELECTOR;
+            }
+            for (uint32_t i = 0; i < (1u << rb); ++i) {
+                uint32_t o = 0;
+                for (uint32_t k = 0; k < ns; ++k)
+                    if ((i >> k) & 1) o ^= off[k];
+                P.lut[i] = (uint16_t)o;
+                P.slut[i] = swz_host(o, cb);
+            }
+            for (int oi : pp.ops) {
+                const PGate& g = sw.ops[oi];
+                SwOp o{};
+                o.type = g.type;
+                o.q0 = (uint8_t)g.q0;
+                o.k0 = g.type == OP_CPH ? (int8_t)-1 : (int8_t)slot_of[g.q0];
+                o.k1 = -1;
+                o.param = g.param;
+                ops.push_back(o);
+            }
+            P.op_end = (uint32_t)ops.size();
+            phases.push_back(P);
+        }
+        d.phase_end = (uint32_t)phases.size();
+        descs.push_back(d);
+    }
+}
+
+// The sweeps of a list of Ry and CZ gates on n qubits for the packed real state of n - 1 (qubit
+// q > 0 is its qubit q - 1, qubit 0 its two parts).  The gates are planned as sweeps over the
+// 2^n amplitudes (mloc local qubits) and run in exactly that order, so every amplitude goes
+// through the same roundings as unpacked: planning the packed gates afresh saves a sweep in four
+// on 16 qubits (5.5 instead of 5.8 ms for 2056 circuits) but its other order of the rotations moves
+// single f32 energies by their whole rounding error.  The order is cut into sweeps of m local packed
+// qubits and phases of rb slots; qubit 0 needs neither.
+inline void packed_program(const std::vector<PGate>& gates, uint32_t n, uint32_t mloc, uint32_t m, uint32_t rb, uint32_t epv,
+                    std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
+    const uint32_t m0 = std::min(n, mloc), c = std::min<uint32_t>(m, 5);
+    std::vector<PGate> order;
+    for (const auto& sw : plan_sweeps(gates, n, m0, std::min<uint32_t>(m0, 5)))
+        for (const auto& pp : plan_phases(sw, rb))
+            for (int k : pp.ops) {
+                PGate g = sw.ops[k];
+                if (g.type == OP_RYP && g.q0 == 0) {
+                    g.type = OP_RY0;
+                } else if (g.type == OP_CZ && g.q0 == 0) {
+                    g.type = OP_CZ0;
+                    g.q0 = g.q1 - 1;
+                } else {
+                    g.q0 -= 1;
+                    if (g.type == OP_CZ) g.q1 -= 1;
+                }
+                order.push_back(g);
+            }
+    const uint64_t base = (1ull << c) - 1;
+    std::vector<Sweep> sweeps;
+    std::vector<std::vector<PhasePlan>> pplans;
+    for (const auto& g : order) {
+        const uint64_t nd = needs(g);
+        if (sweeps.empty() || (uint32_t)__builtin_popcountll(sweeps.back().L | nd) > m) {
+            sweeps.push_back(Sweep{base, {}});
+            pplans.push_back({PhasePlan{0, {}}});
+        }
+        Sweep& sw = sweeps.back();
+        auto& pp = pplans.back();
+        sw.L |= nd;
+        if ((uint32_t)__builtin_popcountll(pp.back().R | nd) > rb) pp.push_back(PhasePlan{0, {}});
+        pp.back().R |= nd;
+        pp.back().ops.push_back((int)sw.ops.size());
+        sw.ops.push_back(g);
+    }
+    for (size_t k = 0; k < sweeps.size(); ++k) {   // fill up the local qubits, then each phase's slots
+        for (uint32_t q = 0; q < n - 1 && (uint32_t)__builtin_popcountll(sweeps[k].L) < m; ++q) sweeps[k].L |= 1ull << q;
+        for (auto& pp : pplans[k])
+            for (uint32_t q = n - 1; q-- > 0 && (uint32_t)__builtin_popcountll(pp.R) < rb;) pp.R |= (1ull << q) & sweeps[k].L;
+    }
+    std::vector<double> mats;
+    build_program(sweeps, n - 1, m, c, rb, epv, descs, phases, ops, mats, false, &pplans);
 }
 
 // ---- dense fusion for the tensor cores ----------------------------------

@@ -179,3 +179,40 @@ def test_repeated_runs_replay_one_graph_with_identical_results():
         eb, gb = plain.gradient(g1, b1)
         assert np.array_equal(ea, eb) and np.array_equal(ga, gb)
         assert a.last_graph()["replayed"] == (it > 0)
+
+
+@pytest.mark.parametrize("prec,sizes", [("f32", (7, 8, 13, 14, 15, 16)), ("f64", (6, 7, 12, 13, 14, 15))])
+def test_states_energies_and_gradients_at_tile_edges(prec, sizes):
+    """Smallest blocks, one tile exactly, one more qubit than a tile, several tiles; even and odd
+    qubit counts, dense and edgeless graphs.  Amplitudes against the oracle's whole state (1e-12 f64,
+    1e-5 f32), energies as above, gradients against central differences of the oracle (step 1e-5: 1e-7,
+    f32 2e-4 per edge)."""
+    r = np.random.default_rng(3)
+    graphs = [(n, [(a, b) for a in range(n) for b in range(a + 1, n) if r.random() < 0.4]) for n in sizes]
+    graphs.append((sizes[2], []))
+    p = 2
+    gam, bet = r.uniform(-1, 1, size=(len(graphs), p)), r.uniform(-1, 1, size=(len(graphs), p))
+    shots, seed = 200, 5
+    for k, (n, e) in enumerate(graphs):
+        qb = QaoaBatch([(n, e)], p, prec)
+        out = qb.run(gam[k:k + 1], bet[k:k + 1], shots=shots, seed=seed)
+        a = qb.state(0)
+        gates = [(0, q, 0, 0.0) for q in range(n)]
+        for l in range(p):
+            gates += [(15, u, v, 2 * gam[k, l]) for u, v in e] + [(8, q, 0, 2 * bet[k, l]) for q in range(n)]
+        o = oracle.OracleState(n, oracle.RQ_F64, 0)
+        o.apply(gates)
+        assert np.max(np.abs(a - o.amplitudes())) < (1e-12 if prec == "f64" else 1e-5)
+        ew = [(u, v, 1.0) for u, v in e]
+        assert abs(out["energies"][0] - oracle.qaoa_cost(n, ew, gam[k], bet[k])) < \
+            (1e-10 if prec == "f64" else 1e-5 * max(1, len(e)))
+        probs = a.real * a.real + a.imag * a.imag
+        assert _best_from_oracle(probs, n, e, seed, shots) == (int(out["best_bits"][0]), int(out["best_cut"][0]))
+        _, grad = qb.gradient(gam[k:k + 1], bet[k:k + 1])
+        for j in (0, p, 2 * p - 1):
+            th = np.concatenate([gam[k], bet[k]])
+            up, dn = th.copy(), th.copy()
+            up[j] += 1e-5
+            dn[j] -= 1e-5
+            want = (oracle.qaoa_cost(n, ew, up[:p], up[p:]) - oracle.qaoa_cost(n, ew, dn[:p], dn[p:])) / 2e-5
+            assert abs(grad[0, j] - want) < (1e-7 if prec == "f64" else 2e-4) * max(1, len(e)), (n, j)
