@@ -218,6 +218,38 @@ __device__ __forceinline__ void op_ry0(V* reg, T c, T s) {
     }
 }
 
+__device__ __forceinline__ float flip_sign(float v, uint32_t m) { return __uint_as_float(__float_as_uint(v) ^ m); }
+__device__ __forceinline__ double flip_sign(double v, uint32_t m) {
+    return __hiloint2double(__double2hiint(v) ^ (int)m, __double2loint(v));
+}
+
+// Sign bits (bit 31) of CZ(q, q + 1), q over the set bits of M, for the registers of one thread: register
+// i stands for the index U | deposit(i) (U with the slot bits zero), whose sign is the parity of
+// x & (x >> 1) & M.  Flipping slot s changes it by its neighbours' bits in U, D[s], and by the slots
+// already set that are neighbours, so the 2^RB sign bits take about two XORs each for any number of
+// gates.  Applying the gates one by one was two thirds of an ansatz sweep (ALU pipe 64 %).
+template <int RB>
+__device__ __forceinline__ void ladder_signs(uint32_t* m, uint32_t M, uint64_t U64, const uint8_t* slot_global) {
+    const uint32_t U = (uint32_t)U64;
+    m[0] = (uint32_t)__popc(U & (U >> 1) & M) << 31;
+#pragma unroll
+    for (int s = 0; s < RB; ++s) {
+        const uint32_t q = slot_global[s], up = M >> q, dn = (M << 1) >> q;   // CZ(q, q + 1), CZ(q - 1, q)
+        const uint32_t D = ((U >> 1 >> q) & up) ^ (((U << 1) >> q) & dn);
+        uint32_t e[1 << RB];                                                   // change by slot s, per subset of slots < s
+        e[0] = D << 31;
+#pragma unroll
+        for (int t = 0; t < s; ++t) {
+            const uint32_t r = slot_global[t];
+            const uint32_t A = ((r == q + 1u ? up : 0u) ^ (r + 1u == q ? dn : 0u)) << 31;
+#pragma unroll
+            for (int i = 0; i < (1 << t); ++i) e[i | (1 << t)] = e[i] ^ A;
+        }
+#pragma unroll
+        for (int i = 0; i < (1 << s); ++i) m[i | (1 << s)] = m[i] ^ e[i];
+    }
+}
+
 template <int NR, typename V, typename T>
 __device__ __forceinline__ void dispatch_ry(int k, V* reg, T c, T s) {
     switch (k) {
@@ -354,14 +386,13 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
                 } else if (op.type == OP_RYP) {
                     const T* r = a.rot + ((size_t)gcirc * a.nparam + op.param) * 2;
                     dispatch_ry<NR>(op.k0, reg, r[0], r[1]);
-                } else if (op.type == OP_CZ) {
-                    const int k0 = op.k0, k1 = op.k1;
-                    const int u0 = (int)((U >> op.q0) & 1ull), u1 = (int)((U >> op.q1) & 1ull);
+                } else if (op.type == OP_CZL) {
+                    uint32_t m[NR];
+                    ladder_signs<RB>(m, op.mat, U, ph.slot_global);
 #pragma unroll
                     for (int i = 0; i < NR; ++i) {
-                        const int b0 = k0 >= 0 ? ((i >> k0) & 1) : u0;
-                        const int b1 = k1 >= 0 ? ((i >> k1) & 1) : u1;
-                        if (b0 & b1) { reg[i].x = -reg[i].x; reg[i].y = -reg[i].y; }
+                        reg[i].x = flip_sign(reg[i].x, m[i]);
+                        reg[i].y = flip_sign(reg[i].y, m[i]);
                     }
                 } else if (op.type == OP_RY0) {
                     const T* r = a.rot + ((size_t)gcirc * a.nparam + op.param) * 2;
@@ -682,19 +713,15 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                             rp[i].y = -rp[i].y;
                             rl[i].y = -rl[i].y;
                         }
-                } else if (op.type == OP_CZ) {   // self-inverse
-                    const int k0 = op.k0, k1 = op.k1;
-                    const int u0 = (int)((U >> op.q0) & 1ull), u1 = (int)((U >> op.q1) & 1ull);
+                } else if (op.type == OP_CZL) {   // self-inverse
+                    uint32_t m[NR];
+                    ladder_signs<RB>(m, op.mat, U, ph.slot_global);
 #pragma unroll
                     for (int i = 0; i < NR; ++i) {
-                        const int b0 = k0 >= 0 ? ((i >> k0) & 1) : u0;
-                        const int b1 = k1 >= 0 ? ((i >> k1) & 1) : u1;
-                        if (b0 & b1) {
-                            rp[i].x = -rp[i].x;
-                            rp[i].y = -rp[i].y;
-                            rl[i].x = -rl[i].x;
-                            rl[i].y = -rl[i].y;
-                        }
+                        rp[i].x = flip_sign(rp[i].x, m[i]);
+                        rp[i].y = flip_sign(rp[i].y, m[i]);
+                        rl[i].x = flip_sign(rl[i].x, m[i]);
+                        rl[i].y = flip_sign(rl[i].y, m[i]);
                     }
                 }
             }
@@ -1072,16 +1099,6 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
 // the sign flips, two conversions and two FP64 FMAs; the grid-stride kernel this replaces read every
 // source amplitude from L2 and summed both complex parts of every string: 19.7 us per 16-qubit
 // circuit and 200 strings (512 circuits), now 3.3 us.
-template <typename T> struct SignBits;
-template <> struct SignBits<float> {
-    static __device__ __forceinline__ float flip(float v, uint32_t m) { return __uint_as_float(__float_as_uint(v) ^ m); }
-};
-template <> struct SignBits<double> {
-    static __device__ __forceinline__ double flip(double v, uint32_t m) {
-        return __hiloint2double(__double2hiint(v) ^ (int)m, __double2loint(v));
-    }
-};
-
 template <typename T, int RBITS>
 __global__ void __launch_bounds__(PK_THREADS, 1)
     k_vqe_apply_h(const typename C2<T>::t* __restrict__ states, typename C2<T>::t* __restrict__ lam, uint32_t n,
@@ -1134,8 +1151,8 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
                         const int i = q ^ (q >> 1);   // Gray-code order: one sign bit changes per element
                         if (q) m ^= ((tm.z >> (PK_TB + gray_bit(q))) & 1u) << 31;
                         const V v = src[P ^ ((uint32_t)i << PK_TB)];
-                        const double vx = (double)SignBits<T>::flip(v.x, m);
-                        const double vy = (double)SignBits<T>::flip(v.y, m ^ tm.z0);
+                        const double vx = (double)flip_sign(v.x, m);
+                        const double vy = (double)flip_sign(v.y, m ^ tm.z0);
                         if (sg.x0) {
                             hx[i] = fma(tm.f, vy, hx[i]);
                             hy[i] = fma(tm.f, vx, hy[i]);

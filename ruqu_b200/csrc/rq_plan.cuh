@@ -29,8 +29,9 @@ namespace rqp {
 // on the tensor cores (param = index of its operand image).
 // RY0, CZ0: Ry on, and CZ with, the qubit that a packed real state keeps in the real and
 // imaginary part of each element (q0 = the other qubit of CZ0); they need no register slot.
+// CZL: CZ(q, q + 1) for every set bit q of mat.
 enum OpType : uint8_t { OP_U1 = 0, OP_D1 = 1, OP_CX = 2, OP_CZ = 3, OP_ZZ = 4, OP_CPH = 5, OP_RXP = 6, OP_RYP = 7,
-                        OP_DENSE = 8, OP_RY0 = 9, OP_CZ0 = 10 };
+                        OP_DENSE = 8, OP_RY0 = 9, OP_CZ0 = 10, OP_CZL = 11 };
 
 constexpr int RBMAX = 5;
 constexpr int MMAX = 14;
@@ -1029,6 +1030,41 @@ inline void symmetric_program(const std::vector<PGate>& gates, uint32_t n, uint3
     }
 }
 
+// Collects the CZ(q, q + 1) of each phase into one op per run: signs are exact, so a CZ may wait until
+// a rotation of one of its qubits comes up.
+inline void merge_ladders(const std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
+    std::vector<SwOp> out;
+    for (const auto& d : descs)
+        for (uint32_t p = d.phase_begin; p < d.phase_end; ++p) {
+            PhaseDesc& ph = phases[p];
+            const uint32_t begin = (uint32_t)out.size();
+            uint32_t mask = 0;
+            auto flush = [&]() {
+                if (!mask) return;
+                SwOp o{};
+                o.type = OP_CZL;
+                o.k0 = o.k1 = -1;
+                o.mat = mask;
+                out.push_back(o);
+                mask = 0;
+            };
+            for (uint32_t k = ph.op_begin; k < ph.op_end; ++k) {
+                const SwOp& o = ops[k];
+                if (o.type == OP_CZ && o.q1 == o.q0 + 1) {
+                    mask ^= 1u << o.q0;
+                    continue;
+                }
+                if (o.type == OP_RYP && (mask & ((1u << o.q0) | (o.q0 ? 1u << (o.q0 - 1) : 0u)))) flush();
+                out.push_back(o);
+            }
+            flush();
+            ph.op_begin = begin;
+            ph.op_end = (uint32_t)out.size();
+        }
+    if (out.empty()) out.push_back(SwOp{});
+    ops.swap(out);
+}
+
 // The sweeps of a list of Ry and CZ gates on n qubits for the packed real state of n - 1 (qubit
 // q > 0 is its qubit q - 1, qubit 0 its two parts).  The gates are planned as sweeps over the
 // 2^n amplitudes (mloc local qubits) and run in exactly that order, so every amplitude goes
@@ -1079,6 +1115,7 @@ inline void packed_program(const std::vector<PGate>& gates, uint32_t n, uint32_t
     }
     std::vector<double> mats;
     build_program(sweeps, n - 1, m, c, rb, epv, descs, phases, ops, mats, false, &pplans);
+    merge_ladders(descs, phases, ops);
 }
 
 // ---- dense fusion for the tensor cores ----------------------------------

@@ -204,17 +204,19 @@ static void check_packed(uint32_t n, uint32_t mloc, uint32_t rb, uint32_t epv, u
     packed_program(g, n, mloc, std::min(n - 1, mloc), rb, epv, descs, phases, ops);
     std::vector<C> st(1ull << (n - 1));
     for (uint64_t j = 0; j < st.size(); ++j) st[j] = C(start[2 * j], start[2 * j + 1]);
-    run_program(descs, phases, ops, rb, epv, st, [&](std::vector<C>& reg, const PhaseDesc&, const SwOp& o, uint64_t U) {
+    run_program(descs, phases, ops, rb, epv, st, [&](std::vector<C>& reg, const PhaseDesc& ph, const SwOp& o, uint64_t U) {
         const double c = std::cos(th[o.param] / 2), s = std::sin(th[o.param] / 2);
         for (uint32_t i = 0; i < reg.size(); ++i) {
             const int b0 = o.k0 >= 0 ? (i >> o.k0) & 1 : (U >> o.q0) & 1;
-            if (o.type == OP_RY0) {
+            if (o.type == OP_CZL) {
+                uint64_t x = U;
+                for (uint32_t s = 0; s < rb; ++s)
+                    if ((i >> s) & 1) x |= 1ull << ph.slot_global[s];
+                if (__builtin_popcountll(x & (x >> 1) & o.mat) & 1) reg[i] = -reg[i];
+            } else if (o.type == OP_RY0) {
                 reg[i] = C(c * reg[i].real() - s * reg[i].imag(), s * reg[i].real() + c * reg[i].imag());
             } else if (o.type == OP_CZ0) {
                 if (b0) reg[i] = std::conj(reg[i]);
-            } else if (o.type == OP_CZ) {
-                const int b1 = o.k1 >= 0 ? (i >> o.k1) & 1 : (U >> o.q1) & 1;
-                if (b0 && b1) reg[i] = -reg[i];
             } else {
                 CHECK(o.k0 >= 0, "Ry without a slot");
                 if (!((i >> o.k0) & 1)) {
