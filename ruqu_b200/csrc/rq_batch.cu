@@ -924,12 +924,14 @@ __global__ void k_bsample(const typename C2<T>::t* __restrict__ amps, const doub
 // x = 2X + x0, Y/Z mask z = 2Z + z0 and an even number of Y factors has, up to its factor,
 //   <P> = sum_j (-1)^|j & Z| (A.x B.x' + (-1)^z0 A.y B.y'),  A = a_j, B = a_(j ^ X),
 // with B's parts swapped when x0 = 1.
-struct PTerm {
-    uint32_t xl;      // X inside a tile of 2^M elements
+template <typename T>
+struct __align__(16) PTerm {
+    uint32_t xb;      // X inside a tile of 2^M elements, as a byte offset
     uint32_t z;       // Z
-    uint32_t z0;      // sign bit (bit 31) of (-1)^z0
-    uint32_t pad;
-    double f;         // energy pass: coefficient and pair factors; H pass: coefficient
+    double f;         // energy pass: coefficient and pair factors
+    double fx, fy;    // H pass: what the source's two parts are multiplied with
+    T sg[4];          // energy pass: +-1, the sign of each register bit
+    T s0, pad[sizeof(T) == 4 ? 3 : 1];   // energy pass: (-1)^z0
 };
 // strings of one kind, [begin, end): top part t of X, x0, and (energy pass) how their pairs are
 // walked -- mode b < RBITS: X has register bit b, walk the elements where it is 0; RBITS: walk all;
@@ -947,11 +949,19 @@ __device__ __forceinline__ float2 fma2(float s, float2 b, float2 c) { return pk_
 __device__ __forceinline__ double2 fma2(double s, double2 b, double2 c) { return make_double2(fma(s, b.x, c.x), fma(s, b.y, c.y)); }
 
 template <typename V>
-__device__ __forceinline__ void pk_load_tile(V* dst, const V* __restrict__ src, uint32_t L, uint32_t tid) {
+__device__ __forceinline__ void pk_load_tile(uint32_t dst, const V* __restrict__ src, uint32_t L, uint32_t tid) {
     constexpr uint32_t EPC = 16 / sizeof(V);
     if (L >= EPC)
-        for (uint32_t e = tid * EPC; e < L; e += PK_THREADS * EPC) bcp_async16(dst + e, src + e);
+        for (uint32_t e = tid * EPC; e < L; e += PK_THREADS * EPC)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + e * (uint32_t)sizeof(V)), "l"(src + e) : "memory");
     asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+// one element from a shared-memory byte address
+__device__ __forceinline__ void lds_pair(float2& v, uint32_t a) {
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+}
+__device__ __forceinline__ void lds_pair(double2& v, uint32_t a) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
 }
 
 // The strings [begin, end) of one segment over the register elements A: per string the products of
@@ -959,59 +969,63 @@ __device__ __forceinline__ void pk_load_tile(V* dst, const V* __restrict__ src, 
 // sign as a factor (at most 16 products in the state's type), then FP64.
 // BIT >= 0: walk the elements whose register bit BIT is HI; BIT < 0: all.
 template <typename T, int RBITS, int BIT, int HI>
-__device__ __forceinline__ double pk_walk(const typename C2<T>::t* A, const typename C2<T>::t* src,
-                                          const PTerm* __restrict__ terms, uint32_t begin, uint32_t end, uint32_t own,
-                                          uint32_t tid, uint32_t L) {
+__device__ __forceinline__ double pk_walk(const typename C2<T>::t* A, uint32_t src, const PTerm<T>* terms, uint32_t begin,
+                                          uint32_t end, uint32_t own, uint32_t tid, bool in) {
     using V = typename C2<T>::t;
     constexpr int NB = BIT >= 0 ? RBITS - 1 : RBITS;   // free register bits
-    constexpr int NW = 1 << NB;
-    const bool in = tid < L;
+    constexpr int NW = 1 << NB, B0 = BIT < 0 ? 0 : BIT;
+    const uint32_t tb = tid * (uint32_t)sizeof(V);
+    const uint32_t idx = own | tid | ((uint32_t)(HI && BIT >= 0) << (PK_TB + B0));
     double acc = 0.0;
-    PTerm nt = terms[begin];
     for (uint32_t k = begin; k < end; ++k) {
-        const PTerm t = nt;
-        if (k + 1 < end) nt = terms[k + 1];
-        const uint32_t P = in ? tid ^ t.xl : 0u;
+        const PTerm<T>& t = terms[k];
+        const uint32_t P = in ? tb ^ t.xb : 0u;
         V v[NW];
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
-            const int i = BIT < 0 ? w : ((w >> BIT) << (BIT + 1)) | (HI << BIT) | (w & ((1 << (BIT < 0 ? 0 : BIT)) - 1));
-            v[w] = mul2(A[i], src[P ^ ((uint32_t)i << PK_TB)]);
+            const int i = BIT < 0 ? w : ((w >> B0) << (B0 + 1)) | (HI << B0) | (w & ((1 << B0) - 1));
+            lds_pair(v[w], src + (P ^ ((uint32_t)i * ((uint32_t)sizeof(V) << PK_TB))));
+            v[w] = mul2(A[i], v[w]);
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-            const int gb = BIT >= 0 && b >= BIT ? b + 1 : b;
-            const T sg = ((t.z >> (PK_TB + gb)) & 1u) ? (T)-1 : (T)1;
+            const T sg = t.sg[BIT >= 0 && b >= BIT ? b + 1 : b];
 #pragma unroll
             for (int w = 0; w < NW; w += 2 << b) v[w] = fma2(sg, v[w + (1 << b)], v[w]);
         }
-        const uint32_t st = (uint32_t)__popc((own | tid | ((uint32_t)(HI && BIT >= 0 ? 1 : 0) << (PK_TB + (BIT < 0 ? 0 : BIT)))) & t.z) & 1u;
-        const T s0 = t.z0 ? (T)-1 : (T)1;
-        const T s = v[0].x + s0 * v[0].y;
-        acc += (st ? -t.f : t.f) * (double)s;
+        const T s = v[0].x + t.s0 * v[0].y;
+        acc = fma(t.f, (double)flip_sign(s, (uint32_t)__popc(idx & t.z) << 31), acc);
     }
     return acc;
 }
 
 template <typename T, int RBITS>
-__device__ __forceinline__ double pk_segment(const PSeg& g, const typename C2<T>::t* A, const typename C2<T>::t* src,
-                                             const PTerm* __restrict__ terms, uint32_t own, bool lower, uint32_t tid,
-                                             uint32_t L) {
+__device__ __forceinline__ double pk_segment(const PSeg& g, const typename C2<T>::t* A, uint32_t src,
+                                             const PTerm<T>* terms, uint32_t own, bool lower, uint32_t tid, bool in) {
     if constexpr (RBITS > 0) {
         if (g.mode > RBITS) {   // pairs across two tiles: the lower tile's CTA takes its elements with top bit 0
             const uint32_t hi = lower ? 0u : 1u ^ (g.mode - RBITS - 1);
-            return hi ? pk_walk<T, RBITS, RBITS - 1, 1>(A, src, terms, g.begin, g.end, own, tid, L)
-                      : pk_walk<T, RBITS, RBITS - 1, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+            return hi ? pk_walk<T, RBITS, RBITS - 1, 1>(A, src, terms, g.begin, g.end, own, tid, in)
+                      : pk_walk<T, RBITS, RBITS - 1, 0>(A, src, terms, g.begin, g.end, own, tid, in);
         }
-        if (g.mode == 0) return pk_walk<T, RBITS, 0, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+        if (g.mode == 0) return pk_walk<T, RBITS, 0, 0>(A, src, terms, g.begin, g.end, own, tid, in);
         if constexpr (RBITS > 1)
-            if (g.mode == 1) return pk_walk<T, RBITS, 1, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+            if (g.mode == 1) return pk_walk<T, RBITS, 1, 0>(A, src, terms, g.begin, g.end, own, tid, in);
         if constexpr (RBITS > 2)
-            if (g.mode == 2) return pk_walk<T, RBITS, 2, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+            if (g.mode == 2) return pk_walk<T, RBITS, 2, 0>(A, src, terms, g.begin, g.end, own, tid, in);
         if constexpr (RBITS > 3)
-            if (g.mode == 3) return pk_walk<T, RBITS, 3, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+            if (g.mode == 3) return pk_walk<T, RBITS, 3, 0>(A, src, terms, g.begin, g.end, own, tid, in);
     }
-    return pk_walk<T, RBITS, -1, 0>(A, src, terms, g.begin, g.end, own, tid, L);
+    return pk_walk<T, RBITS, -1, 0>(A, src, terms, g.begin, g.end, own, tid, in);
+}
+
+// the strings into shared memory (a uniform 16-byte load each; visible after the next barrier)
+template <typename T>
+__device__ __forceinline__ const PTerm<T>* pk_stage_terms(PTerm<T>* dst, const PTerm<T>* __restrict__ src, uint32_t n,
+                                                          uint32_t tid) {
+    const uint32_t nw = n * (uint32_t)(sizeof(PTerm<T>) / 16);
+    for (uint32_t k = tid; k < nw; k += PK_THREADS) reinterpret_cast<uint4*>(dst)[k] = reinterpret_cast<const uint4*>(src)[k];
+    return dst;
 }
 
 // Energy of every (circuit, tile) of a wave: a thread keeps its 2^RBITS elements of the tile in
@@ -1020,20 +1034,23 @@ __device__ __forceinline__ double pk_segment(const PSeg& g, const typename C2<T>
 // and two packed FP32x2 instructions per element walked, and one FP64 FMA: strings add up in FP64
 // per thread and are reduced over the CTA once.  Pairs inside the tile are walked once by a register
 // bit of X (where X has none, all elements are walked and f is halved), pairs between two tiles half
-// by each tile's CTA.  Bound by instruction issue.  The one-warp-per-string walk of complex tiles this
+// by each tile's CTA.  Bound by instruction issue (the strings' sign factors come ready-made from shared
+// memory; forming them per thread had cost another third).  The one-warp-per-string walk of complex tiles this
 // replaces was bound by its index and sign arithmetic: 13.6 us per 16-qubit circuit and 200 strings
-// (2056 circuits), now 1.1 us.
+// (2056 circuits), now 0.8 us.
 template <typename T, int RBITS>
 __global__ void __launch_bounds__(PK_THREADS, 1)
     k_vqe_energy(const typename C2<T>::t* __restrict__ states, uint32_t n, uint32_t M, uint64_t ncirc,
-                 const PSeg* __restrict__ segs, const uint32_t* __restrict__ sofs, const PTerm* __restrict__ terms,
-                 double e0, double* __restrict__ part) {
+                 const PSeg* __restrict__ segs, const uint32_t* __restrict__ sofs, const PTerm<T>* __restrict__ gterms,
+                 uint32_t nterms, double e0, double* __restrict__ part) {
     using V = typename C2<T>::t;
     constexpr int NR = 1 << RBITS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[PK_THREADS / 32];
     const uint32_t L = 1u << M, tid = threadIdx.x;
-    V* buf[2] = {reinterpret_cast<V*>(smem_raw), reinterpret_cast<V*>(smem_raw) + L};
+    const bool in = tid < L;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem_raw), TB = L * (uint32_t)sizeof(V);   // two tiles, then the strings
+    const PTerm<T>* terms = pk_stage_terms(reinterpret_cast<PTerm<T>*>(smem_raw + 2 * TB), gterms, nterms, tid);
     const uint32_t ntile = 1u << (n - M);
     const uint64_t nwork = ncirc * ntile;
     for (uint64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -1053,11 +1070,11 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
         };
         double acc = 0.0;
         uint32_t t = next_t(0), at = 0;
-        if (t < ntile) pk_load_tile<V>(buf[0], a + ((uint64_t)(r ^ t) << M), L, tid);
+        if (t < ntile) pk_load_tile<V>(sbase, a + ((uint64_t)(r ^ t) << M), L, tid);
         while (t < ntile) {
             const uint32_t tn = next_t(t + 1);
             if (tn < ntile) {
-                pk_load_tile<V>(buf[at ^ 1], a + ((uint64_t)(r ^ tn) << M), L, tid);
+                pk_load_tile<V>(sbase + (at ^ 1u) * TB, a + ((uint64_t)(r ^ tn) << M), L, tid);
                 asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             } else {
                 asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -1071,7 +1088,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
                     for (int i = 0; i < NR; ++i) A[i] = V{A[i].y, A[i].x};
                     swapped = sg.x0;
                 }
-                acc += pk_segment<T, RBITS>(sg, A, buf[at], terms, own, r < (r ^ t), tid, L);
+                acc += pk_segment<T, RBITS>(sg, A, sbase + at * TB, terms, own, r < (r ^ t), tid, in);
             }
             if (swapped) {
 #pragma unroll
@@ -1096,20 +1113,43 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
 // lambda = H psi for every (circuit, tile) of a wave (the start of the VQE adjoint pass): a thread
 // owns 2^RBITS output elements (both parts summed in FP64 over the strings), the source tiles r ^ t
 // come through shared memory as in the energy pass.  Per string and element one shared-memory load,
-// the sign flips, two conversions and two FP64 FMAs; the grid-stride kernel this replaces read every
+// two sign flips of the coefficients, two conversions and two FP64 FMAs; the grid-stride kernel this replaces read every
 // source amplitude from L2 and summed both complex parts of every string: 19.7 us per 16-qubit
-// circuit and 200 strings (512 circuits), now 3.3 us.
+// circuit and 200 strings (512 circuits), now 2.1 us, bound by the conversions to FP64 (XU).
+template <typename T, int RBITS>
+__device__ __forceinline__ void pk_accumulate(double* hx, double* hy, uint32_t src, uint32_t P, uint32_t z, double fx,
+                                              double fy) {
+    using V = typename C2<T>::t;
+    uint32_t sb[RBITS > 0 ? RBITS : 1];
+#pragma unroll
+    for (int b = 0; b < RBITS; ++b) sb[b] = (z << (31 - PK_TB - b)) & 0x80000000u;
+#pragma unroll
+    for (int q = 0; q < (1 << RBITS); ++q) {
+        const int i = q ^ (q >> 1);   // Gray-code order: one sign bit changes per element
+        if (q) {
+            fx = flip_sign(fx, sb[gray_bit(q)]);
+            fy = flip_sign(fy, sb[gray_bit(q)]);
+        }
+        V v;
+        lds_pair(v, src + (P ^ ((uint32_t)i * ((uint32_t)sizeof(V) << PK_TB))));
+        hx[i] = fma(fx, (double)v.x, hx[i]);
+        hy[i] = fma(fy, (double)v.y, hy[i]);
+    }
+}
+
 template <typename T, int RBITS>
 __global__ void __launch_bounds__(PK_THREADS, 1)
     k_vqe_apply_h(const typename C2<T>::t* __restrict__ states, typename C2<T>::t* __restrict__ lam, uint32_t n,
                   uint32_t M, uint64_t ncirc, const PSeg* __restrict__ segs, const uint32_t* __restrict__ sofs,
-                  const PTerm* __restrict__ terms) {
+                  const PTerm<T>* __restrict__ gterms, uint32_t nterms, uint32_t term0) {
     using V = typename C2<T>::t;
     constexpr int NR = 1 << RBITS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t L = 1u << M, tid = threadIdx.x;
     const bool in = tid < L;
-    V* buf[2] = {reinterpret_cast<V*>(smem_raw), reinterpret_cast<V*>(smem_raw) + L};
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem_raw), TB = L * (uint32_t)sizeof(V);
+    const PTerm<T>* terms = pk_stage_terms(reinterpret_cast<PTerm<T>*>(smem_raw + 2 * TB), gterms + term0, nterms, tid);
+    const uint32_t tb = tid * (uint32_t)sizeof(V);
     const uint32_t ntile = 1u << (n - M);
     const uint64_t nwork = ncirc * ntile;
     for (uint64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -1124,43 +1164,28 @@ __global__ void __launch_bounds__(PK_THREADS, 1)
             return t;
         };
         uint32_t t = next_t(0), at = 0;
-        if (t < ntile) pk_load_tile<V>(buf[0], a + ((uint64_t)(r ^ t) << M), L, tid);
+        if (t < ntile) pk_load_tile<V>(sbase, a + ((uint64_t)(r ^ t) << M), L, tid);
         while (t < ntile) {
             const uint32_t tn = next_t(t + 1);
             if (tn < ntile) {
-                pk_load_tile<V>(buf[at ^ 1], a + ((uint64_t)(r ^ tn) << M), L, tid);
+                pk_load_tile<V>(sbase + (at ^ 1u) * TB, a + ((uint64_t)(r ^ tn) << M), L, tid);
                 asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             } else {
                 asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             }
             __syncthreads();
-            const V* src = buf[at];
-            const uint32_t top = (r ^ t) << M;
+            const uint32_t src = sbase + at * TB, top = (r ^ t) << M;
             for (uint32_t g = sofs[t]; g < sofs[t + 1]; ++g) {
                 const PSeg sg = segs[g];
-                PTerm nt = terms[sg.begin];
-                for (uint32_t k = sg.begin; k < sg.end; ++k) {
-                    const PTerm tm = nt;
-                    if (k + 1 < sg.end) nt = terms[k + 1];
-                    const uint32_t P = in ? tid ^ tm.xl : 0u;
-                    // sign of the source element (index parity with Z); part b of the source
-                    // carries (-1)^(b z0) and lands in part b ^ x0
-                    uint32_t m = (uint32_t)(__popc((top | P) & tm.z) & 1) << 31;
-#pragma unroll
-                    for (int q = 0; q < NR; ++q) {
-                        const int i = q ^ (q >> 1);   // Gray-code order: one sign bit changes per element
-                        if (q) m ^= ((tm.z >> (PK_TB + gray_bit(q))) & 1u) << 31;
-                        const V v = src[P ^ ((uint32_t)i << PK_TB)];
-                        const double vx = (double)flip_sign(v.x, m);
-                        const double vy = (double)flip_sign(v.y, m ^ tm.z0);
-                        if (sg.x0) {
-                            hx[i] = fma(tm.f, vy, hx[i]);
-                            hy[i] = fma(tm.f, vx, hy[i]);
-                        } else {
-                            hx[i] = fma(tm.f, vx, hx[i]);
-                            hy[i] = fma(tm.f, vy, hy[i]);
-                        }
-                    }
+                for (uint32_t k = sg.begin - term0; k < sg.end - term0; ++k) {
+                    const PTerm<T>& tm = terms[k];
+                    const uint32_t P = in ? tb ^ tm.xb : 0u;
+                    // sign of the source element (index parity with Z), on the coefficients; part b of the
+                    // source carries (-1)^(b z0) (in fy) and lands in part b ^ x0
+                    const uint32_t m = (uint32_t)__popc((top | P / (uint32_t)sizeof(V)) & tm.z) << 31;
+                    double fx = flip_sign(tm.fx, m), fy = flip_sign(tm.fy, m);
+                    if (sg.x0) pk_accumulate<T, RBITS>(hy, hx, src, P, tm.z, fx, fy);
+                    else pk_accumulate<T, RBITS>(hx, hy, src, P, tm.z, fx, fy);
                 }
             }
             __syncthreads();
@@ -2358,7 +2383,8 @@ struct rq_vqe_batch {
     uint32_t em = 0;              // log2 elements of a tile of the energy and H passes
     uint32_t nterms = 0;          // strings as given
     double e0 = 0.0;              // what the strings without a real expectation add (0, or NaN)
-    PTerm* d_terms = nullptr;     // energy strings, then H strings, by segment
+    void* d_terms = nullptr;      // PTerm<T>: energy strings, then H strings, by segment
+    uint32_t neterms = 0, nhterms = 0;
     PSeg* d_segs = nullptr;
     uint32_t* d_sofs = nullptr;   // segments of top part t: [sofs[t], sofs[t + 1]); H pass: after ntile + 1
     double* d_part = nullptr;
@@ -2410,7 +2436,7 @@ template <typename T>
 int vqe_energy(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     using V = typename C2<T>::t;
     const uint32_t ntile = 1u << (b->pn - b->em);
-    const size_t smem = 2 * ((size_t)1 << b->em) * sizeof(V);
+    const size_t smem = 2 * ((size_t)1 << b->em) * sizeof(V) + b->neterms * sizeof(PTerm<T>);
     RQ_TRY(grow(&b->d_part, &b->part_cap, ncirc * ntile));
     const int sms = rq::num_sms(b->device);
     const unsigned grid = (unsigned)std::min<uint64_t>(ncirc * ntile, (uint64_t)sms);
@@ -2418,7 +2444,7 @@ int vqe_energy(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
         auto kern = k_vqe_energy<T, decltype(rbits)::value>;
         RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kern<<<grid, PK_THREADS, smem, b->stream>>>((const V*)b->d_states, b->pn, b->em, ncirc, b->d_segs, b->d_sofs,
-                                                    b->d_terms, b->e0, b->d_part);
+                                                    (const PTerm<T>*)b->d_terms, b->neterms, b->e0, b->d_part);
         RQ_CUDA(cudaGetLastError());
         return (int)RQ_OK;
     }));
@@ -2472,13 +2498,14 @@ int vqe_adjoint(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     constexpr int RBc = std::is_same<T, float>::value ? 4 : 3;
     const int sms = rq::num_sms(b->device);
     const uint32_t ntile = 1u << (b->pn - b->em);
-    const size_t hsmem = 2 * ((size_t)1 << b->em) * sizeof(V);
+    const size_t hsmem = 2 * ((size_t)1 << b->em) * sizeof(V) + b->nhterms * sizeof(PTerm<T>);
     const unsigned hgrid = (unsigned)std::min<uint64_t>(ncirc * ntile, (uint64_t)sms);
     RQ_TRY(with_register_bits<T>(b->em, [&](auto rbits) {
         auto kern = k_vqe_apply_h<T, decltype(rbits)::value>;
         RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
         kern<<<hgrid, PK_THREADS, hsmem, b->stream>>>((const V*)b->d_states, (V*)b->d_lam, b->pn, b->em, ncirc,
-                                                      b->d_segs, b->d_sofs + ntile + 1, b->d_terms);
+                                                      b->d_segs, b->d_sofs + ntile + 1, (const PTerm<T>*)b->d_terms,
+                                                      b->nhterms, b->neterms);
         RQ_CUDA(cudaGetLastError());
         return (int)RQ_OK;
     }));
@@ -2585,7 +2612,11 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
     b->em = std::min<uint32_t>(b->pn, precision == RQ_F32 ? 13 : 12);
     const uint32_t M = b->em, ntile = 1u << (b->pn - M), RBITS = M > (uint32_t)PK_TB ? M - PK_TB : 0;
     // Hamiltonian in mask form, by segment (top part of X, qubit-0 bit of X, walk mode)
-    std::map<std::vector<uint32_t>, std::vector<PTerm>> eseg, hseg;
+    struct HostTerm {
+        uint32_t xl, z, z0;
+        double f;
+    };
+    std::map<std::vector<uint32_t>, std::vector<HostTerm>> eseg, hseg;
     for (uint32_t k = 0; k < nterms; ++k) {
         if (offsets[k + 1] < offsets[k]) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing");
         uint64_t x = 0, z = 0;
@@ -2608,11 +2639,7 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
         }
         const double cf = (ny & 2u) ? -coeffs[k] : coeffs[k];
         const uint32_t x0 = (uint32_t)(x & 1u), X = (uint32_t)(x >> 1), top = X >> M, xl = X & ((1u << M) - 1);
-        PTerm t{};
-        t.xl = xl;
-        t.z = (uint32_t)(z >> 1);
-        t.z0 = (uint32_t)(z & 1u) << 31;
-        t.f = cf;
+        HostTerm t{xl, (uint32_t)(z >> 1), (uint32_t)(z & 1u), cf};
         hseg[{top, x0}].push_back(t);
         uint32_t mode = RBITS;
         const uint32_t xr = xl >> PK_TB;
@@ -2624,11 +2651,11 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
         eseg[{top, x0, mode}].push_back(t);
     }
     // a state that is not finite gives NaN through the strings left out, too
-    if (nterms) eseg[{0u, 0u, RBITS}].push_back(PTerm{});
-    std::vector<PTerm> terms;
+    if (nterms) eseg[{0u, 0u, RBITS}].push_back(HostTerm{});
+    std::vector<HostTerm> terms;
     std::vector<PSeg> segs;
     std::vector<uint32_t> sofs(2 * (ntile + 1), 0);
-    auto lay_out = [&](const std::map<std::vector<uint32_t>, std::vector<PTerm>>& by, uint32_t* ofs) {
+    auto lay_out = [&](const std::map<std::vector<uint32_t>, std::vector<HostTerm>>& by, uint32_t* ofs) {
         auto it = by.begin();
         for (uint32_t t = 0; t < ntile; ++t) {
             ofs[t] = (uint32_t)segs.size();
@@ -2645,15 +2672,35 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
         ofs[ntile] = (uint32_t)segs.size();
     };
     lay_out(eseg, sofs.data());
+    b->neterms = (uint32_t)terms.size();
     lay_out(hseg, sofs.data() + ntile + 1);
+    b->nhterms = (uint32_t)terms.size() - b->neterms;
     if (segs.empty()) segs.push_back(PSeg{});
-    if (terms.empty()) terms.push_back(PTerm{});
+    std::vector<unsigned char> dterms;
+    auto pack = [&](auto sample) {
+        using T = decltype(sample);
+        std::vector<PTerm<T>> out(std::max<size_t>(1, terms.size()));
+        for (size_t k = 0; k < terms.size(); ++k) {
+            const HostTerm& h = terms[k];
+            PTerm<T>& o = out[k];
+            o.xb = h.xl * (uint32_t)(2 * sizeof(T));
+            o.z = h.z;
+            o.f = o.fx = h.f;
+            o.fy = h.z0 ? -h.f : h.f;
+            for (int q = 0; q < 4; ++q) o.sg[q] = (h.z >> (PK_TB + q)) & 1u ? (T)-1 : (T)1;
+            o.s0 = h.z0 ? (T)-1 : (T)1;
+        }
+        dterms.resize(out.size() * sizeof(PTerm<T>));
+        std::memcpy(dterms.data(), out.data(), dterms.size());
+    };
+    if (precision == RQ_F32) pack(0.0f);
+    else pack(0.0);
     RQ_CUDA(cudaMalloc((void**)&b->d_sofs, sofs.size() * sizeof(uint32_t)));
     RQ_CUDA(cudaMemcpy(b->d_sofs, sofs.data(), sofs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     RQ_CUDA(cudaMalloc((void**)&b->d_segs, segs.size() * sizeof(PSeg)));
     RQ_CUDA(cudaMemcpy(b->d_segs, segs.data(), segs.size() * sizeof(PSeg), cudaMemcpyHostToDevice));
-    RQ_CUDA(cudaMalloc((void**)&b->d_terms, terms.size() * sizeof(PTerm)));
-    RQ_CUDA(cudaMemcpy(b->d_terms, terms.data(), terms.size() * sizeof(PTerm), cudaMemcpyHostToDevice));
+    RQ_CUDA(cudaMalloc(&b->d_terms, dterms.size()));
+    RQ_CUDA(cudaMemcpy(b->d_terms, dterms.data(), dterms.size(), cudaMemcpyHostToDevice));
     // the ansatz program
     const uint32_t mloc = precision == RQ_F32 ? 13u : 12u;
     b->m = std::min(b->pn, mloc);
