@@ -25,6 +25,7 @@
 //    keeps the best cut (highest cut, lowest shot index on ties).
 #include "rq_internal.cuh"
 #include "rq_plan.cuh"
+#include "rq_tree.cuh"
 
 
 #include <algorithm>
@@ -806,42 +807,13 @@ __global__ void k_qaoa_tables(const double* __restrict__ gammas, const double* _
 
 // ---- sampling -------------------------------------------------------------
 
-template <typename T>
-__device__ __forceinline__ double pr(const typename C2<T>::t* a, uint64_t i) {
-    auto x = a[i];
-    double re = x.x, im = x.y;
-    return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
-}
-
-// Prefix trees over the kept half of each state (n = its index bits, one less than the qubits; tree of
-// circuit c at tree + c * 2^n): level L holds 2^L sums over the indices with the same low L bits.
-// Level n-1 comes from the amplitudes:
-template <typename T>
-__global__ void k_bleaf(const typename C2<T>::t* __restrict__ amps, uint32_t n, uint64_t ncirc, double* __restrict__ tree) {
-    const uint64_t half = 1ull << (n - 1), per = 1ull << n;
-    const uint64_t total = ncirc * half;
-    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t c = w >> (n - 1), j = w & (half - 1);
-        const typename C2<T>::t* a = amps + c * per;
-        tree[c * per + (half - 1) + j] = __dadd_rn(pr<T>(a, j), pr<T>(a, j + half));
-    }
-}
-
-__global__ void k_bfold(double* __restrict__ tree, uint32_t n, uint64_t ncirc, uint32_t k) {
-    const uint64_t len = 1ull << k, per = 1ull << n;
-    const uint64_t total = ncirc * len;
-    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t c = w >> k, j = w & (len - 1);
-        double* t = tree + c * per;
-        const double* up = t + ((1ull << (k + 1)) - 1);
-        t[(len - 1) + j] = __dadd_rn(up[j], up[j + len]);
-    }
-}
+// Prefix trees (rq_tree.cuh) over the kept half of each state (n = its index bits, one less than the
+// qubits; tree of circuit c at tree + c * 2^n).
 
 // one block per circuit: shots, cut of each, best (max cut, lowest shot).  A shot measures the n + 1
 // qubits in order; p(x) = p(~x), so the mass of a prefix j of L bits is level L at j plus level L at ~j.
 template <typename T>
-__global__ void k_bsample(const typename C2<T>::t* __restrict__ amps, const double* __restrict__ tree, uint32_t n,
+__global__ void __launch_bounds__(1024) k_bsample(const typename C2<T>::t* __restrict__ amps, const double* __restrict__ tree, uint32_t n,
                           uint64_t ncirc, uint64_t circ0, const uint32_t* __restrict__ circ_inst,
                           const uint64_t* __restrict__ user_of,
                           const uint8_t* __restrict__ edges_all, const uint32_t* __restrict__ eoff,
@@ -867,11 +839,11 @@ __global__ void k_bsample(const typename C2<T>::t* __restrict__ amps, const doub
                 double m0, m1;
                 const uint64_t mask = (1ull << (q + 1)) - 1, one = prefix | (1ull << q);
                 if (q == n) {
-                    m0 = pr<T>(a, prefix);
-                    m1 = pr<T>(a, one ^ mask);
+                    m0 = rqt::prob_at<T>(a, prefix);
+                    m1 = rqt::prob_at<T>(a, one ^ mask);
                 } else if (q + 1 == n) {
-                    m0 = __dadd_rn(pr<T>(a, prefix), pr<T>(a, prefix ^ mask));
-                    m1 = __dadd_rn(pr<T>(a, one), pr<T>(a, one ^ mask));
+                    m0 = __dadd_rn(rqt::prob_at<T>(a, prefix), rqt::prob_at<T>(a, prefix ^ mask));
+                    m1 = __dadd_rn(rqt::prob_at<T>(a, one), rqt::prob_at<T>(a, one ^ mask));
                 } else {
                     const double* L = t + mask;
                     m0 = __dadd_rn(L[prefix], L[prefix ^ mask]);
@@ -1570,17 +1542,18 @@ int sample_class(rq_qaoa_batch* b, QClass& K, uint64_t ncirc, uint64_t circ0, vo
     uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(ncirc, tree_budget / (per * sizeof(double))));
     RQ_TRY(grow(&b->d_tree, &b->tree_cap, chunk * per));
     const int sms = rq::num_sms(b->device);
+    rqt::Perm P{};
+    P.n = n;
+    P.identity = 1;
     for (uint64_t c0 = 0; c0 < ncirc; c0 += chunk) {
         const uint64_t cn = std::min<uint64_t>(chunk, ncirc - c0);
         const V* a = (const V*)states + c0 * per;
-        k_bleaf<T><<<rq::grid_for(cn * (per >> 1), TPB, sms), TPB, 0, b->stream>>>(a, n, cn, b->d_tree);
-        RQ_CUDA(cudaGetLastError());
-        for (int k = (int)n - 2; k >= 0; --k) {
-            k_bfold<<<rq::grid_for(cn << k, TPB, sms), TPB, 0, b->stream>>>(b->d_tree, n, cn, (uint32_t)k);
-            RQ_CUDA(cudaGetLastError());
-        }
+        RQ_TRY(rqt::build_trees<T>(a, P, cn, b->d_tree, sms, b->stream));
         const unsigned g = (unsigned)std::min<uint64_t>(cn, (uint64_t)sms * 8);
-        k_bsample<T><<<g, 256, 0, b->stream>>>(a, b->d_tree, n, cn, circ0 + c0, b->d_circ_inst, b->d_user, b->d_edges, b->d_eoff,
+        // a thread per shot up to 1024: a walk is a chain of n dependent loads, so 1024 shots in four
+        // rounds of 256 threads took 45 us on a 22-node class where one round takes 24 us
+        const unsigned threads = std::min<unsigned>(1024, (shots + 31) / 32 * 32);
+        k_bsample<T><<<g, threads, 0, b->stream>>>(a, b->d_tree, n, cn, circ0 + c0, b->d_circ_inst, b->d_user, b->d_edges, b->d_eoff,
                                                b->d_ne, shots, seed, b->d_best_bits, b->d_best_cut);
         RQ_CUDA(cudaGetLastError());
     }

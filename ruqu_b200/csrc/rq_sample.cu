@@ -9,71 +9,24 @@
 // sequential conditional sampling.  FP64 throughout, sums without FMA so a
 // host fold of the same probability vector gives identical bits.
 #include "rq_internal.cuh"
+#include "rq_tree.cuh"
 
 #include <vector>
 
 namespace {
 
 using rqd::C2;
+using rqt::Perm;
+using rqt::prob_at;
+using rqt::unpermute;
 
 constexpr int TPB = 256;
 constexpr int MAXQ = 64;
-
-struct Perm {
-    uint8_t order[MAXQ];   // permuted bit position -> qubit
-    uint8_t pos[MAXQ];     // qubit -> permuted bit position
-    uint32_t n;
-    int identity;
-};
 
 struct Plan {
     uint8_t qubits[MAXQ];  // measurement order (may repeat)
     uint32_t m;
 };
-
-__device__ __forceinline__ uint64_t unpermute(uint64_t j, const Perm& P) {
-    if (P.identity) return j;
-    uint64_t i = 0;
-    for (uint32_t b = 0; b < P.n; ++b) i |= ((j >> b) & 1ull) << P.order[b];
-    return i;
-}
-
-template <typename T>
-__device__ __forceinline__ double prob_at(const typename C2<T>::t* a, uint64_t i) {
-    auto x = a[i];
-    double re = x.x, im = x.y;
-    return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
-}
-
-// level n-1 of the tree straight from the amplitudes
-template <typename T>
-__global__ void k_leaf_fold(const typename C2<T>::t* __restrict__ a, Perm P, double* __restrict__ lvl) {
-    const uint64_t half = 1ull << (P.n - 1);
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < half;
-         j += (uint64_t)gridDim.x * blockDim.x) {
-        double p0 = prob_at<T>(a, unpermute(j, P));
-        double p1 = prob_at<T>(a, unpermute(j + half, P));
-        lvl[j] = __dadd_rn(p0, p1);
-    }
-}
-
-// level k from level k+1 (both 2^k / 2^(k+1) long)
-__global__ void k_fold(const double* __restrict__ up, double* __restrict__ dn, uint64_t len) {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < len;
-         j += (uint64_t)gridDim.x * blockDim.x)
-        dn[j] = __dadd_rn(up[j], up[j + len]);
-}
-
-// all levels from `top` down to 0 in one block (top level has <= 2^12 entries)
-__global__ void k_fold_tail(double* __restrict__ tree, int top) {
-    for (int k = top - 1; k >= 0; --k) {
-        const double* up = tree + ((1ull << (k + 1)) - 1);
-        double* dn = tree + ((1ull << k) - 1);
-        uint64_t len = 1ull << k;
-        for (uint64_t j = threadIdx.x; j < len; j += blockDim.x) dn[j] = __dadd_rn(up[j], up[j + len]);
-        __syncthreads();
-    }
-}
 
 template <typename T>
 __global__ void k_sample(const typename C2<T>::t* __restrict__ a, const double* __restrict__ tree, Perm P,
@@ -165,25 +118,9 @@ int build_tree(rq_state* s, const Perm& P) {
     const uint32_t n = s->nq;
     s->tree_ready = false;
     RQ_TRY(ensure_tree(s, (size_t)1 << n));
-    int sms = num_sms(s->device);
-    double* top = s->tree + ((1ull << (n - 1)) - 1);
-    uint64_t half = 1ull << (n - 1);
-    unsigned g = grid_for(half, TPB, sms);
-    if (s->prec == RQ_F32) k_leaf_fold<float><<<g, TPB, 0, s->stream>>>((const float2*)s->amps, P, top);
-    else k_leaf_fold<double><<<g, TPB, 0, s->stream>>>((const double2*)s->amps, P, top);
-    RQ_CUDA(cudaGetLastError());
-    int k = (int)n - 2;
-    for (; k >= 0 && (1ull << (k + 1)) > 4096; --k) {
-        double* up = s->tree + ((1ull << (k + 1)) - 1);
-        double* dn = s->tree + ((1ull << k) - 1);
-        uint64_t len = 1ull << k;
-        k_fold<<<grid_for(len, TPB, sms), TPB, 0, s->stream>>>(up, dn, len);
-        RQ_CUDA(cudaGetLastError());
-    }
-    if (k >= 0) {
-        k_fold_tail<<<1, 1024, 0, s->stream>>>(s->tree, k + 1);
-        RQ_CUDA(cudaGetLastError());
-    }
+    const int sms = num_sms(s->device);
+    if (s->prec == RQ_F32) RQ_TRY(rqt::build_trees<float>((const float2*)s->amps, P, 1, s->tree, sms, s->stream));
+    else RQ_TRY(rqt::build_trees<double>((const double2*)s->amps, P, 1, s->tree, sms, s->stream));
     for (uint32_t b = 0; b < n; ++b) s->tree_order[b] = P.order[b];
     s->tree_ready = true;
     return RQ_OK;
