@@ -138,6 +138,13 @@ __device__ __forceinline__ void run_phases(typename C2<T>::t* sm, const SweepDes
 #pragma unroll
         for (int i = 0; i < NR; ++i) reg[i] = sm[sb ^ ph.slut[i]];
 
+        // f64: a diagonal on thread or tile bits is one factor for all of a thread's amplitudes, collected
+        // here and applied once at the end of the phase (QAOA of 22 qubits 1136 -> 1087 us; in f32 the extra
+        // registers cost more than the arithmetic)
+        V scal;
+        scal.x = (T)1;
+        scal.y = (T)0;
+        bool scaled = false;
         for (uint32_t o = ph.op_begin; o < ph.op_end; ++o) {
             const SwOp op = ops[o];
             const T* mm = mats + 2 * op.mat;
@@ -148,6 +155,11 @@ __device__ __forceinline__ void run_phases(typename C2<T>::t* sm, const SweepDes
                     const T d0r = mm[0], d0i = mm[1], d1r = mm[2], d1i = mm[3];
                     const int kk = op.k0;
                     const int ub = (int)((U >> op.q0) & 1ull);
+                    if (sizeof(T) == 8 && kk < 0) {
+                        scal = cmul(scal, ub ? d1r : d0r, ub ? d1i : d0i);
+                        scaled = true;
+                        break;
+                    }
 #pragma unroll
                     for (int i = 0; i < NR; ++i) {
                         const int b = kk >= 0 ? ((i >> kk) & 1) : ub;
@@ -174,6 +186,11 @@ __device__ __forceinline__ void run_phases(typename C2<T>::t* sm, const SweepDes
                     const T er = mm[0], ei = mm[1], pr = mm[2], pi = mm[3];
                     const int k0 = op.k0, k1 = op.k1;
                     const int u0 = (int)((U >> op.q0) & 1ull), u1 = (int)((U >> op.q1) & 1ull);
+                    if (sizeof(T) == 8 && k0 < 0 && k1 < 0) {
+                        scal = cmul(scal, u0 != u1 ? pr : er, u0 != u1 ? pi : ei);
+                        scaled = true;
+                        break;
+                    }
 #pragma unroll
                     for (int i = 0; i < NR; ++i) {
                         const int b0 = k0 >= 0 ? ((i >> k0) & 1) : u0;
@@ -185,6 +202,10 @@ __device__ __forceinline__ void run_phases(typename C2<T>::t* sm, const SweepDes
                 }
                 default: break;
             }
+        }
+        if (sizeof(T) == 8 && scaled) {
+#pragma unroll
+            for (int i = 0; i < NR; ++i) reg[i] = cmul(reg[i], scal.x, scal.y);
         }
 #pragma unroll
         for (int i = 0; i < NR; ++i) sm[sb ^ ph.slut[i]] = reg[i];
@@ -290,10 +311,11 @@ __device__ __forceinline__ void run_phases_v1(typename C2<T>::t* sm, const Sweep
     }
 }
 
-template <typename T, int RB, bool PV>
+template <typename T, int RB, bool PV, bool STAGE>
 __global__ void __launch_bounds__(256, 2) k_sweep(typename C2<T>::t* __restrict__ amps, const SweepDesc d,
                                                const PhaseDesc* __restrict__ phases, const SwOp* __restrict__ ops,
-                                               const T* __restrict__ mats, uint64_t ntiles) {
+                                               const T* __restrict__ mats, uint64_t ntiles, uint32_t nops, uint32_t mat0,
+                                               uint32_t nmats) {
     using V = typename C2<T>::t;
     using VV = typename Vec16<T>::t;
     constexpr int NR = 1 << RB;
@@ -303,6 +325,23 @@ __global__ void __launch_bounds__(256, 2) k_sweep(typename C2<T>::t* __restrict_
     V* sm = reinterpret_cast<V*>(smem_raw);
 
     const uint32_t tid = threadIdx.x;
+    // STAGE: the sweep's phases, ops and matrices in shared memory after the tile; an op's record and then
+    // its matrix were dependent loads past the L1 for every warp (12 qubits f64, one tile: 215 -> 156 us;
+    // 24 qubits: 8521 -> 8218)
+    PhaseDesc* sph = reinterpret_cast<PhaseDesc*>(smem_raw + (sizeof(V) << d.m));
+    SwOp* sops = reinterpret_cast<SwOp*>(sph + (d.phase_end - d.phase_begin));
+    T* smats = reinterpret_cast<T*>(sops + nops);
+    if (STAGE) {
+        const uint32_t op0 = phases[d.phase_begin].op_begin;
+        const uint32_t nw = (d.phase_end - d.phase_begin) * (uint32_t)(sizeof(PhaseDesc) / 16);
+        for (uint32_t k = tid; k < nw; k += blockDim.x)
+            reinterpret_cast<uint4*>(sph)[k] = reinterpret_cast<const uint4*>(phases + d.phase_begin)[k];
+        for (uint32_t k = tid; k < nops; k += blockDim.x) sops[k] = ops[op0 + k];
+        for (uint32_t k = tid; k < 2 * nmats; k += blockDim.x) smats[k] = mats[2 * mat0 + k];
+        sops -= op0;
+        smats -= 2 * mat0;
+        sph -= d.phase_begin;
+    }
     const uint64_t cmask = (1ull << d.c) - 1;
 
     // deposit of this thread's vector offset (local bits of EPV*tid) into global positions
@@ -342,6 +381,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep(typename C2<T>::t* __restrict_
 
         // ---- phases ----
         if (PV) run_phases_v1<T, RB>(sm, d, phases, ops, mats, base, tid);
+        else if (STAGE) run_phases<T, RB>(sm, d, sph, sops, smats, base, tid);
         else run_phases<T, RB>(sm, d, phases, ops, mats, base, tid);
 
         // ---- store tile ----
@@ -1311,7 +1351,7 @@ static bool phase_v1() {
 
 template <typename T>
 int launch_sweep(rq_state* s, const SweepDesc& d, const PhaseDesc* ph, const SwOp* ops, const void* mats,
-                 uint64_t ntiles, uint32_t rb, size_t smem) {
+                 uint64_t ntiles, uint32_t rb, size_t smem, uint32_t nops, uint32_t mat0, uint32_t nmats) {
     using V = typename C2<T>::t;
     unsigned threads = 1u << (d.m - rb);
     int sms = rq::num_sms(s->device);
@@ -1329,15 +1369,21 @@ int launch_sweep(rq_state* s, const SweepDesc& d, const PhaseDesc* ph, const SwO
             return RQ_OK;
         }
     }
-    auto kern = phase_v1() ? k_sweep<T, std::is_same<T, float>::value ? 5 : 4, true>
-                           : k_sweep<T, std::is_same<T, float>::value ? 5 : 4, false>;
+    constexpr int RBc = std::is_same<T, float>::value ? 5 : 4;
+    const size_t tables = (d.phase_end - d.phase_begin) * sizeof(PhaseDesc) + nops * sizeof(SwOp) + 2 * (size_t)nmats * sizeof(T);
+    // staged where as many CTAs still fit on an SM: those that 128 registers a thread allow, one where
+    // there are no more tiles than SMs
+    const size_t ctas = ntiles <= (uint64_t)sms ? 1 : 512 / threads;
+    const bool stage = !phase_v1() && ctas * (smem + tables + 1024) <= 228 * 1024;
+    auto kern = phase_v1() ? k_sweep<T, RBc, true, false> : stage ? k_sweep<T, RBc, false, true> : k_sweep<T, RBc, false, false>;
+    if (stage) smem += tables;
     RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // persistent grid: exactly the CTAs that can be resident at once
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
     if (per_sm < 1) return rq::fail(RQ_ERR_CUDA, "sweep kernel does not fit on an SM");
     unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)sms * per_sm);
-    kern<<<grid, threads, smem, s->stream>>>((V*)s->amps, d, ph, ops, (const T*)mats, ntiles);
+    kern<<<grid, threads, smem, s->stream>>>((V*)s->amps, d, ph, ops, (const T*)mats, ntiles, nops, mat0, nmats);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -1357,6 +1403,10 @@ struct rq_plan {
     size_t off_ph = 0, off_ops = 0, off_mat = 0, off_img = 0;
     int tc_passes = 0;                   // > 0: tensor-core sweeps (3 = 3xTF32, 1 = TF32)
     std::vector<PhaseDesc> host_phases;  // tensor-core sweeps: descriptor sizes per launch
+    struct SweepTables {
+        uint32_t nops, mat0, nmats;      // ops, first matrix entry and entries (complex) of a sweep
+    };
+    std::vector<SweepTables> sweep_tables;   // CUDA-core sweeps
     uint64_t ntiles = 0;
     size_t smem = 0;
     uint32_t rb = 0;
@@ -1391,6 +1441,19 @@ static uint32_t sweep_local_qubits(uint32_t nq, int32_t prec) {
         uint32_t cap = prec == RQ_F32 ? 14 : 13;
         if (v >= 8 && (uint32_t)v <= cap) m = (uint32_t)v;
     }
+    return std::min(nq, m);
+}
+
+// Local qubits of the CUDA-core sweeps when the caller names none.  f64: 11 (128-thread CTAs, four an
+// SM), which measured 13-25 % less than 12 on random layers, QAOA and VQE circuits of 12-18 and from 22
+// qubits on: below 19 the smaller tiles reach more SMs (a 16-qubit state has 16 tiles of 2^12; random
+// layers 247 -> 201 us), above 21 four small CTAs overlap each other's loads and barriers better than
+// two (22 qubits: 2102 -> 1856 us).  At 19-21 qubits 12 is as fast or up to 9 % faster (fewer sweeps,
+// and its tiles fill the machine once).  f32: 12 up to 19 qubits (16 qubits: 279 -> 222 us), 13 above (20
+// qubits: 369 against 378 us).
+static uint32_t core_local_qubits(uint32_t nq, int32_t prec) {
+    if (std::getenv("RUQU_SWEEP_LOCAL_QUBITS")) return sweep_local_qubits(nq, prec);
+    const uint32_t m = prec == RQ_F32 ? (nq <= 19 ? 12 : 13) : (nq >= 19 && nq <= 21 ? 12 : 11);
     return std::min(nq, m);
 }
 
@@ -1489,6 +1552,7 @@ int plan_build(const rq_state* s, const rq_gate* gates, uint64_t n, int32_t mode
     // (other 14-qubit requests take 13)
     if (m == 14 && tc_passes != TC_F16) m = 13;
     if (s->prec != RQ_F32 || (m != 12 && m != 13 && !(m == 14 && tc_passes == TC_F16))) tc_passes = 0;
+    if (tc_passes == 0 && !m_override) m = core_local_qubits(nq, s->prec);
     const uint32_t c = std::min<uint32_t>(m, 5);
     std::vector<PGate> pg;
     std::vector<rq_gate> filtered;
@@ -1578,7 +1642,15 @@ int plan_build(const rq_state* s, const rq_gate* gates, uint64_t n, int32_t mode
         return rc;
     }
     P->smem = ((size_t)1 << m) * s->elem_bytes();
-    if (tcp) P->host_phases = phases;
+    if (tcp) {
+        P->host_phases = phases;
+    } else {
+        for (const auto& d : P->descs) {
+            const uint32_t o0 = phases[d.phase_begin].op_begin, o1 = phases[d.phase_end - 1].op_end;
+            const uint32_t end = o1 < ops.size() ? ops[o1].mat : (uint32_t)(mats.size() / 2);
+            P->sweep_tables.push_back({o1 - o0, ops[o0].mat, end - ops[o0].mat});
+        }
+    }
     P->ntiles = 1ull << (nq - m);
     P->rb = rb;
     P->rebindable = true;
@@ -1902,9 +1974,11 @@ static int plan_launch_kernels(rq_state* s, const rq_plan* P) {
         }
         return RQ_OK;
     }
-    for (const auto& d : P->descs) {
-        if (s->prec == RQ_F32) RQ_TRY(launch_sweep<float>(s, d, ph, op, mt, P->ntiles, P->rb, P->smem));
-        else RQ_TRY(launch_sweep<double>(s, d, ph, op, mt, P->ntiles, P->rb, P->smem));
+    for (size_t k = 0; k < P->descs.size(); ++k) {
+        const SweepDesc& d = P->descs[k];
+        const auto& t = P->sweep_tables[k];
+        if (s->prec == RQ_F32) RQ_TRY(launch_sweep<float>(s, d, ph, op, mt, P->ntiles, P->rb, P->smem, t.nops, t.mat0, t.nmats));
+        else RQ_TRY(launch_sweep<double>(s, d, ph, op, mt, P->ntiles, P->rb, P->smem, t.nops, t.mat0, t.nmats));
     }
     return RQ_OK;
 }
