@@ -216,3 +216,25 @@ def test_states_energies_and_gradients_at_tile_edges(prec, sizes):
             dn[j] -= 1e-5
             want = (oracle.qaoa_cost(n, ew, up[:p], up[p:]) - oracle.qaoa_cost(n, ew, dn[:p], dn[p:])) / 2e-5
             assert abs(grad[0, j] - want) < (1e-7 if prec == "f64" else 2e-4) * max(1, len(e)), (n, j)
+
+
+@pytest.mark.parametrize("prec,n,layers", [("f32", 14, 40), ("f32", 14, 64), ("f32", 15, 64), ("f64", 13, 40),
+                                           ("f64", 13, 64)])
+def test_many_layers_with_tables_in_and_out_of_shared_memory(prec, n, layers):
+    """Layers of angle 0 are exact identities, so a deep batch equals the two-layer one up to the order
+    of each thread's 32 (sweep) or 16 (adjoint) terms, whose sum of magnitudes is at most |E| for the energy
+    and 4 |E|^2 for a gradient; the depths lie on both sides of what fits beside a tile."""
+    edges = workloads.random_3regular_graph(n - n % 2, rng.Stream(3, n))
+    ne, eps = len(edges), 2.0 ** (-24 if prec == "f32" else -53)
+    r = np.random.default_rng(layers)
+    gam, bet = np.zeros((3, layers)), np.zeros((3, layers))
+    gam[:, :2], bet[:, :2] = r.uniform(-1, 1, size=(3, 2)), r.uniform(-1, 1, size=(3, 2))
+    graphs = [(n, edges)] * 3
+    want, wgrad = QaoaBatch(graphs, 2, prec).gradient(gam[:, :2], bet[:, :2])
+    qb = QaoaBatch(graphs, layers, prec)
+    got, grad = qb.gradient(gam, bet)
+    assert np.max(np.abs(got - want)) <= 2 * 32 * eps * ne
+    assert np.array_equal(got, qb.run(gam, bet)["energies"])
+    tol = 2 * 16 * eps * 4 * ne * ne
+    assert np.max(np.abs(grad[:, :2] - wgrad[:, :2])) <= tol
+    assert np.max(np.abs(grad[:, layers:layers + 2] - wgrad[:, 2:])) <= tol

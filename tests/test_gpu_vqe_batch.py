@@ -139,3 +139,20 @@ def test_vqe_batch_non_finite_inputs_stay_non_finite():
     p[1, 3] = np.nan
     e = VqeBatch(7, 2, [1.0], [[(1, 2)]], "f32").run(p)
     assert e[0] == 0.0 and np.isnan(e[1])
+
+
+@pytest.mark.parametrize("prec,n,depth", [("f32", 14, 42), ("f32", 14, 102), ("f64", 13, 42), ("f64", 13, 82)])
+def test_many_layers_with_tables_in_and_out_of_shared_memory(prec, n, depth):
+    """Two layers of angle 0 are two CZ ladders, an exact identity, so a deep batch equals the two-layer
+    one up to the order of the sums (f64 1e-12; f32: 32 terms a thread of at most sum |c| in all); the
+    depths lie on both sides of what fits beside a tile."""
+    coeffs, strings = workloads.pauli_hamiltonian(n, 20, 7)
+    params = np.zeros((2, n * depth))
+    params[:, :2 * n] = np.random.default_rng(n).uniform(-math.pi, math.pi, size=(2, 2 * n))
+    want, wgrad = VqeBatch(n, 2, coeffs, strings, prec).run(params[:, :2 * n], gradient="adjoint")
+    vb = VqeBatch(n, depth, coeffs, strings, prec)
+    tol = (1e-12 if prec == "f64" else 2 * 32 * 2.0 ** -24) * float(np.sum(np.abs(coeffs)))
+    assert np.max(np.abs(vb.run(params) - want)) <= tol
+    if n * depth <= 600:   # the adjoint kernel refuses the deeper ones
+        _, grad = vb.run(params, gradient="adjoint")
+        assert np.max(np.abs(grad[:, :2 * n] - wgrad)) <= tol
