@@ -34,6 +34,7 @@ struct rq_state {
     size_t amps_cap = 0;          // bytes allocated for amps
     bool exported = false;        // the device pointer was handed out: its memory is never reused
     bool tc_ran = false;          // a tensor-core sweep was launched since the last check of its waits
+    bool tc_captured = false;     // one was captured in a graph, whose replays the host does not see
     int32_t exec_mode = RQ_EXEC_AUTO;
     size_t elem_bytes() const { return prec == RQ_F32 ? 8 : 16; }
     size_t bytes() const { return (size_t)n * elem_bytes(); }

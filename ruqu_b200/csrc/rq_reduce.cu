@@ -610,7 +610,7 @@ int inner(rq_state* a, rq_state* b, double* re, double* im) {
     unsigned G = reduction_grid(a);
     RQ_TRY(ensure_partials(a, 2 * (size_t)G + 8));
     // b's pending work must be done before a's stream reads it
-    RQ_CUDA(cudaStreamSynchronize(b->stream));
+    RQ_TRY(sync_checked(b));
     if (a->prec == RQ_F32 && b->prec == RQ_F32)
         k_inner<float, float><<<G, TPB, 0, a->stream>>>((const float2*)a->amps, (const float2*)b->amps, a->n, a->partials, G);
     else if (a->prec == RQ_F32)

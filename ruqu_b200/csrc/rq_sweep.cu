@@ -1923,7 +1923,12 @@ static int plan_launch_kernels(rq_state* s, const rq_plan* P);
 // Launch a prepared plan on s's stream; the plan remembers the stream and an event after the
 // launches, so that new matrix tables (plan_rebind) are written only once they have run.
 int plan_launch(rq_state* s, const rq_plan* P) {
-    if (P->mode != RQ_EXEC_PER_GATE && P->tc_passes > 0) s->tc_ran = true;
+    if (P->mode != RQ_EXEC_PER_GATE && P->tc_passes > 0) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        RQ_CUDA(cudaStreamIsCapturing(s->stream, &capture));
+        s->tc_ran = true;
+        if (capture != cudaStreamCaptureStatusNone) s->tc_captured = true;
+    }
     // the plan's last use (launches or new tables) on another stream comes first
     if (P->done && P->done_stream != s->stream) RQ_CUDA(cudaStreamWaitEvent(s->stream, P->done, 0));
     RQ_TRY(plan_launch_kernels(s, P));
@@ -2012,7 +2017,8 @@ int tc_timeout_flag(int* out) {
 
 int sync_checked(rq_state* s) {
     RQ_CUDA(cudaStreamSynchronize(s->stream));
-    if (!s->tc_ran) return RQ_OK;   // nothing on this state waited on the tensor cores: no flag to fetch (27 us)
+    // nothing on this state waited on the tensor cores: no flag to fetch (27 us)
+    if (!s->tc_ran && !s->tc_captured) return RQ_OK;
     s->tc_ran = false;
     int to = 0;
     RQ_TRY(tc_timeout_flag(&to));

@@ -53,6 +53,47 @@ def test_sweep_wait_expiry_reports_timeout_and_state_recovers(mode, lq):
     assert float(np.max(np.abs(st.state_vector() - ref.amplitudes()))) < 1e-5
 
 
+def test_wait_expiry_reaches_the_other_reader_and_every_replay():
+    """An expiry is reported by a fidelity whose second state it hit, and by each read-back after a
+    replay of a graph that captured the plan, also when an earlier read-back found nothing."""
+    import torch
+    n = 15
+    a, st = rq.QuantumState(n, 0, "f32"), rq.QuantumState(n, 0, "f32")
+    plan = rq.Plan(st, workloads.random_layer_circuit(n, 4, 7), rq.RQ_EXEC_SWEEP_TC16)
+    plan.execute(st)
+    st.synchronize()
+    stream = torch.cuda.ExternalStream(st.device_pointer()[1])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        assert _capi.lib.rq_plan_execute(st.handle, plan._h) == _capi.RQ_OK
+    assert _capi.lib.rq_state_synchronize(st.handle) == _capi.RQ_OK
+
+    def expire(launch, read):
+        assert _capi.lib.rq_debug_set_wait_limit(0) == 0
+        try:
+            launch()
+            rc = read()
+        finally:
+            assert _capi.lib.rq_debug_set_wait_limit(DEFAULT) == 0
+        assert rc == _capi.RQ_ERR_TIMEOUT, (rc, _capi.last_error())
+
+    def replay():
+        with torch.cuda.stream(stream):
+            graph.replay()
+
+    out = C.c_double()
+    for _ in range(2):
+        expire(replay, lambda: _capi.lib.rq_state_synchronize(st.handle))
+        assert _capi.lib.rq_state_synchronize(st.handle) == _capi.RQ_OK
+    b = rq.QuantumState(n, 0, "f32")
+    plan_b = rq.Plan(b, workloads.random_layer_circuit(n, 4, 7), rq.RQ_EXEC_SWEEP_TC16)
+    b.synchronize()
+    expire(lambda: _capi.lib.rq_plan_execute(b.handle, plan_b._h),
+           lambda: _capi.lib.rq_state_fidelity(a.handle, b.handle, C.byref(out)))
+    assert _capi.lib.rq_state_synchronize(b.handle) == _capi.RQ_OK
+    del graph
+
+
 def test_gemm_wait_expiry_reports_timeout_and_recovers():
     M, N, K = 128, 64, 128
     r = np.random.default_rng(1)
