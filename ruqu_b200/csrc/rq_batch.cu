@@ -1467,6 +1467,29 @@ TableBytes table_bytes(const std::vector<SweepDesc>& descs, const std::vector<Ph
     return t;
 }
 
+// The sweeps of a QAOA class, with tiles of 2^mloc elements or of half as many; returns the local qubits.
+// A sweep costs passes over the states, so the fewer sweeps win; at the same number the smaller tiles do,
+// whose twice as many CTAs wait less at the barriers between the phases: p = 4, f32, tiles of 2^13 against
+// 2^12, gradients 443 -> 407 us (128 graphs of 15 vertices), 448 -> 420 (64 of 16), 4114 -> 3814 (8 of
+// 22), energies 163 -> 163, 162 -> 159, 1068 -> 995; f64, 2^12 against 2^11, energies 232 -> 219 us (256
+// of 14), 541 -> 486 (8 of 20).  With a sweep more they lose: 329 -> 381 (256 of 14, gradients), 277 -> 319
+// (8 of 20).
+uint32_t plan_symmetric(const std::vector<PGate>& gates, uint32_t n, uint32_t mloc, uint32_t rb, int32_t prec,
+                        std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
+    const uint32_t epv = prec == RQ_F32 ? 2 : 1, m = std::min(n - 1, mloc);
+    symmetric_program(gates, n, m, rb, epv, descs, phases, ops);
+    if (n - 1 < mloc) return m;
+    std::vector<SweepDesc> d;
+    std::vector<PhaseDesc> ph;
+    std::vector<SwOp> o;
+    symmetric_program(gates, n, m - 1, rb, epv, d, ph, o);
+    if (d.size() > descs.size()) return m;
+    descs.swap(d);
+    phases.swap(ph);
+    ops.swap(o);
+    return m - 1;
+}
+
 // Shared memory of a sweep launch: what it needs, or that with its tables (`staged` bytes) where as many
 // CTAs still fit on an SM (228 KB, 1 KB of it per CTA, at most most_per_sm): a CTA less costs half of the
 // warps, the tables give 2 to 5 %.
@@ -1698,9 +1721,6 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
         QClass K;
         K.n = kv.first;
         K.insts = kv.second;
-        K.m = std::min(K.n - 1, mloc);
-        K.ntiles = 1ull << (K.n - 1 - K.m);
-        K.smem = ((size_t)1 << K.m) * elem_size(precision);
         // the circuit of qaoa.rs:125-153 after H^n: per layer the cost phase, then Rx on every qubit
         std::vector<PGate> g;
         for (uint32_t l = 0; l < p; ++l) {
@@ -1721,7 +1741,9 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
         }
         std::vector<PhaseDesc> phases;
         std::vector<SwOp> ops;
-        symmetric_program(g, K.n, K.m, rb, precision == RQ_F32 ? 2 : 1, K.descs, phases, ops);
+        K.m = plan_symmetric(g, K.n, mloc, rb, precision, K.descs, phases, ops);
+        K.ntiles = 1ull << (K.n - 1 - K.m);
+        K.smem = ((size_t)1 << K.m) * elem_size(precision);
         if (precision == RQ_F32) retable_f16(K.descs, phases, rb);   // the conflict-free layout (k_batch_sweep<float>)
         K.tables = table_bytes(K.descs, phases);
         K.descs.front().flags |= SWEEP_INIT_UNIFORM;
@@ -1736,8 +1758,6 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
         {
             // adjoint: per layer in reverse, Rx^-1 on every qubit, then the inverse cost phase
             const uint32_t arb = precision == RQ_F32 ? 4 : 3;
-            K.am = std::min(K.n - 1, mloc);
-            K.antiles = 1ull << (K.n - 1 - K.am);
             std::vector<PGate> ga;
             for (uint32_t l = p; l-- > 0;) {
                 for (uint32_t q = 0; q < K.n; ++q) {
@@ -1755,7 +1775,8 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
             }
             std::vector<PhaseDesc> aph;
             std::vector<SwOp> aops;
-            symmetric_program(ga, K.n, K.am, arb, precision == RQ_F32 ? 2 : 1, K.adescs, aph, aops);
+            K.am = plan_symmetric(ga, K.n, mloc, arb, precision, K.adescs, aph, aops);
+            K.antiles = 1ull << (K.n - 1 - K.am);
             K.atables = table_bytes(K.adescs, aph);
             K.adescs.front().flags |= SWEEP_INIT_LAMBDA;
             K.aoff_ops = (aph.size() * sizeof(PhaseDesc) + 255) & ~size_t(255);
