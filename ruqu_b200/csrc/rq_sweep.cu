@@ -974,6 +974,23 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return r;
 }
 
+// x - h, exact (h = x rounded to FP16): one mixed-precision fma.rn.f32.f16 a component, where converting
+// h back to FP32 first and subtracting took three instructions for the two
+__device__ __forceinline__ float2 residual(float2 x, uint32_t h) {
+    float2 r;
+    asm("{.reg .b16 lo, hi, m;\n\tmov.b32 {lo, hi}, %2;\n\tmov.b16 m, 0xBC00;\n\t"
+        "fma.rn.f32.f16 %0, lo, m, %3;\n\tfma.rn.f32.f16 %1, hi, m, %4;}"
+        : "=f"(r.x), "=f"(r.y) : "r"(h), "f"(x.x), "f"(x.y));
+    return r;
+}
+
+// keeps the uses of registers that a tcgen05.ld fills behind the wait that precedes this
+template <int N>
+__device__ __forceinline__ void landed(float2* r) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) asm volatile("" : "+f"(r[i].x), "+f"(r[i].y));
+}
+
 // bounded wait that lets the thread sleep until the phase completes (or 20 us pass) between
 // polls, so waiting warps take no issue slots from the working ones
 __device__ __forceinline__ bool wait_sleep(uint64_t* bar, uint32_t parity, uint32_t polls) {
@@ -1000,6 +1017,13 @@ __device__ __forceinline__ bool wait_sleep(uint64_t* bar, uint32_t parity, uint3
 // the chain's latency than the earlier image copy does); NTHR = 256: 13 local qubits, two
 // CTAs per SM; NTHR = 512: 14 local qubits, one CTA (four 128-row halves, all 512
 // tensor-memory columns) per SM.  NTHR = 256 and 512 double-buffer the images.
+//
+// What bounds it: the chain of a phase (gather, split, MMAs, read back, scatter, barrier) on 16 warps an SM,
+// at 45 % of the issue slots, 48 % of the shared-memory bandwidth and the board's power limit; about 520
+// instructions of a warp a phase and 1280 a tile.  Reading the accumulator in two parts, the second landing
+// while the first is scattered, and the split's residual in mixed precision: 30 qubits, 20 random layers,
+// 94.5 -> 93.3 ms (12 local qubits), 92.5 -> 90.9 (13), 97.0 -> 95.9 (14); 27 qubits 9.77 -> 9.55, 10.40 ->
+// 10.25, 10.97 -> 10.85.  Two threads a row with 64 registers each (32 warps an SM) took 109 ms in all three.
 template <int NTHR>
 __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restrict__ amps, const SweepDesc d,
                                                      const PhaseDesc* __restrict__ phases,
@@ -1188,7 +1212,7 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
                     for (int j = 0; j < 16; ++j) {
                         const float2 x = reg[16 * c + j];
                         const __half2 h = __float22half2_rn(x);
-                        const __half2 l = __float22half2_rn(tc16::sub2(x, __half22float2(h)));
+                        const __half2 l = __float22half2_rn(tc16::residual(x, *reinterpret_cast<const uint32_t*>(&h)));
                         hw[j] = *reinterpret_cast<const uint32_t*>(&h);
                         lw[j] = *reinterpret_cast<const uint32_t*>(&l);
                     }
@@ -1244,10 +1268,26 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
                 const uint32_t taddr = tmem + lane_base + col_h;
                 tc::ld16(taddr, reg);
                 tc::ld16(taddr + 16, reg + 8);
-                tc::ld16(taddr + 32, reg + 16);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                tc16::landed<NR / 2>(reg);
+                tc::ld16(taddr + 32, reg + 16);   // in flight while the first half is scattered
                 tc::ld16(taddr + 48, reg + 24);
+                const float os = last ? last_scale : mid_scale;
+                const float2 os2 = make_float2(os, os);
+                uint32_t a = sb;
+#pragma unroll
+                for (int g = 0; g < NR / 2; ++g) {
+                    if (g) a ^= S[tc16::ctz5(g)];
+                    sm[a] = tc16::mul2(reg[g ^ (g >> 1)], os2);
+                }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                tc16::landed<NR / 2>(reg + NR / 2);
+#pragma unroll
+                for (int g = NR / 2; g < NR; ++g) {
+                    a ^= S[tc16::ctz5(g)];
+                    sm[a] = tc16::mul2(reg[g ^ (g >> 1)], os2);
+                }
                 if (last) {   // the tile's output norm^2, this thread's part (see the store)
                     float2 o2 = make_float2(0.f, 0.f);
 #pragma unroll
@@ -1256,14 +1296,6 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
 #pragma unroll
                     for (int k = 16; k > 0; k >>= 1) o += __shfl_xor_sync(0xFFFFFFFFu, o, k);
                     if ((tid & 31u) == 0) wsum2[warp] = o;
-                }
-                const float os = last ? last_scale : mid_scale;
-                const float2 os2 = make_float2(os, os);
-                uint32_t a = sb;
-#pragma unroll
-                for (int g = 0; g < NR; ++g) {
-                    if (g) a ^= S[tc16::ctz5(g)];
-                    sm[a] = tc16::mul2(reg[g ^ (g >> 1)], os2);
                 }
             }
             if (__syncthreads_or(failed)) {
