@@ -134,36 +134,6 @@ __device__ __forceinline__ V cmulv(V a, T br, T bi) {
     return r;
 }
 
-// Rx(2 beta) on slot K: [[c, -i s], [-i s, c]]
-template <int K, int NR, typename V, typename T>
-__device__ __forceinline__ void op_rx(V* reg, T c, T s) {
-#pragma unroll
-    for (int i = 0; i < NR; ++i) {
-        if (i & (1 << K)) continue;
-        const int j = i | (1 << K);
-        V x = reg[i], y = reg[j];
-        V o0, o1;
-        o0.x = c * x.x + s * y.y;
-        o0.y = c * x.y - s * y.x;
-        o1.x = s * x.y + c * y.x;
-        o1.y = c * y.y - s * x.x;
-        reg[i] = o0;
-        reg[j] = o1;
-    }
-}
-
-template <int NR, typename V, typename T>
-__device__ __forceinline__ void dispatch_rx(int k, V* reg, T c, T s) {
-    switch (k) {
-        case 0: op_rx<0, NR>(reg, c, s); break;
-        case 1: op_rx<1, NR>(reg, c, s); break;
-        case 2: op_rx<2, NR>(reg, c, s); break;
-        case 3: if constexpr (NR > 8) op_rx<3, NR>(reg, c, s); break;
-        case 4: if constexpr (NR > 16) op_rx<4, NR>(reg, c, s); break;
-        default: break;
-    }
-}
-
 // packed FP32x2 arithmetic: one instruction for both parts of a complex f32 value
 __device__ __forceinline__ float2 pk_mul(float2 a, float2 b) {
     float2 r;
@@ -178,6 +148,65 @@ __device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) {
         "mov.b64 rc, {%6, %7};\n\tfma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;}"
         : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return r;
+}
+
+// f32 QAOA sweeps hold register i with its parts exchanged when i has an odd number of set bits: Rx, which
+// adds real parts to imaginary ones, then acts on both parts alike and runs as packed instructions, four a
+// pair instead of eight, for two moves an odd register in and out of a phase.  With the gradients' overlaps
+// packed as well: QAOA energies of 192 graphs (12-22 vertices) 5244 -> 4964 us, gradients of 256 (12-20)
+// 6537 -> 6138 us; with QAOA and the ansatz as kernels of their own, VQE of 16 qubits: parameter shift
+// 5173 -> 5039 us, adjoint gradients 5253 -> 5103 us.
+template <bool RX, typename T>
+constexpr bool exchanges = RX && std::is_same<T, float>::value;
+
+__host__ __device__ constexpr bool odd_bits(int i) { return ((0x6996 >> (i & 15)) ^ (i >> 4)) & 1; }   // i < 32
+
+template <int NR, typename V>
+__device__ __forceinline__ void exchange_odd(V* reg) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+        if (odd_bits(i)) {
+            const auto x = reg[i].x;
+            reg[i].x = reg[i].y;
+            reg[i].y = x;
+        }
+}
+
+// Rx(2 beta) on slot K: [[c, -i s], [-i s, c]]
+template <int K, int NR, typename V, typename T>
+__device__ __forceinline__ void op_rx(V* reg, T c, T s) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        if (i & (1 << K)) continue;
+        const int j = i | (1 << K);
+        if constexpr (exchanges<true, T>) {
+            const int a = odd_bits(i) ? j : i, b = odd_bits(i) ? i : j;   // b: parts exchanged
+            const float2 c2 = make_float2(c, c), x = reg[a], y = reg[b];
+            reg[a] = pk_fma(c2, x, pk_mul(make_float2(s, -s), y));
+            reg[b] = pk_fma(c2, y, pk_mul(make_float2(-s, s), x));
+        } else {
+            V x = reg[i], y = reg[j];
+            V o0, o1;
+            o0.x = c * x.x + s * y.y;
+            o0.y = c * x.y - s * y.x;
+            o1.x = s * x.y + c * y.x;
+            o1.y = c * y.y - s * x.x;
+            reg[i] = o0;
+            reg[j] = o1;
+        }
+    }
+}
+
+template <int NR, typename V, typename T>
+__device__ __forceinline__ void dispatch_rx(int k, V* reg, T c, T s) {
+    switch (k) {
+        case 0: op_rx<0, NR>(reg, c, s); break;
+        case 1: op_rx<1, NR>(reg, c, s); break;
+        case 2: op_rx<2, NR>(reg, c, s); break;
+        case 3: if constexpr (NR > 8) op_rx<3, NR>(reg, c, s); break;
+        case 4: if constexpr (NR > 16) op_rx<4, NR>(reg, c, s); break;
+        default: break;
+    }
 }
 
 // Ry(theta) on slot K: [[c, -s], [s, c]] with c = cos(theta/2), s = sin(theta/2)
@@ -278,14 +307,15 @@ __device__ __forceinline__ void bcp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 
-// Batched sweep over (circuit, tile) work items of one class.  STAGE: the sweep's ops and, per circuit,
+// Batched sweep over (circuit, tile) work items of one class.  RX: QAOA (Rx and cost phases), else the
+// ansatz (Ry and CZ ladders).  STAGE: the sweep's ops and, per circuit,
 // its rotations and cost phases lie in shared memory after the tile (see staged_smem); an op's record and
 // then its angle were dependent loads past the L1 for every warp.  Bound by issue slots (about half of them
 // used, 512 threads of 128 registers an SM).  Without and with the tables in shared memory: QAOA energies
 // 5744 -> 5549 us, their gradients 6851 -> 6698 us (3-regular graphs of 12 to 22 and 12 to 20 vertices),
 // VQE of 16 qubits, 200 terms: parameter shift 5291 -> 5200 us, adjoint gradients 5591 -> 5299 us, f64 scan of
 // 13 qubits 187 -> 178 us.
-template <typename T, int RB, bool STAGE>
+template <typename T, int RB, bool STAGE, bool RX>
 __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const PhaseDesc* __restrict__ phases,
                                                       const SwOp* __restrict__ ops, QArgs<T> a) {
     using V = typename C2<T>::t;
@@ -334,7 +364,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
         const uint64_t gcirc = a.circ0 + circ;
         V* amps = a.amps + circ * nstate;
         const uint64_t* nb = nullptr;   // the instance's neighbour masks (cost phase and energy)
-        if (a.circ_inst) nb = a.nbr + (size_t)a.circ_inst[gcirc] * NBR_STRIDE;
+        if (RX) nb = a.nbr + (size_t)a.circ_inst[gcirc] * NBR_STRIDE;
         uint64_t base = 0;
         for (uint32_t b = 0; b < d.nonlocal_count; ++b)
             if ((tile >> b) & 1ull) base |= 1ull << d.nonlocal[b];
@@ -399,14 +429,36 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
                     reg[g ^ (g >> 1)] = sm[ad];
                 }
             }
+            if constexpr (exchanges<RX, T>) exchange_odd<NR>(reg);
             auto angle = [&](uint32_t k) {
                 return STAGE ? srot[k] : reinterpret_cast<const V*>(a.rot)[(size_t)gcirc * a.nparam + k];
             };
             for (uint32_t o = ph.op_begin; o < ph.op_end; ++o) {
                 const SwOp op = STAGE ? sops[o - op0] : ops[o];
-                if (op.type == OP_RXP) {
-                    const V r = angle(op.param);
-                    dispatch_rx<NR>(op.k0, reg, r.x, r.y);
+                if constexpr (RX) {
+                    if (op.type == OP_RXP) {
+                        const V r = angle(op.param);
+                        dispatch_rx<NR>(op.k0, reg, r.x, r.y);
+                    } else if (op.type == OP_CPH) {
+                        CutNb<RB> cp;
+                        cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
+                        if (STAGE) {
+                            const V* tab = stab + op.param * a.phs;
+    #pragma unroll
+                            for (int i = 0; i < NR; ++i) {
+                                const V t = tab[cut_nb<RB>(cp, i)];
+                                reg[i] = cmulv(reg[i], t.x, exchanges<RX, T> && odd_bits(i) ? -t.y : t.y);
+                            }
+                        } else {
+                            const T* tab = a.ph + ((size_t)gcirc * a.p + op.param) * a.phs * 2;
+    #pragma unroll
+                            for (int i = 0; i < NR; ++i) {
+                                const int c = cut_nb<RB>(cp, i);
+                                const T ti = tab[2 * c + 1];
+                                reg[i] = cmulv(reg[i], tab[2 * c], exchanges<RX, T> && odd_bits(i) ? -ti : ti);
+                            }
+                        }
+                    }
                 } else if (op.type == OP_RYP) {
                     const V r = angle(op.param);
                     dispatch_ry<NR>(op.k0, reg, r.x, r.y);
@@ -426,27 +478,10 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
 #pragma unroll
                     for (int i = 0; i < NR; ++i)
                         if (op.k0 >= 0 ? ((i >> op.k0) & 1) : u0) reg[i].y = -reg[i].y;
-                } else if (op.type == OP_CPH) {
-                    CutNb<RB> cp;
-                    cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
-                    if (STAGE) {
-                        const V* tab = stab + op.param * a.phs;
-#pragma unroll
-                        for (int i = 0; i < NR; ++i) {
-                            const V t = tab[cut_nb<RB>(cp, i)];
-                            reg[i] = cmulv(reg[i], t.x, t.y);
-                        }
-                    } else {
-                        const T* tab = a.ph + ((size_t)gcirc * a.p + op.param) * a.phs * 2;
-#pragma unroll
-                        for (int i = 0; i < NR; ++i) {
-                            const int c = cut_nb<RB>(cp, i);
-                            reg[i] = cmulv(reg[i], tab[2 * c], tab[2 * c + 1]);
-                        }
-                    }
                 }
             }
-            if ((d.flags & SWEEP_ENERGY) && p + 1 == d.phase_end) {
+            if constexpr (exchanges<RX, T>) exchange_odd<NR>(reg);
+            if (RX && (d.flags & SWEEP_ENERGY) && p + 1 == d.phase_end) {
                 CutNb<RB> cp;
                 cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
                 T e = 0;   // this thread's 2^RB terms in the state's type, then FP64 across threads
@@ -466,7 +501,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_sweep(const SweepDesc d, const
             __syncthreads();
         }
 
-        if (d.flags & SWEEP_ENERGY) {
+        if (RX && (d.flags & SWEEP_ENERGY)) {
             // fixed-order sum over the block (any block size, also < 32 threads)
             red[tid] = energy;
             __syncthreads();
@@ -523,6 +558,17 @@ __global__ void k_energy_finalize(const double* __restrict__ epart, uint64_t nci
 // given launch shape.
 template <int K, int NR, typename V>
 __device__ __forceinline__ double im_x_overlap(const V* p, const V* l) {
+    if constexpr (std::is_same<V, float2>::value) {   // b: parts exchanged (exchange_odd)
+        float2 u = make_float2(0.f, 0.f), v = u;
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            if (i & (1 << K)) continue;
+            const int j = i | (1 << K), a = odd_bits(i) ? j : i, b = odd_bits(i) ? i : j;
+            u = pk_fma(l[a], p[b], u);
+            v = pk_fma(l[b], p[a], v);
+        }
+        return (double)((u.x - v.x) - (u.y - v.y));
+    }
     decltype(p[0].x) acc = 0;   // at most 16 products of one thread, in the state's type
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
@@ -552,6 +598,17 @@ __device__ __forceinline__ double dispatch_im_x(int k, const V* p, const V* l) {
 // part is Re(conj(l_j) p_i) - Re(conj(l_i) p_j).
 template <int K, int NR, typename V>
 __device__ __forceinline__ double im_y_overlap(const V* p, const V* l) {
+    if constexpr (std::is_same<V, float2>::value) {
+        float2 u = make_float2(0.f, 0.f), v = u;
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            if (i & (1 << K)) continue;
+            const int j = i | (1 << K);
+            u = pk_fma(l[j], p[i], u);
+            v = pk_fma(l[i], p[j], v);
+        }
+        return (double)((u.x - v.x) + (u.y - v.y));
+    }
     decltype(p[0].x) acc = 0;   // at most 16 products of one thread, in the state's type
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
@@ -575,7 +632,7 @@ __device__ __forceinline__ double dispatch_im_y(int k, const V* p, const V* l) {
     return 0.0;
 }
 
-template <typename T, int RB, bool STAGE>
+template <typename T, int RB, bool STAGE, bool RX>
 __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, const PhaseDesc* __restrict__ phases,
                                                         const SwOp* __restrict__ ops, QArgs<T> a) {
     using V = typename C2<T>::t;
@@ -723,32 +780,40 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                     rl[g ^ (g >> 1)] = sml[ad];
                 }
             }
+            if constexpr (exchanges<RX, T>) {
+                exchange_odd<NR>(rp);
+                exchange_odd<NR>(rl);
+            }
             auto angle = [&](uint32_t k) {
                 return STAGE ? srot[k] : reinterpret_cast<const V*>(a.rot)[(size_t)gcirc * a.nparam + k];
             };
             for (uint32_t o = ph.op_begin; o < ph.op_end; ++o) {
                 const SwOp op = STAGE ? sops[o - op0] : ops[o];
-                if (op.type == OP_RXP) {
-                    const V r = angle(op.param);
-                    flush(4.0 * dispatch_im_x<NR>(op.k0, rp, rl), a.p + op.param);   // both halves
-                    dispatch_rx<NR>(op.k0, rp, r.x, -r.y);
-                    dispatch_rx<NR>(op.k0, rl, r.x, -r.y);
-                } else if (op.type == OP_CPH) {
-                    CutNb<RB> cp;
-                    cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
-                    const V* tab = STAGE ? stab + op.param * a.phs
-                                         : reinterpret_cast<const V*>(a.ph) + ((size_t)gcirc * a.p + op.param) * a.phs;
-                    T acc = 0;   // this thread's 2^RB terms in the state's type
-#pragma unroll
-                    for (int i = 0; i < NR; ++i) {
-                        const int c = cut_nb<RB>(cp, i);
-                        const T gdiag = (T)((int)ne - 2 * c);
-                        acc += gdiag * (rl[i].x * rp[i].y - rl[i].y * rp[i].x);
-                        const V t = tab[c];
-                        rp[i] = cmulv(rp[i], t.x, -t.y);
-                        rl[i] = cmulv(rl[i], t.x, -t.y);
+                if constexpr (RX) {
+                    if (op.type == OP_RXP) {
+                        const V r = angle(op.param);
+                        flush(4.0 * dispatch_im_x<NR>(op.k0, rp, rl), a.p + op.param);   // both halves
+                        dispatch_rx<NR>(op.k0, rp, r.x, -r.y);
+                        dispatch_rx<NR>(op.k0, rl, r.x, -r.y);
+                    } else if (op.type == OP_CPH) {
+                        CutNb<RB> cp;
+                        cut_plan_nb<RB>(cp, nb, U, ph.slot_global);
+                        const V* tab = STAGE ? stab + op.param * a.phs
+                                             : reinterpret_cast<const V*>(a.ph) + ((size_t)gcirc * a.p + op.param) * a.phs;
+                        T acc = 0;   // this thread's 2^RB terms in the state's type
+    #pragma unroll
+                        for (int i = 0; i < NR; ++i) {
+                            const int c = cut_nb<RB>(cp, i);
+                            const T gdiag = (T)((int)ne - 2 * c);
+                            const bool odd = exchanges<RX, T> && odd_bits(i);
+                            const T im = rl[i].x * rp[i].y - rl[i].y * rp[i].x;
+                            acc += gdiag * (odd ? -im : im);
+                            const V t = tab[c];
+                            rp[i] = cmulv(rp[i], t.x, odd ? t.y : -t.y);
+                            rl[i] = cmulv(rl[i], t.x, odd ? t.y : -t.y);
+                        }
+                        flush(4.0 * (double)acc, op.param);
                     }
-                    flush(4.0 * (double)acc, op.param);
                 } else if (op.type == OP_RYP) {
                     // Ry(theta) = exp(-i theta Y / 2): dE/dtheta = Im <lambda|Y|psi>
                     const V r = angle(op.param);
@@ -782,6 +847,10 @@ __global__ void __launch_bounds__(512, 1) k_batch_adjoint(const SweepDesc d, con
                         rl[i].y = flip_sign(rl[i].y, m[i]);
                     }
                 }
+            }
+            if constexpr (exchanges<RX, T>) {
+                exchange_odd<NR>(rp);
+                exchange_odd<NR>(rl);
             }
             {
                 uint32_t ad = sb;
@@ -1570,7 +1639,7 @@ int launch_class(rq_qaoa_batch* b, QClass& K, uint64_t ncirc, uint64_t circ0, vo
     const size_t angles = (b->p + (size_t)b->p * b->phs) * sizeof(V);
     const size_t smem = staged_smem(K.smem + K.tables.phases, K.smem + K.tables.all + angles, 2048,
                                     std::max(1u, 512u / threads), &stage);
-    auto kern = stage ? k_batch_sweep<T, RBc, true> : k_batch_sweep<T, RBc, false>;
+    auto kern = stage ? k_batch_sweep<T, RBc, true, true> : k_batch_sweep<T, RBc, false, true>;
     RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
@@ -1620,7 +1689,7 @@ int adjoint_class(rq_qaoa_batch* b, QClass& K, uint64_t ncirc, uint64_t circ0, v
     const size_t need = 2 * ((size_t)1 << K.am) * sizeof(V) + ((size_t)ngroup * P2 + 1) / 2 * 16;
     const size_t smem = staged_smem(need, need + K.atables.all + (b->p + (size_t)b->p * b->phs) * sizeof(V), 0,
                                     std::max(1u, 512u / threads), &stage);
-    auto kern = stage ? k_batch_adjoint<T, RBc, true> : k_batch_adjoint<T, RBc, false>;
+    auto kern = stage ? k_batch_adjoint<T, RBc, true, true> : k_batch_adjoint<T, RBc, false, true>;
     RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
@@ -2550,7 +2619,7 @@ int vqe_wave(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     bool stage = false;
     const size_t smem = staged_smem(b->smem + b->tables.phases, b->smem + b->tables.all + b->P * sizeof(V), 2048,
                                     std::max(1u, 512u / threads), &stage);
-    auto kern = stage ? k_batch_sweep<T, RBc, true> : k_batch_sweep<T, RBc, false>;
+    auto kern = stage ? k_batch_sweep<T, RBc, true, false> : k_batch_sweep<T, RBc, false, false>;
     RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
@@ -2609,7 +2678,7 @@ int vqe_adjoint(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0) {
     bool stage = false;
     const size_t need = 2 * ((size_t)1 << b->am) * sizeof(V) + ((size_t)ngroup * b->P + 1) / 2 * 16;
     const size_t smem = staged_smem(need, need + b->atables.all + b->P * sizeof(V), 0, std::max(1u, 512u / threads), &stage);
-    auto kern = stage ? k_batch_adjoint<T, RBc, true> : k_batch_adjoint<T, RBc, false>;
+    auto kern = stage ? k_batch_adjoint<T, RBc, true, false> : k_batch_adjoint<T, RBc, false, false>;
     RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
