@@ -124,7 +124,9 @@ struct GemmArgs {
     int out;                     // EPI_MSE: columns that count
     float* F;                    // EPI_RELU_BACK, EPI_MSE: [M x N] f32 (row stride ldh)
     float* losspart;             // EPI_MSE: [row tiles * column tiles]
+    int early;                   // EARLY_A, EARLY_B: operands that the launch just before does not write
 };
+constexpr int EARLY_A = 1, EARLY_B = 2;
 
 // Programmatic dependent launch: a kernel of the training chain starts while its predecessor
 // drains, sets up its tensor memory and barriers, and waits here for the predecessor's results
@@ -132,6 +134,9 @@ struct GemmArgs {
 // visible; it returns at once in a kernel launched without the attribute).  What a predecessor
 // writes is read past the L1 cache (cp.async.cg, __ldcg): the reading kernel may have begun before
 // the write, so the read-only path would be free to return or to fetch early a stale line.
+// A kernel starts once every CTA of its predecessor is past its own wait, so what the launch before
+// that one wrote, or an older one, is there already: such operands (GemmArgs::early) are read before
+// the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -228,7 +233,10 @@ __device__ void column_sums(const ColSum& s, int block, float* stage, int tid) {
 // 8) took 80 us each on a B200 with 256-column tiles and 64-wide chunks (two CTAs, a wait after
 // every chunk) and take 8 us; the ReLU mask and the bias gradients, two kernels of 135 us that
 // walked the batch serially per column, run in this epilogue and beside the products.  A step with
-// Adam: 900 -> 65 us, and 50 us with each launch's set-up overlapping its predecessor (pdl_wait).
+// Adam: 900 -> 65 us, and 56 us with each launch's set-up overlapping its predecessor (pdl_wait).
+// Loading the 80 KB of operands took 4 us of a product's 8 (a few bytes in flight a thread over 1 us of
+// latency): with the operand that is older than the predecessor read before the wait, both chunks in
+// flight at once and the epilogue's operands fetched beside them, a step takes 44 us.
 template <int NT, int KC>
 __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, const ColSum cs, int tiles0,
                                                      int tiles1) {
@@ -268,44 +276,90 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
+    const int nk = (g.K + KC - 1) / KC;
+    auto load_a = [&](int kc) {
+        unsigned char* sA = smem + (kc & 1) * (ABYTES + BBYTES);
+        const int k0 = kc * KC, kw = min(KC, g.K - k0);   // multiple of 16
+        if (g.at) load_mn_major<BM, KC>(sA, g.A, g.lda, row0, g.M, k0, kw, g.arows, tid);
+        else load_k_major<BM, KC>(sA, g.A, g.lda, row0, g.arows, k0, kw, tid);
+    };
+    auto load_b = [&](int kc) {
+        unsigned char* sB = smem + (kc & 1) * (ABYTES + BBYTES) + ABYTES;
+        const int k0 = kc * KC, kw = min(KC, g.K - k0);
+        if (g.bt) load_mn_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, g.at ? g.arows : g.K, tid);
+        else load_k_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, tid);
+    };
+    // what the epilogue adds, masks with or compares with, for 16 columns of this thread's row
+    const int rl = (warp & 3) * 32 + lane, r = row0 + rl, half = warp >> 2;
+    float eb[16], et[16];
+    uint4 em[2];
+    auto fetch = [&](int c) {
+        if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) eb[j] = c + j < g.nbias ? __ldcg(g.bias + c + j) : 0.f;
+        }
+        if (g.epi == EPI_MSE) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) et[j] = r < g.valid && c + j < g.out ? g.target[(size_t)r * g.out + c + j] : 0.f;
+        }
+        if (g.epi == EPI_RELU_BACK) {
+            em[0] = em[1] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < g.M && c < g.N && r < g.valid) {   // N is a multiple of 16 here
+                const uint4* mp = reinterpret_cast<const uint4*>(g.mask + (size_t)r * g.ldh + c);
+                em[0] = __ldcg(mp);
+                em[1] = __ldcg(mp + 1);
+            }
+        }
+    };
+
+    // the first two chunks into the two buffers: what the predecessor does not write, then the rest
+    const int pre = min(nk, 2);
+    for (int kc = 0; kc < pre; ++kc) {
+        if (g.early & EARLY_A) load_a(kc);
+        if (g.early & EARLY_B) load_b(kc);
+    }
     pdl_wait();
     pdl_go();
+    for (int kc = 0; kc < pre; ++kc) {
+        if (!(g.early & EARLY_A)) load_a(kc);
+        if (!(g.early & EARLY_B)) load_b(kc);
+    }
+    if (NT == 32) fetch(col0 + half * 16);   // lands while the operands do
 
-    const int nk = (g.K + KC - 1) / KC;
     int issued = 0;                       // chunks whose MMAs have been issued
     for (int kc = 0; kc < nk; ++kc) {
         const int buf = kc & 1;
-        unsigned char* sA = smem + buf * (ABYTES + BBYTES);
-        unsigned char* sB = sA + ABYTES;
         if (kc >= 2) {                    // the MMAs of chunk kc - 2 read this buffer
             if (!mbar_wait(&mbar[buf], (uint32_t)((kc >> 1) - 1) & 1u, g_mma_wait_polls)) timed_out = 1;
             __syncthreads();
             if (timed_out) break;
+            load_a(kc);
+            load_b(kc);
         }
-        const int k0 = kc * KC;
-        const int kw = min(KC, g.K - k0);   // multiple of 16
-        if (g.at) load_mn_major<BM, KC>(sA, g.A, g.lda, row0, g.M, k0, kw, g.arows, tid);
-        else load_k_major<BM, KC>(sA, g.A, g.lda, row0, g.arows, k0, kw, tid);
-        if (g.bt) load_mn_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, g.at ? g.arows : g.K, tid);
-        else load_k_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, tid);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        // make the generic-proxy writes visible to the tensor core (async proxy)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (kc != 1) {                    // chunk 1 landed with chunk 0
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            // make the generic-proxy writes visible to the tensor core (async proxy)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncthreads();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
         if (tid == 0) {
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-            for (int ks = 0; ks < kw / 16; ++ks) {
-                const uint64_t ad = sdesc(a0 + ks * 2 * LBO, KC * 16);
-                const uint64_t bd = sdesc(b0 + ks * 2 * LBO, KC * 16);
-                const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
+            const uint32_t a0 = smem_u32(smem + buf * (ABYTES + BBYTES));
+            uint64_t ad = sdesc(a0, KC * 16), bd = sdesc(a0 + ABYTES, KC * 16);
+            const int steps = min(KC, g.K - kc * KC) / 16;
+            uint32_t acc = kc > 0 ? 1u : 0u;
+#pragma unroll 4
+            for (int ks = 0; ks < steps; ++ks) {
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
                     ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc_bf16(NT)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
                     : "memory");
+                ad += 2 * LBO >> 4;       // the address field: the next 16 of K
+                bd += 2 * LBO >> 4;
+                acc = 1u;
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_u32(&mbar[buf]))
@@ -329,7 +383,6 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
     } else {
         // epilogue: warps w and w + 4 read the tensor-memory lanes 32 (w % 4).. (rows of the tile),
         // the lower four warps the first half of the columns, the upper four the second
-        const int rl = (warp & 3) * 32 + lane, r = row0 + rl, half = warp >> 2;
         float loss = 0.f;
         const float inv = g.epi == EPI_MSE ? 1.f / (float)(g.valid * g.out) : 0.f;
         for (int c0 = half * (NT / 2); c0 < (half + 1) * (NT / 2); c0 += 16) {
@@ -345,12 +398,13 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
 #pragma unroll
             for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
             const int c = col0 + c0;
+            if (NT != 32) fetch(c);
             const bool in = r < g.M && c < g.N;
             const bool full = in && c + 16 <= g.N;
             if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
-                    if (c + j < g.nbias) x[j] += __ldcg(g.bias + c + j);
+                    if (c + j < g.nbias) x[j] += eb[j];
             }
             if (g.epi == EPI_F32 || g.epi == EPI_BIAS) {
                 float* o = g.C + (size_t)r * g.ldc + c;
@@ -369,13 +423,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
 #pragma unroll
                 for (int j = 0; j < 16; ++j) x[j] = x[j] > 0.f ? x[j] : 0.f;
             } else if (g.epi == EPI_RELU_BACK) {
-                uint4 mk[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-                if (in && r < g.valid) {   // N is a multiple of 16 here
-                    const uint4* mp = reinterpret_cast<const uint4*>(g.mask + (size_t)r * g.ldh + c);
-                    mk[0] = __ldcg(mp);
-                    mk[1] = __ldcg(mp + 1);
-                }
-                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(mk);
+                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(em);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) x[j] = __bfloat162float(mb[j]) > 0.f ? x[j] : 0.f;
             } else {   // EPI_MSE
@@ -383,7 +431,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
                 for (int j = 0; j < 16; ++j) {
                     float gr = 0.f;
                     if (r < g.valid && c + j < g.out) {
-                        const float d = x[j] - g.target[(size_t)r * g.out + c + j];
+                        const float d = x[j] - et[j];
                         loss += d * d;
                         gr = 2.f * d;
                     }
@@ -733,8 +781,8 @@ int mlp_pack_rows(rq_mlp* m, const float* src, size_t rows, __nv_bfloat16* dst) 
     return RQ_OK;
 }
 
-// hidden layers on B packed rows X: H1, H2
-int mlp_hidden(rq_mlp* m, const __nv_bfloat16* X, int B) {
+// hidden layers on B packed rows X: H1, H2 (settled: X is older than the launch before)
+int mlp_hidden(rq_mlp* m, const __nv_bfloat16* X, int B, bool settled) {
     const int Bp = (B + 127) & ~127;
     GemmArgs g{};
     g.A = X; g.lda = m->inp; g.arows = B;
@@ -743,7 +791,9 @@ int mlp_hidden(rq_mlp* m, const __nv_bfloat16* X, int B) {
     g.bias = m->P + m->off_b1; g.nbias = m->h1;
     g.H = m->H1; g.ldh = m->h1;
     g.epi = EPI_BIAS_RELU;
+    g.early = settled ? EARLY_A : 0;
     RQ_TRY(gemm(m->stream, g));
+    g.early = EARLY_B;
     g.A = m->H1; g.lda = m->h1; g.arows = Bp;
     g.B = m->W2b; g.ldb = m->h1;
     g.N = m->h2; g.K = m->h1;
@@ -761,14 +811,15 @@ GemmArgs output_layer(rq_mlp* m, int B) {
     g.bias = m->P + m->off_b3; g.nbias = m->out;
     g.C = m->Y; g.ldc = m->outp;
     g.epi = EPI_BIAS;
+    g.early = EARLY_B;
     return g;
 }
 
 // forward and backward pass on B packed rows X with targets T (device): weight gradients into m->G,
 // bias gradients into m->db1..3, the loss as per-tile sums
-int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) {
+int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B, bool settled) {
     const int Bp = (B + 127) & ~127;
-    RQ_TRY(mlp_hidden(m, X, B));
+    RQ_TRY(mlp_hidden(m, X, B, settled));
     // output layer with the loss: dY = 2 (Y - T) / (B out)
     GemmArgs y = output_layer(m, B);
     y.N = m->outp;                     // W3b's padding rows are zero; columns past out become zero in dY
@@ -785,6 +836,7 @@ int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) 
     w.M = m->h2; w.N = m->outp; w.K = Bp; w.arows = B;
     w.C = m->G + m->g_w3t; w.ldc = m->outp;
     w.epi = EPI_F32;
+    w.early = EARLY_A;
     GemmArgs d{};
     d.A = m->dY; d.lda = m->outp; d.arows = Bp;
     d.B = m->W3b; d.ldb = m->h2; d.bt = 1;
@@ -792,12 +844,14 @@ int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B) 
     d.H = m->dZ2; d.ldh = m->h2; d.mask = m->H2;
     d.valid = B; d.F = m->F2;
     d.epi = EPI_RELU_BACK;
+    d.early = EARLY_B;
     const ColSum b3{m->F3, m->outp, m->out, B, 1.f / (float)(B * m->out), m->db3};
     RQ_TRY(gemm(m->stream, w, &d, &b3));
     // dW2 [h2 x h1] = dZ2^T H1, and dZ1 [Bp x h1] = (dZ2 W2) where H1 > 0
     w.A = m->dZ2; w.lda = m->h2;
     w.B = m->H1; w.ldb = m->h1;
     w.M = m->h2; w.N = m->h1;
+    w.early = EARLY_B;
     w.C = m->G + m->g_w2; w.ldc = m->h1;
     d.A = m->dZ2; d.lda = m->h2;
     d.B = m->W2b; d.ldb = m->h1;
@@ -938,7 +992,7 @@ int rq_mlp_forward(rq_mlp* m, const float* x, int32_t B, float* y) {
     RQ_TRY(mlp_reserve(m, B));
     RQ_CUDA(cudaMemcpyAsync(m->Xf, x, (size_t)B * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     RQ_TRY(mlp_pack_rows(m, m->Xf, B, m->X));
-    RQ_TRY(mlp_hidden(m, m->X, B));
+    RQ_TRY(mlp_hidden(m, m->X, B, false));
     RQ_TRY(gemm(m->stream, output_layer(m, B)));
     RQ_CUDA(cudaMemcpy2DAsync(y, m->out * sizeof(float), m->Y, m->outp * sizeof(float), m->out * sizeof(float), B,
                               cudaMemcpyDeviceToHost, m->stream));
@@ -957,7 +1011,7 @@ int rq_mlp_gradients(rq_mlp* m, const float* x, const float* t, int32_t B, float
     RQ_CUDA(cudaMemcpyAsync(m->Xf, x, (size_t)B * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     RQ_CUDA(cudaMemcpyAsync(m->Tf, t, (size_t)B * m->out * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     RQ_TRY(mlp_pack_rows(m, m->Xf, B, m->X));
-    RQ_TRY(mlp_gradients_dev(m, m->X, m->Tf, B));
+    RQ_TRY(mlp_gradients_dev(m, m->X, m->Tf, B, false));
     float* dflat = nullptr;
     RQ_TRY(dalloc(&dflat, m->nparam));
     k_gather<<<rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0, m->stream>>>(
@@ -992,7 +1046,7 @@ int rq_mlp_train(rq_mlp* m, const float* x, const float* t, int32_t n, int32_t B
     for (int s = 0; s < steps && rc == RQ_OK; ++s) {
         const long r0 = ((long)s * B) % n;
         const int take = (int)std::min<long>(B, n - r0);
-        rc = mlp_gradients_dev(m, m->txb + r0 * m->inp, m->tt + r0 * m->out, take);
+        rc = mlp_gradients_dev(m, m->txb + r0 * m->inp, m->tt + r0 * m->out, take, s > 0);
         if (rc == RQ_OK) rc = mlp_adam(m, take, lr, 0.9f, 0.999f, 1e-8f);
     }
     if (rc == RQ_OK && last_loss) {

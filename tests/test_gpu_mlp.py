@@ -132,3 +132,29 @@ def test_mlp_edge_shapes_match_oracle(dims, B):
         # an activation whose BF16 rounding or ReLU sign differs moves single entries: 1e-2 of the norm
         assert np.linalg.norm(a - b) <= 1e-2 * (np.linalg.norm(b) + 1e-12), (n, np.linalg.norm(a - b), np.linalg.norm(b))
         k += n
+
+
+@pytest.mark.parametrize("M,N,chunk", [(100, 40, 256), (2400, 500, 192), (2400, 1000, 192), (2400, 2000, 128)])
+def test_gemm_bf16_chunk_counts(M, N, chunk):
+    """One chunk of K, the two that are loaded together, and those that follow into their buffers, full
+    and with a remainder, at each tile width.  Whole numbers of at most 2: every sum is exact."""
+    r = np.random.default_rng(M + N)
+    for K in (16, chunk, chunk + 16, 2 * chunk, 2 * chunk + 16, 3 * chunk, 4 * chunk + 48):
+        out, ref = gemm(r.integers(-2, 3, size=(M, K)).astype(np.float32), r.integers(-2, 3, size=(N, K)).astype(np.float32))
+        assert np.array_equal(out, ref), K
+
+
+@pytest.mark.parametrize("dims,B", [((325, 256, 256, 8), 256), ((600, 64, 272, 3), 129), ((9, 528, 16, 20), 300),
+                                    ((325, 256, 256, 8), 1)])
+def test_mlp_steps_in_a_row_equal_single_steps(dims, B):
+    """Steps whose products start before their predecessors end give the parameters of the same steps
+    run one call at a time, to the bit."""
+    r = np.random.default_rng(B)
+    x = r.normal(size=(B, dims[0])).astype(np.float32)
+    t = r.uniform(0, 1.5, size=(B, dims[3])).astype(np.float32)
+    a, b = Mlp(*dims, seed=3), Mlp(*dims, seed=3)
+    for _ in range(3):
+        la = a.train(x, t, batch=B, steps=8)
+        for _ in range(8):
+            lb = b.train(x, t, batch=B, steps=1)
+        assert la == lb and np.array_equal(a.get_params(), b.get_params())
