@@ -31,7 +31,6 @@
 
 namespace {
 
-constexpr int BM = 128;      // rows per CTA (UMMA M)
 constexpr int GT = 256;      // threads per CTA
 constexpr int LBO = 128;     // bytes between core matrices along K
 
@@ -51,13 +50,13 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t sbo) {
     return d;                 // base offset 0, lbo mode 0, layout type 0 (no swizzle)
 }
 
-// instruction descriptor: BF16 x BF16 -> F32, A and B K-major, M = 128, N = n
-__host__ __device__ constexpr uint32_t idesc_bf16(int n) {
+// instruction descriptor: BF16 x BF16 -> F32, A and B K-major, M = m (64 or 128), N = n
+__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
     return (1u << 4)               // D format F32
          | (1u << 7)               // A format BF16
          | (1u << 10)              // B format BF16
          | ((uint32_t)(n >> 3) << 17)
-         | ((uint32_t)(BM >> 4) << 24);
+         | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -226,8 +225,9 @@ __device__ void column_sums(const ColSum& s, int block, float* stage, int tid) {
 }
 
 // One launch covers the tiles of g0 and, after them, those of g1 (independent products that
-// become ready together; tiles0 and tiles1 = their tiles), then the column sums cs.  A tile is rows [128 i, +128) x columns
-// [NT j, +NT) of C.  The warm-start products are small (256 x 256 x 256-336): what bounds them is
+// become ready together; tiles0 and tiles1 = their tiles), then the column sums cs.  A tile is rows [BM i, +BM) x columns
+// [NT j, +NT) of C (BM 128 or 64; the accumulator of 64 rows lies in the first 16 tensor-memory lanes of
+// each warp).  The warm-start products are small (256 x 256 x 256-336): what bounds them is
 // the latency of load -> MMA -> epilogue, so narrow tiles (more CTAs, each loading little) and the
 // whole K in at most two chunks.  The products of a training step (batch 256, 336 -> 256 -> 256 ->
 // 8) took 80 us each on a B200 with 256-column tiles and 64-wide chunks (two CTAs, a wait after
@@ -236,8 +236,9 @@ __device__ void column_sums(const ColSum& s, int block, float* stage, int tid) {
 // Adam: 900 -> 65 us, and 56 us with each launch's set-up overlapping its predecessor (pdl_wait).
 // Loading the 80 KB of operands took 4 us of a product's 8 (a few bytes in flight a thread over 1 us of
 // latency): with the operand that is older than the predecessor read before the wait, both chunks in
-// flight at once and the epilogue's operands fetched beside them, a step takes 44 us.
-template <int NT, int KC>
+// flight at once and the epilogue's operands fetched beside them, a step takes 44 us, and with 64-row
+// tiles 36 us.
+template <int BM, int NT, int KC>
 __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, const ColSum cs, int tiles0,
                                                      int tiles1) {
     static_assert(NT % 32 == 0 && NT >= 32 && NT <= 256, "tile N");
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
         else load_k_major<NT, KC>(sB, g.B, g.ldb, col0, g.N, k0, kw, tid);
     };
     // what the epilogue adds, masks with or compares with, for 16 columns of this thread's row
-    const int rl = (warp & 3) * 32 + lane, r = row0 + rl, half = warp >> 2;
+    const int r = row0 + (warp & 3) * (BM / 4) + lane, half = warp >> 2;
     float eb[16], et[16];
     uint4 em[2];
     auto fetch = [&](int c) {
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                    ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc_bf16(NT)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                    ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc_bf16(BM, NT)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
                     : "memory");
                 ad += 2 * LBO >> 4;       // the address field: the next 16 of K
                 bd += 2 * LBO >> 4;
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
             atomicExch(&g_mma_timeout, 1);
         }
     } else {
-        // epilogue: warps w and w + 4 read the tensor-memory lanes 32 (w % 4).. (rows of the tile),
+        // epilogue: warps w and w + 4 read the tensor-memory lanes 32 (w % 4).. (BM / 4 rows of the tile),
         // the lower four warps the first half of the columns, the upper four the second
         float loss = 0.f;
         const float inv = g.epi == EPI_MSE ? 1.f / (float)(g.valid * g.out) : 0.f;
@@ -399,7 +400,8 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
             for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
             const int c = col0 + c0;
             if (NT != 32) fetch(c);
-            const bool in = r < g.M && c < g.N;
+            const bool row_ok = lane < BM / 4;
+            const bool in = row_ok && r < g.M && c < g.N;
             const bool full = in && c + 16 <= g.N;
             if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
 #pragma unroll
@@ -430,7 +432,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     float gr = 0.f;
-                    if (r < g.valid && c + j < g.out) {
+                    if (row_ok && r < g.valid && c + j < g.out) {
                         const float d = x[j] - et[j];
                         loss += d * d;
                         gr = 2.f * d;
@@ -438,7 +440,7 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
                     x[j] = gr;
                 }
             }
-            if (r < g.M && c + 16 <= g.ldh) {     // ldh is a multiple of 16: whole 16-column groups
+            if (row_ok && r < g.M && c + 16 <= g.ldh) {     // ldh is a multiple of 16: whole 16-column groups
                 const size_t at = (size_t)r * g.ldh + c;
                 if (g.epi != EPI_BIAS_RELU) {
 #pragma unroll
@@ -489,25 +491,27 @@ int launch_chained(cudaStream_t stream, void (*kern)(KA...), unsigned grid, unsi
     return RQ_OK;
 }
 
-template <int NT, int KC>
+template <int BM, int NT, int KC>
 int launch_gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1, const ColSum* cs) {
     auto tiles = [](const GemmArgs& g) { return ((g.M + BM - 1) / BM) * ((g.N + NT - 1) / NT); };
     constexpr int smem = 2 * (BM + NT) * KC * 2;
     const int t0 = tiles(g0), t1 = g1 ? tiles(*g1) : 0, tc = cs ? (cs->cols + 31) / 32 : 0;
-    RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<NT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    return launch_chained(stream, k_gemm_bf16<NT, KC>, t0 + t1 + tc, GT, smem, g0, g1 ? *g1 : g0,
+    RQ_CUDA(cudaFuncSetAttribute(k_gemm_bf16<BM, NT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return launch_chained(stream, k_gemm_bf16<BM, NT, KC>, t0 + t1 + tc, GT, smem, g0, g1 ? *g1 : g0,
                           cs ? *cs : ColSum{}, t0, t1);
 }
 
 // Tile width by the number of CTAs it leaves: the widest tile whose grid still has a CTA for
-// every SM (A is re-read once per column tile, so large products want wide tiles), else 32
-// columns, where a small product spreads over the most SMs.
+// every SM (A is re-read once per column tile, so large products want wide tiles); where even 32
+// columns leave SMs idle, 64 rows by 32 columns, whose CTAs each load 48 KB instead of 80 (64
+// training steps of batch 256: 2.76 -> 2.30 ms).
 int gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1 = nullptr, const ColSum* cs = nullptr) {
-    const long mt = (g0.M + BM - 1) / BM;
-    if (!g1 && mt * ((g0.N + 255) / 256) >= 148) return launch_gemm<256, 128>(stream, g0, g1, cs);
-    if (!g1 && mt * ((g0.N + 127) / 128) >= 148) return launch_gemm<128, 192>(stream, g0, g1, cs);
-    if (!g1 && mt * ((g0.N + 63) / 64) >= 148) return launch_gemm<64, 192>(stream, g0, g1, cs);
-    return launch_gemm<32, 256>(stream, g0, g1, cs);
+    const long mt = (g0.M + 127) / 128;
+    if (!g1 && mt * ((g0.N + 255) / 256) >= 148) return launch_gemm<128, 256, 128>(stream, g0, g1, cs);
+    if (!g1 && mt * ((g0.N + 127) / 128) >= 148) return launch_gemm<128, 128, 192>(stream, g0, g1, cs);
+    if (!g1 && mt * ((g0.N + 63) / 64) >= 148) return launch_gemm<128, 64, 192>(stream, g0, g1, cs);
+    if (!g1 && mt * ((g0.N + 31) / 32) >= 148) return launch_gemm<128, 32, 256>(stream, g0, g1, cs);
+    return launch_gemm<64, 32, 256>(stream, g0, g1, cs);
 }
 
 }  // namespace
@@ -737,7 +741,7 @@ int mlp_reserve(rq_mlp* m, int B) {
         *p = nullptr;
         return dalloc(p, n);
     };
-    const size_t b = (size_t)Bp, nt = b / BM;
+    const size_t b = (size_t)Bp, nt = b / 64;
     RQ_TRY(regrow(&m->X, b * m->inp));
     RQ_TRY(regrow(&m->H1, b * m->h1));
     RQ_TRY(regrow(&m->H2, b * m->h2));
@@ -828,7 +832,7 @@ int mlp_gradients_dev(rq_mlp* m, const __nv_bfloat16* X, const float* T, int B, 
     y.nbias = m->out;
     y.valid = B; y.out = m->out; y.target = T;
     y.F = m->F3; y.losspart = m->losspart;
-    RQ_TRY((launch_gemm<32, 256>(m->stream, y, nullptr, nullptr)));
+    RQ_TRY((launch_gemm<64, 32, 256>(m->stream, y, nullptr, nullptr)));
     // dW3^T [h2 x outp] = H2^T dY, and dZ2 [Bp x h2] = (dY W3) where H2 > 0
     GemmArgs w{};
     w.A = m->H2; w.lda = m->h2; w.at = 1;
@@ -879,7 +883,8 @@ ParamMap param_map(const rq_mlp* m) {
     return k;
 }
 
-int loss_tiles(const rq_mlp* m, int B) { return ((B + BM - 1) / BM) * ((m->outp + 31) / 32); }
+// tiles of the output layer (64 rows of the padded batch, 32 columns)
+int loss_tiles(const rq_mlp* m, int B) { return ((B + 127) / 128 * 2) * ((m->outp + 31) / 32); }
 
 // one Adam step over every parameter from the gradients of the last mlp_gradients_dev (B rows)
 int mlp_adam(rq_mlp* m, int B, float lr, float b1, float b2, float eps) {

@@ -134,7 +134,7 @@ def test_mlp_edge_shapes_match_oracle(dims, B):
         k += n
 
 
-@pytest.mark.parametrize("M,N,chunk", [(100, 40, 256), (2400, 500, 192), (2400, 1000, 192), (2400, 2000, 128)])
+@pytest.mark.parametrize("M,N,chunk", [(100, 40, 256), (63, 8, 256), (65, 100, 256), (19000, 24, 256), (2400, 500, 192), (2400, 1000, 192), (2400, 2000, 128)])
 def test_gemm_bf16_chunk_counts(M, N, chunk):
     """One chunk of K, the two that are loaded together, and those that follow into their buffers, full
     and with a remainder, at each tile width.  Whole numbers of at most 2: every sum is exact."""
@@ -144,7 +144,7 @@ def test_gemm_bf16_chunk_counts(M, N, chunk):
         assert np.array_equal(out, ref), K
 
 
-@pytest.mark.parametrize("dims,B", [((325, 256, 256, 8), 256), ((600, 64, 272, 3), 129), ((9, 528, 16, 20), 300),
+@pytest.mark.parametrize("dims,B", [((325, 256, 256, 8), 256), ((600, 64, 272, 3), 129), ((9, 528, 16, 40), 300),
                                     ((325, 256, 256, 8), 1)])
 def test_mlp_steps_in_a_row_equal_single_steps(dims, B):
     """Steps whose products start before their predecessors end give the parameters of the same steps
