@@ -236,8 +236,9 @@ __device__ void column_sums(const ColSum& s, int block, float* stage, int tid) {
 // Adam: 900 -> 65 us, and 56 us with each launch's set-up overlapping its predecessor (pdl_wait).
 // Loading the 80 KB of operands took 4 us of a product's 8 (a few bytes in flight a thread over 1 us of
 // latency): with the operand that is older than the predecessor read before the wait, both chunks in
-// flight at once and the epilogue's operands fetched beside them, a step takes 44 us, and with 64-row
-// tiles 36 us.
+// flight at once and the epilogue's operands fetched beside them, a step takes 44 us, with 64-row
+// tiles 36 us, and with Adam's parameters and moments read before its wait 35 us.  Of a product's 4.5 us
+// 1.3 are the hand-over between launches, 1.2 the late operand, 0.9 the MMAs, 0.6 the epilogue.
 template <int BM, int NT, int KC>
 __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, const ColSum cs, int tiles0,
                                                      int tiles1) {
@@ -249,6 +250,8 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
     __shared__ int timed_out;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int uwarp = __shfl_sync(0xffffffffu, warp, 0);
+    const uint32_t leader = lane == 0 ? 1u : 0u;
     if ((int)blockIdx.x >= tiles0 + tiles1) {
         pdl_wait();
         pdl_go();
@@ -292,12 +295,12 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
     };
     // what the epilogue adds, masks with or compares with, for 16 columns of this thread's row
     const int r = row0 + (warp & 3) * (BM / 4) + lane, half = warp >> 2;
-    float eb[16], et[16];
+    float eb = 0.f, et[16];   // eb: lanes 0-15 hold the columns' biases
     uint4 em[2];
     auto fetch = [&](int c) {
         if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) eb[j] = c + j < g.nbias ? __ldcg(g.bias + c + j) : 0.f;
+            const int b = c + (lane & 15);
+            eb = b < g.nbias ? __ldcg(g.bias + b) : 0.f;
         }
         if (g.epi == EPI_MSE) {
 #pragma unroll
@@ -345,7 +348,8 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
             __syncthreads();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        if (tid == 0) {
+        // the whole of warp 0 steps the descriptors, so that they stay in uniform registers; one lane issues
+        if (uwarp == 0) {
             const uint32_t a0 = smem_u32(smem + buf * (ABYTES + BBYTES));
             uint64_t ad = sdesc(a0, KC * 16), bd = sdesc(a0 + ABYTES, KC * 16);
             const int steps = min(KC, g.K - kc * KC) / 16;
@@ -353,18 +357,21 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
 #pragma unroll 4
             for (int ks = 0; ks < steps; ++ks) {
                 asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
+                    "{\n\t.reg .pred p, e;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                    ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc_bf16(BM, NT)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                    "setp.ne.b32 e, %9, 0;\n\t"
+                    "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+                    ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc_bf16(BM, NT)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u),
+                    "r"(leader)
                     : "memory");
                 ad += 2 * LBO >> 4;       // the address field: the next 16 of K
                 bd += 2 * LBO >> 4;
                 acc = 1u;
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&mbar[buf]))
-                         : "memory");
+            if (leader)
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 smem_u32(&mbar[buf]))
+                             : "memory");
         }
         issued = kc + 1;
     }
@@ -405,8 +412,10 @@ __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const Ge
             const bool full = in && c + 16 <= g.N;
             if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU || g.epi == EPI_MSE) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (c + j < g.nbias) x[j] += eb[j];
+                for (int j = 0; j < 16; ++j) {
+                    const float b = __shfl_sync(0xffffffffu, eb, j);
+                    if (c + j < g.nbias) x[j] += b;
+                }
             }
             if (g.epi == EPI_F32 || g.epi == EPI_BIAS) {
                 float* o = g.C + (size_t)r * g.ldc + c;
@@ -612,65 +621,92 @@ struct ParamMap {
     __nv_bfloat16 *W1b, *W2b, *W3b;
 };
 
-// gradient of parameter w; *copy = where its BF16 copy lives (null for a bias)
-__device__ __forceinline__ float grad_of(const ParamMap& m, long w, __nv_bfloat16** copy) {
+// where the gradient of parameter w lies; *copy = where its BF16 copy lives (null for a bias)
+__device__ __forceinline__ const float* grad_of(const ParamMap& m, long w, __nv_bfloat16** copy) {
     *copy = nullptr;
     if (w < m.b1) {
         const int r = (int)(w / m.in), k = (int)(w - (long)r * m.in);
         *copy = m.W1b + (long)r * m.inp + k;
-        return __ldcg(m.g1 + (long)r * m.inp + k);
+        return m.g1 + (long)r * m.inp + k;
     } else if (w < m.w2) {
-        return __ldcg(m.db1 + (w - m.b1));
+        return m.db1 + (w - m.b1);
     } else if (w < m.b2) {
         *copy = m.W2b + (w - m.w2);
-        return __ldcg(m.g2 + (w - m.w2));
+        return m.g2 + (w - m.w2);
     } else if (w < m.w3) {
-        return __ldcg(m.db2 + (w - m.b2));
+        return m.db2 + (w - m.b2);
     } else if (w < m.b3) {
         const int r = (int)((w - m.w3) / m.h2), k = (int)((w - m.w3) - (long)r * m.h2);
         *copy = m.W3b + (long)r * m.h2 + k;
-        return __ldcg(m.g3t + (long)k * m.outp + r);
+        return m.g3t + (long)k * m.outp + r;
     }
-    return __ldcg(m.db3 + (w - m.b3));
+    return m.db3 + (w - m.b3);
+}
+
+// a warp's sum of the tiles' losses, added in tile order
+__device__ __forceinline__ float loss_sum(const float* losspart, int nloss) {
+    const int lane = threadIdx.x & 31;
+    float s = 0.f;
+    for (int k0 = 0; k0 < nloss; k0 += 32) {
+        const float v = k0 + lane < nloss ? __ldcg(losspart + k0 + lane) : 0.f;
+        for (int k = 0; k < min(32, nloss - k0); ++k) s += __shfl_sync(0xffffffffu, v, k);
+    }
+    return s;
 }
 
 // One Adam step over every parameter, and the BF16 copies the next step's products read.  One
 // launch for the six blocks (they were six Adam launches, three copies and two transposes); the
-// loss of the step from its per-tile sums on the way.
+// loss of the step from its per-tile sums by the last CTA.  Parameters, moments and the places of the
+// gradients are older than the predecessor and come before the wait (64 training steps 2.31 -> 2.25 ms).
 __global__ void k_adam(ParamMap map, float* p, float* m, float* v, float lr,
                        float b1, float b2, float eps, float c1, float c2, const float* losspart, int nloss,
                        float inv, float* loss) {
-    pdl_wait();
-    pdl_go();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        float s = 0.f;
-        for (int k = 0; k < nloss; ++k) s += __ldcg(losspart + k);
-        *loss = s * inv;
+    const long w0 = (long)blockIdx.x * blockDim.x + threadIdx.x, step = (long)(gridDim.x - 1) * blockDim.x;
+    if (blockIdx.x == gridDim.x - 1) {
+        pdl_wait();
+        pdl_go();
+        if (threadIdx.x < 32) {
+            const float s = loss_sum(losspart, nloss);
+            if (threadIdx.x == 0) *loss = s * inv;
+        }
+        return;
     }
-    for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < map.total; w += (long)gridDim.x * blockDim.x) {
+    bool waited = false;
+    for (long w = w0; w < map.total; w += step) {
         __nv_bfloat16* copy;
-        const float gr = grad_of(map, w, &copy);
-        const float mm = b1 * __ldcg(m + w) + (1.f - b1) * gr;
-        const float vv = b2 * __ldcg(v + w) + (1.f - b2) * gr * gr;
+        const float* grad = grad_of(map, w, &copy);
+        const float mo = __ldcg(m + w), vo = __ldcg(v + w), po = __ldcg(p + w);
+        if (!waited) {
+            pdl_wait();
+            pdl_go();
+            waited = true;
+        }
+        const float gr = __ldcg(grad);
+        // roundings spelled out: training amplifies a last-bit difference, so they must not move with the code
+        const float mm = __fmaf_rn(1.f - b1, gr, __fmul_rn(b1, mo));
+        const float vv = __fmaf_rn(__fmul_rn(1.f - b2, gr), gr, __fmul_rn(b2, vo));
         m[w] = mm;
         v[w] = vv;
-        const float np = __ldcg(p + w) - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+        const float np = po - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
         p[w] = np;
         if (copy) *copy = __float2bfloat16_rn(np);
+    }
+    if (!waited) {
+        pdl_wait();
+        pdl_go();
     }
 }
 
 // gradients in the caller's flat layout, and the loss
 __global__ void k_gather(ParamMap map, const float* __restrict__ losspart, int nloss, float inv, float* __restrict__ out,
                          float* __restrict__ loss) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        float s = 0.f;
-        for (int k = 0; k < nloss; ++k) s += __ldcg(losspart + k);
-        *loss = s * inv;
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        const float s = loss_sum(losspart, nloss);
+        if (threadIdx.x == 0) *loss = s * inv;
     }
     for (long w = (long)blockIdx.x * blockDim.x + threadIdx.x; w < map.total; w += (long)gridDim.x * blockDim.x) {
         __nv_bfloat16* copy;
-        out[w] = grad_of(map, w, &copy);
+        out[w] = __ldcg(grad_of(map, w, &copy));
     }
 }
 
@@ -890,7 +926,7 @@ int loss_tiles(const rq_mlp* m, int B) { return ((B + 127) / 128 * 2) * ((m->out
 int mlp_adam(rq_mlp* m, int B, float lr, float b1, float b2, float eps) {
     m->step += 1;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    return launch_chained(m->stream, k_adam, rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)), 256, 0,
+    return launch_chained(m->stream, k_adam, rq::grid_for((uint64_t)m->nparam, 256, rq::num_sms(m->device)) + 1, 256, 0,
                           param_map(m), m->P, m->Mo, m->Vo, lr, b1, b2, eps, c1, c2, m->losspart, loss_tiles(m, B),
                           1.f / (float)(B * m->out), m->loss);
 }
