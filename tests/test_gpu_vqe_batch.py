@@ -156,3 +156,21 @@ def test_many_layers_with_tables_in_and_out_of_shared_memory(prec, n, depth):
     if n * depth <= 600:   # the adjoint kernel refuses the deeper ones
         _, grad = vb.run(params, gradient="adjoint")
         assert np.max(np.abs(grad[:, :2 * n] - wgrad)) <= tol
+
+
+@pytest.mark.parametrize("prec,n,depth,sets", [("f32", 8, 3, 3), ("f32", 14, 2, 5), ("f32", 16, 8, 3), ("f32", 20, 2, 8),
+                                               ("f32", 24, 2, 1), ("f64", 12, 3, 2), ("f64", 13, 3, 4), ("f64", 16, 3, 40)])
+def test_shift_rule_equals_explicitly_shifted_runs(prec, n, depth, sets):
+    """A shifted circuit begins with the sweep of its parameter, on the unshifted circuit's state: to the bit
+    what running it from the start gives.  One sweep and several; one wave and several; one group of sets
+    and several (20 qubits); a state too large to keep between the sweeps (24 qubits)."""
+    coeffs, strings = workloads.pauli_hamiltonian(n, 12, 3)
+    params = np.random.default_rng(n).uniform(-math.pi, math.pi, size=(sets, n * depth))
+    vb = VqeBatch(n, depth, coeffs, strings, prec)
+    e, g = vb.run(params, gradient="shift")
+    assert np.array_equal(e, vb.run(params))
+    for k in sorted({0, 1, n - 1, n, n * depth // 2, n * depth - n, n * depth - 1}):
+        up, dn = params.copy(), params.copy()
+        up[:, k] += math.pi / 2
+        dn[:, k] -= math.pi / 2
+        assert np.array_equal(g[:, k], (vb.run(up) - vb.run(dn)) / 2.0), k
