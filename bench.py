@@ -238,8 +238,9 @@ def qaoa_batch_leg(a, ws, rank, with_cpu):
                         "achieved": sweep_gbs, "peak": peak, "unit": "GB/s", "frac": sweep_gbs / peak,
                         "peak_kind": peak_kind, "bytes": prof["sweep_bytes"], "kernel_ms": prof["sweep_ms"],
                         "bytes_definition": "per circuit and sweep: S written by the initialising sweep, 2S "
-                                            "(read + write) for every other sweep; S = 2^n x 8 B"},
-           "sampling": {"kernels": "k_leaf_fold / k_fold / k_sample (1024 shots per circuit)",
+                                            "(read + write) for every other sweep; S = 2^(n-1) x 8 B, the half "
+                                            "of a state that its bit-flip symmetry leaves free"},
+           "sampling": {"kernels": "k_tree_leaf / k_tree_fold / k_tree_tail / k_bsample (1024 shots per circuit)",
                         "achieved_gbs": sample_gbs, "bytes": prof["sample_bytes"], "kernel_ms": prof["sample_ms"],
                         "frac": sample_gbs / peak},
            "device_ms_outside_kernels": dev_ms - prof["sweep_ms"] - prof["sample_ms"]}
@@ -333,8 +334,8 @@ def vqe_batch_leg(a, ws, rank, with_cpu):
            "energy_pass": {"kernel": "k_vqe_energy", "flops": prof["energy_flops"],
                            "kernel_ms": prof["energy_ms"],
                            "achieved_tflops": prof["energy_flops"] / (prof["energy_ms"] / 1e3) / 1e12,
-                           "flops_definition": "8 per Pauli string and amplitude: one complex product "
-                                               "conj(a[i^x]) a[i] and its FP64 accumulation (CUDA cores, FP32 "
+                           "flops_definition": "2 per Pauli string and pair of the ansatz's real amplitudes: one "
+                                               "product a[i^x] a[i] and its accumulation (CUDA cores, FP32 "
                                                "products, FP64 sums; no measured peak for this mix)"},
            "adjoint": {"device_ms": min(ams), "gradient_sets_per_s": len(params) * ws / (min(ams) / 1e3),
                        "kernel_ms": aprof["adjoint_ms"], "bytes": aprof["adjoint_bytes"],

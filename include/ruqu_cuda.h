@@ -500,8 +500,8 @@ RQ_API int rq_qaoa_batch_last_ms(const rq_qaoa_batch* b, float* ms);
  * kind (no counterpart in the reference): out6 = {sweep HBM bytes, sweep ms, sampling
  * bytes, sampling ms, adjoint bytes, adjoint ms}.  Bytes are algorithmic: per circuit
  * and sweep, S written by an initialising sweep and 2S for a read and a write otherwise
- * (two states in the adjoint pass), and per sampled circuit S + 2^n x 16 bytes for the
- * prefix tree; times are CUDA events around each class's launches. */
+ * (two states in the adjoint pass), and per sampled circuit S + 2^(n-1) x 16 bytes for the
+ * prefix tree, S being the 2^(n-1) amplitudes that are kept; times are CUDA events around each class's launches. */
 RQ_API int rq_qaoa_batch_last_profile(const rq_qaoa_batch* b, double* out6);
 
 /* CUDA graphs of the batched runs (rq_qaoa_batch_run / _gradient, rq_vqe_batch_run): the
@@ -554,8 +554,8 @@ RQ_API int rq_vqe_batch_run(rq_vqe_batch* b, uint32_t nsets, const double* param
 
 RQ_API int rq_vqe_batch_last_ms(const rq_vqe_batch* b, float* ms);
 /* As rq_qaoa_batch_last_profile for the last rq_vqe_batch_run: {evolution sweep bytes,
- * evolution ms, energy-pass floating-point operations (8 per string and amplitude),
- * energy ms, adjoint bytes (the H pass and the backward program over two states),
+ * evolution ms, energy-pass floating-point operations (2 per string and pair of the real
+ * amplitudes; strings with an odd number of Y factors need none), energy ms, adjoint bytes (the H pass and the backward program over two states),
  * adjoint ms}.  The waves are sized to stay in L2, so the sweep bytes are mostly L2
  * traffic.  No counterpart in the reference. */
 RQ_API int rq_vqe_batch_last_profile(const rq_vqe_batch* b, double* out6);

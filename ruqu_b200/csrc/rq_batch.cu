@@ -2683,9 +2683,9 @@ int vqe_wave(rq_vqe_batch* b, uint64_t ncirc, uint64_t circ0, uint64_t first, ui
     b->prof.end(ev, b->stream, 0, bytes);
     ev = b->prof.begin(b->stream);
     RQ_TRY(vqe_energy<T>(b, ncirc, circ0));
-    // per string and amplitude: one complex product conj(a[i ^ x]) a[i] (6 flops) and its
-    // FP64 accumulation (2 flops)
-    b->prof.end(ev, b->stream, 1, (double)ncirc * (double)b->nterms * (double)((size_t)1 << b->n) * 8.0);
+    // per string with an even number of Y factors (the others are zero in a real state) and pair of
+    // amplitudes: one product and its accumulation
+    b->prof.end(ev, b->stream, 1, (double)ncirc * (double)b->neterms * (double)((size_t)1 << b->n));
     return RQ_OK;
 }
 
