@@ -1812,18 +1812,15 @@ uint64_t structure_hash(const rq_gate* g, uint64_t n) {
     return h;
 }
 
-// device time of one execution of P on a scratch state shaped like t (after one warm-up run)
+// device time of one execution of P on a scratch state shaped like t
 int time_plan(const rq_state& t, const rq_plan* P, float* ms) {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     RQ_CUDA(cudaEventCreate(&e0));
     RQ_CUDA(cudaEventCreate(&e1));
     rq_state u = t;
+    cudaEventRecord(e0, t.stream);
     int rc = plan_launch(&u, P);
-    if (rc == RQ_OK) {
-        cudaEventRecord(e0, t.stream);
-        rc = plan_launch(&u, P);
-        cudaEventRecord(e1, t.stream);
-    }
+    cudaEventRecord(e1, t.stream);
     cudaError_t e = cudaEventSynchronize(e1);
     if (rc == RQ_OK && e != cudaSuccess) rc = cuda_fail(e, "autotune timing");
     if (rc == RQ_OK) cudaEventElapsedTime(ms, e0, e1);
@@ -1889,8 +1886,33 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cudaMemsetAsync(scratch, 0, s->bytes(), s->stream);
         const float one[2] = {1.f, 0.f};   // complex f32 amplitude 0 (pageable: staged before the call returns)
         cudaMemcpyAsync(scratch, one, sizeof(one), cudaMemcpyHostToDevice, s->stream);
-        for (size_t k = 0; k < cands.size() && rc == RQ_OK; ++k)
-            if (cands[k].plan) rc = time_plan(t, cands[k].plan, &cands[k].ms);
+        // Each candidate runs once to warm up and is then timed; a long first run that is already a quarter
+        // slower than the best is enough. Those within 10 % of the best are timed twice more in turn and
+        // count with their median: a single time each, taken while the clock was still settling under the
+        // power limit, picked the 14-qubit plan of a 30-qubit random-layer circuit (95.9 ms) before the
+        // 13-qubit one (90.9 ms) in one process of two.
+        float least = 0.f;
+        auto timed = [&](Cand& c) {
+            if (!c.plan || rc != RQ_OK) return;
+            rc = time_plan(t, c.plan, &c.ms);
+            if (rc == RQ_OK && !(c.ms > 50.f && least > 0.f && c.ms > 1.25f * least)) rc = time_plan(t, c.plan, &c.ms);
+            if (rc == RQ_OK && (least == 0.f || c.ms < least)) least = c.ms;
+        };
+        timed(cands[2]);   // the FP16 sweep first: the slow ones then need one run
+        for (size_t k = 0; k < cands.size(); ++k)
+            if (k != 2) timed(cands[k]);
+        std::vector<std::vector<float>> again(cands.size());
+        for (int round = 0; round < 2; ++round)
+            for (size_t k = 0; k < cands.size() && rc == RQ_OK; ++k)
+                if (cands[k].plan && cands[k].ms <= 1.1f * least) {
+                    float ms = 0.f;
+                    rc = time_plan(t, cands[k].plan, &ms);
+                    again[k].push_back(ms);
+                }
+        for (size_t k = 0; k < cands.size(); ++k)
+            if (again[k].size() == 2)
+                cands[k].ms = std::max(std::min(again[k][0], again[k][1]),
+                                       std::min(std::max(again[k][0], again[k][1]), cands[k].ms));
         // a later candidate must be more than 2 % faster than the best so far: near-equal plans
         // (the 12- and 13-qubit FP16 plans of a 30-qubit random-layer circuit are within 1 %)
         // then keep the earlier one, which has fewer sweeps, instead of following timing noise
