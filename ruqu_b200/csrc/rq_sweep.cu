@@ -1024,6 +1024,8 @@ __device__ __forceinline__ bool wait_sleep(uint64_t* bar, uint32_t parity, uint3
 // while the first is scattered, and the split's residual in mixed precision: 30 qubits, 20 random layers,
 // 94.5 -> 93.3 ms (12 local qubits), 92.5 -> 90.9 (13), 97.0 -> 95.9 (14); 27 qubits 9.77 -> 9.55, 10.40 ->
 // 10.25, 10.97 -> 10.85.  Two threads a row with 64 registers each (32 warps an SM) took 109 ms in all three.
+// Fewer address instructions a tile (next tile's base by one addition, constant offsets): 91.3 -> 89.3 ms with
+// 13 local qubits, 95.9 -> 92.9 with 14, 93.6 -> 92.9 with 12.
 template <int NTHR>
 __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restrict__ amps, const SweepDesc d,
                                                      const PhaseDesc* __restrict__ phases,
@@ -1044,6 +1046,7 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
     __shared__ uint32_t tmem_base;
     __shared__ float wmax[NTHR / 32], wsum[NTHR / 32], wsum2[NTHR / 32];
     __shared__ int half_failed[NTHR / 128];
+    __shared__ uint64_t walk[2];   // the tile's own bits; the grid's size spread over the others
 
     const uint32_t tid = threadIdx.x;
     const uint32_t T_ = blockDim.x;
@@ -1059,6 +1062,12 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
+        uint64_t own = 0, step = 0;
+        for (uint32_t k = 0; k < d.m; ++k) own |= 1ull << d.local_global[k];
+        for (uint32_t k = 0; k < d.nonlocal_count; ++k)
+            if (((uint64_t)gridDim.x >> k) & 1u) step |= 1ull << d.nonlocal[k];
+        walk[0] = own;
+        walk[1] = step;
         for (int k = 0; k < NTHR / 128; ++k) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_u32(&mbar[k])), "r"(1u) : "memory");
             half_failed[k] = 0;
@@ -1116,8 +1125,21 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
     }
     for (; tile < ntiles && !failed; tile += gridDim.x) {
         const uint64_t next = tile + gridDim.x;
-        const uint64_t nbase = next < ntiles ? tile_base(next) : 0;
-        issue_tile<float>(sm, amps, d, base, dep_tid, stid);
+        // the grid's size added to the tile number, with the tile's own bits set for the carries to pass
+        const uint64_t nbase = next < ntiles ? ((base | walk[0]) + walk[1]) & ~walk[0] : 0;
+        // one base address and constant offsets take fewer instructions than OR-ing each index; in the
+        // 128-thread kernel they cost registers that it lacks (27 qubits: 9.57 -> 9.72 ms)
+        if constexpr (ONE_BUF) {
+            issue_tile<float>(sm, amps, d, base, dep_tid, stid);
+        } else {
+            const float2* mine = amps + (base | dep_tid);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const uint32_t se = stid ^ d.sgj[j];
+                cp_async8(sm + se, mine + d.gj[j]);
+                cp_async8(sm + (se ^ 1u), mine + d.gj[j] + 1);
+            }
+        }
         cp_async_commit();
         if (next < ntiles) {
             // Pull the next tile into L2 while this one runs its phases: thread t prefetches the
@@ -1322,9 +1344,9 @@ __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restr
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const uint32_t se = stid ^ d.sgj[j];
-            const uint64_t g = base | dep_tid | d.gj[j];
+            float2* g = ONE_BUF ? amps + (base | dep_tid | d.gj[j]) : amps + (base | dep_tid) + d.gj[j];
             const float2 a = tc16::mul2(sm[se], fix2), b = tc16::mul2(sm[se ^ 1u], fix2);
-            __stcs(reinterpret_cast<VV*>(amps + g), make_float4(a.x, a.y, b.x, b.y));
+            __stcs(reinterpret_cast<VV*>(g), make_float4(a.x, a.y, b.x, b.y));
         }
         __syncthreads();
         base = nbase;

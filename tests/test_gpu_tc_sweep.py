@@ -292,3 +292,20 @@ def test_tiled_plan_rejects_bad_tile_sizes():
             rq.Plan(g, gates, mode, local_qubits=lq)
     with pytest.raises(rq.InvalidArgument):
         rq.Plan(QuantumState(16, 0, "f64"), gates, rq.RQ_EXEC_SWEEP_TC16, local_qubits=13)
+
+
+@pytest.mark.parametrize("n", [22, 23])
+@pytest.mark.parametrize("lq", [12, 13, 14])
+def test_tc16_ctas_walk_several_tiles(lq, n):
+    """Several tiles for every CTA (at least 256 tiles of 14 local qubits on 148 CTAs), so that the step
+    from a tile to the next carries across the qubits outside it: against the complex f64 sweep of the same
+    circuit, in the 2-norm.  A phase rounds to about 2^-21 of the norm (22-bit operands, FP32 sums); at most
+    60 phases: 3e-5."""
+    gates = workloads.random_layer_circuit(n, 6, 11)
+    ref = rq.QuantumState(n, 0, "f64")
+    rq.Plan(ref, gates).execute(ref)
+    st = rq.QuantumState(n, 0, "f32")
+    plan = rq.Plan(st, gates, rq.RQ_EXEC_SWEEP_TC16, local_qubits=lq)
+    assert plan.stats()["dense_ops"] <= 60
+    plan.execute(st)
+    assert np.linalg.norm(st.state_vector() - ref.state_vector()) < 3e-5
