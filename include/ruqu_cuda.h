@@ -378,7 +378,9 @@ RQ_API int rq_state_expectation_hamiltonian(rq_state* s, const double* coeffs,
  *   - runs on `stream` (a cudaStream_t, NULL = the legacy default stream) on
  *     the current device; it blocks the host: it copies the sums back and
  *     synchronises `stream` before it returns with the results in out[];
- *   - a NULL `ops` with a non-empty string is rejected (RQ_ERR_INVALID_ARGUMENT).
+ *   - a NULL `ops` with a non-empty string is rejected (RQ_ERR_INVALID_ARGUMENT);
+ *   - device_amps needs the alignment of an amplitude (8 bytes f32, 16 bytes f64; any
+ *     other address is rejected); f32 at 16 bytes is read with wider loads.
  * It calls no cudaMalloc / cudaFree and no allocating library routine. */
 #define RQ_NOALLOC_MAX_STRINGS 128u
 #define RQ_NOALLOC_MAX_BLOCKS 1024u

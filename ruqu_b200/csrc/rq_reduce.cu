@@ -129,7 +129,22 @@ template <typename T> struct Vec16;
 template <> struct Vec16<float> { using t = float4; };
 template <> struct Vec16<double> { using t = double2; };
 
-template <typename T, int KT>
+// 16 bytes of amplitudes (two f32, one f64).  PAIRS: a caller's f32 array that is only 8-byte aligned
+// (rq_expectation_batch_noalloc), two loads of 8 bytes.
+template <bool PAIRS>
+__device__ __forceinline__ float4 load16(const float4* p) {
+    if constexpr (PAIRS) {
+        const float2 x = __ldcs(reinterpret_cast<const float2*>(p)), y = __ldcs(reinterpret_cast<const float2*>(p) + 1);
+        return make_float4(x.x, x.y, y.x, y.y);
+    }
+    return __ldcs(p);
+}
+template <bool PAIRS>
+__device__ __forceinline__ double2 load16(const double2* p) {
+    return __ldcs(p);
+}
+
+template <typename T, int KT, bool PAIRS>
 __global__ void __launch_bounds__(ZT, KT > 16 ? 2 : 3) k_pauli_z(const typename C2<T>::t* __restrict__ a, uint64_t ntiles,
                                                    const __grid_constant__ ZPasses zp, double* __restrict__ partials,
                                                    uint32_t stride) {
@@ -151,7 +166,7 @@ __global__ void __launch_bounds__(ZT, KT > 16 ? 2 : 3) k_pauli_z(const typename 
         if constexpr (F) {   // register bit 0 = element bit 0, register bits 1-3 = element bits 9-11
             VV v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = __ldcs(src + u * ZT + tid);
+            for (int u = 0; u < 8; ++u) v[u] = load16<PAIRS>(src + u * ZT + tid);
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 p[2 * u] = (double)v[u].x * v[u].x + (double)v[u].y * v[u].y;
@@ -160,7 +175,7 @@ __global__ void __launch_bounds__(ZT, KT > 16 ? 2 : 3) k_pauli_z(const typename 
         } else {             // register bits 0-3 = element bits 8-11
             VV v[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) v[u] = __ldcs(src + u * ZT + tid);
+            for (int u = 0; u < 16; ++u) v[u] = load16<PAIRS>(src + u * ZT + tid);
 #pragma unroll
             for (int u = 0; u < 16; ++u) p[u] = v[u].x * v[u].x + v[u].y * v[u].y;
         }
@@ -271,7 +286,7 @@ __device__ __forceinline__ double span_string(const double* ar, const double* ai
     return span_walk<T, RB, -1, ODD>(ar, ai, tile, tid, s);
 }
 
-template <typename T>
+template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(ST, 1) k_pauli_span(const typename C2<T>::t* __restrict__ a, uint32_t tile_bits,
                                                       const __grid_constant__ SpanPasses sp,
                                                       double* __restrict__ partials, uint32_t stride) {
@@ -304,7 +319,13 @@ __global__ void __launch_bounds__(ST, 1) k_pauli_span(const typename C2<T>::t* _
             if (j & 2) g ^= P.basis[6];
             if (j & 4) g ^= P.basis[7];
             const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + (((tid >> 4) + 32 * j) << C) + piece);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(a + g + piece) : "memory");
+            const V* p = a + g + piece;
+            if constexpr (PAIRS) {   // 8-byte aligned f32 (load16)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(p) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + 8), "l"(p + 1) : "memory");
+            } else {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(p) : "memory");
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -516,7 +537,7 @@ void plan_strings(uint32_t n, int32_t prec, int sms, const rq::PauliMask* terms,
     P.stride = std::max(P.zblocks, P.sblocks);
 }
 
-template <typename T>
+template <typename T, bool PAIRS>
 int launch_strings_t(const PauliPlan& P, const void* amps, uint32_t n, cudaStream_t st, double* partials, double* out) {
     using V = typename C2<T>::t;
     const V* a = (const V*)amps;
@@ -547,19 +568,19 @@ int launch_strings_t(const PauliPlan& P, const void* amps, uint32_t n, cudaStrea
             }
         }
         double* part = partials + (size_t)p0 * ZK * P.stride;
-        auto kern = nz <= 8 ? k_pauli_z<T, 8> : nz <= 16 ? k_pauli_z<T, 16> : k_pauli_z<T, ZK>;
+        auto kern = nz <= 8 ? k_pauli_z<T, 8, PAIRS> : nz <= 16 ? k_pauli_z<T, 16, PAIRS> : k_pauli_z<T, ZK, PAIRS>;
         kern<<<dim3(P.zblocks, np), ZT, 0, st>>>(a, 1ull << (n - 12), zp, part, P.stride);
         RQ_CUDA(cudaGetLastError());
     }
     constexpr int smem = 2 * (1 << (SpanShape<T>::C + 8)) * (int)sizeof(V) + SK * ST * (int)sizeof(double);
     if (!P.spans.empty())
-        RQ_CUDA(cudaFuncSetAttribute(k_pauli_span<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        RQ_CUDA(cudaFuncSetAttribute(k_pauli_span<T, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     for (size_t p0 = 0; p0 < P.spans.size(); p0 += SPASSES) {
         SpanPasses sp{};
         const size_t np = std::min<size_t>(SPASSES, P.spans.size() - p0);
         for (size_t p = 0; p < np; ++p) sp.p[p] = P.spans[p0 + p];
-        k_pauli_span<T><<<dim3(P.sblocks, (unsigned)np), ST, smem, st>>>(a, n - SpanShape<T>::C - 8, sp, partials,
-                                                                       P.stride);
+        k_pauli_span<T, PAIRS><<<dim3(P.sblocks, (unsigned)np), ST, smem, st>>>(a, n - SpanShape<T>::C - 8, sp, partials,
+                                                                              P.stride);
         RQ_CUDA(cudaGetLastError());
     }
     k_finalize<<<P.rows, TPB, 0, st>>>(partials, nz, P.zblocks, P.sblocks, P.stride, out);
@@ -571,8 +592,9 @@ int launch_strings_t(const PauliPlan& P, const void* amps, uint32_t n, cudaStrea
 // P.rows * P.stride doubles
 int launch_strings(const PauliPlan& P, const void* amps, uint32_t n, int32_t prec, cudaStream_t st, double* partials,
                    double* out) {
-    return prec == RQ_F32 ? launch_strings_t<float>(P, amps, n, st, partials, out)
-                          : launch_strings_t<double>(P, amps, n, st, partials, out);
+    if (prec != RQ_F32) return launch_strings_t<double, false>(P, amps, n, st, partials, out);
+    return reinterpret_cast<uintptr_t>(amps) % 16 == 0 ? launch_strings_t<float, false>(P, amps, n, st, partials, out)
+                                                       : launch_strings_t<float, true>(P, amps, n, st, partials, out);
 }
 
 }  // namespace
@@ -696,6 +718,9 @@ extern "C" int rq_expectation_batch_noalloc(const void* device_amps, uint32_t nu
                                                      std::to_string(RQ_NOALLOC_MAX_STRINGS) + " Pauli strings per call, got " +
                                                      std::to_string(nstrings));
     if (nstrings == 0) return RQ_OK;
+    const size_t align = precision == RQ_F32 ? sizeof(float2) : sizeof(double2);
+    if (reinterpret_cast<uintptr_t>(device_amps) % align)   // a load would fault
+        return rq::fail(RQ_ERR_INVALID_ARGUMENT, "device_amps must be aligned to an amplitude (" + std::to_string(align) + " bytes)");
     if (!ops && offsets[nstrings] > offsets[0]) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "null pointer");
     // Pauli strings in mask form (same rules as rq_state_expectation_batch)
     std::vector<rq::PauliMask> terms(nstrings);
