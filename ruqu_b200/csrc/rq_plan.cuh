@@ -1065,13 +1065,21 @@ inline void merge_ladders(const std::vector<SweepDesc>& descs, std::vector<Phase
     ops.swap(out);
 }
 
+// Phases that one batched sweep may have: their descriptors lie in shared memory after the tile of 2^m
+// elements (227 KB a CTA, 2 KB of it static).  Only an ansatz whose state is a single tile gets there:
+// 643 phases for 2^13 f32 or 2^12 f64 elements, about 570 layers of 14 qubits f32 or 420 of 13 f64.
+// symmetric_program needs no cut: at most 64 layers of four phases.
+inline uint32_t sweep_phase_limit(uint32_t m, uint32_t epv) {
+    return (uint32_t)(((227u << 10) - 2048u - ((16u / epv) << m)) / sizeof(PhaseDesc));
+}
+
 // The sweeps of a list of Ry and CZ gates on n qubits for the packed real state of n - 1 (qubit
 // q > 0 is its qubit q - 1, qubit 0 its two parts).  The gates are planned as sweeps over the
 // 2^n amplitudes (mloc local qubits) and run in exactly that order, so every amplitude goes
 // through the same roundings as unpacked: planning the packed gates afresh saves a sweep in four
 // on 16 qubits (5.5 instead of 5.8 ms for 2056 circuits) but its other order of the rotations moves
 // single f32 energies by their whole rounding error.  The order is cut into sweeps of m local packed
-// qubits and phases of rb slots; qubit 0 needs neither.
+// qubits and phases of rb slots; qubit 0 needs neither.  A cut moves no gate, so it changes no result.
 inline void packed_program(const std::vector<PGate>& gates, uint32_t n, uint32_t mloc, uint32_t m, uint32_t rb, uint32_t epv,
                     std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
     const uint32_t m0 = std::min(n, mloc), c = std::min<uint32_t>(m, 5);
@@ -1092,11 +1100,14 @@ inline void packed_program(const std::vector<PGate>& gates, uint32_t n, uint32_t
                 order.push_back(g);
             }
     const uint64_t base = (1ull << c) - 1;
+    const uint32_t limit = sweep_phase_limit(m, epv);
     std::vector<Sweep> sweeps;
     std::vector<std::vector<PhasePlan>> pplans;
     for (const auto& g : order) {
         const uint64_t nd = needs(g);
-        if (sweeps.empty() || (uint32_t)__builtin_popcountll(sweeps.back().L | nd) > m) {
+        const bool full = !sweeps.empty() && pplans.back().size() == limit &&
+                          (uint32_t)__builtin_popcountll(pplans.back().back().R | nd) > rb;
+        if (sweeps.empty() || full || (uint32_t)__builtin_popcountll(sweeps.back().L | nd) > m) {
             sweeps.push_back(Sweep{base, {}});
             pplans.push_back({PhasePlan{0, {}}});
         }
