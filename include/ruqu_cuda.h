@@ -209,6 +209,10 @@ RQ_API int rq_state_synchronize(rq_state* s);
 #define RQ_WAIT_LIMIT_DEFAULT 0xFFFFFFFFu
 RQ_API int rq_debug_set_wait_limit(uint32_t polls);
 
+/* What destroyed states have left for later ones (rq_state_destroy): the number of sets of
+ * resources and their device and pinned bytes.  No counterpart in the reference. */
+RQ_API int rq_debug_state_pool(uint64_t* sets, uint64_t* bytes);
+
 /* ------------------------------------------------------------------------ */
 /* gates (state.rs:158-276)                                                  */
 /* ------------------------------------------------------------------------ */

@@ -68,6 +68,7 @@ SIGNATURES = {
     "rq_state_device_ptr": (C.c_int, [_vp, _P(_vp), _P(_vp)]),
     "rq_state_synchronize": (C.c_int, [_vp]),
     "rq_debug_set_wait_limit": (C.c_int, [_u32]),
+    "rq_debug_state_pool": (C.c_int, [_P(_u64), _P(_u64)]),
     "rq_state_apply": (C.c_int, [_vp, _P(RqGate), _u64, _P(RqMeasurement), _u64, _P(_u64)]),
     "rq_state_apply_mode": (C.c_int, [_vp, _P(RqGate), _u64, _i32, _P(RqMeasurement), _u64, _P(_u64)]),
     "rq_state_apply_noisy": (C.c_int, [_vp, _P(RqGate), _u64, _P(RqNoiseModel), _P(RqMeasurement), _u64, _P(_u64)]),

@@ -107,7 +107,7 @@ int check_create(uint32_t nq, int32_t prec) {
 // evaluate_qaoa_cost, run_shots) spent 3-30 ms per evaluation in cudaMalloc, cudaFree,
 // cudaMallocHost, cudaFreeHost and stream creation -- the calls serialise with every process on
 // the machine's GPUs -- against 0.2 ms on the device.  Bounds: POOL_ENTRIES sets, POOL_STATE_BYTES
-// of device memory each, POOL_TOTAL_BYTES in all; sets unused for POOL_IDLE_S are freed at the next
+// of memory each (device and pinned), POOL_TOTAL_BYTES in all; sets unused for POOL_IDLE_S are freed at the next
 // create or destroy, all of them when an allocation fails (device_malloc).  A set enters the pool
 // with its stream drained, and never with amplitudes whose device pointer was handed out
 // (rq_state_device_ptr): another stream may still use those.
@@ -122,7 +122,7 @@ struct PoolEntry {
     unsigned long long ctx = 0;       // context they belong to
     double since = 0.0;
     size_t bytes() const {
-        return (r.amps ? r.amps_cap : 0) + r.scratch_cap + (r.partials_cap + r.tree_cap) * sizeof(double);
+        return (r.amps ? r.amps_cap : 0) + r.scratch_cap + (r.partials_cap + r.tree_cap + r.hbuf_cap) * sizeof(double);
     }
 };
 
@@ -1096,6 +1096,16 @@ int rq_state_fidelity(rq_state* a, rq_state* b, double* out) {
     double re = 0, im = 0;
     RQ_TRY(rq::inner(a, b, &re, &im));
     *out = re * re + im * im;
+    return RQ_OK;
+}
+
+int rq_debug_state_pool(uint64_t* sets, uint64_t* bytes) {
+    std::lock_guard<std::mutex> lk(pool().mu);
+    if (sets) *sets = pool().entries.size();
+    if (bytes) {
+        *bytes = 0;
+        for (const auto& e : pool().entries) *bytes += e.bytes();
+    }
     return RQ_OK;
 }
 

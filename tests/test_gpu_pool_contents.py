@@ -1,0 +1,109 @@
+"""What the pool of destroyed states' resources holds (needs a GPU; rq_debug_state_pool).
+
+An ordinary state leaves one set; one whose device pointer was handed out leaves none, since another
+stream may still use its memory; the sets stay within 16, 64 MiB each and 256 MiB in all.
+"""
+import contextlib
+import ctypes as C
+import gc
+
+import numpy as np
+import pytest
+
+import ruqu_b200 as rq
+from ruqu_b200 import _capi
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+def _pool():
+    sets, size = C.c_uint64(), C.c_uint64()
+    assert _capi.lib.rq_debug_state_pool(C.byref(sets), C.byref(size)) == _capi.RQ_OK
+    return sets.value, size.value
+
+
+@contextlib.contextmanager
+def little_memory(leave=64 * MIB):
+    """The rest of the device's memory taken, but for less than `leave` bytes."""
+    from cuda.bindings import runtime as rt
+    taken = []
+    try:
+        for chunk in (1 << 30, leave // 2):
+            while rt.cudaMemGetInfo()[1] >= chunk + leave // 2:
+                err, ptr = rt.cudaMalloc(chunk)
+                if int(err) != 0:
+                    break
+                taken.append(ptr)
+        yield rt.cudaMemGetInfo()[1]
+    finally:
+        for ptr in taken:
+            rt.cudaFree(ptr)
+
+
+def test_only_memory_that_was_not_handed_out_is_kept():
+    held = [rq.QuantumState(3, 0, "f64") for _ in range(17)]   # takes what small states left
+    st = rq.QuantumState(10, 1, "f64")
+    before = _pool()[0]
+    st.device_pointer()
+    del st
+    gc.collect()
+    assert _pool()[0] == before
+    st = rq.QuantumState(10, 1, "f64")
+    before = _pool()[0]
+    del st
+    gc.collect()
+    assert _pool()[0] == before + 1
+    del held
+
+
+def test_limits():
+    states = [rq.QuantumState(20, 1, "f64") for _ in range(18)]        # 16 MiB each
+    del states
+    gc.collect()
+    sets, size = _pool()
+    assert 0 < sets <= 16 and size <= 256 * MIB
+    states = [rq.QuantumState(4, 1, "f64") for _ in range(40)]
+    del states
+    gc.collect()
+    sets, size = _pool()
+    assert sets == 16 and size <= 256 * MIB
+    before = _pool()
+    big = rq.QuantumState(23, 1, "f64")                                # 128 MiB: its amplitudes are not kept
+    big.norm_sq()
+    del big
+    gc.collect()
+    assert _pool()[1] <= before[1] + MIB
+
+
+def test_pinned_staging_counts():
+    """2^20 + 1 Pauli strings need 8 MiB of pinned results."""
+    with little_memory():
+        with pytest.raises(rq.MemoryAllocationFailed):
+            rq.QuantumState(26, 1, "f64")
+    assert _pool() == (0, 0)
+    st = rq.QuantumState(1, 1, "f64")
+    count = (1 << 20) + 1
+    off = np.zeros(count + 1, dtype=np.uint32)
+    out = np.zeros(count)
+    ops = (_capi.RqPauliOp * 1)()
+    rc = _capi.lib.rq_state_expectation_batch(st.handle, ops, off.ctypes.data_as(C.POINTER(C.c_uint32)), count,
+                                              out.ctypes.data_as(C.POINTER(C.c_double)))
+    assert rc == 0 and np.all(out == 1.0)
+    del st
+    gc.collect()
+    assert _pool()[1] >= 8 * MIB
+
+
+def test_a_failed_allocation_empties_the_pool():
+    held = [rq.QuantumState(14, 1, "f64") for _ in range(4)]
+    del held
+    gc.collect()
+    assert _pool()[0] >= 4
+    with little_memory() as free:
+        assert free < 128 * MIB
+        with pytest.raises(rq.MemoryAllocationFailed):
+            rq.QuantumState(26, 1, "f64")                              # 1 GiB
+        assert _pool()[0] == 0
+    assert rq.QuantumState(26, 1, "f64").norm_sq() == 1.0
