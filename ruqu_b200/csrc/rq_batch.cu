@@ -1842,7 +1842,7 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
         std::vector<unsigned char> host(total);
         std::memcpy(host.data(), phases.data(), phases.size() * sizeof(PhaseDesc));
         std::memcpy(host.data() + K.off_ops, ops.data(), ops.size() * sizeof(SwOp));
-        RQ_CUDA(cudaMalloc((void**)&K.prog, total));
+        RQ_CUDA(rq::device_malloc((void**)&K.prog, total));
         RQ_CUDA(cudaMemcpy(K.prog, host.data(), total, cudaMemcpyHostToDevice));
         {
             // adjoint: per layer in reverse, Rx^-1 on every qubit, then the inverse cost phase
@@ -1873,20 +1873,20 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
             std::vector<unsigned char> ah(atotal);
             std::memcpy(ah.data(), aph.data(), aph.size() * sizeof(PhaseDesc));
             std::memcpy(ah.data() + K.aoff_ops, aops.data(), aops.size() * sizeof(SwOp));
-            RQ_CUDA(cudaMalloc((void**)&K.aprog, atotal));
+            RQ_CUDA(rq::device_malloc((void**)&K.aprog, atotal));
             RQ_CUDA(cudaMemcpy(K.aprog, ah.data(), atotal, cudaMemcpyHostToDevice));
         }
         b->classes.push_back(std::move(K));
     }
     // graph data
     if (ed.empty()) ed.push_back(0);
-    RQ_CUDA(cudaMalloc((void**)&b->d_edges, ed.size()));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_edges, ed.size()));
     RQ_CUDA(cudaMemcpy(b->d_edges, ed.data(), ed.size(), cudaMemcpyHostToDevice));
     std::vector<uint32_t> eoff(ninst + 1, 0);
     for (uint32_t k = 0; k < ninst; ++k) eoff[k + 1] = eoff[k] + b->ne_of[k];
-    RQ_CUDA(cudaMalloc((void**)&b->d_eoff, (ninst + 1) * sizeof(uint32_t)));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_eoff, (ninst + 1) * sizeof(uint32_t)));
     RQ_CUDA(cudaMemcpy(b->d_eoff, eoff.data(), (ninst + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    RQ_CUDA(cudaMalloc((void**)&b->d_ne, std::max<uint32_t>(1, ninst) * sizeof(uint32_t)));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_ne, std::max<uint32_t>(1, ninst) * sizeof(uint32_t)));
     if (ninst) RQ_CUDA(cudaMemcpy(b->d_ne, b->ne_of.data(), ninst * sizeof(uint32_t), cudaMemcpyHostToDevice));
     std::vector<uint64_t> nbr((size_t)std::max<uint32_t>(1, ninst) * NBR_STRIDE, 0);
     for (uint32_t k = 0; k < ninst; ++k)
@@ -1895,7 +1895,7 @@ int rq_qaoa_batch_create(uint32_t ninst, const uint32_t* num_nodes, const uint32
             nbr[(size_t)k * NBR_STRIDE + u] |= 1ull << v;
             nbr[(size_t)k * NBR_STRIDE + v] |= 1ull << u;
         }
-    RQ_CUDA(cudaMalloc((void**)&b->d_nbr, nbr.size() * sizeof(uint64_t)));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_nbr, nbr.size() * sizeof(uint64_t)));
     RQ_CUDA(cudaMemcpy(b->d_nbr, nbr.data(), nbr.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
     // the copies above (from pageable memory) may return before their DMA lands, and the
     // batch's stream is not ordered after them: wait here, once, before any run
@@ -2893,11 +2893,11 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
     };
     if (precision == RQ_F32) pack(0.0f);
     else pack(0.0);
-    RQ_CUDA(cudaMalloc((void**)&b->d_sofs, sofs.size() * sizeof(uint32_t)));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_sofs, sofs.size() * sizeof(uint32_t)));
     RQ_CUDA(cudaMemcpy(b->d_sofs, sofs.data(), sofs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    RQ_CUDA(cudaMalloc((void**)&b->d_segs, segs.size() * sizeof(PSeg)));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_segs, segs.size() * sizeof(PSeg)));
     RQ_CUDA(cudaMemcpy(b->d_segs, segs.data(), segs.size() * sizeof(PSeg), cudaMemcpyHostToDevice));
-    RQ_CUDA(cudaMalloc(&b->d_terms, dterms.size()));
+    RQ_CUDA(rq::device_malloc(&b->d_terms, dterms.size()));
     RQ_CUDA(cudaMemcpy(b->d_terms, dterms.data(), dterms.size(), cudaMemcpyHostToDevice));
     // the ansatz program
     const uint32_t mloc = precision == RQ_F32 ? 13u : 12u;
@@ -2938,14 +2938,14 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
             }
         b->upto.push_back((uint32_t)b->order.size());
     }
-    RQ_CUDA(cudaMalloc((void**)&b->d_order, std::max<size_t>(1, b->order.size()) * sizeof(uint32_t)));
+    RQ_CUDA(rq::device_malloc((void**)&b->d_order, std::max<size_t>(1, b->order.size()) * sizeof(uint32_t)));
     RQ_CUDA(cudaMemcpy(b->d_order, b->order.data(), b->order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     b->off_ops = (phases.size() * sizeof(PhaseDesc) + 255) & ~size_t(255);
     const size_t total = b->off_ops + opsv.size() * sizeof(SwOp);
     std::vector<unsigned char> host(total);
     std::memcpy(host.data(), phases.data(), phases.size() * sizeof(PhaseDesc));
     std::memcpy(host.data() + b->off_ops, opsv.data(), opsv.size() * sizeof(SwOp));
-    RQ_CUDA(cudaMalloc((void**)&b->prog, total));
+    RQ_CUDA(rq::device_malloc((void**)&b->prog, total));
     RQ_CUDA(cudaMemcpy(b->prog, host.data(), total, cudaMemcpyHostToDevice));
     {
         // the adjoint program: per layer in reverse, the CZ ladder, then Ry^-1 on every qubit
@@ -2966,7 +2966,7 @@ int rq_vqe_batch_create(uint32_t num_qubits, uint32_t depth, const double* coeff
         std::vector<unsigned char> ah(atotal);
         std::memcpy(ah.data(), aph.data(), aph.size() * sizeof(PhaseDesc));
         std::memcpy(ah.data() + b->aoff_ops, aops.data(), aops.size() * sizeof(SwOp));
-        RQ_CUDA(cudaMalloc((void**)&b->aprog, atotal));
+        RQ_CUDA(rq::device_malloc((void**)&b->aprog, atotal));
         RQ_CUDA(cudaMemcpy(b->aprog, ah.data(), atotal, cudaMemcpyHostToDevice));
     }
     RQ_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));

@@ -176,6 +176,13 @@ void pool_drop(F drop) {
     cudaSetDevice(cur);
 }
 
+// all of it back, after an allocation failed (whose error is cleared)
+bool pool_release() {
+    cudaGetLastError();
+    pool_drop([](const PoolEntry&) { return true; });
+    return true;
+}
+
 void pool_drop_idle() {
     const double t = now_s();
     pool_drop([t](const PoolEntry& e) { return t - e.since > POOL_IDLE_S; });
@@ -444,7 +451,9 @@ int ensure_tree(rq_state* s, size_t nd) {
 
 int scratch_get(rq_state* s, size_t bytes, void** out) {
     if (bytes > SCRATCH_KEEP_BYTES) {
-        RQ_CUDA(cudaMallocAsync(out, bytes, s->stream));
+        cudaError_t e = cudaMallocAsync(out, bytes, s->stream);
+        if (e == cudaErrorMemoryAllocation && pool_release()) e = cudaMallocAsync(out, bytes, s->stream);
+        RQ_CUDA(e);
         return RQ_OK;
     }
     if (s->scratch_cap < bytes) {
@@ -469,10 +478,8 @@ void scratch_put(rq_state* s, void* p) {
 
 cudaError_t device_malloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
-    pool_drop([](const PoolEntry&) { return true; });
-    return cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && pool_release()) e = cudaMalloc(p, bytes);
+    return e;
 }
 
 // Unique id of the current CUDA context (cuCtxGetId, reached through the runtime's

@@ -570,9 +570,9 @@ int rq_gemm_bf16(const uint16_t* A, const uint16_t* B, int32_t M, int32_t N, int
     if (!A || !B || !C) return rq::fail(RQ_ERR_INVALID_ARGUMENT, "null pointer");
     __nv_bfloat16 *dA = nullptr, *dB = nullptr;
     float* dC = nullptr;
-    RQ_CUDA(cudaMalloc(&dA, (size_t)M * K * 2));
-    RQ_CUDA(cudaMalloc(&dB, (size_t)N * K * 2));
-    RQ_CUDA(cudaMalloc(&dC, (size_t)M * N * 4));
+    RQ_CUDA(rq::device_malloc((void**)&dA, (size_t)M * K * 2));
+    RQ_CUDA(rq::device_malloc((void**)&dB, (size_t)N * K * 2));
+    RQ_CUDA(rq::device_malloc((void**)&dC, (size_t)M * N * 4));
     int rc = RQ_OK;
     cudaError_t e = cudaMemcpy(dA, A, (size_t)M * K * 2, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(dB, B, (size_t)N * K * 2, cudaMemcpyHostToDevice);

@@ -1675,7 +1675,7 @@ int plan_build(const rq_state* s, const rq_gate* gates, uint64_t n, int32_t mode
     // Upload in stream order on the state's stream: a synchronous copy from pageable memory may
     // return before its DMA lands, and the state's stream (non-blocking) is not ordered after
     // the legacy stream, so the kernels below could otherwise read the tables half-written.
-    cudaError_t e = cudaMalloc((void**)&P->dev, total);
+    cudaError_t e = device_malloc((void**)&P->dev, total);
     if (e == cudaSuccess) e = cudaMemcpyAsync(P->dev, host.data(), total, cudaMemcpyHostToDevice, s->stream);
     if (e != cudaSuccess) {
         if (P->dev) {
@@ -1899,7 +1899,7 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
     const bool any_tc = std::any_of(cands.begin() + 1, cands.end(), [](const Cand& c) {
         return c.plan && c.plan->stats.dense_ops > 0;
     });
-    if (any_tc && cudaMalloc(&scratch, s->bytes()) == cudaSuccess) {
+    if (any_tc && device_malloc(&scratch, s->bytes()) == cudaSuccess) {
         rq_state t = *s;
         t.amps = scratch;
         // |0...0>: the circuit's first layers spread it into a dense state, so the candidates are

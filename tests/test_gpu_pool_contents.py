@@ -107,3 +107,29 @@ def test_a_failed_allocation_empties_the_pool():
             rq.QuantumState(26, 1, "f64")                              # 1 GiB
         assert _pool()[0] == 0
     assert rq.QuantumState(26, 1, "f64").norm_sq() == 1.0
+
+
+def test_calls_that_need_memory_get_what_the_pool_holds():
+    """Scratch above 64 MiB (stream-ordered), the tuner's scratch state and a plan's tables: 128 MiB are
+    free only with the pool's 192 MiB."""
+    from ruqu_b200 import workloads
+    n = 24
+    st = rq.QuantumState(n, 1, "f64")
+    f32 = rq.QuantumState(n, 1, "f32")
+    pooled = [rq.QuantumState(21, 1, "f64") for _ in range(6)]
+    with little_memory() as free:
+        assert free < 128 * MIB
+        del pooled
+        gc.collect()
+        assert _pool()[0] >= 6
+        assert st.probabilities()[0] == 1.0                # 128 MiB
+        assert _pool()[0] == 0
+    pooled = [rq.QuantumState(21, 1, "f64") for _ in range(6)]
+    with little_memory() as free:
+        assert free < 128 * MIB
+        del pooled
+        gc.collect()
+        assert _pool()[0] >= 6
+        plan = rq.Plan(f32, workloads.random_layer_circuit(n, 13, 5))
+        assert plan.stats()["dense_ops"] > 0               # tuned: the tensor-core sweep
+        assert _pool()[0] == 0
