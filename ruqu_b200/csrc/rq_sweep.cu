@@ -1884,8 +1884,10 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cands.push_back({TC_F16, 12, nullptr, 0.f});
         if (s->nq > 14) cands.push_back({TC_F16, 14, nullptr, 0.f});
     }
+    bool keep = true;   // a choice made for want of memory is made again at the next call
     for (auto& c : cands)
-        if (plan_build(s, gates, n, RQ_EXEC_SWEEP, &c.plan, c.passes, 2, c.m) != RQ_OK) {
+        if (const int prc = plan_build(s, gates, n, RQ_EXEC_SWEEP, &c.plan, c.passes, 2, c.m)) {
+            if (prc != RQ_ERR_CIRCUIT) keep = false;   // its tables found no memory
             if (c.passes == 0) {   // the CUDA-core plan is the reference point
                 for (auto& d : cands) plan_free(d.plan);
                 return fail(RQ_ERR_CIRCUIT, "circuit error: the gate list cannot be planned");
@@ -1951,15 +1953,17 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cudaFree(scratch);
     } else {
         cudaGetLastError();   // no room for a scratch state (or nothing to compare): CUDA-core sweep
+        if (any_tc) keep = false;
     }
     const int choice_passes = cands[best].passes;
     const uint32_t choice_m = cands[best].m;
     for (auto& c : cands) plan_free(c.plan);
     RQ_TRY(rc);
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[key] = std::make_pair(choice_passes, choice_m);
     *passes = choice_passes;
     *m_out = choice_m;
+    if (!keep) return RQ_OK;
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    g_tune[key] = std::make_pair(choice_passes, choice_m);
     return RQ_OK;
 }
 

@@ -133,3 +133,17 @@ def test_calls_that_need_memory_get_what_the_pool_holds():
         plan = rq.Plan(f32, workloads.random_layer_circuit(n, 13, 5))
         assert plan.stats()["dense_ops"] > 0               # tuned: the tensor-core sweep
         assert _pool()[0] == 0
+
+
+def test_a_choice_made_without_memory_is_made_again():
+    """No room for the tuner's scratch state: the CUDA-core sweep, for that call only."""
+    from ruqu_b200 import workloads
+    n = 24
+    f32 = rq.QuantumState(n, 1, "f32")
+    gates = workloads.random_layer_circuit(n, 14, 5)
+    with little_memory() as free:
+        assert free < 128 * MIB
+        with pytest.raises(rq.MemoryAllocationFailed):     # and none in the pool
+            rq.QuantumState(26, 1, "f64")
+        assert rq.Plan(f32, gates).stats()["dense_ops"] == 0
+    assert rq.Plan(f32, gates).stats()["dense_ops"] > 0
