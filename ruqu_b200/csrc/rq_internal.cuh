@@ -163,7 +163,7 @@ int mma_timeout_flag(int* out);
 // polls before an mbarrier wait counts as expired (0: the default), current device
 int mma_set_wait_polls(uint32_t polls);
 // the tensor-core sweeps' equivalents (rq_sweep.cu)
-int tc_timeout_flag(int* out);
+int tc_timeout_flag(int* out, bool clear = true);
 int tc_set_wait_polls(uint32_t polls);
 // synchronise the state's stream, then report (and clear) an expired tensor-core wait as
 // RQ_ERR_TIMEOUT: the read-back paths call this, so a sweep that gave up is never read as

@@ -1884,7 +1884,7 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cands.push_back({TC_F16, 12, nullptr, 0.f});
         if (s->nq > 14) cands.push_back({TC_F16, 14, nullptr, 0.f});
     }
-    bool keep = true;   // a choice made for want of memory is made again at the next call
+    bool keep = true;   // a choice made for want of memory, or after a wait ran out, is made again at the next call
     for (auto& c : cands)
         if (const int prc = plan_build(s, gates, n, RQ_EXEC_SWEEP, &c.plan, c.passes, 2, c.m)) {
             if (prc != RQ_ERR_CIRCUIT) keep = false;   // its tables found no memory
@@ -1915,6 +1915,8 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         // count with their median: a single time each, taken while the clock was still settling under the
         // power limit, picked the 14-qubit plan of a 30-qubit random-layer circuit (95.9 ms) before the
         // 13-qubit one (90.9 ms) in one process of two.
+        int pending = 0, expired = 0;   // a flag that is up already is for the state it belongs to
+        rc = tc_timeout_flag(&pending, false);
         float least = 0.f;
         auto timed = [&](Cand& c) {
             if (!c.plan || rc != RQ_OK) return;
@@ -1937,10 +1939,14 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
             if (again[k].size() == 2)
                 cands[k].ms = std::max(std::min(again[k][0], again[k][1]),
                                        std::min(std::max(again[k][0], again[k][1]), cands[k].ms));
+        // a candidate whose wait ran out gave up early: no time counts, and nobody else hears of it
+        if (rc == RQ_OK) rc = tc_timeout_flag(&expired, !pending);
         // a later candidate must be more than 2 % faster than the best so far: near-equal plans
         // (the 12- and 13-qubit FP16 plans of a 30-qubit random-layer circuit are within 1 %)
         // then keep the earlier one, which has fewer sweeps, instead of following timing noise
-        if (rc == RQ_OK) {
+        if (expired) {
+            keep = false;
+        } else if (rc == RQ_OK) {
             float ms[8];
             bool ok[8];
             const size_t nc = std::min<size_t>(cands.size(), 8);   // at most six candidates
@@ -2084,10 +2090,10 @@ void plan_free(rq_plan* P) {
 
 rq_plan_stats plan_stats(const rq_plan* p) { return p->stats; }
 
-int tc_timeout_flag(int* out) {
+int tc_timeout_flag(int* out, bool clear) {
     int v = 0, zero = 0;
     RQ_CUDA(cudaMemcpyFromSymbol(&v, tc::g_tc_timeout, sizeof(int)));
-    if (v) {
+    if (v && clear) {
         RQ_CUDA(cudaMemcpyToSymbol(tc::g_tc_timeout, &zero, sizeof(int)));
         RQ_CUDA(cudaDeviceSynchronize());
     }
