@@ -1910,25 +1910,26 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cudaMemsetAsync(scratch, 0, s->bytes(), s->stream);
         const float one[2] = {1.f, 0.f};   // complex f32 amplitude 0 (pageable: staged before the call returns)
         cudaMemcpyAsync(scratch, one, sizeof(one), cudaMemcpyHostToDevice, s->stream);
-        // Each candidate runs once to warm up and is then timed; a long first run that is already a quarter
-        // slower than the best is enough. Those within 10 % of the best are timed twice more in turn and
-        // count with their median: a single time each, taken while the clock was still settling under the
-        // power limit, picked the 14-qubit plan of a 30-qubit random-layer circuit (95.9 ms) before the
-        // 13-qubit one (90.9 ms) in one process of two.
+        // Each candidate runs once to warm up and is then timed.  Where the runs are long enough for the
+        // clock to settle under the power limit meanwhile (LONG_MS), a single time is not enough: those within
+        // 10 % of the best are timed twice more in turn and count with their median, and a first run that is
+        // already a quarter slower than the best is not repeated.  Short runs are timed once: timing them
+        // again made the first call of a 24- to 26-qubit circuit 4 to 8 % slower.
+        constexpr float LONG_MS = 50.f;
         int pending = 0, expired = 0;   // a flag that is up already is for the state it belongs to
         rc = tc_timeout_flag(&pending, false);
         float least = 0.f;
         auto timed = [&](Cand& c) {
             if (!c.plan || rc != RQ_OK) return;
             rc = time_plan(t, c.plan, &c.ms);
-            if (rc == RQ_OK && !(c.ms > 50.f && least > 0.f && c.ms > 1.25f * least)) rc = time_plan(t, c.plan, &c.ms);
+            if (rc == RQ_OK && !(c.ms > LONG_MS && least > 0.f && c.ms > 1.25f * least)) rc = time_plan(t, c.plan, &c.ms);
             if (rc == RQ_OK && (least == 0.f || c.ms < least)) least = c.ms;
         };
         timed(cands[2]);   // the FP16 sweep first: the slow ones then need one run
         for (size_t k = 0; k < cands.size(); ++k)
             if (k != 2) timed(cands[k]);
         std::vector<std::vector<float>> again(cands.size());
-        for (int round = 0; round < 2; ++round)
+        for (int round = 0; round < 2 && least > LONG_MS; ++round)
             for (size_t k = 0; k < cands.size() && rc == RQ_OK; ++k)
                 if (cands[k].plan && cands[k].ms <= 1.1f * least) {
                     float ms = 0.f;
