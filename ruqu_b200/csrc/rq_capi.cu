@@ -9,6 +9,7 @@
 #include "rq_internal.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -140,8 +141,11 @@ double now_s() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
+std::atomic<size_t> g_scratch_kept{0};   // bytes of scratch that states and pooled sets keep (scratch_get)
+
 // free a set's resources (its device current); a set of a context that is gone is only forgotten
 void release_resources(rq_state& r, unsigned long long ctx) {
+    g_scratch_kept -= r.scratch_cap;
     if (ctx != rq::current_context_id()) return;
     if (r.amps) cudaFree(r.amps);
     if (r.partials) cudaFree(r.partials);
@@ -450,25 +454,35 @@ int ensure_tree(rq_state* s, size_t nd) {
 }
 
 int scratch_get(rq_state* s, size_t bytes, void** out) {
-    if (bytes > SCRATCH_KEEP_BYTES) {
-        cudaError_t e = cudaMallocAsync(out, bytes, s->stream);
-        if (e == cudaErrorMemoryAllocation && pool_release()) e = cudaMallocAsync(out, bytes, s->stream);
-        RQ_CUDA(e);
-        return RQ_OK;
-    }
-    if (s->scratch_cap < bytes) {
-        if (s->scratch) {
-            RQ_CUDA(cudaStreamSynchronize(s->stream));
-            cudaFree(s->scratch);
-            s->scratch = nullptr;
-            s->scratch_cap = 0;
-        }
+    if (s->scratch_cap < bytes && bytes <= SCRATCH_KEEP_BYTES) {
         size_t cap = (size_t)64 << 10;
         while (cap < bytes) cap <<= 1;
-        RQ_CUDA(device_malloc(&s->scratch, cap));
-        s->scratch_cap = cap;
+        // room for it among what all states keep: not reserved from two threads at once
+        size_t kept = g_scratch_kept.load();
+        while (kept - s->scratch_cap + cap <= SCRATCH_TOTAL_BYTES &&
+               !g_scratch_kept.compare_exchange_weak(kept, kept - s->scratch_cap + cap)) {
+        }
+        if (kept - s->scratch_cap + cap <= SCRATCH_TOTAL_BYTES) {
+            const cudaError_t se = s->scratch ? cudaStreamSynchronize(s->stream) : cudaSuccess;
+            if (s->scratch) cudaFree(s->scratch);
+            s->scratch = nullptr;
+            s->scratch_cap = cap;
+            const cudaError_t e = se == cudaSuccess ? device_malloc(&s->scratch, cap) : se;
+            if (e != cudaSuccess) {
+                s->scratch = nullptr;
+                s->scratch_cap = 0;
+                g_scratch_kept -= cap;
+                RQ_CUDA(e);
+            }
+        }
     }
-    *out = s->scratch;
+    if (bytes <= s->scratch_cap) {
+        *out = s->scratch;
+        return RQ_OK;
+    }
+    cudaError_t e = cudaMallocAsync(out, bytes, s->stream);
+    if (e == cudaErrorMemoryAllocation && pool_release()) e = cudaMallocAsync(out, bytes, s->stream);
+    RQ_CUDA(e);
     return RQ_OK;
 }
 

@@ -75,8 +75,10 @@ int ensure_partials(rq_state* s, size_t ndoubles);
 int ensure_hbuf(rq_state* s, size_t ndoubles);
 int ensure_tree(rq_state* s, size_t ndoubles);
 // `bytes` of device scratch for one call on s's stream: the state's own buffer up to
-// SCRATCH_KEEP_BYTES (kept for the next call), a stream-ordered allocation above that.
+// SCRATCH_KEEP_BYTES (kept for the next call, SCRATCH_TOTAL_BYTES over all states), a stream-ordered
+// allocation above that.
 constexpr size_t SCRATCH_KEEP_BYTES = (size_t)64 << 20;
+constexpr size_t SCRATCH_TOTAL_BYTES = (size_t)256 << 20;
 int scratch_get(rq_state* s, size_t bytes, void** out);
 void scratch_put(rq_state* s, void* p);
 // cudaMalloc that gives the memory of destroyed states back and tries again before it fails

@@ -23,6 +23,7 @@
 
 #include <cuda_bf16.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -732,10 +733,11 @@ struct rq_mlp {
     float *F1 = nullptr, *F2 = nullptr, *F3 = nullptr;     // f32 dZ1, dZ2 and 2 (Y - T): summed over rows into
     float *db1 = nullptr, *db2 = nullptr, *db3 = nullptr;  // the bias gradients
     float* losspart = nullptr;                             // per-tile sums of squares
-    // a training set on the device (kept between calls up to TRAIN_KEEP_BYTES)
+    // a training set on the device (kept between calls: keep_training_rows)
     float *tx = nullptr, *tt = nullptr;
     __nv_bfloat16* txb = nullptr;
     size_t train_rows = 0;
+    size_t train_kept = 0;        // bytes of it counted in g_train_kept
     float* G = nullptr;           // gradients: dW1 [h1 x inp], dW2 [h2 x h1], dW3t [h2 x outp]
     long g_w1 = 0, g_w2 = 0, g_w3t = 0, g_total = 0;
     float* loss = nullptr;
@@ -753,7 +755,8 @@ int dalloc(P** p, size_t n) {
     return RQ_OK;
 }
 
-constexpr size_t TRAIN_KEEP_BYTES = (size_t)256 << 20;
+constexpr size_t TRAIN_KEEP_BYTES = (size_t)256 << 20;   // training sets kept on the device, all networks together
+std::atomic<size_t> g_train_kept{0};
 
 int mlp_refresh_bf16(rq_mlp* m) {
     const int sms = rq::num_sms(m->device);
@@ -801,6 +804,21 @@ void train_release(rq_mlp* m) {
     m->tx = m->tt = nullptr;
     m->txb = nullptr;
     m->train_rows = 0;
+    g_train_kept -= m->train_kept;
+    m->train_kept = 0;
+}
+
+// after a call: the training set stays for the next one if there is room for it, else it is freed
+void keep_training_rows(rq_mlp* m) {
+    if (m->train_kept) return;
+    const size_t bytes = m->train_rows * (m->in * sizeof(float) + m->out * sizeof(float) + m->inp * sizeof(__nv_bfloat16));
+    size_t kept = g_train_kept.load();
+    while (kept + bytes <= TRAIN_KEEP_BYTES)
+        if (g_train_kept.compare_exchange_weak(kept, kept + bytes)) {
+            m->train_kept = bytes;
+            return;
+        }
+    train_release(m);
 }
 
 int train_reserve(rq_mlp* m, size_t n) {
@@ -1095,7 +1113,7 @@ int rq_mlp_train(rq_mlp* m, const float* x, const float* t, int32_t n, int32_t B
         if (e != cudaSuccess) rc = rq::cuda_fail(e, "cudaMemcpyAsync");
     }
     e = cudaStreamSynchronize(m->stream);
-    if ((size_t)n * (m->in * 4 + m->out * 4 + m->inp * 2) > TRAIN_KEEP_BYTES) train_release(m);
+    keep_training_rows(m);
     RQ_TRY(rc);
     RQ_CUDA(e);
     int to = 0;
