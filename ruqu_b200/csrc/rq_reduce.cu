@@ -6,6 +6,7 @@
 // for f32 states) and is deterministic: a fixed grid writes one partial per
 // block and term, and a second kernel sums the partials in a fixed order.
 #include "rq_internal.cuh"
+#include "rq_pauli_plan.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -16,6 +17,7 @@ namespace {
 
 using rqd::C2;
 using rqd::insert0;
+using namespace rqs;
 
 constexpr int TPB = 256;
 
@@ -72,7 +74,6 @@ __global__ void k_prob(const typename C2<T>::t* __restrict__ a, uint64_t count, 
 //   k_pauli_z      up to ZK strings with x == 0 per read of the state;
 //   k_pauli_span   up to SK strings with x != 0 per read of the state.
 
-constexpr uint32_t SMALL_QUBITS = 13;
 constexpr int SMALL_STRINGS = 480;
 struct SmallStrings {
     uint32_t x[SMALL_STRINGS], z[SMALL_STRINGS];
@@ -230,19 +231,8 @@ __global__ void __launch_bounds__(ZT, KT > 16 ? 2 : 3) k_pauli_z(const typename 
 // CTA's tiles.  Bound by the FP64 conversions (XU 60 %, issue 47 %): 64 random strings of 24 qubits
 // f32 in 0.59 ms against 2.8 ms for a read of the state
 // per string.
-constexpr int SK = 16, SPASSES = 10, ST = 512, STB = 9;
-struct SpanString {
-    uint64_t z;
-    uint16_t lx, lz;     // X and sign masks on the tile's local bits
-    uint8_t mode, odd;   // mode: register bit held at 0, or the number of register bits: walk all
-    uint16_t pad;
-};
-struct SpanPass {
-    uint64_t basis[8];   // bits above the run
-    uint8_t free_bit[24];   // the other bits above the run, low to high: the tile number's bits
-    uint32_t k, row0;       // its strings, and the row of the first
-    SpanString s[SK];
-};
+constexpr int SPASSES = 10, ST = 512;
+static_assert(ST == 1 << STB, "a tile index is a thread and a register");
 struct SpanPasses {
     SpanPass p[SPASSES];
 };
@@ -428,113 +418,6 @@ int finish(rq_state* s, unsigned nblocks, unsigned stride, unsigned nout, double
     RQ_TRY(rq::sync_checked(s));
     for (unsigned k = 0; k < nout; ++k) host[k] = s->hbuf[k];
     return RQ_OK;
-}
-
-inline double re_ipow(uint32_t k) {
-    switch (k & 3u) {
-        case 0: return 1.0;
-        case 2: return -1.0;
-        default: return 0.0;
-    }
-}
-
-// Which kernel sums which string, into which row of the partials.
-struct PauliPlan {
-    bool small = false;
-    std::vector<uint32_t> zs;             // strings of k_pauli_z in row order
-    std::vector<SpanPass> spans;
-    uint32_t rows = 0;                    // one per string
-    uint32_t zblocks = 0, sblocks = 0, stride = 0;
-    std::vector<uint32_t> row_of;         // string -> row
-    std::vector<double> factor;           // string -> factor of its sum
-    const rq::PauliMask* terms = nullptr;
-};
-
-void plan_strings(uint32_t n, int32_t prec, int sms, const rq::PauliMask* terms, uint32_t nterms, PauliPlan& P) {
-    P.terms = terms;
-    P.rows = nterms;
-    P.row_of.assign(nterms, 0);
-    P.factor.resize(nterms);
-    for (uint32_t k = 0; k < nterms; ++k) {
-        const rq::PauliMask& t = terms[k];
-        const bool odd = __builtin_popcountll(t.xmask & t.pmask) & 1;
-        P.factor[k] = t.xmask == 0 ? re_ipow(t.ny) : 2.0 * re_ipow(odd ? t.ny + 1 : t.ny);
-    }
-    if (n <= SMALL_QUBITS) {
-        P.small = true;
-        for (uint32_t k = 0; k < nterms; ++k) P.row_of[k] = k;
-        return;
-    }
-    std::vector<uint32_t> left;
-    for (uint32_t k = 0; k < nterms; ++k) {
-        if (terms[k].xmask == 0) {
-            P.row_of[k] = (uint32_t)P.zs.size();
-            P.zs.push_back(k);
-        } else {
-            left.push_back(k);
-        }
-    }
-    uint32_t row = (uint32_t)P.zs.size();
-    const uint32_t C = prec == RQ_F32 ? 5 : 4, RB = prec == RQ_F32 ? 4 : 3;
-    const uint64_t low = (1ull << C) - 1;
-    while (!left.empty()) {
-        SpanPass sp{};
-        sp.row0 = row;
-        uint64_t pivot[8];
-        uint32_t dim = 0;
-        auto reduced = [&](uint64_t x) {
-            for (uint32_t b = 0; b < dim; ++b)
-                if (x & pivot[b]) x ^= sp.basis[b];
-            return x;
-        };
-        auto add = [&](uint64_t v) {   // v reduced and not zero: clear its pivot from the others
-            const uint64_t pv = 1ull << (63 - __builtin_clzll(v));
-            for (uint32_t b = 0; b < dim; ++b)
-                if (sp.basis[b] & pv) sp.basis[b] ^= v;
-            pivot[dim] = pv;
-            sp.basis[dim++] = v;
-        };
-        std::vector<uint32_t> take, rest;
-        for (uint32_t k : left) {
-            const uint64_t r = take.size() < (size_t)SK ? reduced(terms[k].xmask & ~low) : ~0ull;
-            if (take.size() == (size_t)SK || (r && dim == 8)) {
-                rest.push_back(k);
-                continue;
-            }
-            if (r) add(r);
-            take.push_back(k);
-        }
-        for (uint32_t q = C; dim < 8; ++q)
-            if (const uint64_t r = reduced(1ull << q)) add(r);
-        uint64_t pivots = 0;
-        for (uint32_t b = 0; b < 8; ++b) pivots |= pivot[b];
-        uint32_t nf = 0;
-        for (uint32_t q = C; q < n; ++q)
-            if (!((pivots >> q) & 1)) sp.free_bit[nf++] = (uint8_t)q;
-        for (uint32_t k : take) {
-            const rq::PauliMask& t = terms[k];
-            SpanString& ss = sp.s[sp.k];
-            uint32_t lx = (uint32_t)(t.xmask & low), lz = (uint32_t)(t.pmask & low);
-            for (uint32_t b = 0; b < 8; ++b) {
-                if (t.xmask & pivot[b]) lx |= 1u << (C + b);
-                if (__builtin_popcountll(sp.basis[b] & t.pmask) & 1) lz |= 1u << (C + b);
-            }
-            ss.z = t.pmask;
-            ss.lx = (uint16_t)lx;
-            ss.lz = (uint16_t)lz;
-            ss.odd = (uint8_t)(__builtin_popcountll(t.xmask & t.pmask) & 1);
-            const uint32_t xr = lx >> STB;
-            ss.mode = (uint8_t)(xr ? 31 - __builtin_clz(xr) : RB);
-            if (!xr) P.factor[k] *= 0.5;   // walked from both ends
-            P.row_of[k] = row++;
-            ++sp.k;
-        }
-        P.spans.push_back(sp);
-        left.swap(rest);
-    }
-    P.zblocks = P.zs.empty() ? 0 : (uint32_t)std::min<uint64_t>(1ull << (n - 12), (uint64_t)sms * 2);
-    P.sblocks = P.spans.empty() ? 0 : (uint32_t)std::min<uint64_t>(1ull << (n - C - 8), (uint64_t)sms);
-    P.stride = std::max(P.zblocks, P.sblocks);
 }
 
 template <typename T, bool PAIRS>
