@@ -1565,18 +1565,18 @@ TableBytes table_bytes(const std::vector<SweepDesc>& descs, const std::vector<Ph
 // (8 of 20).
 uint32_t plan_symmetric(const std::vector<PGate>& gates, uint32_t n, uint32_t mloc, uint32_t rb, int32_t prec,
                         std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
-    const uint32_t epv = prec == RQ_F32 ? 2 : 1, m = std::min(n - 1, mloc);
-    symmetric_program(gates, n, m, rb, epv, descs, phases, ops);
-    if (n - 1 < mloc) return m;
-    std::vector<SweepDesc> d;
-    std::vector<PhaseDesc> ph;
-    std::vector<SwOp> o;
-    symmetric_program(gates, n, m - 1, rb, epv, d, ph, o);
-    if (d.size() > descs.size()) return m;
-    descs.swap(d);
-    phases.swap(ph);
-    ops.swap(o);
-    return m - 1;
+    const uint32_t epv = prec == RQ_F32 ? 2 : 1;
+    uint32_t m = std::min(n - 1, mloc);
+    auto sweeps = symmetric_sweeps(gates, n, m);
+    if (n - 1 >= mloc) {
+        auto smaller = symmetric_sweeps(gates, n, m - 1, sweeps.size());
+        if (smaller.size() <= sweeps.size()) {
+            sweeps.swap(smaller);
+            --m;
+        }
+    }
+    symmetric_program(sweeps, n, m, rb, epv, descs, phases, ops);
+    return m;
 }
 
 // Shared memory of a sweep launch: what it needs, or that with its tables (`staged` bytes) where as many

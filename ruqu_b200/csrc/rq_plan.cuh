@@ -169,12 +169,13 @@ inline std::vector<Sweep> plan_sweeps_first_come(const std::vector<PGate>& gates
     std::vector<char> taken(gates.size(), 0);
     size_t first = 0;
     const uint64_t base = (c >= 64) ? ~0ull : ((1ull << c) - 1);
+    const uint64_t allq = (n >= 64) ? ~0ull : ((1ull << n) - 1);
     while (first < gates.size()) {
         Sweep sw;
         sw.L = base;
         uint64_t blocked = 0;
         std::vector<int> last(n, -1);   // index in sw.ops of the last op on each qubit
-        for (size_t k = first; k < gates.size(); ++k) {
+        for (size_t k = first; k < gates.size() && blocked != allq; ++k) {
             if (taken[k]) continue;
             const PGate& g = gates[k];
             uint64_t qm = qmask(g);
@@ -204,19 +205,30 @@ inline std::vector<Sweep> plan_sweeps_first_come(const std::vector<PGate>& gates
     return out;
 }
 
+// a gate's qubits, and those that must be local
+struct GateMask {
+    uint64_t qm, need;
+};
+
+inline std::vector<GateMask> gate_masks(const std::vector<PGate>& gates) {
+    std::vector<GateMask> out;
+    out.reserve(gates.size());
+    for (const PGate& g : gates) out.push_back({qmask(g), needs(g, false)});
+    return out;
+}
+
 // Gates a sweep with the fixed local set L would take from the remaining list (per-qubit
 // order kept: a gate that cannot run holds its qubits back for the rest of the list);
 // marks them in *mark when given.  Stops once every qubit is held back.
-inline int sweep_closure(const std::vector<PGate>& gates, const std::vector<char>& taken, size_t first, uint64_t L,
+inline int sweep_closure(const std::vector<GateMask>& gates, const std::vector<char>& taken, size_t first, uint64_t L,
                          uint64_t allq, std::vector<char>* mark) {
     uint64_t blocked = 0;
     int cnt = 0;
     for (size_t k = first; k < gates.size(); ++k) {
         if (taken[k]) continue;
-        const PGate& g = gates[k];
-        const uint64_t qm = qmask(g);
-        if ((qm & blocked) || (needs(g, false) & ~L)) {
-            blocked |= qm;
+        const GateMask& g = gates[k];
+        if ((g.qm & blocked) || (g.need & ~L)) {
+            blocked |= g.qm;
             if ((blocked & allq) == allq) break;
             continue;
         }
@@ -229,16 +241,17 @@ inline int sweep_closure(const std::vector<PGate>& gates, const std::vector<char
 // Candidate local sets for the next sweep: the first-come set (padded to m qubits) and
 // every window of m - c consecutive qubits above the always-local low c qubits (the
 // shape that follows nearest-neighbour circuits as their light cones move).
-inline std::vector<uint64_t> sweep_candidates(const std::vector<PGate>& gates, const std::vector<char>& taken,
+inline std::vector<uint64_t> sweep_candidates(const std::vector<GateMask>& gates, const std::vector<char>& taken,
                                               size_t first, uint32_t n, uint32_t m, uint32_t c) {
     const uint64_t base = (c >= 64) ? ~0ull : ((1ull << c) - 1);
     std::vector<uint64_t> out;
+    const uint64_t allq = (n >= 64) ? ~0ull : ((1ull << n) - 1);
     uint64_t L = base, blocked = 0;
-    for (size_t k = first; k < gates.size(); ++k) {
+    for (size_t k = first; k < gates.size() && blocked != allq; ++k) {
         if (taken[k]) continue;
-        const uint64_t qm = qmask(gates[k]);
+        const uint64_t qm = gates[k].qm;
         if (qm & blocked) { blocked |= qm; continue; }
-        const uint64_t L2 = L | needs(gates[k], false);
+        const uint64_t L2 = L | gates[k].need;
         if ((uint32_t)__builtin_popcountll(L2) > m) { blocked |= qm; continue; }
         L = L2;
     }
@@ -255,25 +268,27 @@ inline std::vector<uint64_t> sweep_candidates(const std::vector<PGate>& gates, c
 
 // Lookahead local sets: each sweep takes the candidate set that maximises the gates it
 // runs plus the most the following sweep could then run (two-step lookahead over the
-// candidates of sweep_candidates).
-inline std::vector<Sweep> plan_sweeps_lookahead(const std::vector<PGate>& gates, uint32_t n, uint32_t m, uint32_t c) {
+// candidates of sweep_candidates).  Stops, unfinished, past `most` sweeps.
+inline std::vector<Sweep> plan_sweeps_lookahead(const std::vector<PGate>& gates, uint32_t n, uint32_t m, uint32_t c,
+                                                size_t most = SIZE_MAX) {
     std::vector<Sweep> out;
-    std::vector<char> taken(gates.size(), 0);
+    std::vector<char> taken(gates.size(), 0), t2;
+    const auto masks = gate_masks(gates);
     const uint64_t allq = (n >= 64) ? ~0ull : ((1ull << n) - 1);
     size_t first = 0;
-    while (first < gates.size()) {
-        const auto cands = sweep_candidates(gates, taken, first, n, m, c);
+    while (first < gates.size() && out.size() <= most) {
+        const auto cands = sweep_candidates(masks, taken, first, n, m, c);
         double best = -1.0;
         uint64_t bestL = cands[0];
         for (uint64_t L : cands) {
-            std::vector<char> t2 = taken;
-            double score = sweep_closure(gates, taken, first, L, allq, &t2);
+            t2 = taken;
+            double score = sweep_closure(masks, taken, first, L, allq, &t2);
             size_t f2 = first;
             while (f2 < gates.size() && t2[f2]) ++f2;
             int next = 0;
             if (f2 < gates.size())
-                for (uint64_t L2 : sweep_candidates(gates, t2, f2, n, m, c))
-                    next = std::max(next, sweep_closure(gates, t2, f2, L2, allq, nullptr));
+                for (uint64_t L2 : sweep_candidates(masks, t2, f2, n, m, c))
+                    next = std::max(next, sweep_closure(masks, t2, f2, L2, allq, nullptr));
             score += 0.999 * next;   // ties go to the set that runs more gates now
             if (score > best) {
                 best = score;
@@ -284,7 +299,7 @@ inline std::vector<Sweep> plan_sweeps_lookahead(const std::vector<PGate>& gates,
         sw.L = bestL;
         std::vector<int> last(n, -1);   // index in sw.ops of the last op on each qubit
         uint64_t blocked = 0;
-        for (size_t k = first; k < gates.size(); ++k) {
+        for (size_t k = first; k < gates.size() && blocked != allq; ++k) {
             if (taken[k]) continue;
             const PGate& g = gates[k];
             const uint64_t qm = qmask(g);
@@ -356,20 +371,48 @@ inline std::vector<PhasePlan> plan_phases_first_come(const Sweep& sw, uint32_t r
     return out;
 }
 
+// What the phase planners look at, once per sweep: each op's qubits, those of them that must be register
+// slots and those outside the tile that count (tensor-core plans), and the windows of rb consecutive local
+// qubits.
+struct PhaseOps {
+    struct Op {
+        uint64_t qm, need, out;
+    };
+    std::vector<Op> ops;
+    std::vector<uint64_t> windows;
+    std::vector<uint32_t> loc;
+    uint64_t allq = 0;   // qubits of the ops: once all are held back, no later op runs
+    uint32_t rb;
+    PhaseOps(const Sweep& sw, uint32_t slots, bool all_slots) : rb(slots) {
+        ops.reserve(sw.ops.size());
+        for (const PGate& g : sw.ops) {
+            const uint64_t qm = qmask(g);
+            ops.push_back({qm, needs(g, false) | (all_slots ? (qm & sw.L) : 0ull), all_slots ? (qm & ~sw.L) : 0ull});
+            allq |= qm;
+        }
+        for (uint32_t q = 0; q < 64; ++q)
+            if ((sw.L >> q) & 1) loc.push_back(q);
+        for (size_t a0 = 0; a0 + rb <= loc.size(); ++a0) {
+            uint64_t W = 0;
+            for (size_t j = a0; j < a0 + rb; ++j) W |= 1ull << loc[j];
+            windows.push_back(W);
+        }
+    }
+};
+
 // Ops of the sweep a phase with slot set R would take (per-qubit order kept), with the
 // same rules as plan_phases_first_come; marks them in *mark when given.
-inline int phase_closure(const Sweep& sw, const std::vector<char>& taken, size_t first, uint64_t R, bool all_slots,
+inline int phase_closure(const PhaseOps& po, const std::vector<char>& taken, size_t first, uint64_t R,
                          std::vector<int>* mark) {
     uint64_t blocked = 0, outside = 0;
     int cnt = 0;
-    for (size_t k = first; k < sw.ops.size(); ++k) {
+    for (size_t k = first; k < po.ops.size(); ++k) {
         if (taken[k]) continue;
-        const PGate& g = sw.ops[k];
-        const uint64_t qm = qmask(g);
-        const uint64_t need = needs(g, false) | (all_slots ? (qm & sw.L) : 0ull);
-        const uint64_t out2 = all_slots ? (outside | (qm & ~sw.L)) : 0ull;
-        if ((qm & blocked) || (need & ~R) || __builtin_popcountll(out2) > DENSE_MAX_VQ_PLAN) {
-            blocked |= qm;
+        const PhaseOps::Op& g = po.ops[k];
+        const uint64_t out2 = outside | g.out;
+        if ((g.qm & blocked) || (g.need & ~R) || __builtin_popcountll(out2) > DENSE_MAX_VQ_PLAN) {
+            blocked |= g.qm;
+            if (blocked == po.allq) break;
             continue;
         }
         outside = out2;
@@ -379,59 +422,55 @@ inline int phase_closure(const Sweep& sw, const std::vector<char>& taken, size_t
     return cnt;
 }
 
+// Slot sets for the next phase: the first-come set for the remaining ops, and the windows.
+inline void phase_candidates(const PhaseOps& po, const std::vector<char>& taken, size_t first, std::vector<uint64_t>& c) {
+    uint64_t R = 0, blocked = 0, outside = 0;
+    for (size_t k = first; k < po.ops.size() && blocked != po.allq; ++k) {
+        if (taken[k]) continue;
+        const PhaseOps::Op& g = po.ops[k];
+        const uint64_t R2 = R | g.need, out2 = outside | g.out;
+        if ((g.qm & blocked) || (uint32_t)__builtin_popcountll(R2) > po.rb || __builtin_popcountll(out2) > DENSE_MAX_VQ_PLAN) {
+            blocked |= g.qm;
+            continue;
+        }
+        R = R2;
+        outside = out2;
+    }
+    for (uint32_t q : po.loc)
+        if ((uint32_t)__builtin_popcountll(R) < po.rb && !((R >> q) & 1)) R |= 1ull << q;
+    c.clear();
+    c.push_back(R);
+    for (uint64_t W : po.windows)
+        if (W != R) c.push_back(W);
+}
+
 // Lookahead register slots: candidates are the first-come slot set and every window of
 // rb consecutive local qubits; each phase takes the one maximising the ops it runs plus
 // the most the next phase could then run.
 inline std::vector<PhasePlan> plan_phases_lookahead(const Sweep& sw, uint32_t rb, bool all_slots) {
     std::vector<PhasePlan> out;
-    std::vector<char> taken(sw.ops.size(), 0);
-    std::vector<uint32_t> loc;
-    for (uint32_t q = 0; q < 64; ++q)
-        if ((sw.L >> q) & 1) loc.push_back(q);
-    auto cands = [&](const std::vector<char>& tk, size_t f) {
-        std::vector<uint64_t> c;
-        // the first-come choice for the remaining ops
-        uint64_t R = 0, blocked = 0, outside = 0;
-        for (size_t k = f; k < sw.ops.size(); ++k) {
-            if (tk[k]) continue;
-            const PGate& g = sw.ops[k];
-            const uint64_t qm = qmask(g);
-            if (qm & blocked) { blocked |= qm; continue; }
-            const uint64_t R2 = R | needs(g, false) | (all_slots ? (qm & sw.L) : 0ull);
-            const uint64_t out2 = all_slots ? (outside | (qm & ~sw.L)) : 0ull;
-            if ((uint32_t)__builtin_popcountll(R2) > rb || __builtin_popcountll(out2) > DENSE_MAX_VQ_PLAN) {
-                blocked |= qm;
-                continue;
-            }
-            R = R2;
-            outside = out2;
-        }
-        for (uint32_t q : loc)
-            if ((uint32_t)__builtin_popcountll(R) < rb && !((R >> q) & 1)) R |= 1ull << q;
-        c.push_back(R);
-        for (size_t a0 = 0; a0 + rb <= loc.size(); ++a0) {
-            uint64_t W = 0;
-            for (size_t j = a0; j < a0 + rb; ++j) W |= 1ull << loc[j];
-            if (W != R) c.push_back(W);
-        }
-        return c;
-    };
+    std::vector<char> taken(sw.ops.size(), 0), t2;
+    const PhaseOps po(sw, rb, all_slots);
+    std::vector<uint64_t> c, c2;
+    std::vector<int> got;
     size_t first = 0;
     while (first < sw.ops.size()) {
-        const auto c = cands(taken, first);
+        phase_candidates(po, taken, first, c);
         double best = -1.0;
         uint64_t bestR = c[0];
         for (uint64_t R : c) {
-            std::vector<int> got;
-            double score = phase_closure(sw, taken, first, R, all_slots, &got);
+            got.clear();
+            double score = phase_closure(po, taken, first, R, &got);
             if (got.empty()) continue;
-            std::vector<char> t2 = taken;
+            t2 = taken;
             for (int k : got) t2[k] = 1;
             size_t f2 = first;
             while (f2 < sw.ops.size() && t2[f2]) ++f2;
             int next = 0;
-            if (f2 < sw.ops.size())
-                for (uint64_t R2 : cands(t2, f2)) next = std::max(next, phase_closure(sw, t2, f2, R2, all_slots, nullptr));
+            if (f2 < sw.ops.size()) {
+                phase_candidates(po, t2, f2, c2);
+                for (uint64_t R2 : c2) next = std::max(next, phase_closure(po, t2, f2, R2, nullptr));
+            }
             score += 0.999 * next;   // ties go to the set that runs more ops now
             if (score > best) {
                 best = score;
@@ -440,7 +479,7 @@ inline std::vector<PhasePlan> plan_phases_lookahead(const Sweep& sw, uint32_t rb
         }
         PhasePlan ph;
         ph.R = bestR;
-        if (phase_closure(sw, taken, first, bestR, all_slots, &ph.ops) == 0) return {};   // no progress: give up
+        if (phase_closure(po, taken, first, bestR, &ph.ops) == 0) return {};   // no progress: give up
         for (int k : ph.ops) taken[k] = 1;
         while (first < sw.ops.size() && taken[first]) ++first;
         out.push_back(std::move(ph));
@@ -461,36 +500,8 @@ inline std::vector<PhasePlan> plan_phases_beam(const Sweep& sw, uint32_t rb, boo
         int done;
         std::vector<PhasePlan> phases;
     };
-    std::vector<uint32_t> loc;
-    for (uint32_t q = 0; q < 64; ++q)
-        if ((sw.L >> q) & 1) loc.push_back(q);
-    auto cands = [&](const std::vector<char>& tk, size_t f) {
-        std::vector<uint64_t> c;
-        uint64_t R = 0, blocked = 0, outside = 0;
-        for (size_t k = f; k < sw.ops.size(); ++k) {
-            if (tk[k]) continue;
-            const PGate& g = sw.ops[k];
-            const uint64_t qm = qmask(g);
-            if (qm & blocked) { blocked |= qm; continue; }
-            const uint64_t R2 = R | needs(g, false) | (all_slots ? (qm & sw.L) : 0ull);
-            const uint64_t out2 = all_slots ? (outside | (qm & ~sw.L)) : 0ull;
-            if ((uint32_t)__builtin_popcountll(R2) > rb || __builtin_popcountll(out2) > DENSE_MAX_VQ_PLAN) {
-                blocked |= qm;
-                continue;
-            }
-            R = R2;
-            outside = out2;
-        }
-        for (uint32_t q : loc)
-            if ((uint32_t)__builtin_popcountll(R) < rb && !((R >> q) & 1)) R |= 1ull << q;
-        c.push_back(R);
-        for (size_t a0 = 0; a0 + rb <= loc.size(); ++a0) {
-            uint64_t W = 0;
-            for (size_t j = a0; j < a0 + rb; ++j) W |= 1ull << loc[j];
-            if (W != R) c.push_back(W);
-        }
-        return c;
-    };
+    const PhaseOps po(sw, rb, all_slots);
+    std::vector<uint64_t> c;
     if (sw.ops.empty()) return {};
     std::vector<Partial> beam(1);
     beam[0].taken.assign(sw.ops.size(), 0);
@@ -499,11 +510,12 @@ inline std::vector<PhasePlan> plan_phases_beam(const Sweep& sw, uint32_t rb, boo
     for (size_t depth = 1; depth <= sw.ops.size(); ++depth) {
         std::vector<Partial> next;
         std::vector<std::vector<char>> seen;
-        for (const Partial& p : beam)
-            for (uint64_t R : cands(p.taken, p.first)) {
+        for (const Partial& p : beam) {
+            phase_candidates(po, p.taken, p.first, c);
+            for (uint64_t R : c) {
                 PhasePlan ph;
                 ph.R = R;
-                if (phase_closure(sw, p.taken, p.first, R, all_slots, &ph.ops) == 0) continue;
+                if (phase_closure(po, p.taken, p.first, R, &ph.ops) == 0) continue;
                 Partial t{p.taken, p.first, p.done + (int)ph.ops.size(), p.phases};
                 for (int k : ph.ops) t.taken[k] = 1;
                 while (t.first < sw.ops.size() && t.taken[t.first]) ++t.first;
@@ -513,6 +525,7 @@ inline std::vector<PhasePlan> plan_phases_beam(const Sweep& sw, uint32_t rb, boo
                 seen.push_back(t.taken);
                 next.push_back(std::move(t));
             }
+        }
         std::stable_sort(next.begin(), next.end(), [](const Partial& a, const Partial& b) { return a.done > b.done; });
         if (next.size() > width) next.resize(width);
         if (next.empty()) return {};
@@ -602,12 +615,13 @@ inline std::vector<Sweep> plan_sweeps_costed(const std::vector<PGate>& gates, ui
                                              uint32_t rb, double rate, SweepCost cost = COST_TF32) {
     std::vector<Sweep> out;
     std::vector<char> taken(gates.size(), 0);
+    const auto masks = gate_masks(gates);
     size_t first = 0;
     while (first < gates.size()) {
         double best = -1e300;
         uint64_t bestL = 0;
         bool found = false;
-        for (uint64_t L : sweep_candidates(gates, taken, first, n, m, c)) {
+        for (uint64_t L : sweep_candidates(masks, taken, first, n, m, c)) {
             std::vector<char> t2 = taken;
             Sweep sw = take_sweep(gates, t2, first, L, n, m);
             if (sw.ops.empty()) continue;
@@ -645,6 +659,7 @@ inline std::vector<Sweep> plan_sweeps_beam(const std::vector<PGate>& gates, uint
         std::vector<uint64_t> sets;
     };
     if (gates.empty()) return {};
+    const auto masks = gate_masks(gates);
     std::vector<Partial> beam(1);
     beam[0].taken.assign(gates.size(), 0);
     beam[0].first = 0;
@@ -656,7 +671,7 @@ inline std::vector<Sweep> plan_sweeps_beam(const std::vector<PGate>& gates, uint
         std::vector<Partial> next;
         std::vector<std::vector<char>> seen;
         for (const Partial& p : beam)
-            for (uint64_t L : sweep_candidates(gates, p.taken, p.first, n, m, c)) {
+            for (uint64_t L : sweep_candidates(masks, p.taken, p.first, n, m, c)) {
                 Partial t{p.taken, p.first, p.cost, p.done, p.sets};
                 const Sweep sw = take_sweep(gates, t.taken, p.first, L, n, m);
                 if (sw.ops.empty()) continue;
@@ -702,11 +717,12 @@ inline std::vector<Sweep> plan_sweeps_beam(const std::vector<PGate>& gates, uint
 // beam-search plans, keeping the plan of least modelled cost (the fewest-sweeps plan on a
 // tie, then the cost-aware one).  A gate qubit that stays outside a sweep's
 // local set is uniform over each tile, for CUDA-core and tensor-core plans alike.
+// most: the caller drops a plan of more sweeps, which then may be unfinished.
 inline std::vector<Sweep> plan_sweeps(const std::vector<PGate>& gates, uint32_t n, uint32_t m, uint32_t c,
-                                      bool all_slots = false, SweepCost k = COST_TF32) {
+                                      bool all_slots = false, SweepCost k = COST_TF32, size_t most = SIZE_MAX) {
     auto a = plan_sweeps_first_come(gates, n, m, c);
-    auto b = plan_sweeps_lookahead(gates, n, m, c);
-    auto best = b.size() < a.size() ? b : a;
+    auto b = plan_sweeps_lookahead(gates, n, m, c, most);
+    auto best = std::move(b.size() < a.size() ? b : a);
     if (!all_slots || gates.empty()) return best;
     const uint32_t rb = 5;
     const double cost_best = plan_cost(best, n, m, rb, k);
@@ -945,12 +961,17 @@ inline void build_program(std::vector<Sweep>& sweeps, uint32_t nq, uint32_t m, u
 //  * flipping the n-1 index bits changes the cut as flipping vertex n-1 does, so for the cost phase the
 //    complement slot is that vertex.
 // Rx is the same from either end of a pair, so no signs change.
-inline void symmetric_program(const std::vector<PGate>& gates, uint32_t n, uint32_t m, uint32_t rb, uint32_t epv,
+inline std::vector<Sweep> symmetric_sweeps(const std::vector<PGate>& gates, uint32_t n, uint32_t m,
+                                           size_t most = SIZE_MAX) {
+    return plan_sweeps(gates, n, m == n - 1 ? n : m, std::min<uint32_t>(m, 5), false, COST_TF32, most);
+}
+
+inline void symmetric_program(const std::vector<Sweep>& sweeps, uint32_t n, uint32_t m, uint32_t rb, uint32_t epv,
                        std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
     const uint32_t N = n - 1, c = std::min<uint32_t>(m, 5), cb = epv == 2 ? 4 : 3, t = m - rb;
     const bool whole = m == N;
     const uint64_t G = 1ull << N;
-    for (auto& sw : plan_sweeps(gates, n, whole ? n : m, c)) {
+    for (const auto& sw : sweeps) {
         const bool pairs = (sw.L & G) && !whole;          // tiles with their complements
         uint64_t real = sw.L & (G - 1);
         const uint32_t want = pairs ? m - 1 : m;
@@ -1028,6 +1049,11 @@ inline void symmetric_program(const std::vector<PGate>& gates, uint32_t n, uint3
         d.phase_end = (uint32_t)phases.size();
         descs.push_back(d);
     }
+}
+
+inline void symmetric_program(const std::vector<PGate>& gates, uint32_t n, uint32_t m, uint32_t rb, uint32_t epv,
+                       std::vector<SweepDesc>& descs, std::vector<PhaseDesc>& phases, std::vector<SwOp>& ops) {
+    symmetric_program(symmetric_sweeps(gates, n, m), n, m, rb, epv, descs, phases, ops);
 }
 
 // Collects the CZ(q, q + 1) of each phase into one op per run: signs are exact, so a CZ may wait until
