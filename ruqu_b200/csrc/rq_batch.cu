@@ -3001,15 +3001,13 @@ int rq_vqe_batch_run(rq_vqe_batch* b, uint32_t nsets, const double* params, int3
     RQ_TRY(grow_bytes(&b->d_states, &b->states_cap, wave * state_bytes));
     // the unshifted states of a group's sets between the sweeps: as many sets as fit the size of a wave; a
     // state too large for that, or no memory for them, and every circuit runs from the start
-    VqeOrder o{V, V == 1 ? nsets : 1, nsets, b->d_order};
+    VqeOrder o{V, nsets, nsets, b->d_order};   // one group where nothing is shared: its waves are filled from all sets
     const size_t keep = (b->descs.size() - 1) * state_bytes;   // per set
     bool share = V > 1 && keep > 0 && keep <= b->wave_bytes;
     if (share) {
-        o.group = (uint32_t)std::min<uint64_t>({nsets, wave, b->wave_bytes / keep});
-        if (grow_bytes(&b->d_snap, &b->snap_cap, o.group * keep) != RQ_OK) {
-            share = false;
-            o.group = 1;
-        }
+        const uint32_t group = (uint32_t)std::min<uint64_t>({nsets, wave, b->wave_bytes / keep});
+        share = grow_bytes(&b->d_snap, &b->snap_cap, group * keep) == RQ_OK;
+        if (share) o.group = group;
     }
     if (adj) {
         RQ_TRY(grow_bytes(&b->d_lam, &b->lam_cap, wave * state_bytes));
