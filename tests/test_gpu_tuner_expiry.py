@@ -17,7 +17,8 @@ DEFAULT = 0xFFFFFFFF
 
 def test_a_wait_that_expires_in_a_candidate_stays_there():
     n = 14
-    gates = workloads.random_layer_circuit(n, 4, 21)
+    # a structure that no other test has tuned: the choice is kept per process
+    gates = workloads.random_layer_circuit(n, 4, 21) + [(12, 3, 11, 0.0), (12, 9, 0, 0.0), (12, 1, 12, 0.0)]
     other = rq.QuantumState(n, 0, "f32")
     rq.Plan(other, workloads.random_layer_circuit(n, 4, 7), rq.RQ_EXEC_SWEEP_TC16).execute(other)
     st = rq.QuantumState(n, 0, "f32")
