@@ -177,9 +177,10 @@ RQ_API int rq_state_from_amplitudes(const double* interleaved, uint64_t len,
                              uint32_t num_qubits, int32_t precision,
                              uint64_t seed, rq_state** out);
 
-/* Ends the state.  Its stream and small device buffers are kept for a later state of the
- * same size on that device (bounded; freed when idle or when memory runs out), unless
- * rq_state_device_ptr handed the memory out. */
+/* Ends the state.  Its stream, pinned staging and small device buffers are kept for a later
+ * state of the same size on that device, unless rq_state_device_ptr handed the memory out:
+ * at most 16 sets, 64 MiB each and 256 MiB in all, freed when an allocation of this library
+ * finds no memory, and, once unused for 30 s, when a state is next created or destroyed. */
 RQ_API int rq_state_destroy(rq_state* s);
 
 /* Back to |0...0>, measurement stream rewound to draw 0 of the same seed.

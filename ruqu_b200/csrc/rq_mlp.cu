@@ -6,8 +6,8 @@
 // qaoa.rs:221-222); it is trained on angles the batched simulator optimises.
 //
 // k_gemm_bf16 computes C[M x N] = A[M x K] * B[N x K]^T (+ epilogue) on the
-// 5th-generation tensor cores: each CTA owns a 128-row tile of C and NT
-// columns; K is consumed in chunks of KC through two shared-memory buffers, so
+// 5th-generation tensor cores: each CTA owns a tile of C of BM (128 or 64) rows
+// and NT columns; K is consumed in chunks of KC through two shared-memory buffers, so
 // a chunk loads while the previous one's MMAs run.  Operands sit in shared
 // memory in the no-swizzle K-major "core matrix" layout (8 rows x 16 bytes per
 // core matrix; element (r, k) of a tile at byte (r/8)*SBO + (k/8)*128 +
@@ -230,16 +230,10 @@ __device__ void column_sums(const ColSum& s, int block, float* stage, int tid) {
 // [NT j, +NT) of C (BM 128 or 64; the accumulator of 64 rows lies in the first 16 tensor-memory lanes of
 // each warp).  The warm-start products are small (256 x 256 x 256-336): what bounds them is
 // the latency of load -> MMA -> epilogue, so narrow tiles (more CTAs, each loading little) and the
-// whole K in at most two chunks.  The products of a training step (batch 256, 336 -> 256 -> 256 ->
-// 8) took 80 us each on a B200 with 256-column tiles and 64-wide chunks (two CTAs, a wait after
-// every chunk) and take 8 us; the ReLU mask and the bias gradients, two kernels of 135 us that
-// walked the batch serially per column, run in this epilogue and beside the products.  A step with
-// Adam: 900 -> 65 us, and 56 us with each launch's set-up overlapping its predecessor (pdl_wait).
-// Loading the 80 KB of operands took 4 us of a product's 8 (a few bytes in flight a thread over 1 us of
-// latency): with the operand that is older than the predecessor read before the wait, both chunks in
-// flight at once and the epilogue's operands fetched beside them, a step takes 44 us, with 64-row
-// tiles 36 us, and with Adam's parameters and moments read before its wait 35 us.  Of a product's 4.5 us
-// 1.3 are the hand-over between launches, 1.2 the late operand, 0.9 the MMAs, 0.6 the epilogue.
+// whole K in at most two chunks.  The operand that is older than the predecessor is read before the wait
+// for it, both chunks are in flight at once, and the epilogue's operands come in beside them: a training
+// step (batch 256, 336 -> 256 -> 256 -> 8, with Adam) takes 35 us.  Of a product's 4.5 us 1.3 are the
+// hand-over between launches, 1.2 the late operand, 0.9 the MMAs, 0.6 the epilogue.
 template <int BM, int NT, int KC>
 __global__ void __launch_bounds__(GT, 1) k_gemm_bf16(const GemmArgs g0, const GemmArgs g1, const ColSum cs, int tiles0,
                                                      int tiles1) {
@@ -511,10 +505,12 @@ int launch_gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1, con
                           cs ? *cs : ColSum{}, t0, t1);
 }
 
-// Tile width by the number of CTAs it leaves: the widest tile whose grid still has a CTA for
-// every SM (A is re-read once per column tile, so large products want wide tiles); where even 32
-// columns leave SMs idle, 64 rows by 32 columns, whose CTAs each load 48 KB instead of 80 (64
-// training steps of batch 256: 2.76 -> 2.30 ms).
+// Tile of a single product by the number of CTAs it leaves: the widest whose grid still has a CTA for
+// every SM (A is re-read once per column tile, so large products want wide tiles); where even 32 columns
+// leave SMs idle, 64 rows by 32 columns, whose CTAs each load 48 KB instead of 80 (64 training steps of
+// batch 256: 2.30 against 2.76 ms).  Two products in one launch, and the output layer, always take the
+// small tile: they are made for the warm start's widths.  Wider networks re-read their operands by it (4096
+// wide, batch 4096: 7.7 ms a step).
 int gemm(cudaStream_t stream, const GemmArgs& g0, const GemmArgs* g1 = nullptr, const ColSum* cs = nullptr) {
     const long mt = (g0.M + 127) / 128;
     if (!g1 && mt * ((g0.N + 255) / 256) >= 148) return launch_gemm<128, 256, 128>(stream, g0, g1, cs);
@@ -655,10 +651,9 @@ __device__ __forceinline__ float loss_sum(const float* losspart, int nloss) {
     return s;
 }
 
-// One Adam step over every parameter, and the BF16 copies the next step's products read.  One
-// launch for the six blocks (they were six Adam launches, three copies and two transposes); the
-// loss of the step from its per-tile sums by the last CTA.  Parameters, moments and the places of the
-// gradients are older than the predecessor and come before the wait (64 training steps 2.31 -> 2.25 ms).
+// One Adam step over every parameter, and the BF16 copies the next step's products read, in one
+// launch; the loss of the step from its per-tile sums by the last CTA.  Parameters, moments and the places
+// of the gradients are older than the predecessor and come before the wait.
 __global__ void k_adam(ParamMap map, float* p, float* m, float* v, float lr,
                        float b1, float b2, float eps, float c1, float c2, const float* losspart, int nloss,
                        float inv, float* loss) {

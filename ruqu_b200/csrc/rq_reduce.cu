@@ -79,8 +79,8 @@ struct SmallStrings {
     uint32_t x[SMALL_STRINGS], z[SMALL_STRINGS];
 };
 
-// One launch for all strings, each summed by one CTA straight into out[]: the 8-qubit VQE energy's
-// 32 strings took 30 launches of 3.1 us and a reduction.
+// One launch for all strings, each summed by one CTA straight into out[]: a launch takes as long as
+// such a sum (3 us).
 template <typename T>
 __global__ void k_pauli_small(const typename C2<T>::t* __restrict__ a, uint32_t n, const __grid_constant__ SmallStrings ss,
                               double* __restrict__ out) {
@@ -113,8 +113,7 @@ __global__ void k_pauli_small(const typename C2<T>::t* __restrict__ a, uint32_t 
 // mask on those bits selects, with the sign of the other bits: five instructions per string and 16
 // amplitudes.  The sums go through the thread's own column of shared memory, as a register cannot be
 // selected at run time.  Bound by HBM: 30 single-Z strings of 30 qubits f32 in 1.43 ms (a copy-rate read takes
-// 1.31 ms) against 2.65 ms
-// for per-string sums of each warp's 1024 amplitudes.
+// 1.31 ms).
 constexpr int ZK = 32, ZPASSES = 11, ZT = 256;
 struct ZPass {
     uint64_t z[ZK];
@@ -229,8 +228,7 @@ __global__ void __launch_bounds__(ZT, KT > 16 ? 2 : 3) k_pauli_z(const typename 
 // pair is walked once, by a register bit of the local X mask held at 0 (all elements where it has none:
 // the sum is then halved by the caller).  Sums per string and thread live in shared memory across the
 // CTA's tiles.  Bound by the FP64 conversions (XU 60 %, issue 47 %): 64 random strings of 24 qubits
-// f32 in 0.59 ms against 2.8 ms for a read of the state
-// per string.
+// f32 in 0.59 ms (one read of the state per string: 2.8 ms).
 constexpr int SPASSES = 10, ST = 512;
 static_assert(ST == 1 << STB, "a tile index is a thread and a register");
 struct SpanPasses {

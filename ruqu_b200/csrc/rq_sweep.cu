@@ -1019,13 +1019,13 @@ __device__ __forceinline__ bool wait_sleep(uint64_t* bar, uint32_t parity, uint3
 // tensor-memory columns) per SM.  NTHR = 256 and 512 double-buffer the images.
 //
 // What bounds it: the chain of a phase (gather, split, MMAs, read back, scatter, barrier) on 16 warps an SM,
-// at 45 % of the issue slots, 48 % of the shared-memory bandwidth and the board's power limit; about 520
-// instructions of a warp a phase and 1280 a tile.  Reading the accumulator in two parts, the second landing
-// while the first is scattered, and the split's residual in mixed precision: 30 qubits, 20 random layers,
-// 94.5 -> 93.3 ms (12 local qubits), 92.5 -> 90.9 (13), 97.0 -> 95.9 (14); 27 qubits 9.77 -> 9.55, 10.40 ->
-// 10.25, 10.97 -> 10.85.  Two threads a row with 64 registers each (32 warps an SM) took 109 ms in all three.
-// Fewer address instructions a tile (next tile's base by one addition, constant offsets): 91.3 -> 89.3 ms with
-// 13 local qubits, 95.9 -> 92.9 with 14, 93.6 -> 92.9 with 12.
+// at 45 % of the issue slots and 48 % of the shared-memory bandwidth (no unit above 50 %); about 520
+// instructions of a warp a phase and 1280 a tile.  The board draws 880-940 W of its 1000 meanwhile, which
+// costs up to 5 % of the clock.  The accumulator is read in two parts, the second landing while the
+// first is scattered (1-2 %); two threads a row with 64 registers each (32 warps an SM) took 109 ms for 30
+// qubits, 20 random layers, and the next tile's base by one addition with constant offsets saves 1-3 %.
+// 30 qubits, 20 random layers, in turn on one box: 88.7 ms with 12 local qubits, 92.8 with 13, 94.2 with 14
+// (on others 92.9, 89.5 and 92.7); 27 qubits 9.52, 10.06 and 10.51.
 template <int NTHR>
 __global__ void __launch_bounds__(NTHR, 512 / NTHR) k_sweep_tc16(float2* __restrict__ amps, const SweepDesc d,
                                                      const PhaseDesc* __restrict__ phases,
@@ -1499,11 +1499,11 @@ static uint32_t sweep_local_qubits(uint32_t nq, int32_t prec) {
 }
 
 // Local qubits of the CUDA-core sweeps when the caller names none.  f64: 11 (128-thread CTAs, four an
-// SM), which measured 13-25 % less than 12 on random layers, QAOA and VQE circuits of 12-18 and from 22
-// qubits on: below 19 the smaller tiles reach more SMs (a 16-qubit state has 16 tiles of 2^12; random
-// layers 247 -> 201 us), above 21 four small CTAs overlap each other's loads and barriers better than
-// two (22 qubits: 2102 -> 1856 us).  At 19-21 qubits 12 is as fast or up to 9 % faster (fewer sweeps,
-// and its tiles fill the machine once).  f32: 12 up to 19 qubits (16 qubits: 279 -> 222 us), 13 above (20
+// SM).  Random layers, QAOA and VQE circuits of 12-27 qubits take with 11 instead of 12: 12-18 qubits 6 to 31 %
+// less (the smaller tiles reach more SMs: a 16-qubit state has 16 tiles of 2^12; random layers 205 against
+// 249 us), 19-21 qubits between 5 % less and 3 % more (12 needs fewer sweeps and its tiles fill the machine once),
+// 22 qubits 11-14 % less (1853 against 2089 us), 23-27 qubits 2-6 % less (four small CTAs overlap each other's
+// loads and barriers better than two).  f32: 12 up to 19 qubits (16 qubits: 222 against 279 us), 13 above (20
 // qubits: 369 against 378 us).
 static uint32_t core_local_qubits(uint32_t nq, int32_t prec) {
     if (std::getenv("RUQU_SWEEP_LOCAL_QUBITS")) return sweep_local_qubits(nq, prec);
@@ -1943,7 +1943,7 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         // a candidate whose wait ran out gave up early: no time counts, and nobody else hears of it
         if (rc == RQ_OK) rc = tc_timeout_flag(&expired, !pending);
         // a later candidate must be more than 2 % faster than the best so far: near-equal plans
-        // (the 12- and 13-qubit FP16 plans of a 30-qubit random-layer circuit are within 1 %)
+        // (the 13- and 14-qubit FP16 plans of a 30-qubit random-layer circuit)
         // then keep the earlier one, which has fewer sweeps, instead of following timing noise
         if (expired) {
             keep = false;

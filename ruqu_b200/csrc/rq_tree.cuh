@@ -57,9 +57,8 @@ __device__ __forceinline__ void store_three(double* __restrict__ tree, uint32_t 
 }
 
 // Levels n-1, n-2 and n-3 from the amplitudes: eight probabilities of a thread, all loads in flight, and
-// no level is read back.  One launch a level read every level again and cost a launch each: 12 kernels
-// and 62 us for a 23-qubit f64 state, against 5 kernels and 43 us
-// (a copy-rate read of the amplitudes alone: 20 us).
+// no level is read back.  A 23-qubit f64 state takes 5 kernels and 43 us (a copy-rate read of the
+// amplitudes alone: 20 us); a launch a level, which reads every level again, 12 kernels and 62 us.
 template <typename T>
 __global__ void __launch_bounds__(TREE_TPB) k_tree_leaf(const typename C2<T>::t* __restrict__ amps, const Perm P,
                                                         double* __restrict__ tree) {
