@@ -42,8 +42,15 @@ def little_memory(leave=64 * MIB):
             rt.cudaFree(ptr)
 
 
+def _empty():
+    with little_memory():
+        with pytest.raises(rq.MemoryAllocationFailed):
+            rq.QuantumState(26, 1, "f64")                              # 1 GiB
+    assert _pool() == (0, 0)
+
+
 def test_only_memory_that_was_not_handed_out_is_kept():
-    held = [rq.QuantumState(3, 0, "f64") for _ in range(17)]   # takes what small states left
+    _empty()
     st = rq.QuantumState(10, 1, "f64")
     before = _pool()[0]
     st.device_pointer()
@@ -55,7 +62,6 @@ def test_only_memory_that_was_not_handed_out_is_kept():
     del st
     gc.collect()
     assert _pool()[0] == before + 1
-    del held
 
 
 def test_limits():
@@ -79,10 +85,7 @@ def test_limits():
 
 def test_pinned_staging_counts():
     """2^20 + 1 Pauli strings need 8 MiB of pinned results."""
-    with little_memory():
-        with pytest.raises(rq.MemoryAllocationFailed):
-            rq.QuantumState(26, 1, "f64")
-    assert _pool() == (0, 0)
+    _empty()
     st = rq.QuantumState(1, 1, "f64")
     count = (1 << 20) + 1
     off = np.zeros(count + 1, dtype=np.uint32)
@@ -97,6 +100,7 @@ def test_pinned_staging_counts():
 
 
 def test_a_failed_allocation_empties_the_pool():
+    _empty()
     held = [rq.QuantumState(14, 1, "f64") for _ in range(4)]
     del held
     gc.collect()
@@ -113,6 +117,7 @@ def test_calls_that_need_memory_get_what_the_pool_holds():
     """Scratch above 64 MiB (stream-ordered), the tuner's scratch state and a plan's tables: 128 MiB are
     free only with the pool's 192 MiB."""
     from ruqu_b200 import workloads
+    _empty()
     n = 24
     st = rq.QuantumState(n, 1, "f64")
     f32 = rq.QuantumState(n, 1, "f32")
