@@ -31,6 +31,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 
 namespace {
@@ -1818,6 +1819,10 @@ int apply_one_gate(rq_state* s, const rq_gate& g);   // rq_capi.cu
 namespace {
 std::mutex g_tune_mu;
 std::map<std::tuple<int, uint32_t, uint64_t>, std::pair<int, uint32_t>> g_tune;
+// Structures that could not be timed for want of memory: CUDA-core sweeps, until the device has room for a
+// scratch state and TUNE_SLACK of tables (planning the candidates takes 0.1 to 1 s, so not at every call).
+std::set<std::tuple<int, uint32_t, uint64_t>> g_untuned;
+constexpr size_t TUNE_SLACK = (size_t)64 << 20;
 
 uint64_t structure_hash(const rq_gate* g, uint64_t n) {
     uint64_t h = 1469598103934665603ull;
@@ -1868,6 +1873,9 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
             *m_out = it->second.second;
             return RQ_OK;
         }
+        size_t room = 0, total = 0;
+        if (g_untuned.count(key) && (cudaMemGetInfo(&room, &total) != cudaSuccess || room < s->bytes() + TUNE_SLACK))
+            return RQ_OK;
     }
     // candidates: CUDA-core sweep; 3xTF32 and FP16-split tensor-core sweeps with the default
     // tile and with one local qubit fewer (twice the CTAs per SM, more sweeps); the FP16 sweep
@@ -1884,10 +1892,11 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cands.push_back({TC_F16, 12, nullptr, 0.f});
         if (s->nq > 14) cands.push_back({TC_F16, 14, nullptr, 0.f});
     }
-    bool keep = true;   // a choice made for want of memory, or after a wait ran out, is made again at the next call
+    bool keep = true;       // a choice made for want of memory, or after a wait ran out, is not final
+    bool memory = true;
     for (auto& c : cands)
         if (const int prc = plan_build(s, gates, n, RQ_EXEC_SWEEP, &c.plan, c.passes, 2, c.m)) {
-            if (prc != RQ_ERR_CIRCUIT) keep = false;   // its tables found no memory
+            if (prc != RQ_ERR_CIRCUIT) memory = false;   // its tables found none
             if (c.passes == 0) {   // the CUDA-core plan is the reference point
                 for (auto& d : cands) plan_free(d.plan);
                 return fail(RQ_ERR_CIRCUIT, "circuit error: the gate list cannot be planned");
@@ -1960,7 +1969,7 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
         cudaFree(scratch);
     } else {
         cudaGetLastError();   // no room for a scratch state (or nothing to compare): CUDA-core sweep
-        if (any_tc) keep = false;
+        if (any_tc) memory = false;
     }
     const int choice_passes = cands[best].passes;
     const uint32_t choice_m = cands[best].m;
@@ -1968,8 +1977,10 @@ int autotune_tc(const rq_state* s, const rq_gate* gates, uint64_t n, int* passes
     RQ_TRY(rc);
     *passes = choice_passes;
     *m_out = choice_m;
-    if (!keep) return RQ_OK;
     std::lock_guard<std::mutex> lk(g_tune_mu);
+    if (!memory) g_untuned.insert(key);
+    if (!keep || !memory) return RQ_OK;
+    g_untuned.erase(key);
     g_tune[key] = std::make_pair(choice_passes, choice_m);
     return RQ_OK;
 }

@@ -152,3 +152,23 @@ def test_a_choice_made_without_memory_is_made_again():
             rq.QuantumState(26, 1, "f64")
         assert rq.Plan(f32, gates).stats()["dense_ops"] == 0
     assert rq.Plan(f32, gates).stats()["dense_ops"] > 0
+
+
+def test_calls_without_memory_do_not_plan_every_candidate_again():
+    """The second call of a structure that found no memory takes the CUDA-core sweep without planning the
+    candidates (0.1 s and more for 24 qubits, 15 layers); it is a small part of the first."""
+    import time
+
+    from ruqu_b200 import workloads
+    n = 24
+    f32 = rq.QuantumState(n, 1, "f32")
+    gates = workloads.random_layer_circuit(n, 15, 5)
+    times = []
+    with little_memory() as free:
+        assert free < 128 * MIB
+        for _ in range(3):
+            t = time.perf_counter()
+            assert rq.Plan(f32, gates).stats()["dense_ops"] == 0
+            times.append(time.perf_counter() - t)
+    assert max(times[1:]) < 0.5 * times[0], times
+    assert rq.Plan(f32, gates).stats()["dense_ops"] > 0
